@@ -146,7 +146,7 @@ struct UnitConsts
 //   A' = fp16(1.732421875 / Mb),  C' = fp16(((N / Mb) K0 + K0) - 1024 A'),  K0 = -3.453125, 1 / Mb rounded first.
 __device__ __forceinline__ uint32_t block_multipliers(uint32_t block_word)
 {
-    const float inv = __fdiv_rn(1.0f, (float)(block_word & 0xFFu));
+    const float inv = __frcp_rn((float)(block_word & 0xFFu));      // 1 / Mb, correctly rounded like the division it stands for
     const __half a = __float2half_rn(__fmul_rn(1.732421875f, inv));
     const float ratio = __fmul_rn((float)((block_word >> 8) & 0xFFu), inv);
     const float c = __fsub_rn(__fadd_rn(__fmul_rn(ratio, -3.453125f), -3.453125f), __fmul_rn(1024.0f, __half2float(a)));

@@ -1,32 +1,39 @@
 // Decode path of the MoE layer (1..32 tokens): routing, input rotation, gate|up GEMV + SwiGLU, down GEMV + combine, in
-// ONE persistent launch whose warps pull work pieces from a queue.
+// ONE persistent launch of one 640-thread CTA per SM.
 //
 // Replaces moe_forward() of the reference (sm120/nqmoe.cu:858-907 and the kernels it launches, :375-824).  Every routing,
 // level and pointer decision is read on the device (graph-capturable).
 //
 //   route      every CTA groups the picks into runs (one expert + the tokens that picked it, level 4 first) in its own
 //              shared memory: no CTA waits for another one's routing.
-//   pieces     the queue holds, in this order,
-//                rotation pieces   (pick, 4 blocks of 128): x * su -> WHT128 -> fp16 for the gate and the up scale, stored in
-//                                  the k order the GEMV lanes read (see "operand order");
-//                gate|up pieces    (run, 16-row strip, k-slice): one warp streams the strip's packed planes from HBM through
-//                                  its cp.async ring, decodes them in registers and feeds mma.m16n8k16 with the run's tokens
-//                                  as N; the last warp to finish a (run, 128-column group) sums the k-slices in a fixed
-//                                  order and applies WHT128, sv, SwiGLU, su_d, WHT128 -> h (fp16);
-//                down pieces       the same stream / decode / MMA over h; the last warp to finish a (token, 128-row group)
-//                                  combines out[b] = sum_k rw * sv_o * WHT128(y).
-//              A warp is the unit of scheduling (no CTA-wide barrier inside the loop), so the tail of the launch is at
-//              most one piece per warp.  Pieces are handed out heaviest first.
-//   waits      gate|up pieces need the rotated inputs (one global counter), down pieces need h of their run (one counter
-//              per run).  A piece is claimed only after every piece it depends on has been claimed by a warp that is
-//              already running and waits for nothing that comes later in the queue, so the waits cannot deadlock; they are
-//              bounded all the same (2 s, then status[0] = 1 and the launch drains).
+//   lists      the 16 x 128 units of the runs, in storage order, form up to four lists that every CTA goes through in order:
+//              gate|up of the first half of the runs, gate|up of the rest, down of the first half, down of the rest.  When a CTA
+//              gets to a down list the h it needs was finished while it worked on the list in between.
+//   shares     a list is cut by cost into one share per CTA, at piece boundaries (a piece = 16-row strip x k-slice), and a share
+//              into one range per warp, at unit boundaries.  The cut points follow from the run list, so a CTA computes its
+//              own: no queue, and a warp walks a contiguous range of each plane.  (A share whose token rows do not fit into
+//              shared memory is worked off in several jobs.)
+//   rows       the token rows a job multiplies with sit in shared memory: for gate|up x * su -> WHT128 -> fp16, computed by every
+//              CTA for the runs of its share (1 to 2 rows of a 1-token call), for down copies of h; both in the k order the
+//              lanes read (see "operand order").
+//   units      a warp decodes a unit in registers and feeds mma.m16n8k16 with the run's tokens as N.  A piece that spans warps is
+//              added up in warp order through shared memory.  The last piece of a (run, 128-column group) of gate|up to arrive
+//              sums the k-slices in a fixed order and applies WHT128, sv, SwiGLU, su_d, WHT128 -> h (fp16); the last piece of
+//              a (token, 128-row group) of down combines out[b] = sum_k rw * sv_o * WHT128(y).
+//   waits      down jobs need h of their runs (one counter per run), a piece that spans warps needs the following warps'
+//              first units.  CTAs draw their shares from counters and leave a list only when no share of it is left, so
+//              whatever a warp waits for is in the hands of a running CTA, however many CTAs are resident (with all of them
+//              resident each draws one share of every list).  The waits are bounded all the same (2 s, then status[0] = 1
+//              and the launch drains).
 //   operand order   inside a 128-wide chunk the fp16 element k = 16 T + 2 t4 + 8 hi + e sits at position 32 t4 + 4 T + 2 hi + e,
 //              so lane (g, t4) finds the B fragments of all 8 k-steps of a unit in 64 contiguous bytes.
 // Split-k partial sums go to separate buffers and are added in a fixed order, so results are bitwise repeatable
 // (the reference accumulates with fp32 atomics and is not, sm120/check.py:21).
-// HBM-bound by design (0.25 B per level-2 weight, ~0.52 B per level-4 weight); in practice the integer decode
-// issue rate bounds it.
+//
+// Bound: the integer decode.  A loop that does nothing but decode and multiply units from registers runs at 382 clocks per
+// unit and SM sub-partition at level 2 and 645 at level 4 (the multiplies and byte sums on the FMA-heavy pipe, half rate,
+// are 320 and 576 of them, 8 legacy MMAs that overlap with nothing 64), whatever the number of warps from 8 on; HBM would
+// allow 70 and 140.
 #include "nq_common.cuh"
 #include "nq_rotate.cuh"
 #include "nq_unit.cuh"
@@ -37,20 +44,21 @@ namespace nq {
 #ifndef NQ_GEMV_CODES
 #define NQ_GEMV_CODES 0x3FF
 #endif
-#ifndef NQ_GEMV_DEPTH
-#define NQ_GEMV_DEPTH 3          // stages of the plane ring per warp
-#endif
-#ifndef NQ_GEMV_WARPS
-#define NQ_GEMV_WARPS 10         // warps per CTA (independent of one another; the first 8 also build the run list)
-#endif
-#ifndef NQ_GEMV_MINBLOCKS
-#define NQ_GEMV_MINBLOCKS 2      // resident CTAs per SM the kernel is compiled for: 20 warps per SM at <= 96 registers
-#endif
-constexpr int kDepth = NQ_GEMV_DEPTH;
-constexpr int kWarps = NQ_GEMV_WARPS, kThreads = 32 * kWarps;
+// One CTA of 20 warps per SM, 96 registers per thread.  Clocks per unit and sub-partition of the unit loop (level 2 / level 4 with
+// residual code 0 / 7) on data in L2: 408 / 662 / 677 with 20 warps; 432 / 681 / 769 with 16 warps of 128 registers; 24 warps
+// of 80 registers gain under 2 %.  Token fragments read through L1 instead of shared memory: 424 / 694 / 732, through a
+// generic pointer 449 / 712 / 746; copied per unit through a cp.async ring, as an earlier version of this kernel did,
+// 530 / 777 / 802.
+constexpr int kWarps = 20, kThreads = 32 * kWarps;
 static_assert(kThreads >= NQ_MAX_PICKS, "the run list is built by one thread per pick");
-constexpr int kRunTiles = 4;     // column tiles (8 tokens each) of mma.m16n8k16 per run
-constexpr int kRunTokens = 8 * kRunTiles;
+// Shared memory of the CTA: route, slots, token rows.  It stays below 164 KB, which leaves 64 KB of L1: registers that the
+// decoder functions save live in local memory, and with all 227 KB taken every access to it went to L2 (a 1-token call
+// spent ~45 us outside the unit loop instead of ~20).
+constexpr int kGemvSmem = 160 * 1024;
+constexpr int kRunTiles = 4;     // most column tiles (8 tokens each) of mma.m16n8k16 per run
+constexpr int kTileFloats = 4 * 32;      // accumulators of a column tile
+constexpr int kRowStep = 272;    // a token row in shared memory: 256 bytes per chunk, 272 from chunk to chunk (the eight chunks that
+                                 // a warp stores at once fall on different banks)
 constexpr unsigned long long kWaitNs = 2000000000ull;
 constexpr int kEpRanks = 8, kEpTokens = NQ_MAX_TOKENS, kEpGroups = 64;   // limits of the in-kernel all-reduce
 
@@ -60,15 +68,15 @@ struct MoeArgs
 {
     const __half* x; const int64_t* sel; const __half* rw;
     int B, topk, E, H, I, nm_gu, nm_dn, force_level, ks_gu, ks_dn, which;
+    int run_cap, slot_floats;    // most tokens of a run (their rows fit into shared memory), floats of a slot
     const int64_t* table;
     int* status;       // [0] != 0: a device-side wait ran out
-    __half* xrot;      // [S][2][H] rotated inputs (gate scale, up scale), operand order
     float* part_gu;    // [ks_gu][S][2I]
     __half* h;         // [S][I], operand order
     float* part_d;     // [ks_dn][S][H]
     int* cnt_gu;       // [S * I/128] (run, group) arrivals, [S * I/128] (run, 512-block) arrivals, [S] finished groups per run
     int* cnt_d;        // [B][H/128] (token, group) arrivals
-    int* wq;           // [0] piece queue, [1] CTAs that left, [2] finished rotation pieces, [3] queue of the all-reduce tasks
+    int* wq;           // [0], [2] shares drawn so far of lists 0 | 1 << 16 and 2 | 3 << 16, [1] CTAs that left ([3] unused)
     float* zd;         // [S][I/128][4] down low-rank partials
     float* out;        // [B][H]
     int* hits;         // optional [E] pick counters (may be host-mapped)
@@ -79,15 +87,18 @@ struct MoeArgs
     int* epoch;              // this rank's call counter (device): its parity picks the half of recv / rcnt
 };
 
-__device__ __forceinline__ bool pick_valid(const MoeArgs& a, int s, int* expert, int* level)
+// What a pick refers to.  The fields of the table row are fetched together, not one decision after the other.
+struct Pick { int expert, level; const __half *scales, *lr; bool masked_gu, masked_dn; };
+__device__ __forceinline__ bool read_pick(const MoeArgs& a, int s, Pick& p)
 {
     const int64_t e = a.sel[s];
-    if (e < 0 || e >= a.E || __half2float(a.rw[s]) == 0.f) return false;
-    int lv = (int)a.table[e * kTableWidth];
-    if (lv <= 0) return false;
-    if (a.force_level > 0) lv = a.force_level;
-    *expert = (int)e; *level = lv;
-    return true;
+    const __half w = a.rw[s];
+    if (e < 0 || e >= a.E) return false;
+    const int64_t* row = a.table + e * kTableWidth;
+    const int64_t lv = row[0], fg = row[4], fd = row[8], sc = row[9], lr = row[14];
+    p.expert = (int)e; p.level = a.force_level > 0 ? a.force_level : (int)lv; p.scales = (const __half*)sc; p.lr = (const __half*)lr;
+    p.masked_gu = fg != 0; p.masked_dn = fd != 0;
+    return (int)lv > 0 && __half2float(w) != 0.f;
 }
 
 // Programmatic dependent launch: a kernel lets its successor in the stream start launching early (launch_dependents)
@@ -102,66 +113,180 @@ __device__ __forceinline__ int ld_acquire(const int* p)
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ int add_acq_rel(int* p, int v)
+// Arrival on a counter: publishes what the warp stored before it.  The one that finds itself last acquires (ld_acquire on the
+// counter) before it reads what the others published; everybody else keeps its L1, which an acquire drops.
+__device__ __forceinline__ int add_release(int* p, int v)
 {
     int prev;
-    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(prev) : "l"(p), "r"(v) : "memory");
+    asm volatile("atom.add.release.gpu.global.s32 %0, [%1], %2;" : "=r"(prev) : "l"(p), "r"(v) : "memory");
     return prev;
 }
-// every lane polls (one broadcast transaction) until *p >= target; false = gave up (status raised by this or another warp)
+// Every lane polls (one broadcast transaction) until *p >= target; false = gave up (status raised by this or another warp).
+// The polls are relaxed: an acquiring load drops the SM's L1, where the other warps find their token rows.
+__device__ __forceinline__ int ld_relaxed(const int* p)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ bool wait_counter(const int* p, int target, int* status)
 {
     unsigned long long t0 = 0;
     for (uint32_t i = 0;; ++i)
     {
-        if (ld_acquire(p) >= target) return true;
+        if (ld_relaxed(p) >= target) { ld_acquire(p); return true; }
         if ((i & 63u) == 63u)
         {
-            if (ld_acquire(status) != 0) return false;
+            if (ld_relaxed(status) != 0) return false;
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             if (t0 == 0) t0 = t;
             else if (t - t0 > kWaitNs) break;
         }
-        __nanosleep(100);
+        __nanosleep(32);
     }
     atomicExch(status, 1);
     return false;
 }
 
 // ---------------------------------------------------------------- shared state of a CTA
+// Relative cost of a unit, by which the lists are cut: measured clocks of the unit loop, 410 at level 2 and 690 at level 4, and 64
+// (8 legacy MMAs) for a further column tile.
+constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f;
+constexpr int kUndecided = -1, kDeciding = -2, kLists = 4, kCachedRows = 2;
+// The units [at, stop) of list positions that this CTA is working on, and the token rows it needs for them.
+struct Job
+{
+    int share, next;                 // share in work; the one to follow (kUndecided until the first warp is done)
+    int at, stop, end;               // this job; the end of the share
+    int seq;                         // number of the job (of any list), never 0
+    int staged;                      // the rows are in place already
+    int run0, row0, nrows, rows_at;  // first run, its first row's number, rows, byte offset behind the slots
+    int bound[kWarps + 1];           // the warps' ranges
+    int64_t row[kCachedRows][kTableWidth];   // table rows of run0 and the runs behind it
+};
+struct Shape
+{
+    int S, ng, ngH, KSg, KSd, nruns, split;      // split: runs of the first of the two lists of a phase
+    int nu_gu, nu_dn;                // units per run of the two projections (0: that half is not wanted)
+};
+// What a warp does with (part of) a piece: read by the decoder functions.
+struct StripJob
+{
+    ProjPlanes P;
+    size_t nrec, res_nrec;           // records of the base and of the residual plane
+    size_t unit0, res0;              // plane index of the first unit, of the strip's first refined unit
+    unsigned long long flags;        // mask mode: refined chunks of the strip
+    int c0, n;                       // first chunk, units
+    uint32_t x;                      // shared-space address of the run's first token row
+    int row_bytes, count;            // bytes from row to row, tokens of the run
+    // what becomes of the sums: list, run, strip, k-slice, units of the piece behind the warp's range, whether it begins in it
+    int l, r, strip, ks, left, starts;
+};
+// The state of a CTA, at the start of its shared memory.  (Reached through route(): the functions that are not inlined get
+// neither pointers nor structures, which would go through local memory.)
 struct Route
 {
+    MoeArgs a;
+    Shape sh;
+    int par;
+    StripJob strip[kWarps];
     int key[NQ_MAX_PICKS];                // expert of a valid pick, else -1 - pick
     RunRec runs[NQ_MAX_PICKS];
+    const __half* scales[NQ_MAX_PICKS];   // scale vector of a valid pick's expert
+    const __half* lr[NQ_MAX_PICKS];       // its low-rank plane, or null
     short lead[NQ_MAX_PICKS];             // run ordinal (by first pick) -> its first pick
     short first_of[NQ_MAX_PICKS];         // first pick of a run -> offset of the run in order[]
     unsigned char lvl[NQ_MAX_PICKS], order[NQ_MAX_PICKS], nvalid[NQ_MAX_TOKENS];
     int warp_sum[NQ_MAX_PICKS / 32], nruns;
+    float cost[2][NQ_MAX_PICKS];          // cost of one unit of a run (gate|up, down)
+    float base[2][NQ_MAX_PICKS + 1];      // cost of the units before a run
+    int ks[2];                            // k-slices per strip in use
+    int draws[2];                         // this CTA's first shares of the lists, packed as in wq
+    __align__(16) float zg[NQ_MAX_PICKS][4];   // low-rank inputs x V_gu^T of the picks of this CTA's gate|up shares
+    int slot_seq[2][kWarps];              // job whose share of a piece is in the warp's slot (lists 0, 2 and 1, 3)
+    Job job[kLists];
 };
+constexpr int kRouteBytes = (sizeof(Route) + 127) / 128 * 128;
+extern __shared__ __align__(128) uint8_t nq_gemv_smem[];      // Route, [3][kWarps][slot_floats], token rows
+__device__ __forceinline__ Route& route() { return *(Route*)nq_gemv_smem; }
+// slots of a warp: 0, 1 its share of a piece that an earlier warp adds up (lists 0, 2 and 1, 3), 2 the sums of its current
+// piece; fragment order [tile][i][lane]
+__device__ __forceinline__ float* slot_of(const Route& R, int which, int warp) { return (float*)(nq_gemv_smem + kRouteBytes) + (which * kWarps + warp) * R.a.slot_floats; }
+__device__ __forceinline__ uint32_t rows_base(const Route& R) { return smem_addr(nq_gemv_smem) + kRouteBytes + 3 * kWarps * R.a.slot_floats * 4; }
+__host__ __device__ constexpr int rows_room(int slot_floats) { return kGemvSmem - kRouteBytes - 3 * kWarps * slot_floats * 4; }
+
+// quotient of small non-negative integers (a < 2^20) without the ~130 clocks of an integer division
+__device__ __forceinline__ int quot(int a, int b) { return (int)__fdividef((float)a + 0.5f, (float)b); }
+__device__ __forceinline__ int quot_any(int a, int b) { return a < (1 << 20) ? quot(a, b) : a / b; }
 
 // Group the picks into runs: a run = one expert and up to 32 of its picks in pick order; runs are numbered by first
-// pick, then ordered level 4 before level 2 (heavier pieces are handed out first).  Thread t = pick t (t < 256); every thread
-// of the CTA must call it.
-__device__ __forceinline__ void build_route(const MoeArgs& a, Route& R)
+// pick, then ordered level 4 before level 2.  A run has at most run_cap picks.
+__device__ __forceinline__ void set_costs(const MoeArgs& a, Route& R, int rank, const Pick& p, int count)
+{
+    const int C[2] = {a.H / 128, a.I / 128}, nm[2] = {a.nm_gu, a.nm_dn};
+#pragma unroll
+    for (int d = 0; d < 2; ++d)
+    {
+        const bool masked = d ? p.masked_dn : p.masked_gu;
+        const float refined = p.level < 4 ? 0.f : masked ? fminf(__fdividef((float)nm[d], (float)C[d]), 1.f) : 1.f;
+        R.cost[d][rank] = kCostUnit + kCostRefined * refined + kCostTile * (float)((count - 1) >> 3);
+    }
+}
+// up to 32 picks, none of them more than run_cap times the same expert (false otherwise): one warp, a lane per pick
+__device__ __forceinline__ bool build_route_warp(const MoeArgs& a, Route& R, int lane)
+{
+    const int S = a.B * a.topk;
+    Pick p{-1, 0, nullptr, nullptr, false, false};
+    const bool tv = lane < S && read_pick(a, lane, p);
+    const unsigned valid = __ballot_sync(0xffffffffu, tv), below = (1u << lane) - 1u;
+    const unsigned same = __match_any_sync(0xffffffffu, tv ? p.expert : -1 - lane);
+    const int pos = __popc(same & below), count = __popc(same), leader = __ffs(same) - 1;
+    if (__any_sync(0xffffffffu, count > a.run_cap)) return false;
+    const bool lead = tv && pos == 0;
+    const unsigned lead4 = __ballot_sync(0xffffffffu, lead && p.level >= 4), lead2 = __ballot_sync(0xffffffffu, lead && p.level < 4);
+    const int rank = p.level >= 4 ? __popc(lead4 & below) : __popc(lead4) + __popc(lead2 & below), nruns = __popc(lead4 | lead2);
+    // picks of the runs before this one: the leaders' counts, in run order, added up
+    if (lead) R.first_of[rank] = (short)count;
+    __syncwarp();
+    const int mine_count = lane < nruns ? R.first_of[lane] : 0;
+    int sum = mine_count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += u; }
+    const int first = __shfl_sync(0xffffffffu, sum - mine_count, rank & 31);
+    if (lead) { R.runs[rank] = RunRec{p.expert, p.level, first, count}; set_costs(a, R, rank, p, count); }
+    const int base = __shfl_sync(0xffffffffu, first, leader);
+    if (lane < S) { R.key[lane] = tv ? p.expert : -1 - lane; R.lvl[lane] = (unsigned char)p.level; R.scales[lane] = p.scales; R.lr[lane] = p.lr; }
+    if (tv) R.order[base + pos] = (unsigned char)lane;
+    if (lane < a.B)
+    {
+        const unsigned mine = a.topk >= 32 ? 0xffffffffu : ((1u << a.topk) - 1u) << (lane * a.topk);
+        R.nvalid[lane] = (unsigned char)__popc(valid & mine);
+    }
+    if (lane == 0) R.nruns = nruns;
+    return true;
+}
+// up to 256 picks: thread t = pick t; every thread of the CTA must call it
+__device__ __forceinline__ void build_route_cta(const MoeArgs& a, Route& R)
 {
     const int S = a.B * a.topk, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const bool in = t < NQ_MAX_PICKS;
-    int e = -1, lv = 0;
-    const bool tv = t < S && pick_valid(a, t, &e, &lv);
-    if (in) { R.key[t] = tv ? e : -1 - t; R.lvl[t] = (unsigned char)lv; }
+    Pick p{-1, 0, nullptr, nullptr, false, false};
+    const bool tv = t < S && read_pick(a, t, p);
+    const int e = p.expert, lv = p.level;
+    if (in) { R.key[t] = tv ? e : -1 - t; R.lvl[t] = (unsigned char)lv; R.scales[t] = p.scales; R.lr[t] = p.lr; }
     __syncthreads();
     int pos = 0, cnt = 0, first_pick = t;
     if (tv)
         for (int q = 0; q < S; ++q)
             if (R.key[q] == e) { if (cnt == 0) first_pick = q; ++cnt; pos += q < t; }
-    const bool lead = tv && (pos % kRunTokens) == 0;
+    const bool lead = tv && pos % a.run_cap == 0;
     const unsigned bal = __ballot_sync(0xffffffffu, lead);
     if (lane == 0 && in) R.warp_sum[warp] = __popc(bal);
     __syncthreads();
     int ord = __popc(bal & ((1u << lane) - 1u)), nruns = 0;
     for (int w = 0; w < NQ_MAX_PICKS / 32; ++w) { const int c = R.warp_sum[w]; ord += w < warp ? c : 0; nruns += c; }
-    const int my_count = cnt - pos < kRunTokens ? cnt - pos : kRunTokens;
+    const int my_count = cnt - pos < a.run_cap ? cnt - pos : a.run_cap;
     if (lead) { R.lead[ord] = (short)t; R.first_of[t] = (short)my_count; }      // first_of holds the run's size until the ranks are known
     if (t == 0) R.nruns = nruns;
     __syncthreads();
@@ -174,16 +299,16 @@ __device__ __forceinline__ void build_route(const MoeArgs& a, Route& R)
             rank += before; first += before ? (int)R.first_of[lp] : 0;
         }
     __syncthreads();
-    if (lead) { R.runs[rank] = RunRec{e, lv, first, my_count}; R.first_of[t] = (short)first; }
+    if (lead) { R.runs[rank] = RunRec{e, lv, first, my_count}; R.first_of[t] = (short)first; set_costs(a, R, rank, p, my_count); }
     __syncthreads();
     if (tv)
     {
         int lp = first_pick;
-        const int want = pos - pos % kRunTokens;
-        if (want)                                   // an expert with more than 32 picks: find the first pick of my run
+        const int want = pos - pos % a.run_cap;
+        if (want)                                   // an expert with more than one run: find the first pick of my run
             for (int q = 0, seen = 0; q < S; ++q)
                 if (R.key[q] == e) { if (seen == want) { lp = q; break; } ++seen; }
-        R.order[R.first_of[lp] + pos % kRunTokens] = (unsigned char)t;
+        R.order[R.first_of[lp] + pos % a.run_cap] = (unsigned char)t;
     }
     if (t < a.B)
     {
@@ -203,184 +328,121 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
 }
 
 // Tokens of the run as the N operand: lane (g, t4) supplies k = 16 T + 2 t4 (+8) of token 8 nt + g, i.e. column g of the
-// tile.  A tile column without a token reads the run's first token instead: MMA columns are independent, so whatever is
-// multiplied there lands in accumulators that are never stored.
-//
-// One column tile (runs of up to 8 tokens, the 1..8-token decode case): the 8 k-steps' (b0, b1) pairs of a unit are 64
-// contiguous bytes per lane, copied into the plane ring by cp.async together with the unit's records (lanes whose column
-// has a token only), so they are in shared memory when the unit is decoded.  A lane's four 16-byte pieces go to four
-// lane-indexed arrays (piece i of lane l at 512 i + 16 l): conflict-free, and addressed from the same per-lane register
-// as the base records.
-constexpr int kStageTokens = kStageBytes;            // offset of the token fragments inside a GEMV stage
-constexpr int kGemvStage = kStageBytes + 4 * 512;    // bytes per GEMV stage
-struct TokenSink1
-{
-    float (&acc)[4];
-    uint32_t frag;     // shared-space address of this stage's token fragments + 16 lane
-    template <int T>
-    __device__ __forceinline__ void operator()(std::integral_constant<int, T>, const uint32_t (&a)[4]) const
-    {
-        const uint2 b = lds64(frag + 512 * (T >> 1) + 8 * (T & 1));
-        mma_16816(acc, a, b.x, b.y);
-    }
-};
-// Up to NT column tiles: B fragments fetched from global memory per k-step.
+// tile: 64 contiguous bytes per unit in shared memory, read 16 bytes per two k-steps.  A tile column without a token reads the
+// run's first token instead: MMA columns are independent, so whatever is multiplied there lands in accumulators that are
+// never stored.
 template <int NT>
-struct TokenSinkN
+struct TokenSink
 {
     float (&acc)[NT][4];
-    const uint8_t* x0;           // token rows (bytes)
-    const uint32_t (&xoff)[NT];  // byte offset of the tile's row for this lane (+ 64 t4)
-    int ntiles, off;             // off = 256 * chunk
+    const uint32_t (&x)[NT];     // shared-space address of this lane's 64 bytes per tile, at chunk 0
+    uint32_t off;                // kRowStep * chunk
+    uint4 (&b)[NT];              // fragments of k-steps T and T + 1 (T even)
     template <int T>
     __device__ __forceinline__ void operator()(std::integral_constant<int, T>, const uint32_t (&a)[4]) const
     {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
         {
-            if (nt >= ntiles) break;      // warp-uniform
-            const uint2 b = *(const uint2*)(x0 + xoff[nt] + off + T * 8);
-            mma_16816(acc[nt], a, b.x, b.y);
+            if constexpr ((T & 1) == 0) { b[nt] = lds128(x[nt] + off + T * 8); mma_16816(acc[nt], a, b[nt].x, b[nt].y); }
+            else mma_16816(acc[nt], a, b[nt].z, b[nt].w);
         }
     }
 };
 
-// What one warp does with one strip: filled in by the caller, read once by strip_gemv.
-struct StripJob
+// n units of one strip: stream, decode, multiply; the 16 x (8 NT) partial sums go to the warp's slot 2.  MODE 0: level 2, 1: level 4, 2: level 4 in
+// mask mode (chunks without a flag decode as level 2).  The records of the next unit are fetched into registers while the
+// current one is decoded.
+// Not inlined on purpose: each of the decoder variants gets a register allocation of its own, and the caller's state is
+// saved once per piece around the call instead of being squeezed into the unit loop (an inlined loop saves 10 to 35
+// clocks per unit, a loop that shares its function with the piece bookkeeping loses 200 to spills).
+template <int MODE, int RC, int BK, int NT>
+__device__ __noinline__ void strip_gemv()
 {
-    ProjPlanes P;
-    StripRef sr;
-    int C, NS, c0, c1;               // chunks per strip, strips of the projection, chunk range [c0, c1)
-    const uint8_t* x0;               // token rows (operand order), as bytes
-    uint32_t xoff[kRunTiles];        // per column tile: byte offset of this lane's token row + 64 t4
-    int ntiles;
-    bool has_token;                  // this lane's column of tile 0 holds a token
-    uint32_t ring;                   // shared-space address of the warp's kDepth stages
-    const int* gate; int gate_target; int* status;   // counter to wait for before the first multiply (or null)
-};
-
-// One warp, one strip, chunks [c0, c1): stream, decode, multiply; acc = the 16 x (8 NT) partial sums.  REFINED: the expert
-// is at level 4.  false = the wait on the gate counter ran out.
-// Not inlined on purpose: each of the decoder variants gets a register allocation of its own, and the bookkeeping of the
-// piece loop is saved once per piece around the call instead of being squeezed into the decode loop.
-template <bool REFINED, int RC, int BK, int NT>
-__device__ __noinline__ bool strip_gemv(const StripJob& J, float (&out)[NT][4])
-{
-    const int lane = threadIdx.x & 31, c0 = J.c0, c1 = J.c1;
-    const unsigned long long flags = J.sr.flags;
-    RecordCursor<BK> cb;
-    cb.init(J.P.base, (size_t)J.NS * J.C * 32, J.sr.unit0 + c0, lane);
-    RecordCursor<RC> cr;
-    int issued = 0;                       // refined units whose copies are issued
-    if constexpr (REFINED) cr.init(J.P.p4, J.sr.res_nrec, J.sr.res0 + refined_before(J.sr, c0), lane);
-    const uint32_t ring = J.ring;
-    const uint8_t* xin = J.x0 + J.xoff[0] + (size_t)c0 * 256;       // next token fragment to copy (one column tile)
-    const bool has_token = J.has_token;
-    auto issue_planes = [&](int ch, uint32_t st) {
-        cb.copy(st, ch - c0, lane);
-        if constexpr (REFINED)
-            if ((flags >> ch) & 1ull) cr.copy(st + kStageBase, issued++, lane);
-    };      // (prologue only; the loop below tests its flags from a block-local copy)
-    auto issue_tokens = [&](uint32_t st) {
-        if constexpr (NT == 1)
-        {
-            if (has_token)
-            {
-                const uint32_t dst = st + kStageTokens + lane * 16;
-                cp_async16_at<0, 0>(dst, xin); cp_async16_at<512, 16>(dst, xin);
-                cp_async16_at<1024, 32>(dst, xin); cp_async16_at<1536, 48>(dst, xin);
-            }
-            xin += 256;
-        }
-    };
-    // the planes can be fetched before the inputs exist (gate), the token fragments only after
-#pragma unroll
-    for (int d = 0; d < kDepth - 1; ++d)
-        if (c0 + d < c1) issue_planes(c0 + d, ring + d * kGemvStage);
-    bool ok = true;
-    if (J.gate) ok = wait_counter(J.gate, J.gate_target, J.status);
-#pragma unroll
-    for (int d = 0; d < kDepth - 1; ++d)
+    const StripJob& J = route().strip[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, nxt = ring_successor(lane), n = J.n;
+    RecordReader<BK> rb;
+    rb.init(J.P.base, J.nrec, J.unit0, lane);
+    rb.fetch();
+    RecordReader<RC> rr;
+    const int c0 = MODE == 2 ? J.c0 : 0;
+    unsigned long long flags = 0;
+    size_t res = 0;                                       // residual index of the first refined unit at or behind c0
+    if constexpr (MODE == 1) res = J.res0 + J.c0;
+    if constexpr (MODE == 2) { flags = J.flags; res = J.res0 + __popcll(flags & ((1ull << c0) - 1ull)); flags >>= c0; }
+    if constexpr (MODE > 0)
     {
-        if (c0 + d < c1) issue_tokens(ring + d * kGemvStage);
-        cp_async_commit();
+        rr.init(J.P.p4, J.res_nrec, res, lane);
+        if (MODE == 1 || (flags & 1ull)) rr.fetch();
     }
+    uint32_t x[NT];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+    {
+        const int j = nt * 8 + (lane >> 2);
+        x[nt] = J.x + (j < J.count ? j : 0) * J.row_bytes + (lane & 3) * 64;
+    }
+    uint32_t off = J.c0 * kRowStep;
     float acc[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
-    uint32_t st = ring;                                   // stage to consume; the stage before it (cyclically) is filled
-    const int nxt = ring_successor(lane);
-    for (int cs = c0; cs < c1; cs += 32)
+    for (int s = 0; s < n; s += 32)
     {
-        // per-unit scalars of chunks cs .. cs + 31, one chunk per lane: ring signs, block word and its multipliers;
-        // fl: refinement flags of chunks cs .. cs + 31 (+ kDepth - 1 for the copies that run ahead)
-        const unsigned long long fl = flags >> cs;
-        uint32_t var_b = 0, ac = 0, mbn = 0;
+        // per-unit scalars of units s .. s + 31, one unit per lane: ring signs and block word (meta = word | signs << 16) and the
+        // block word's multipliers
+        uint32_t meta = 0, ac = 0;
+        const int m = n - s < 32 ? n - s : 32;
+        const uint32_t now = MODE == 2 ? (uint32_t)(flags >> s) : 0u;
+        const unsigned long long after = MODE == 2 ? flags >> s >> 1 : 0ull;     // bit i: the unit behind unit s + i is refined
+        if (lane < m)
         {
-            const int cl = cs + lane;
-            if (cl < c1)
+            if (J.P.var) meta = (uint32_t)__ldg(J.P.var + J.unit0 + s + lane) << 16;
+            if (MODE == 1 || (MODE == 2 && (now >> lane & 1u)))
             {
-                if (J.P.var) var_b = __ldg(J.P.var + J.sr.unit0 + cl);
-                if constexpr (REFINED)
-                    if ((fl >> lane) & 1ull)
-                    {
-                        mbn = __ldg(J.P.d4 + J.sr.res0 + refined_before(J.sr, cl)) & 0xFFFFu;
-                        ac = block_multipliers(mbn);
-                    }
+                const size_t at = MODE == 1 ? res + s + lane : res + __popcll(flags & ((1ull << (s + lane)) - 1ull));
+                const uint32_t word = __ldg(J.P.d4 + at) & 0xFFFFu;
+                meta |= word;
+                ac = block_multipliers(word);
             }
         }
-        const int n = c1 - cs < 32 ? c1 - cs : 32;
-        for (int i = 0; i < n; ++i)
+#pragma unroll 1
+        for (int i = 0; i < m; ++i)
         {
-            const int ch = cs + i;
-            if (ch + kDepth - 1 < c1)
-            {
-                const uint32_t st_in = st == ring ? ring + (kDepth - 1) * kGemvStage : st - kGemvStage;
-                cb.copy(st_in, ch + kDepth - 1 - c0, lane);
-                if constexpr (REFINED)
-                    if ((fl >> (i + kDepth - 1)) & 1ull) cr.copy(st_in + kStageBase, issued++, lane);
-                issue_tokens(st_in);
-            }
-            cp_async_commit();
-            cp_async_wait<kDepth - 1>();
-            const uint32_t sign2 = sign_mask(__shfl_sync(0xffffffffu, var_b, i), lane);
             uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
-            RecordCursor<BK>::read(wb, st, lane);
+            bool refined = MODE == 1;
+            if constexpr (MODE == 2) refined = now >> i & 1u;
+            rb.words(wb, lane);
+            if constexpr (MODE > 0)
+                if (refined) rr.words(wr, lane);
+            if (s + i + 1 < n)
+            {
+                rb.fetch();
+                if constexpr (MODE > 0)
+                    if (MODE == 1 || ((uint32_t)after >> i & 1u)) rr.fetch();
+            }
             continue_stream<Pattern<BK>::kBits>(wb, __shfl_sync(0xffffffffu, wb[0], nxt));
-            bool refined = false;
-            if constexpr (REFINED) refined = (fl >> i) & 1ull;
-            UnitConsts k;
-            if (refined)
+            const uint32_t um = __shfl_sync(0xffffffffu, meta, i), sign2 = sign_mask(um >> 16, lane);
+            uint4 b[NT];
+            const TokenSink<NT> sink{acc, x, off, b};
+            if (MODE > 0 && refined)
             {
-                const uint32_t acw = __shfl_sync(0xffffffffu, ac, i), mb = __shfl_sync(0xffffffffu, mbn, i);
-                RecordCursor<RC>::read(wr, st + kStageBase, lane);
-                continue_stream<Pattern<RC>::kBits>(wr, __shfl_sync(0xffffffffu, wr[0], nxt));
-                k = consts_level4(acw, mb, sign2);
+                if constexpr (MODE > 0)
+                {
+                    continue_stream<Pattern<RC>::kBits>(wr, __shfl_sync(0xffffffffu, wr[0], nxt));
+                    decode_words<true, RC, BK>(wb, wr, consts_level4(__shfl_sync(0xffffffffu, ac, i), um, sign2), sink);
+                }
             }
-            else k = consts_level2(sign2);
-            if constexpr (NT == 1)
-            {
-                const TokenSink1 sink{acc[0], st + kStageTokens + lane * 16};
-                if (refined) decode_words<true, RC, BK>(wb, wr, k, sink);
-                else decode_words<false, 0, BK>(wb, wr, k, sink);
-            }
-            else
-            {
-                const TokenSinkN<NT> sink{acc, J.x0, J.xoff, J.ntiles, ch * 256};
-                if (refined) decode_words<true, RC, BK>(wb, wr, k, sink);
-                else decode_words<false, 0, BK>(wb, wr, k, sink);
-            }
-            st = st + kGemvStage == ring + kDepth * kGemvStage ? ring : st + kGemvStage;
+            else if constexpr (MODE != 1) decode_words<false, 0, BK>(wb, wr, consts_level2(sign2), sink);
+            off += kRowStep;
         }
     }
-    cp_async_wait<0>();
+    float* out = slot_of(route(), 2, threadIdx.x >> 5) + lane;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) out[nt][i] = acc[nt][i];
-    return ok;
+        for (int i = 0; i < 4; ++i) out[(nt * 4 + i) * 32] = acc[nt][i];
 }
 
 // 4 consecutive elements k = 4 lane + i of a 128-chunk -> operand order (two 4-byte stores)
@@ -392,98 +454,178 @@ __device__ __forceinline__ void store4h_operand(__half* chunk, int lane, const f
     w[16] = *(const uint32_t*)&b;
 }
 
-struct Shape
+// A list: units of the runs [run0, run1) of phase d; position p of the list is unit p mod NU of run run0 + p / NU.
+struct List { int d, run0, run1, C, NU, cps, NH; };        // chunks per strip, units per run, chunks per piece, units of a half (gate, up)
+__device__ __forceinline__ List list_of(const MoeArgs& a, const Shape& sh, int l)
 {
-    int S, ng, ngH, KSg, KSd, nparts, rot_blocks, nruns;
-    int n_rot, n_gu, n_dn, per_run_gu, per_run_dn;
-};
-
-// ---------------------------------------------------------------- rotation piece: (pick, blocks [rb part, rb part + rb))
-// rb = 1 whenever there are at least as many warps as (pick, block) pairs: every gate|up piece waits for the rotations, so
-// they are spread as thin as possible, and the inputs of the next block are fetched before the current one is transformed.
-struct RotIn { uint2 x, g, u; };
-__device__ __forceinline__ RotIn rot_fetch(const __half* xr, const __half* scales, const __half* su_u, int k)
-{
-    return RotIn{*(const uint2*)(xr + k), *(const uint2*)(scales + k), *(const uint2*)(su_u + k)};
+    List L;
+    L.d = l >> 1;
+    L.run0 = l & 1 ? sh.split : 0; L.run1 = l & 1 ? sh.nruns : sh.split;
+    L.C = (L.d ? a.I : a.H) >> 7; L.NU = L.d ? sh.nu_dn : sh.nu_gu; L.NH = L.d ? L.NU : L.NU >> 1;
+    const int KS = L.d ? sh.KSd : sh.KSg;
+    L.cps = KS == 1 ? L.C : quot(L.C, KS);
+    return L;
 }
+
+// ---------------------------------------------------------------- token rows
 __device__ __forceinline__ void unpack4h(const uint2& w, float (&f)[4])
 {
     const __half2 a = *(const __half2*)&w.x, b = *(const __half2*)&w.y;
     f[0] = __low2float(a); f[1] = __high2float(a); f[2] = __low2float(b); f[3] = __high2float(b);
 }
-__device__ __forceinline__ void rotate_piece(const MoeArgs& a, const Shape& sh, const Route& R, int piece, int lane)
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// Rows are numbered run by run: gate|up has the gate rows of a run's picks, then their up rows, down one row per pick.
+__device__ __forceinline__ int row_id(const RunRec& run, int d, int up) { return d ? run.first : 2 * run.first + up * run.count; }
+// The rows of a gate|up job.  A warp task = eight blocks of 128 of one row: lanes 4 v .. 4 v + 3 hold block v (wht128_x8, map H).
+// Returns the number of warp tasks; w0: the warp that takes the first one.
+__device__ __forceinline__ int rotate_rows(const MoeArgs& a, const Shape& sh, const Route& R, const Job& job, uint32_t rows, int w0, int lane, int warp)
 {
-    const int s = piece / sh.nparts, part = piece - s * sh.nparts;
-    const int e = R.key[s];
-    if (e >= 0)
+    const int oct = (sh.ngH + 7) >> 3, n = job.nrows * oct, q = lane & 3;
+    int run = job.run0;
+    for (int t = warp >= w0 ? warp - w0 : warp + kWarps - w0; t < n; t += kWarps)
     {
-        const __half* scales = (const __half*)a.table[(int64_t)e * kTableWidth + 9];
-        const __half* su_u = scales + 2 * a.H + 3 * a.I;
-        const __half* xr = a.x + (size_t)(s / a.topk) * a.H;
-        __half* dst = a.xrot + (size_t)s * 2 * a.H;
-        const int b0 = part * sh.rot_blocks, b1 = b0 + sh.rot_blocks < sh.ngH ? b0 + sh.rot_blocks : sh.ngH;
-        RotIn in = rot_fetch(xr, scales, su_u, b0 * 128 + lane * 4);
-        for (int blk = b0; blk < b1; ++blk)
+        const int p = quot(t, oct), blk = (t - p * oct) * 8 + (lane >> 2);
+        while (job.row0 + p >= 2 * (R.runs[run].first + R.runs[run].count)) ++run;
+        const RunRec rr = R.runs[run];
+        const int at = job.row0 + p - 2 * rr.first, u = at >= rr.count ? 1 : 0, s = R.order[rr.first + at - u * rr.count];
+        const bool live = blk < sh.ngH;
+        float v[32];
+        if (live)
         {
-            const RotIn cur = in;
-            if (blk + 1 < b1) in = rot_fetch(xr, scales, su_u, (blk + 1) * 128 + lane * 4);
-            float f[4], g[4], u[4];
-            unpack4h(cur.x, f); unpack4h(cur.g, g); unpack4h(cur.u, u);
-            float vg[4] = {f[0] * g[0], f[1] * g[1], f[2] * g[2], f[3] * g[3]};
-            float vu[4] = {f[0] * u[0], f[1] * u[1], f[2] * u[2], f[3] * u[3]};
-            wht128(vg, lane); wht128(vu, lane);
-            store4h_operand(dst + blk * 128, lane, vg);
-            store4h_operand(dst + a.H + blk * 128, lane, vu);
+            uint32_t xw[16], sw[16];
+            load16w_mapH(a.x + (size_t)quot(s, a.topk) * a.H + blk * 128, q, xw);
+            load16w_mapH(R.scales[s] + (u ? 2 * a.H + 3 * a.I : 0) + blk * 128, q, sw);
+            mul32w_mapH(xw, sw, v);
+        }
+        else
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = 0.f;
+        wht128_x8(v, lane);
+        if (!live) continue;
+        // element 32 j + 8 q + 2 t4 + e of the block -> operand position 32 t4 + 8 j + 2 q + e
+        const uint32_t dst = rows + (p * sh.ngH + blk) * kRowStep + 4 * q;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int t4 = 0; t4 < 4; ++t4)
+            {
+                const __half2 h = __floats2half2_rn(v[8 * j + 2 * t4], v[8 * j + 2 * t4 + 1]);
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + 64 * t4 + 16 * j), "r"(*(const uint32_t*)&h) : "memory");
+            }
+    }
+    return n;
+}
+// low-rank inputs x V_gu^T (unrotated input) of a gate|up job's picks, a warp per pick
+__device__ __forceinline__ void low_rank_inputs(const MoeArgs& a, Route& R, int p0, int p1, int lane, int warp)
+{
+    for (int p = p0 + warp; p < p1; p += kWarps)
+    {
+        const int s = R.order[p];
+        const __half* lr = R.lr[s];
+        if (!lr) continue;
+        const int rg = (int)a.table[(int64_t)R.key[s] * kTableWidth + 16];
+        const __half* xr = a.x + (size_t)(s / a.topk) * a.H;
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int k = lane * 4; k < a.H; k += 128)
+        {
+            float f[4], w[4];
+            load4h(xr + k, f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q < rg)
+                {
+                    load4h(lr + (size_t)q * a.H + k, w);
+                    d[q] += f[0] * w[0] + f[1] * w[1] + f[2] * w[2] + f[3] * w[3];
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int o = 16; o; o >>= 1) d[q] += __shfl_xor_sync(0xffffffffu, d[q], o);
+        if (lane == 0) *(float4*)R.zg[s] = make_float4(d[0], d[1], d[2], d[3]);
+    }
+}
+// The rows of a down job: h of its runs, once they are complete.  A warp task = 512 bytes of a row.  false = the wait ran out.
+__device__ __forceinline__ bool copy_rows(const MoeArgs& a, const Shape& sh, const Route& R, const Job& job, uint32_t rows, int lane, int warp)
+{
+    const int per = (sh.ng + 1) >> 1, n = job.nrows * per;
+    int run = job.run0, seen = -1;
+    for (int t = warp; t < n; t += kWarps)
+    {
+        const int p = quot(t, per), blk = (t - p * per) * 2 + (lane >> 4);
+        while (job.row0 + p >= R.runs[run].first + R.runs[run].count) ++run;
+        if ((a.which & 1) && run != seen)
+        {
+            if (!wait_counter(a.cnt_gu + 2 * sh.S * sh.ng + run, sh.ng, a.status)) return false;
+            seen = run;
+        }
+        if (blk < sh.ng)
+        {
+            const uint4 v = __ldcg((const uint4*)(a.h + (size_t)R.order[job.row0 + p] * a.I + blk * 128) + (lane & 15));
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(rows + (p * sh.ng + blk) * kRowStep + (lane & 15) * 16), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
         }
     }
-    __syncwarp();                      // the lanes' stores happen before lane 0's release below
-    if (lane == 0) add_acq_rel(a.wq + 2, 1);
+    return true;
 }
 
 // ---------------------------------------------------------------- finishers
-// (run, group) complete: WHT128, sv, (+ low rank), SwiGLU, su_d, WHT128 -> h, one token after the other.
-__device__ __forceinline__ void finish_gate_up(const MoeArgs& a, const Shape& sh, const Route& R, int r, int grp, int lane)
+// (run, group) complete: WHT128, sv, (+ low rank), SwiGLU, su_d, WHT128 -> h, one token after the other; the sums of the
+// next token are fetched while the current one is transformed.
+__device__ __forceinline__ float4 sum_slices(const float* p, size_t stride, int KS)
 {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < KS; ++q)
+    {
+        const float4 f = __ldcg((const float4*)(p + q * stride));
+        v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+    }
+    return v;
+}
+__device__ __noinline__ void finish_gate_up(int r, int grp)
+{
+    const Route& R = route();
+    const MoeArgs& a = R.a;
+    const Shape& sh = R.sh;
+    const int lane = threadIdx.x & 31;
     __syncwarp();        // lane 0's acquiring arrival is ordered before every lane's loads below
     const RunRec run = R.runs[r];
     const int64_t* row = a.table + (int64_t)run.expert * kTableWidth;
     const int S = sh.S, N = 2 * a.I, KS = sh.KSg, ng = sh.ng;
-    const __half* scales = (const __half*)row[9];
-    const __half *sv_g = scales + a.H, *sv_u = sv_g + a.I, *su_d = sv_u + a.I;
-    const __half* lr = (const __half*)row[14];
-    const int rg = lr ? (int)row[16] : 0, rd = lr ? (int)row[17] : 0, hw = (int)row[18];
-    const __half* lr4 = run.level == 4 ? (const __half*)row[15] : nullptr;
+    const size_t slice = (size_t)S * N;
     const int col = grp * 128 + lane * 4;
+    const float* part = a.part_gu + col;
+    int slot = R.order[run.first];
+    float4 fg = sum_slices(part + (size_t)slot * N, slice, KS), fu = sum_slices(part + (size_t)slot * N + a.I, slice, KS);
+    const __half* scales = R.scales[slot];
+    const uint2 sv_g = *(const uint2*)(scales + a.H + col), sv_u = *(const uint2*)(scales + a.H + a.I + col),
+                su_d = *(const uint2*)(scales + a.H + 2 * a.I + col);
+    const __half* lr = R.lr[slot];
+    const int rg = lr ? (int)row[16] : 0, rd = lr ? (int)row[17] : 0, hw = (int)row[18];
+    const __half* lr4 = lr && run.level == 4 ? (const __half*)row[15] : nullptr;
+#pragma unroll 1
     for (int j = 0; j < run.count; ++j)
     {
-        const int slot = R.order[run.first + j];
-        float z[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int q = 0; q < rg; ++q)          // z = x V_gu^T on the unrotated input
+        const float4 cur[2] = {fg, fu};
+        const int now = slot;
+        if (j + 1 < run.count)
         {
-            const __half* xr = a.x + (size_t)(slot / a.topk) * a.H;
-            float d = 0.f;
-            for (int k = lane * 4; k < a.H; k += 128)
-            {
-                float f[4], w[4];
-                load4h(xr + k, f); load4h(lr + (size_t)q * a.H + k, w);
-                d += f[0] * w[0] + f[1] * w[1] + f[2] * w[2] + f[3] * w[3];
-            }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            z[q] = d;
+            slot = R.order[run.first + j + 1];
+            fg = sum_slices(part + (size_t)slot * N, slice, KS); fu = sum_slices(part + (size_t)slot * N + a.I, slice, KS);
+        }
+        float z[4] = {0.f, 0.f, 0.f, 0.f};
+        if (rg)
+        {
+            const float4 f = *(const float4*)R.zg[now];
+            z[0] = f.x; z[1] = f.y; z[2] = f.z; z[3] = f.w;
         }
         float gu[2][4];
 #pragma unroll
         for (int u = 0; u < 2; ++u)
         {
-            float v[4] = {0.f, 0.f, 0.f, 0.f}, sc[4];
-            for (int q = 0; q < KS; ++q)
-            {
-                const float4 f = __ldcg((const float4*)(a.part_gu + ((size_t)q * S + slot) * N + u * a.I + col));
-                v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
-            }
+            float v[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w}, sc[4];
             wht128(v, lane);
-            load4h((u ? sv_u : sv_g) + col, sc);
+            unpack4h(u ? sv_u : sv_g, sc);
 #pragma unroll
             for (int i = 0; i < 4; ++i) v[i] *= sc[i];
             for (int q = 0; q < rg; ++q)
@@ -499,7 +641,7 @@ __device__ __forceinline__ void finish_gate_up(const MoeArgs& a, const Shape& sh
             for (int i = 0; i < 4; ++i) gu[u][i] = v[i];
         }
         float v[4], sc[4];
-        load4h(su_d + col, sc);
+        unpack4h(su_d, sc);
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] = silu(gu[0][i]) * gu[1][i];
         for (int q = 0; q < rd; ++q)          // this group's share of z_dn = sw V_dn^T
@@ -509,13 +651,13 @@ __device__ __forceinline__ void finish_gate_up(const MoeArgs& a, const Shape& sh
             float d = v[0] * w[0] + v[1] * w[1] + v[2] * w[2] + v[3] * w[3];
 #pragma unroll
             for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (lane == 0) a.zd[((size_t)slot * ng + grp) * 4 + q] = d;
+            if (lane == 0) a.zd[((size_t)now * ng + grp) * 4 + q] = d;
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] *= sc[i];
         wht128(v, lane);
-        if (hw <= 128) store4h_operand(a.h + (size_t)slot * a.I + grp * 128, lane, v);
-        else __stcg((float4*)(a.part_gu + (size_t)slot * N + col), make_float4(v[0], v[1], v[2], v[3]));   // fp32 stage: gate columns, k-slice 0
+        if (hw <= 128) store4h_operand(a.h + (size_t)now * a.I + grp * 128, lane, v);
+        else __stcg((float4*)(a.part_gu + (size_t)now * N + col), make_float4(v[0], v[1], v[2], v[3]));   // fp32 stage: gate columns, k-slice 0
     }
     int done = 1;       // groups of this run whose h is now complete
     if (hw > 128)
@@ -527,8 +669,8 @@ __device__ __forceinline__ void finish_gate_up(const MoeArgs& a, const Shape& sh
         if (lane == 0)
         {
             int* ch = a.cnt_gu + S * ng + r * ng + b0;
-            last = add_acq_rel(ch, 1) == nb - 1;
-            if (last) *ch = 0;
+            last = add_release(ch, 1) == nb - 1;
+            if (last) { ld_acquire(ch); *ch = 0; }
         }
         last = __shfl_sync(0xffffffffu, last, 0);
         done = 0;
@@ -557,7 +699,7 @@ __device__ __forceinline__ void finish_gate_up(const MoeArgs& a, const Shape& sh
     if (done)
     {
         __syncwarp();
-        if (lane == 0) add_acq_rel(a.cnt_gu + 2 * S * ng + r, done);
+        if (lane == 0) add_release(a.cnt_gu + 2 * S * ng + r, done);
     }
 }
 
@@ -610,124 +752,473 @@ __device__ __forceinline__ bool ep_sum(const MoeArgs& a, const Shape& sh, int pa
     return true;
 }
 
-// output rows [grp * 128, +128) of token b are complete in every k-slice of every pick: weighted combine
-__device__ __forceinline__ void finish_down(const MoeArgs& a, const Shape& sh, const Route& R, int b, int grp, int lane, int par)
+// output rows [grp * 128, +128) of token b are complete in every k-slice of every pick: weighted combine, four picks at a time
+// (their loads and their rotations overlap).
+__device__ __noinline__ void finish_down(int b, int grp)
 {
+    const Route& R = route();
+    const MoeArgs& a = R.a;
+    const Shape& sh = R.sh;
+    const int lane = threadIdx.x & 31;
     __syncwarp();        // the acquiring arrival (some lane's) is ordered before every lane's loads below
-    const int S = sh.S, N = a.H, KS = sh.KSd, col = grp * 128 + lane * 4;
+    const int N = a.H, KS = sh.KSd, col = grp * 128 + lane * 4, s0 = b * a.topk;
+    const size_t slice = (size_t)sh.S * N;
     float o[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k = 0; k < a.topk; ++k)
+    for (int k0 = 0; k0 < a.topk; k0 += 4)
     {
-        const int s = b * a.topk + k, e = R.key[s];
-        if (e < 0) continue;
-        const int lv = R.lvl[s];
-        const float w = __half2float(a.rw[s]);
-        const int64_t* erow = a.table + (int64_t)e * kTableWidth;
-        const __half* sv_o = (const __half*)erow[9] + a.H + 3 * a.I;
-        float v[4] = {0.f, 0.f, 0.f, 0.f}, sc[4];
-        for (int q = 0; q < KS; ++q)
-        {
-            const float4 f = __ldcg((const float4*)(a.part_d + ((size_t)q * S + s) * N + col));
-            v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
-        }
-        wht128(v, lane);
-        load4h(sv_o + col, sc);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] *= sc[i];
-        const __half* lr = (const __half*)erow[14];
-        const int rd = lr ? (int)erow[17] : 0;
-        if (rd)
-        {
-            const int rg = (int)erow[16], ng = sh.ng;
-            const __half* lr4 = lv == 4 ? (const __half*)erow[15] : nullptr;
-            const size_t ou = (size_t)rg * a.H + 2 * (size_t)rg * a.I + (size_t)rd * a.I;
-            for (int q = 0; q < rd; ++q)
-            {
-                float z = 0.f;
-                for (int gq = 0; gq < ng; ++gq) z += __ldcg(a.zd + ((size_t)s * ng + gq) * 4 + q);
-                float u2[4], u4[4] = {0.f, 0.f, 0.f, 0.f};
-                load4h(lr + ou + (size_t)q * a.H + col, u2);
-                if (lr4) load4h(lr4 + 2 * (size_t)rg * a.I + (size_t)q * a.H + col, u4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] += z * u2[i] + z * u4[i];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] += w * v[i];
-    }
-    if (a.world > 1) ep_send(a, sh, par, b, grp, lane, o);
-    else *(float4*)(a.out + (size_t)b * a.H + col) = make_float4(o[0], o[1], o[2], o[3]);
-}
-
-// ---------------------------------------------------------------- GEMV pieces
-// One warp's piece: strip `strip` of the projection over chunks [c0, c1) for the run's tokens; the partial sums go to
-// part[ks][slot][row].  false = a wait ran out.
-template <int NT>
-__device__ __forceinline__ bool gemv_piece(const MoeArgs& a, const Shape& sh, const Route& R, const RunRec& run, int DOWN, int strip, int c0, int c1,
-                                           int up, int ks, const int* gate_counter, int gate_target, uint32_t ring, int lane)
-{
-    const int g = lane >> 2, t4 = lane & 3;
-    const int N = DOWN ? a.H : 2 * a.I, K = DOWN ? a.I : a.H;
-    const int64_t* row = a.table + (int64_t)run.expert * kTableWidth;
-    const int rc = (int)row[10 + DOWN], nm = DOWN ? a.nm_dn : a.nm_gu, bk = (int)(row[19] >> (8 * DOWN)) & 0xFF;
-    const bool level4 = run.level >= 4;
-    StripJob J;
-    J.P = planes_from_row(row, DOWN);
-    J.C = K / 128; J.NS = N / 16; J.c0 = c0; J.c1 = c1;
-    J.sr = locate_strip(J.P, strip, J.C, J.NS, nm, level4);
-    J.ntiles = (run.count + 7) >> 3;
-    J.has_token = g < run.count;
-    J.x0 = (const uint8_t*)(DOWN ? a.h : a.xrot);
-#pragma unroll
-    for (int nt = 0; nt < kRunTiles; ++nt)
-    {
-        const int j = nt * 8 + g;
-        const int slot = R.order[run.first + (j < run.count ? j : 0)];
-        J.xoff[nt] = (uint32_t)((DOWN ? (size_t)slot * a.I : ((size_t)slot * 2 + up) * a.H) * 2 + t4 * 64);
-    }
-    J.ring = ring; J.gate = gate_counter; J.gate_target = gate_target; J.status = a.status;
-    float acc[NT][4];
-    bool ok = true;
-#define NQ_RUN(RES, RCV, BKV) ok = strip_gemv<RES, RCV, BKV, NT>(J, acc)
-    NQ_WITH_CODES(level4, rc, bk, NQ_GEMV_CODES, NQ_RUN);
-#undef NQ_RUN
-    if (!ok) return false;
-    float* part = DOWN ? a.part_d : a.part_gu;
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+        float v[4][4], w[4];
+        uint2 sv[4];
+        bool any_lr = false;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
         {
-            const int j = nt * 8 + t4 * 2 + (i & 1), rr = strip * 16 + g + (i >> 1) * 8;
-            if (j < run.count) __stcg(part + ((size_t)ks * sh.S + R.order[run.first + j]) * N + rr, acc[nt][i]);
+            const int s = s0 + k0 + i;
+            const bool on = k0 + i < a.topk && R.key[s] >= 0;
+            w[i] = on ? __half2float(a.rw[s]) : 0.f;
+            sv[i] = on ? *(const uint2*)(R.scales[s] + a.H + 3 * a.I + col) : make_uint2(0u, 0u);
+            const float4 f = on ? sum_slices(a.part_d + (size_t)s * N + col, slice, KS) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i][0] = f.x; v[i][1] = f.y; v[i][2] = f.z; v[i][3] = f.w;
+            any_lr = any_lr || (on && R.lr[s] != nullptr);
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) wht128(v[i], lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            float sc[4];
+            unpack4h(sv[i], sc);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[i][e] *= sc[e];
+        }
+        if (any_lr)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const int s = s0 + k0 + i;
+                if (k0 + i >= a.topk || R.key[s] < 0) continue;
+                const __half* lr = R.lr[s];
+                if (!lr) continue;
+                const int64_t* erow = a.table + (int64_t)R.key[s] * kTableWidth;
+                const int rd = (int)erow[17], rg = (int)erow[16], ng = sh.ng;
+                const __half* lr4 = R.lvl[s] == 4 ? (const __half*)erow[15] : nullptr;
+                const size_t ou = (size_t)rg * a.H + 2 * (size_t)rg * a.I + (size_t)rd * a.I;
+                float z[4] = {0.f, 0.f, 0.f, 0.f};           // z_dn: the column groups' shares, a lane per group
+                for (int gq = lane; gq < ng; gq += 32)
+                {
+                    const float* zp = a.zd + ((size_t)s * ng + gq) * 4;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q < rd) z[q] += __ldcg(zp + q);
+                }
+                for (int q = 0; q < rd; ++q)
+                {
+                    float zq = q == 0 ? z[0] : q == 1 ? z[1] : q == 2 ? z[2] : z[3];
+#pragma unroll
+                    for (int m = 16; m; m >>= 1) zq += __shfl_xor_sync(0xffffffffu, zq, m);
+                    float u2[4], u4[4] = {0.f, 0.f, 0.f, 0.f};
+                    load4h(lr + ou + (size_t)q * a.H + col, u2);
+                    if (lr4) load4h(lr4 + 2 * (size_t)rg * a.I + (size_t)q * a.H + col, u4);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[i][e] += zq * u2[e] + zq * u4[e];
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] += w[i] * v[i][e];
+    }
+    if (a.world > 1) ep_send(a, sh, R.par, b, grp, lane, o);
+    else *(float4*)(a.out + (size_t)b * a.H + col) = make_float4(o[0], o[1], o[2], o[3]);
+}
+
+// ---------------------------------------------------------------- shares and jobs
+// k-slices actually used, a divisor of the caller's: the fewest that keep the fullest CTA within 3 % of what any divisor
+// gives it (every slice adds arrivals and partial sums; calls for one half of the layer use the caller's count, whose
+// partial sums stay readable).  A lane per candidate; a count beyond 32 stands as it is.
+__device__ __forceinline__ int choose_ksplit(int strips, int C, int ks, int ctas, int lane)
+{
+    if (ks == 1) return 1;
+    const int d = lane + 1, q = quot(ks, d);
+    int load = 0x7fffffff;
+    if (ks <= 32 && q * d == ks)
+    {
+        const int share = quot_any(strips * d + ctas - 1, ctas) * quot(C, d);
+        load = share < kWarps ? kWarps : share;
+    }
+    const int best = __reduce_min_sync(0xffffffffu, load);
+    const unsigned good = __ballot_sync(0xffffffffu, load != 0x7fffffff && load * 32 <= best * 33);
+    return good ? __ffs(good) : ks;
+}
+__device__ __forceinline__ Shape make_shape(const MoeArgs& a, int nruns, int ctas)
+{
+    Shape sh;
+    sh.S = a.B * a.topk; sh.ng = a.I >> 7; sh.ngH = a.H >> 7; sh.nruns = nruns;
+    sh.nu_gu = (a.which & 1) ? (a.I >> 3) * sh.ngH : 0;
+    sh.nu_dn = (a.which & 2) ? (a.H >> 4) * sh.ng : 0;
+    sh.KSg = sh.KSd = 1;             // filled in once the lists are cut
+    // Two lists per phase hide the hand-over of h (the way from the last gate|up piece to the first down unit) but cost rows and
+    // barriers of their own: worth it from about a dozen units per warp on.
+    sh.split = a.which == 3 && nruns > 1 && nruns * (sh.nu_dn >> 2) >= ctas * kWarps ? (nruns + 1) >> 1 : nruns;
+    return sh;
+}
+// costs of the units before each run of phase d, by one warp
+__device__ __forceinline__ void prefix_costs(const Shape& sh, Route& R, int d, float NU, int lane)
+{
+    float run = 0.f;
+    for (int r0 = 0; r0 < sh.nruns; r0 += 32)
+    {
+        const int r = r0 + lane;
+        const float own = r < sh.nruns ? R.cost[d][r] * NU : 0.f;
+        float v = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+        if (r < sh.nruns) R.base[d][r] = run + v - own;
+        run += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) R.base[d][sh.nruns] = run;
+    __syncwarp();
+}
+// list position at which `cost` (counted from the phase's first run) has been passed, rounded to whole steps of `step` units.  The
+// arithmetic is approximate, but every CTA evaluates the same expression for the same cut.
+__device__ __forceinline__ int position_at(const Route& R, const List& L, float cost, int step)
+{
+    const float* base = R.base[L.d];
+    int lo = L.run0, hi = L.run1;                // base[lo] <= cost < base[hi + 1]
+    while (lo < hi)
+    {
+        const int mid = (lo + hi + 1) >> 1;
+        if (base[mid] <= cost) lo = mid; else hi = mid - 1;
+    }
+    const int at = (lo - L.run0) * L.NU;
+    if (lo >= L.run1) return at;
+    const int n = __float2int_rn(__fdividef(cost - base[lo], R.cost[L.d][lo] * (float)step)) * step;
+    return at + (n < 0 ? 0 : n < L.NU ? n : L.NU);
+}
+__device__ __forceinline__ float cost_at(const Route& R, const List& L, int p)
+{
+    const int r = quot_any(p, L.NU);
+    return R.base[L.d][L.run0 + r] + (L.run0 + r < L.run1 ? (float)(p - r * L.NU) * R.cost[L.d][L.run0 + r] : 0.f);
+}
+// The job that starts at position `at` of the share in work, by one warp: how far its rows fit, the warps' ranges, the table rows
+// of its first runs.  rows_at: byte offset of its rows behind the slots.
+__device__ __forceinline__ void cut_job(const MoeArgs& a, const Shape& sh, Route& R, const List& L, Job& job, int l, int at, int rows_at, int lane)
+{
+    int stop = job.end, run0 = 0, row0 = 0, nrows = 0;
+    if (at < stop)
+    {
+        const int row_bytes = (L.d ? sh.ng : sh.ngH) * kRowStep, room = quot(rows_room(a.slot_floats) - rows_at, row_bytes);
+        int h = quot_any(at, L.NH), up = L.d ? 0 : h & 1, run = L.run0 + (L.d ? h : h >> 1);
+        run0 = run; row0 = row_id(R.runs[run], L.d, up);
+        for (; h * L.NH < stop; ++h)           // (run) or (run, gate / up) by (run, gate / up)
+        {
+            const int c = R.runs[run].count;
+            if (nrows + c > room) { stop = h * L.NH; break; }
+            nrows += c;
+            if (L.d || up) { ++run; up = 0; } else up = 1;
+        }
+    }
+    if (lane <= kWarps)
+    {
+        int g = at;
+        if (at < stop)
+        {
+            const float ca = cost_at(R, L, at), cb = cost_at(R, L, stop);
+            g = lane == 0 ? at : lane == kWarps ? stop : position_at(R, L, ca + (cb - ca) * ((float)lane / kWarps), 1);
+            g = g < at ? at : g > stop ? stop : g;
+        }
+        job.bound[lane] = g;
+    }
+    if (at < stop)
+        for (int i = lane; i < kCachedRows * kTableWidth; i += 32)
+        {
+            const int k = i / kTableWidth, run = run0 + k;
+            if (run < L.run1) job.row[k][i - k * kTableWidth] = a.table[(int64_t)R.runs[run].expert * kTableWidth + i - k * kTableWidth];
+        }
+    if (lane == 0)
+    {
+        job.at = at; job.stop = stop; job.seq += kLists; job.staged = 0;
+        job.run0 = run0; job.row0 = row0; job.nrows = nrows; job.rows_at = rows_at;
+    }
+    __syncwarp();
+}
+// share k of a list (an empty one if k >= the number of CTAs), by one warp
+__device__ __forceinline__ void cut_share(const MoeArgs& a, const Shape& sh, Route& R, const List& L, Job& job, int l, int k, int lane)
+{
+    const float c0 = R.base[L.d][L.run0], each = __fdividef(R.base[L.d][L.run1] - c0, (float)gridDim.x);
+    const bool any = k < (int)gridDim.x && L.NU > 0 && L.run0 < L.run1;
+    const int A = any ? position_at(R, L, fmaf(each, (float)k, c0), L.cps) : 0;
+    const int B = !any ? 0 : k + 1 == (int)gridDim.x ? (L.run1 - L.run0) * L.NU : position_at(R, L, fmaf(each, (float)(k + 1), c0), L.cps);
+    if (lane == 0) { job.share = k; job.next = kUndecided; job.end = B; }
+    __syncwarp();
+    cut_job(a, sh, R, L, job, l, A < B ? A : B, 0, lane);
+}
+// this CTA's next share of a list (>= the number of CTAs: none left), decided once per share by the first warp that gets here
+__device__ __forceinline__ int next_share(const MoeArgs& a, Job& job, int l, int lane)
+{
+    int v = 0;
+    if (lane == 0)
+    {
+        const int ctas = (int)gridDim.x, shift = 16 * (l & 1);
+        v = atomicCAS(&job.next, kUndecided, kDeciding);
+        if (v == kUndecided)
+        {
+            // with every CTA resident all shares are drawn by now: a plain read tells
+            int* q = a.wq + (l & 2);
+            v = (ld_relaxed(q) >> shift & 0xFFFF) < ctas ? atomicAdd(q, 1 << shift) >> shift & 0xFFFF : ctas;
+            *(volatile int*)&job.next = v;
+        }
+        while (v == kDeciding) v = *(volatile int*)&job.next;
+    }
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// ---------------------------------------------------------------- a warp's share of a job
+__device__ __forceinline__ int ld_slot_seq(const int* p)
+{
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
+    return v;
+}
+// Part of a piece is through.  The warp in whose range the piece starts owns it: it adds the following warps' shares (if the
+// piece goes on behind its range), stores the sums to part[ks][slot][row] and counts the piece; the others leave theirs in
+// their slot (fragment order [tile][i][lane]).  false = a wait ran out.
+template <int NT>
+__device__ __noinline__ bool piece_done()
+{
+    Route& R = route();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const StripJob& pc = R.strip[warp];
+    const MoeArgs& a = R.a;
+    const Shape& sh = R.sh;
+    const Job& job = R.job[pc.l];
+    const int g = lane >> 2, t4 = lane & 3, d = pc.l >> 1, N = d ? a.H : 2 * a.I, buf = pc.l & 1;
+    const RunRec run = R.runs[pc.r];
+    float acc[NT][4];
+    {
+        const float* from = slot_of(R, 2, warp) + lane;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[nt][i] = from[(nt * 4 + i) * 32];
+    }
+    if (!pc.starts)
+    {
+        float* to = slot_of(R, buf, warp) + lane;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) to[(nt * 4 + i) * 32] = acc[nt][i];
+        __syncwarp();
+        if (lane == 0) asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(&R.slot_seq[buf][warp])), "r"(job.seq) : "memory");
+        return true;
+    }
+    int left = pc.left;
+    for (int v = warp + 1; left > 0 && v < kWarps; ++v)
+    {
+        const int n = job.bound[v + 1] - job.bound[v];
+        if (n <= 0) continue;
+        unsigned long long t0 = 0;
+        for (uint32_t i = 0; ld_slot_seq(&R.slot_seq[buf][v]) != job.seq; ++i)
+            if ((i & 63u) == 63u)
+            {
+                if (ld_relaxed(a.status) != 0) return false;
+                unsigned long long t;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+                if (t0 == 0) t0 = t;
+                else if (t - t0 > kWaitNs) { atomicExch(a.status, 1); return false; }
+            }
+        __syncwarp();
+        const float* from = slot_of(R, buf, v) + lane;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[nt][i] += from[(nt * 4 + i) * 32];
+        left -= n;
+    }
+    float* part = (d ? a.part_d : a.part_gu) + (size_t)pc.ks * sh.S * N + pc.strip * 16 + g;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+        {
+            const int j = nt * 8 + t4 * 2 + e;
+            if (j < run.count)
+            {
+                float* to = part + (size_t)R.order[run.first + j] * N;
+                __stcg(to, acc[nt][e]);
+                __stcg(to + 8, acc[nt][e + 2]);
+            }
+        }
+    // Every arrival below is a releasing atomic issued after this warp barrier: the barrier orders all lanes' partial-sum
+    // stores before it, the release publishes them, the acquire of the last one to arrive sees everybody's.
+    __syncwarp();
+    int last = 0;
+    if (!d)
+    {
+        const int half = a.I >> 4, grp = (pc.strip >= half ? pc.strip - half : pc.strip) >> 3;
+        if (lane == 0)
+        {
+            int* cnt = a.cnt_gu + pc.r * sh.ng + grp;
+            last = add_release(cnt, 1) == 2 * sh.KSg * 8 - 1;
+            if (last) { ld_acquire(cnt); *cnt = 0; }
+        }
+        if (__shfl_sync(0xffffffffu, last, 0)) finish_gate_up(pc.r, grp);
+    }
+    else
+    {
+        // one arrival per token of the run on its (token, group) counter
+        const int grp = pc.strip >> 3;
+        int b = 0;
+        if (lane < run.count)
+        {
+            b = quot(R.order[run.first + lane], a.topk);
+            int* cnt = a.cnt_d + b * sh.ngH + grp;
+            last = add_release(cnt, 1) == (int)R.nvalid[b] * sh.KSd * 8 - 1;
+            if (last) { ld_acquire(cnt); *cnt = 0; }
+        }
+        unsigned todo = __ballot_sync(0xffffffffu, last);
+        while (todo)
+        {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            finish_down(__shfl_sync(0xffffffffu, b, src), grp);
+        }
+    }
     return true;
 }
 
-__device__ __forceinline__ Shape make_shape(const MoeArgs& a, int nruns, int nwarps)
+// this warp's range of a job, piece by piece; false = a wait ran out
+template <int NT>
+__device__ __forceinline__ bool run_piece(int mode, int rc, int bk)
 {
-    Shape sh;
-    sh.S = a.B * a.topk; sh.ng = a.I / 128; sh.ngH = a.H / 128; sh.KSg = a.ks_gu; sh.KSd = a.ks_dn;
-    sh.rot_blocks = (sh.S * sh.ngH + nwarps - 1) / nwarps;
-    sh.nparts = (sh.ngH + sh.rot_blocks - 1) / sh.rot_blocks; sh.nruns = nruns;
-    sh.per_run_gu = sh.ng * 2 * sh.KSg * 8; sh.per_run_dn = sh.ngH * sh.KSd * 8;
-    sh.n_rot = (a.which & 1) ? sh.S * sh.nparts : 0;
-    sh.n_gu = (a.which & 1) ? nruns * sh.per_run_gu : 0;
-    sh.n_dn = (a.which & 2) ? nruns * sh.per_run_dn : 0;
-    return sh;
+#define NQ_RUN(RES, RCV, BKV) do { if (RES && mode == 2) strip_gemv<RES ? 2 : 0, RCV, BKV, NT>(); else strip_gemv<RES ? 1 : 0, RCV, BKV, NT>(); } while (0)
+    NQ_WITH_CODES(mode > 0, rc, bk, NQ_GEMV_CODES, NQ_RUN);
+#undef NQ_RUN
+    return piece_done<NT>();
+}
+__device__ __noinline__ bool run_job(int l)
+{
+    Route& R = route();
+    const MoeArgs& a = R.a;
+    const List L = list_of(a, R.sh, l);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Job& job = R.job[l];
+    StripJob& J = R.strip[warp];
+    const int d = L.d, row_bytes = ((d ? a.I : a.H) >> 7) * kRowStep, NS = (d ? a.H : 2 * a.I) >> 4;
+    const uint32_t rows = rows_base(R) + job.rows_at;
+    const int end = job.bound[warp + 1];
+    for (int at = job.bound[warp]; at < end;)
+    {
+        const int k = quot_any(at, L.NU), r = L.run0 + k, u = at - k * L.NU, s = quot(u, L.C), ch = u - s * L.C, up = u >= L.NH;
+        const int ks = L.cps == L.C ? 0 : quot(ch, L.cps), stop = (ks + 1) * L.cps, n = stop - ch < end - at ? stop - ch : end - at;
+        at += n;
+        const RunRec run = R.runs[r];
+        const int64_t* row = a.table + (int64_t)run.expert * kTableWidth;
+        const bool cached = r - job.run0 < kCachedRows;
+        const int64_t* crow = job.row[cached ? r - job.run0 : 0];
+        const int rc = (int)(cached ? crow[10 + d] : row[10 + d]), bk = (int)((cached ? crow[19] : row[19]) >> (8 * d)) & 0xFF;
+        const ProjPlanes P = cached ? planes_from_row(crow, d) : planes_from_row(row, d);
+        const int mode = run.level < 4 ? 0 : P.flags ? 2 : 1, nm = mode == 2 ? (d ? a.nm_dn : a.nm_gu) : L.C;
+        if (lane == 0)
+        {
+            J.P = P;
+            J.nrec = (size_t)NS * L.C * 32; J.res_nrec = (size_t)NS * nm * 32;
+            J.unit0 = (size_t)s * L.C + ch; J.res0 = (size_t)s * nm;
+            J.flags = mode == 2 ? (unsigned long long)__ldg((const unsigned long long*)P.flags + s) : 0ull;
+            J.c0 = ch; J.n = n;
+            J.x = rows + (row_id(run, d, up) - job.row0) * row_bytes; J.row_bytes = row_bytes; J.count = run.count;
+            J.l = l; J.r = r; J.strip = s; J.ks = ks; J.left = stop - ch - n; J.starts = ch == ks * L.cps;
+        }
+        __syncwarp();
+        bool ok;
+        if (run.count <= 8) ok = run_piece<1>(mode, rc, bk);
+        else if (run.count <= 16) ok = run_piece<2>(mode, rc, bk);
+        else ok = run_piece<kRunTiles>(mode, rc, bk);
+        if (!ok) return false;
+        __syncwarp();
+    }
+    return true;
+}
+// the first unit of this warp's range on its way to L2, and the output scales of the strips of the job
+__device__ __forceinline__ void prefetch_job(const MoeArgs& a, const Route& R, const List& L, const Job& job, int lane, int warp)
+{
+    const int at = job.bound[warp];
+    if (at >= job.bound[warp + 1]) return;
+    const int k = quot_any(at, L.NU), u = at - k * L.NU, r = L.run0 + k;
+    const RunRec run = R.runs[r];
+    const int64_t* row = r - job.run0 < kCachedRows ? job.row[r - job.run0] : a.table + (int64_t)run.expert * kTableWidth;
+    const ProjPlanes P = planes_from_row(row, L.d);
+    // (the first sub-array of a plane holds 16 bytes per record, 8 for the codes below 128 bits)
+    prefetch_l2((const uint8_t*)P.base + ((size_t)u * 32 + lane) * ((row[19] >> (8 * L.d) & 0xFF) ? 8 : 16));
+    if (run.level >= 4 && !P.flags) prefetch_l2(P.p4 + ((size_t)u * 32 + lane) * (0x29D >> (int)row[10 + L.d] & 1 ? 16 : 8));
+    const __half* sc = (const __half*)row[9];
+    const int col = quot(u, L.C) * 16;
+    if (lane == 0) prefetch_l2(L.d ? sc + a.H + 3 * a.I + col : sc + a.H + col);
+    if (lane == 1 && !L.d) prefetch_l2(sc + a.H + 2 * a.I + (col >= a.I ? col - a.I : col));
 }
 
-// persistent CTAs of independent warps
-__global__ void __launch_bounds__(kThreads, NQ_GEMV_MINBLOCKS) moe_decode_kernel(MoeArgs a)
+// one CTA per SM, warps independent of one another inside a job
+__global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_constant__ MoeArgs a)
 {
-    extern __shared__ __align__(16) uint8_t smem_ring[];   // [kWarps][kDepth][kGemvStage]
-    __shared__ Route R;
+    Route& R = route();
+    __shared__ int s_small;
     launch_dependents();
     grid_dependency_wait();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    build_route(a, R);
-    const int nwarps = (int)gridDim.x * kWarps;
-    const Shape sh = make_shape(a, R.nruns, nwarps);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ctas = (int)gridDim.x, nwarps = ctas * kWarps;
+    if (warp == kWarps - 1)
+    {
+        // this CTA's shares: one of each list that there is
+        if (lane < 2) R.draws[lane] = (a.which >> lane & 1) ? atomicAdd(a.wq + 2 * lane, 0x10001) : ctas | ctas << 16;
+        for (int i = lane; i < 2 * kWarps; i += 32) (&R.slot_seq[0][0])[i] = 0;
+        if (lane < kLists) R.job[lane].seq = lane;
+        for (int i = lane; i < (int)sizeof(MoeArgs) / 4; i += 32) ((int*)&R.a)[i] = ((const int*)&a)[i];
+    }
+    if (a.B * a.topk <= 32)
+    {
+        if (warp == 0)
+        {
+            const bool done = build_route_warp(a, R, lane);
+            if (lane == 0) s_small = done;
+        }
+        __syncthreads();
+    }
+    else if (threadIdx.x == 0) s_small = 0;
+    if (a.B * a.topk > 32 || !s_small) build_route_cta(a, R);
+    Shape sh = make_shape(a, R.nruns, ctas);
+    if (warp < kLists)
+    {
+        // a warp per list
+        const int l = warp, d = l >> 1, ks = d ? a.ks_dn : a.ks_gu;
+        const int use = a.which == 3 ? choose_ksplit(sh.nruns * (d ? a.H >> 4 : a.I >> 3), d ? sh.ng : sh.ngH, ks, ctas, lane) : ks;
+        if (lane == 0) R.ks[d] = use;                 // (the two warps of a phase store the same)
+        sh.KSg = sh.KSd = use;
+        prefix_costs(sh, R, d, (float)(d ? sh.nu_dn : sh.nu_gu), lane);
+        cut_share(a, sh, R, list_of(a, sh, l), R.job[l], l, R.draws[d] >> (16 * (l & 1)) & 0xFFFF, lane);
+    }
+    __syncthreads();
+    sh.KSg = R.ks[0]; sh.KSd = R.ks[1];
+    const uint32_t rows = rows_base(R);
+    // the rows of both gate|up lists are prepared together when they fit
+    const bool both = R.job[0].stop == R.job[0].end && (R.job[0].nrows + R.job[1].nrows) * (sh.ngH * kRowStep) <= rows_room(a.slot_floats);
+    const int rows1 = both ? R.job[0].nrows * (sh.ngH * kRowStep) : 0;
+    if (threadIdx.x == 0)
+    {
+        R.sh = sh;
+        R.job[0].staged = 1; R.job[1].staged = both; R.job[1].rows_at = rows1;
+    }
+    if (a.which & 1)
+    {
+        int w0 = 0;
+        for (int l = 0; l < 1 + both; ++l)
+        {
+            const Job& job = R.job[l];
+            if (job.at >= job.stop) continue;
+            w0 += rotate_rows(a, sh, R, job, rows + (l ? rows1 : 0), w0 % kWarps, lane, warp);
+            const RunRec hi = R.runs[list_of(a, sh, l).run0 + quot_any(job.stop - 1, sh.nu_gu)];
+            low_rank_inputs(a, R, R.runs[job.run0].first, hi.first + hi.count, lane, warp);
+        }
+        prefetch_job(a, R, list_of(a, sh, 0), R.job[0], lane, warp);
+    }
     if (blockIdx.x == 0 && a.hits && (int)threadIdx.x < sh.S)
     {
         const int64_t es = a.sel[threadIdx.x];
@@ -735,111 +1226,79 @@ __global__ void __launch_bounds__(kThreads, NQ_GEMV_MINBLOCKS) moe_decode_kernel
     }
     const bool ep = a.world > 1 && a.which == 3;
     const int par = ep ? (*(volatile int*)a.epoch & 1) : 0;
+    if (threadIdx.x == 0) R.par = par;
+    const int gw = warp * ctas + (int)blockIdx.x;    // tasks below are dealt out CTA by CTA
     // rows of tokens none of whose picks is resident here are defined as zero (nothing else writes them); under expert
     // parallelism this rank's slice of such a token is a zero slice, sent like any other
     if (a.which & 2)
     {
         if (!ep)
         {
-            for (int b = blockIdx.x; b < a.B; b += gridDim.x)
+            for (int b = blockIdx.x; b < a.B; b += ctas)
                 if (R.nvalid[b] == 0)
                     for (int i = threadIdx.x; i < a.H; i += kThreads) a.out[(size_t)b * a.H + i] = 0.f;
         }
         else
         {
             const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int task = (int)blockIdx.x * kWarps + warp; task < a.B * sh.ngH; task += (int)gridDim.x * kWarps)
+            for (int task = gw; task < a.B * sh.ngH; task += nwarps)
                 if (R.nvalid[task / sh.ngH] == 0) ep_send(a, sh, par, task / sh.ngH, task % sh.ngH, lane, zero);
         }
     }
-
-    const uint32_t ring = smem_addr(smem_ring) + warp * (kDepth * kGemvStage);
-    const int total = sh.n_rot + sh.n_gu + sh.n_dn;
-    bool rotated = false;      // this warp has seen every rotation piece finished
-    int ready_run = -1;        // the run whose h this warp has seen complete
-    // a warp's first piece is its own index (thousands of warps start at once: no burst of atomics on one address); later
-    // ones come from the queue counter, which therefore counts from the number of warps
-    for (int round = 0;; ++round)
+    __syncthreads();
+    bool ok = true;
+#pragma unroll 1
+    for (int l = 0; l < kLists; ++l)
     {
-        int piece = (int)blockIdx.x * kWarps + warp;
-        if (round)
+        if (!(a.which >> (l >> 1) & 1)) continue;
+        const List L = list_of(a, sh, l);
+        if (L.run0 >= L.run1) continue;
+        Job& job = R.job[l];
+        for (;;)
         {
-            if (lane == 0) piece = nwarps + atomicAdd(a.wq, 1);
-            else if (lane == 1) piece = ld_acquire(a.status);
-            const int raised = __shfl_sync(0xffffffffu, piece, 1);
-            piece = __shfl_sync(0xffffffffu, piece, 0);
-            if (raised) break;
-        }
-        if (piece >= total) break;
-        if (piece < sh.n_rot) { rotate_piece(a, sh, R, piece, lane); continue; }
-        piece -= sh.n_rot;
-        // gate|up: (run, group, gate / up, k-slice, strip of the group); down: (run, group, k-slice, strip of the group)
-        const int down = piece >= sh.n_gu;
-        if (down) piece -= sh.n_gu;
-        const int per_run = down ? sh.per_run_dn : sh.per_run_gu, KS = down ? sh.KSd : sh.KSg;
-        const int r = piece / per_run, rem = piece - r * per_run;
-        const int per_grp = (down ? 1 : 2) * KS * 8, grp = rem / per_grp, rem2 = rem - grp * per_grp;
-        const int up = rem2 / (KS * 8), rem3 = rem2 - up * (KS * 8), ks = rem3 >> 3, s8 = rem3 & 7;
-        const RunRec run = R.runs[r];
-        const int C = (down ? a.I : a.H) / 128, c0 = ks * (C / KS), c1 = c0 + C / KS;
-        const int strip = down ? grp * 8 + s8 : (up * a.I + grp * 128) / 16 + s8;
-        const int* gate = nullptr;
-        int target = 0;
-        if (!down) { if (!rotated) { gate = a.wq + 2; target = sh.n_rot; } }
-        else if ((a.which & 1) && ready_run != r) { gate = a.cnt_gu + 2 * sh.S * sh.ng + r; target = sh.ng; }
-        bool ok;
-        if (run.count <= 8) ok = gemv_piece<1>(a, sh, R, run, down, strip, c0, c1, up, ks, gate, target, ring, lane);
-        else ok = gemv_piece<kRunTiles>(a, sh, R, run, down, strip, c0, c1, up, ks, gate, target, ring, lane);
-        if (!ok) break;
-        // Every arrival below is an acq_rel atomic issued after this warp barrier: the barrier orders all lanes' partial-sum
-        // stores before it, the release half publishes them, the acquire half of the last arrival sees everybody's.
-        __syncwarp();
-        if (!down)
-        {
-            rotated = true;
-            int last = 0;
-            if (lane == 0)
+            if (job.at < job.stop)
             {
-                int* cnt = a.cnt_gu + r * sh.ng + grp;
-                last = add_acq_rel(cnt, 1) == 2 * KS * 8 - 1;
-                if (last) *cnt = 0;
+                if (!job.staged)
+                {
+                    if (l >= 2) prefetch_job(a, R, L, job, lane, warp);
+                    __syncthreads();            // the rows of the job before are no longer needed
+                    if (l < 2)
+                    {
+                        rotate_rows(a, sh, R, job, rows + job.rows_at, 0, lane, warp);
+                        const RunRec hi = R.runs[L.run0 + quot_any(job.stop - 1, L.NU)];
+                        low_rank_inputs(a, R, R.runs[job.run0].first, hi.first + hi.count, lane, warp);
+                    }
+                    else ok = copy_rows(a, sh, R, job, rows + job.rows_at, lane, warp) && ok;
+                    __syncthreads();
+                }
+                if (ok) ok = run_job(l);
             }
-            if (__shfl_sync(0xffffffffu, last, 0)) finish_gate_up(a, sh, R, r, grp, lane);
-        }
-        else
-        {
-            ready_run = r;
-            // one arrival per token of the run on its (token, group) counter
-            int last = 0, b = 0;
-            if (lane < run.count)
+            // the rest of the share, or (only if some CTA is not resident) a share that nobody has drawn
+            const bool rest = job.stop < job.end;
+            int k = 0;
+            if (!rest && (k = next_share(a, job, l, lane)) >= ctas) break;
+            __syncthreads();
+            if (warp == 0)
             {
-                b = R.order[run.first + lane] / a.topk;
-                int* cnt = a.cnt_d + b * sh.ngH + grp;
-                last = add_acq_rel(cnt, 1) == (int)R.nvalid[b] * KS * 8 - 1;
-                if (last) *cnt = 0;
+                if (rest) cut_job(a, sh, R, L, job, l, job.stop, 0, lane);
+                else cut_share(a, sh, R, L, job, l, k, lane);
             }
-            unsigned todo = __ballot_sync(0xffffffffu, last);
-            while (todo)
-            {
-                const int src = __ffs(todo) - 1;
-                todo &= todo - 1;
-                finish_down(a, sh, R, __shfl_sync(0xffffffffu, b, src), grp, lane, par);
-            }
+            __syncthreads();
         }
     }
-    // this rank's pieces are done (or handed out): add up the slices of all ranks, one (token, group) at a time
-    // (tasks are dealt out by warp index: there are more warps than tasks for every supported shape, and no counter to fight over)
+    // this rank's units are done: add up the slices of all ranks, one (token, group) at a time (tasks are dealt out by warp
+    // index: there are more warps than tasks for every supported shape, and no counter to fight over)
     if (ep)
-        for (int task = (int)blockIdx.x * kWarps + warp; task < a.B * sh.ngH; task += nwarps)
+        for (int task = gw; task < a.B * sh.ngH; task += nwarps)
             if (!ep_sum(a, sh, par, task / sh.ngH, task % sh.ngH, lane)) break;
-    // the last CTA to leave resets the queue and the per-run counters (graph replays start from zero)
+    // the last CTA to leave resets the counters (graph replays start from zero)
     __syncthreads();
     if (threadIdx.x == 0)
     {
         __threadfence();
-        if (atomicAdd(a.wq + 1, 1) == (int)gridDim.x - 1)
+        if (atomicAdd(a.wq + 1, 1) == ctas - 1)
         {
-            a.wq[0] = 0; a.wq[1] = 0; a.wq[2] = 0; a.wq[3] = 0;
+            a.wq[0] = 0; a.wq[1] = 0; a.wq[2] = 0;
             if (ep) *a.epoch = *(volatile int*)a.epoch + 1;
             for (int r = 0; r < sh.nruns; ++r) a.cnt_gu[2 * sh.S * sh.ng + r] = 0;
             if (ld_acquire(a.status) != 0)      // a wait ran out: leave every counter clean all the same
@@ -852,7 +1311,6 @@ __global__ void __launch_bounds__(kThreads, NQ_GEMV_MINBLOCKS) moe_decode_kernel
     }
 }
 
-constexpr int kGemvSmem = kWarps * kDepth * kGemvStage;
 constexpr int kMaxDevices = 64;
 
 // CTAs that fit on the current device at once (the kernel is persistent); the first call on a device also opts the kernel
@@ -866,8 +1324,21 @@ static int resident_ctas()
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (cudaFuncSetAttribute((const void*)moe_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmem) != cudaSuccess) return 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)moe_decode_kernel, kThreads, kGemvSmem);
-    cached[dev] = sms * (per > 0 ? per : 1);
+    cached[dev] = per > 0 ? sms : 0;
     return cached[dev];
+}
+
+// Most tokens of a run: their rows (of H or I halves) have to fit into shared memory behind the slots, whose size goes with the
+// number of column tiles.  Calls of up to 8 tokens have one tile.
+static void run_limits(int B, int H, int I, int* run_cap, int* slot_floats)
+{
+    const int row = (H > I ? H : I) / 128 * kRowStep;
+    *run_cap = 0;
+    for (int tiles = 1; tiles <= (B <= 8 ? 1 : kRunTiles); tiles *= 2)
+    {
+        const int fit = rows_room(tiles * kTileFloats) / row, cap = fit < 8 * tiles ? fit : 8 * tiles;
+        if (cap > *run_cap) { *run_cap = cap; *slot_floats = tiles * kTileFloats; }
+    }
 }
 
 }  // namespace nq
@@ -882,7 +1353,7 @@ int nq_moe_workspace(int B, int topk, int H, int I, int ks_gu, int ks_dn, NqMoeW
     NQ_REQUIRE(ks_gu >= 1 && (H / 128) % ks_gu == 0 && ks_dn >= 1 && (I / 128) % ks_dn == 0, "nq_moe_workspace: k-splits %d / %d must divide %d / %d chunks", ks_gu, ks_dn, H / 128, I / 128);
     const size_t S = (size_t)B * topk;
     w->acc_gu_floats = (size_t)ks_gu * S * 2 * I;
-    w->h_halves = S * I + S * 2 * H;                    // h [S][I], then the rotated inputs [S][2][H]
+    w->h_halves = S * I + S * 2 * H;                    // h [S][I], the rest is spare
     w->acc_d_floats = (size_t)ks_dn * S * H;
     w->cnt_gu_ints = 2 * S * (I / 128) + S;
     w->cnt_d_ints = (size_t)B * (H / 128);
@@ -915,9 +1386,10 @@ static int moe_forward(const NqMoeForward* p, const NqMoeEp* ep, void* stream)
     a.x = (const __half*)p->x; a.sel = p->sel; a.rw = (const __half*)p->rw;
     a.B = p->B; a.topk = p->topk; a.E = p->E; a.H = p->H; a.I = p->I; a.nm_gu = p->nm_gu; a.nm_dn = p->nm_dn;
     a.force_level = p->force_level; a.ks_gu = p->ks_gu; a.ks_dn = p->ks_dn; a.which = p->which & 3; a.table = p->table;
-    a.status = p->cnt_h; a.h = (__half*)p->h; a.xrot = a.h + (size_t)p->B * p->topk * p->I;
+    a.status = p->cnt_h; a.h = (__half*)p->h; 
     a.part_gu = p->acc_gu; a.part_d = p->acc_d; a.zd = p->zd; a.cnt_gu = p->cnt_gu; a.cnt_d = p->cnt_d; a.wq = p->wq; a.out = p->out; a.hits = p->hits;
     a.world = 1; a.rank = 0;
+    nq::run_limits(p->B, p->H, p->I, &a.run_cap, &a.slot_floats);
     if (ep && ep->world > 1)
     {
         NQ_REQUIRE(ep->world <= nq::kEpRanks && ep->rank >= 0 && ep->rank < ep->world, "nq_moe_forward_ep: rank %d of %d", ep->rank, ep->world);

@@ -69,8 +69,8 @@ int nq_moe_forward_static(const void* x, const int64_t* sel, const void* rw, con
     const size_t o_cnt_gu = off; off = align256(off + w.cnt_gu_ints * 4);
     const size_t o_cnt_d = off; off = align256(off + w.cnt_d_ints * 4);
     const size_t o_wq = off; off = align256(off + w.wq_ints * 4);
-    const size_t counters_end = off;
     const size_t o_cnt_h = off; off = align256(off + w.cnt_h_ints * 4);
+    const size_t counters_end = off;
     const size_t o_zd = off; off = align256(off + w.zd_floats * 4);
     const size_t o_acc_gu = off; off = align256(off + w.acc_gu_floats * 4);
     const size_t o_h = off; off = align256(off + w.h_halves * 2);

@@ -131,4 +131,81 @@ struct RecordCursor
     }
 };
 
+// The same records read straight into registers, one unit ahead of their use (the decode-path kernel): a warp that decodes
+// for ~1 us between two loads needs no deeper pipeline, and the copies into shared memory, their stage addresses and the
+// reads back are gone.  Plane bytes are used once: they bypass L1, which holds the token rows.
+__device__ __forceinline__ uint4 ldg_stream128(const void* p)
+{
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ldg_stream64(const void* p)
+{
+    uint2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ldg_stream32(const void* p)
+{
+    uint32_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ldg_stream16(const void* p)
+{
+    uint16_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+
+template <int CODE>
+struct RecordReader
+{
+    using L = RecordLayout<CODE>;
+    const uint8_t *p128, *p64, *p32, *p16, *ptail;
+    uint4 v128; uint2 v64, vtail; uint32_t v32, v16;      // pieces in flight
+
+    __device__ __forceinline__ void init(const void* plane, size_t nrec, size_t unit0, int lane)
+    {
+        const uint8_t* p = (const uint8_t*)plane;
+        if constexpr (L::n128) { p128 = p + unit0 * 512 + lane * 16; p += nrec * 16; }
+        if constexpr (L::has64) { p64 = p + unit0 * 256 + lane * 8; p += nrec * 8; }
+        if constexpr (L::has32) { p32 = p + unit0 * 128 + lane * 4; p += nrec * 4; }
+        if constexpr (L::has16) { p16 = p + unit0 * 64 + lane * 2; p += nrec * 2; }
+        if constexpr (L::T != 0) ptail = p + unit0 * (4 * L::T) + ((lane * L::T) >> 5) * 4;
+    }
+    // fetch the unit at the read position and move on
+    __device__ __forceinline__ void fetch()
+    {
+        if constexpr (L::n128) { v128 = ldg_stream128(p128); p128 += 512; }
+        if constexpr (L::has64) { v64 = ldg_stream64(p64); p64 += 256; }
+        if constexpr (L::has32) { v32 = ldg_stream32(p32); p32 += 128; }
+        if constexpr (L::has16) { v16 = ldg_stream16(p16); p16 += 64; }
+        if constexpr (L::T != 0)
+        {
+            vtail.x = ldg_stream32(ptail);
+            if constexpr (L::tail2) vtail.y = ldg_stream32(ptail + 4);
+            ptail += 4 * L::T;
+        }
+    }
+    // the fetched record as stream words w[0 .. kWords), bits past the record zero
+    __device__ __forceinline__ void words(uint32_t* w, int lane) const
+    {
+        int k = 0;
+        if constexpr (L::n128) { w[k++] = v128.x; w[k++] = v128.y; w[k++] = v128.z; w[k++] = v128.w; }
+        if constexpr (L::has64) { w[k++] = v64.x; w[k++] = v64.y; }
+        if constexpr (L::has32) w[k++] = v32;
+        if constexpr (L::has16) w[k++] = v16;
+        if constexpr (L::T != 0)
+        {
+            const int sh = (lane * L::T) & 31;
+            uint32_t v = L::tail2 ? __funnelshift_r(vtail.x, vtail.y, sh) : vtail.x >> sh;
+            v &= (1u << L::T) - 1u;
+            if constexpr (L::tail_joins) w[k - 1] |= v << 16;
+            else w[k++] = v;
+        }
+    }
+};
+
 }  // namespace nq
