@@ -194,11 +194,13 @@ __device__ __forceinline__ void tc_mma_kblock2(uint32_t tmem_d0, uint32_t tmem_d
         "}"
         ::"r"(tmem_d0), "r"(tmem_d1), "r"(tmem_a), "r"(b_lo0), "r"(b_lo1), "r"(b_hi), "r"(idesc0), "r"(idesc1), "r"(first) : "memory");
 }
-// 16 lanes x 256 bits of tensor memory from a warp: lane (g, t4) supplies lane g columns 2 t4, 2 t4 + 1 (r0, r1) and
-// lane g + 8, same columns (r2, r3) - the layout of an m16n8 fragment
-__device__ __forceinline__ void tmem_st_16x256b(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3)
+// 16 lanes x 4 x 256 bits of tensor memory from a warp, for columns 8 i .. 8 i + 7: lane (g, t4) supplies lane g columns
+// 2 t4, 2 t4 + 1 (r[4 i], r[4 i + 1]) and lane g + 8, same columns (r[4 i + 2], r[4 i + 3]) - the layout of m16n8 fragments
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t* r)
 {
-    asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                   "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // shared-memory operand descriptor: start address, leading / stride byte offsets (all >> 4), descriptor version 1,
@@ -240,33 +242,31 @@ __device__ __forceinline__ int b_stage_boxes(int nbox) { return nbox <= 2 ? 2 : 
 __device__ __forceinline__ int b_stages(int nbox) { return nbox <= 2 ? 8 : nbox <= 4 ? 5 : nbox <= 5 ? 4 : 3; }
 
 // A unit is decoded whole (8 k-steps) by one warp: k-steps 0..3 fill the weight tile of k-block 2 c, k-steps 4..7 the
-// tile of k-block 2 c + 1.  The sink does the stage hand-over in between: wait until the MMAs that last read the
-// stage are done, store the fragments, wait for the stores, signal "full".
+// tile of k-block 2 c + 1.  The sink keeps the fragments of four k-steps in registers and hands them over as one: wait until
+// the MMAs that last read the stage are done, one 32-column store, wait for the store, signal "full".  The four k-steps are
+// one straight run of arithmetic with nothing to wait for in it (a store and a branch after every k-step cut the unit into
+// ten pieces that were scheduled one by one).
 struct UnitSink
 {
     uint32_t tmem_a;      // tensor-memory address of the warp's 16 lanes in weight-tile stage 0
-    PfShared* sh; uint32_t it0; int lane; bool* ok;
+    PfShared* sh; uint32_t it0; int lane; bool* ok; uint32_t* frag;      // frag: 16 registers
     template <int T>
     __device__ __forceinline__ void operator()(std::integral_constant<int, T>, const uint32_t (&a)[4]) const
     {
-        const uint32_t it = it0 + (T >> 2), sa = it % kPfAStages;
-        if constexpr ((T & 3) == 0)
+        // a[0], a[2]: row g, k = 2 t4 + {0,1} and 8 + 2 t4 + {0,1}; a[1], a[3]: row g + 8
+        constexpr int o = 4 * (T & 3);
+        frag[o] = a[0]; frag[o + 1] = a[2]; frag[o + 2] = a[1]; frag[o + 3] = a[3];
+        if constexpr ((T & 3) == 3)
         {
-            if (*ok && !mbar_wait(&sh->empty_a[sa], ((it / kPfAStages) & 1u) ^ 1u, &sh->abort_flag)) *ok = false;
-            *ok = __shfl_sync(0xffffffffu, (int)*ok, 0) != 0;
+            const uint32_t it = it0 + (T >> 2), sa = it % kPfAStages;
+            if (*ok) *ok = mbar_wait_warp(&sh->empty_a[sa], ((it / kPfAStages) & 1u) ^ 1u, &sh->abort_flag);
             tc_fence_after();
-        }
-        if (*ok)      // warp-uniform
-        {
-            // a[0], a[2]: row g, k = 2 t4 + {0,1} and 8 + 2 t4 + {0,1}; a[1], a[3]: row g + 8
-            tmem_st_16x256b(tmem_a + sa * kPfACols + (T & 3) * 8, a[0], a[2], a[1], a[3]);
-            if constexpr ((T & 3) == 3)
-            {
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh->full_a[sa]);
-            }
+            // an aborted launch stores too (the columns are this CTA's until the end, the results are discarded) but signals nothing
+            tmem_st_16x256b_x4(tmem_a + sa * kPfACols, frag);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (*ok && lane == 0) mbar_arrive(&sh->full_a[sa]);
         }
     }
 };
@@ -321,7 +321,8 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         const uint32_t sign2 = sign_mask(__shfl_sync(0xffffffffu, var_b, i), lane);
         uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
         RecordCursor<BK>::read(wb, st, lane);
-        const UnitSink sink{tmem_a, sh, it_base + 2 * (uint32_t)ch, lane, &ok};
+        uint32_t frag[16];
+        const UnitSink sink{tmem_a, sh, it_base + 2 * (uint32_t)ch, lane, &ok, frag};
         bool refined = false;
         if constexpr (REFINED) refined = chunk_refined(sr, ch);
         if (refined)
