@@ -24,6 +24,7 @@
 #include <cuda.h>
 
 #include "nq_common.cuh"
+#include "nq_scan.cuh"
 #include "nq_unit.cuh"
 
 namespace nq {
@@ -499,46 +500,56 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
 }
 
 // ---------------------------------------------------------------- pass plan (device side, no host sync)
-// counts[e] = routed pairs of expert e (pairs are sorted by expert).  A pass = one expert x up to 384 of its pairs;
-// experts at level 0 get none.  plan: [0] passes, [1] pairs covered, then PfPass records from int 4 on.
-__global__ void pf_plan_kernel(const int* __restrict__ counts, const int64_t* __restrict__ table, int E, int* plan, int max_passes)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    PfPass* out = (PfPass*)(plan + 4);
-    int n = 0, row = 0, covered = 0;
-    for (int e = 0; e < E; ++e)
-    {
-        const int c = counts[e];
-        if (c > 0 && table[(int64_t)e * kTableWidth] > 0)
-            for (int t0 = 0; t0 < c && n < max_passes; t0 += kPfTokens)
-            {
-                out[n].expert = e; out[n].row0 = row + t0; out[n].ntok = c - t0 < kPfTokens ? c - t0 : kPfTokens; out[n].pad = 0;
-                covered += out[n].ntok; ++n;
-            }
-        row += c;
-    }
-    plan[0] = n; plan[1] = covered; plan[2] = plan[3] = 0;
-}
+// A pass = one expert x up to 384 of its pairs (pairs are sorted by expert); experts at level 0 get none.  plan: [0] passes,
+// [1] pairs covered, then PfPass records from int 4 on, in expert order.
+//   WINDOW = false  from[e] = routed pairs of expert e, in the order of the pair list; the plan covers the whole list
+//   WINDOW = true   from[e] = first pair of expert e in the sorted list (from[E] = end of the last expert's pairs); the plan covers
+//                   the pairs [pair0, pair0 + npairs) with rows counted from pair0
+// One CTA, a thread per expert: sums over the CTA (passes before the expert, pairs before it) place every record.  One thread
+// that walks the experts alone pays two dependent loads for each of them.
+constexpr int kPlanThreads = 1024;
 
-// The same from the sorted pair list of a whole window: start[e] = first pair of expert e (start[E] = end of the last
-// expert's pairs); the plan covers the pairs [pair0, pair0 + npairs) with rows counted from pair0.
-__global__ void pf_plan_window_kernel(const int* __restrict__ start, const int64_t* __restrict__ table, int E, int pair0, int npairs,
-                                      int* plan, int max_passes)
+template <bool WINDOW>
+__global__ void __launch_bounds__(kPlanThreads) pf_plan_kernel(const int* __restrict__ from, const int64_t* __restrict__ table, int E,
+                                                               int pair0, int npairs, int* plan, int max_passes)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ int s_warp[kPlanThreads / 32];
     PfPass* out = (PfPass*)(plan + 4);
-    int n = 0, covered = 0;
-    for (int e = 0; e < E; ++e)
+    int n = 0, rows = 0, covered = 0;     // passes, pairs and covered pairs of the experts handled so far
+    for (int e0 = 0; e0 < E; e0 += kPlanThreads)
     {
-        const int a = max(start[e], pair0), b = min(start[e + 1], pair0 + npairs), c = b - a;
-        if (c > 0 && table[(int64_t)e * kTableWidth] > 0)
-            for (int t0 = 0; t0 < c && n < max_passes; t0 += kPfTokens)
+        const int e = e0 + (int)threadIdx.x;
+        int first = 0, c = 0, total;
+        bool live = false;
+        if (e < E)
+        {
+            live = table[(int64_t)e * kTableWidth] > 0;
+            if constexpr (WINDOW)
             {
-                out[n].expert = e; out[n].row0 = a - pair0 + t0; out[n].ntok = c - t0 < kPfTokens ? c - t0 : kPfTokens; out[n].pad = 0;
-                covered += out[n].ntok; ++n;
+                const int a = max(from[e], pair0), b = min(from[e + 1], pair0 + npairs);
+                first = a - pair0; c = b - a;
             }
+            else c = from[e];
+        }
+        if constexpr (!WINDOW)
+        {
+            first = rows + cta_exclusive_sum(c, s_warp, total);
+            rows += total;
+        }
+        const int np = live && c > 0 ? (c + kPfTokens - 1) / kPfTokens : 0;
+        const int at = n + cta_exclusive_sum(np, s_warp, total);
+        const int kept = max(min(np, max_passes - at), 0);
+        for (int i = 0; i < kept; ++i)
+        {
+            PfPass ps;
+            ps.expert = e; ps.row0 = first + i * kPfTokens; ps.ntok = min(c - i * kPfTokens, kPfTokens); ps.pad = 0;
+            out[at + i] = ps;
+        }
+        n = min(n + total, max_passes);
+        cta_exclusive_sum(kept > 0 ? min(c, kept * kPfTokens) : 0, s_warp, total);
+        covered += total;
     }
-    plan[0] = n; plan[1] = covered; plan[2] = plan[3] = 0;
+    if (threadIdx.x == 0) { plan[0] = n; plan[1] = covered; plan[2] = plan[3] = 0; }
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -576,7 +587,7 @@ int nq_pf_plan(const int32_t* counts, const int64_t* table, int E, int pairs, in
 {
     NQ_REQUIRE(counts && table && plan && E > 0 && pairs >= 0, "nq_pf_plan: bad arguments");
     NQ_REQUIRE(plan_ints >= nq_pf_plan_ints(E, pairs), "nq_pf_plan: plan needs %d ints", nq_pf_plan_ints(E, pairs));
-    nq::pf_plan_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(counts, table, E, plan, (plan_ints - 4) / 4);
+    nq::pf_plan_kernel<false><<<1, nq::kPlanThreads, 0, (cudaStream_t)stream>>>(counts, table, E, 0, 0, plan, (plan_ints - 4) / 4);
     return nq::check_launch("nq_pf_plan");
 }
 
@@ -584,7 +595,7 @@ int nq_pf_plan_window(const int32_t* start, const int64_t* table, int E, int pai
 {
     NQ_REQUIRE(start && table && plan && E > 0 && pair0 >= 0 && npairs >= 0, "nq_pf_plan_window: bad arguments");
     NQ_REQUIRE(plan_ints >= nq_pf_plan_ints(E, npairs), "nq_pf_plan_window: plan needs %d ints", nq_pf_plan_ints(E, npairs));
-    nq::pf_plan_window_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(start, table, E, pair0, npairs, plan, (plan_ints - 4) / 4);
+    nq::pf_plan_kernel<true><<<1, nq::kPlanThreads, 0, (cudaStream_t)stream>>>(start, table, E, pair0, npairs, plan, (plan_ints - 4) / 4);
     return nq::check_launch("nq_pf_plan_window");
 }
 

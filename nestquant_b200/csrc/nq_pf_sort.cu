@@ -1,15 +1,18 @@
-// Prefill path, the permutation: the (token, pick) pairs of a window sorted by expert, as a stable counting sort in three
-// small kernels and without a host sync.
+// Prefill path, the permutation: the (token, pick) pairs of a window sorted by expert, as a stable counting sort in one kernel
+// (up to 8,192 picks) or three, and without a host sync.
 //
 // Replaces the host side of the reference's prefill (sm120/moe.py:293-298: torch.argsort of the flattened expert ids,
 // scatter_add for the counts, a .cpu() of the counts) and this library's earlier use of the same torch operators.
 //   bins     expert id 0 .. E - 1, plus bin E for the picks that contribute nothing (id outside [0, E), expert not resident
 //            on this GPU, routing weight 0): they sort behind every real pair and no kernel touches their rows.
-//   slices   a warp owns 256 consecutive picks.  Pass 1 counts its picks per bin; pass 2 (one CTA) turns the counts into the
-//            offset of every (slice, bin) and the start of every bin; pass 3 walks the slice again, 32 picks at a time in pick
+//   slices   a warp owns up to 256 consecutive picks.  Pass 1 counts its picks per bin; pass 2 turns the counts into the
+//            offset of every (slice, bin) and the size of every bin; pass 3 walks the slice again, 32 picks at a time in pick
 //            order, and places each pick at start[bin] + offset[slice][bin] + its rank among the slice's earlier picks of that
 //            bin (match.any gives the lanes of a step that share a bin).  Equal experts keep pick order: the result does
-//            not depend on timing.
+//            not depend on timing, nor on where the slices are cut.
+// Everything here is latency (65,536 picks are 0.7 MB), so every pass loads independently: with pass 2 as one CTA whose threads
+// walked the slices, and a pass list written by one thread, sort and pass list of the full layer (256 experts) took 80 us
+// longer at 8,000 picks and 130 us longer at 65,536 (whole prefill call, same GPU).
 // Outputs: pe[p] = expert (or E) and pt[p] = token of sorted pair p, pos[t * topk + k] = sorted index of a pick,
 // start[0 .. E + 1] = first pair of each bin (start[E] = number of live pairs, start[E + 1] = all pairs), and, optionally,
 // the routing-hit counts of this call (every pick with a valid id and a non-zero weight, whatever the expert's level) added
@@ -18,12 +21,14 @@
 
 #include "nq_common.cuh"
 #include "nq_format.cuh"
+#include "nq_scan.cuh"
 
 namespace nq {
 
 constexpr int kSortSlice = 256;      // picks per warp
 constexpr int kSortWarps = 8;        // warps per CTA
 constexpr int kSortMaxBins = 1025;   // experts + 1
+constexpr size_t kSortSmallShared = 48 * 1024 - 256;      // the one-kernel form stays within the default shared memory of a CTA
 
 __device__ __forceinline__ int pick_bin(const int64_t* __restrict__ sel, const __half* __restrict__ rw, const int64_t* __restrict__ table,
                                         int E, int i, bool* hit)
@@ -56,59 +61,133 @@ __global__ void __launch_bounds__(32 * kSortWarps) sort_count_kernel(const int64
         for (int b = lane; b < nb; b += 32) hist[(size_t)slice * nb + b] = h[b];
 }
 
-// pass 2 (one CTA): hist[slice][bin] -> offset of the slice inside the bin; start[bin] = first pair of the bin
-__global__ void __launch_bounds__(1024) sort_scan_kernel(int* hist, int nslices, int E, int* start)
+// pass 2: hist[slice][bin] -> picks of the bin in earlier slices; the row of slice 0, whose offsets are zero, takes the size of
+// the bin instead.  A CTA takes 32 bins (a lane each), its 32 warps equal runs of slices: every load is independent.
+__global__ void __launch_bounds__(1024) sort_offset_kernel(int* hist, int nslices, int E)
 {
-    __shared__ int s_total[kSortMaxBins + 1];
-    const int nb = E + 1;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    {
-        int run = 0;
-        for (int s = 0; s < nslices; ++s)
-        {
-            const int c = hist[(size_t)s * nb + b];
-            hist[(size_t)s * nb + b] = run;
-            run += c;
-        }
-        s_total[b] = run;
-    }
+    __shared__ int s_sum[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = E + 1, b = blockIdx.x * 32 + lane;
+    const int per = (nslices + 31) / 32, s0 = warp * per, s1 = min(s0 + per, nslices);
+    int sum = 0;
+    if (b < nb)
+#pragma unroll 8
+        for (int s = s0; s < s1; ++s) sum += __ldcg(hist + (size_t)s * nb + b);
+    s_sum[warp][lane] = sum;
     __syncthreads();
-    if (threadIdx.x == 0)
+    int run = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < 32; ++w)
     {
-        int run = 0;
-        for (int b = 0; b < nb; ++b) { start[b] = run; run += s_total[b]; }
-        start[nb] = run;
+        const int v = s_sum[w][lane];
+        run += w < warp ? v : 0;
+        total += v;
+    }
+    if (b >= nb) return;
+    for (int s = s0; s < s1; ++s)
+    {
+        const int c = hist[(size_t)s * nb + b];
+        hist[(size_t)s * nb + b] = s ? run : total;
+        run += c;
     }
 }
 
-// pass 3: place every pick
+// size[b] -> s_start[b] = picks of earlier bins, s_start[nb] = all picks; whole CTA.  size and s_start may be the same array.
+__device__ __forceinline__ void scan_bins(const int* size, int nb, int* s_start, int* s_warp)
+{
+    const int per = (nb + (int)blockDim.x - 1) / (int)blockDim.x, b0 = (int)threadIdx.x * per, b1 = min(b0 + per, nb);
+    int sum = 0, total;
+    for (int b = b0; b < b1; ++b) sum += size[b];
+    int run = cta_exclusive_sum(sum, s_warp, total);
+    for (int b = b0; b < b1; ++b) { const int c = size[b]; s_start[b] = run; run += c; }
+    if (threadIdx.x == 0) s_start[nb] = total;
+    __syncthreads();
+}
+
+// 32 picks of a warp (pick i of bin b per lane; lanes without one: b < 0 and different from every other lane's) take their
+// places: nx[bin] = next free place of the bin for this warp
+__device__ __forceinline__ void place_picks(int* nx, int b, int i, int topk, int lane, int* pe, int* pt, int* pos)
+{
+    const unsigned same = __match_any_sync(0xffffffffu, b);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    int p = 0;
+    if (b >= 0) p = nx[b] + rank;
+    __syncwarp();
+    if (b >= 0 && rank == __popc(same) - 1) nx[b] = p + 1;                     // the last lane of each bin moves the bin on
+    __syncwarp();
+    if (b >= 0) { pe[p] = b; pt[p] = i / topk; pos[i] = p; }
+}
+
+// pass 3: place every pick.  Every CTA adds up the bin sizes itself (row 0 of hist); CTA 0 writes them out as start.
 __global__ void __launch_bounds__(32 * kSortWarps) sort_place_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
                                                                     const int64_t* __restrict__ table, int P, int E, int topk,
-                                                                    const int* __restrict__ hist, const int* __restrict__ start,
-                                                                    int* pe, int* pt, int* pos)
+                                                                    const int* __restrict__ hist, int* start, int* pe, int* pt, int* pos)
 {
     extern __shared__ int s_next[];      // [kSortWarps][E + 1]: next free place of each bin for this slice
+    __shared__ int s_start[kSortMaxBins + 1], s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slice = blockIdx.x * kSortWarps + warp, nb = E + 1;
+    scan_bins(hist, nb, s_start, s_warp);
+    if (blockIdx.x == 0)
+        for (int b = threadIdx.x; b <= nb; b += blockDim.x) start[b] = s_start[b];
     int* nx = s_next + warp * nb;
     const int i0 = slice * kSortSlice;
     if (i0 >= P) return;                 // warp-uniform
-    for (int b = lane; b < nb; b += 32) nx[b] = start[b] + hist[(size_t)slice * nb + b];
+    for (int b = lane; b < nb; b += 32) nx[b] = s_start[b] + (slice ? hist[(size_t)slice * nb + b] : 0);
     __syncwarp();
     for (int base = i0; base < i0 + kSortSlice && base < P; base += 32)
     {
         const int i = base + lane;
-        const bool in = i < P;
         bool hit;
-        const int b = in ? pick_bin(sel, rw, table, E, i, &hit) : -1 - lane;      // idle lanes get bins of their own
-        const unsigned same = __match_any_sync(0xffffffffu, b);
-        const int rank = __popc(same & ((1u << lane) - 1u));
-        int p = 0;
-        if (in) p = nx[b] + rank;
-        __syncwarp();
-        if (in && rank == __popc(same) - 1) nx[b] = p + 1;                         // the last lane of each bin moves the bin on
-        __syncwarp();
-        if (in) { pe[p] = b; pt[p] = i / topk; pos[i] = p; }
+        place_picks(nx, i < P ? pick_bin(sel, rw, table, E, i, &hit) : -1 - lane, i, topk, lane, pe, pt, pos);
     }
+}
+
+// The three passes in one CTA of 32 warps, the counts in shared memory: up to 32 slices (8,192 picks).  A slice is a multiple of
+// 32 picks, no longer than needed, and a lane keeps its picks' bins in registers between the passes.
+constexpr int kSortSmallPicks = 32 * kSortSlice;
+__global__ void __launch_bounds__(1024) sort_small_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
+                                                          const int64_t* __restrict__ table, int P, int E, int topk, int* start, int* hits,
+                                                          int* pe, int* pt, int* pos)
+{
+    extern __shared__ int s_hist[];      // [32][E + 1] counts, then next free places; [E + 2] bin sizes, then starts
+    __shared__ int s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = E + 1;
+    const int slice = (P + 1023) / 1024 * 32, i0 = warp * slice;
+    int* h = s_hist + warp * nb;
+    int* s_start = s_hist + 32 * nb;
+    int bin[kSortSlice / 32];
+    for (int b = lane; b < nb; b += 32) h[b] = 0;
+#pragma unroll
+    for (int j = 0; j < kSortSlice / 32; ++j)
+    {
+        const int i = i0 + 32 * j + lane;
+        bin[j] = -1 - lane;
+        if (32 * j < slice && i < P)
+        {
+            bool hit;
+            bin[j] = pick_bin(sel, rw, table, E, i, &hit);
+            if (hits && hit) atomicAdd(hits + (int)sel[i], 1);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kSortSlice / 32; ++j)
+        if (bin[j] >= 0) atomicAdd(h + bin[j], 1);
+    __syncthreads();
+    for (int b = threadIdx.x; b < nb; b += blockDim.x)
+    {
+        int run = 0;
+#pragma unroll 8
+        for (int w = 0; w < 32; ++w) { const int c = s_hist[w * nb + b]; s_hist[w * nb + b] = run; run += c; }
+        s_start[b] = run;
+    }
+    __syncthreads();
+    scan_bins(s_start, nb, s_start, s_warp);
+    for (int b = threadIdx.x; b <= nb; b += blockDim.x) start[b] = s_start[b];
+    for (int b = lane; b < nb; b += 32) h[b] += s_start[b];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kSortSlice / 32; ++j)
+        if (32 * j < slice) place_picks(h, bin[j], i0 + 32 * j + lane, topk, lane, pe, pt, pos);
 }
 
 }  // namespace nq
@@ -134,12 +213,18 @@ int nq_pf_sort(const int64_t* sel, const void* rw, const int64_t* table, int T, 
     if (P == 0) return cudaMemsetAsync(start, 0, sizeof(int32_t) * (E + 2), st) == cudaSuccess ? NQ_OK : nq::fail(NQ_ERR_CUDA, "nq_pf_sort: memset failed");
     NQ_REQUIRE(sel && rw && table && pe && pt && pos && scratch, "nq_pf_sort: null pointer");
     NQ_REQUIRE(scratch_ints >= nq_pf_sort_scratch_ints(P, E), "nq_pf_sort: scratch needs %d ints", nq_pf_sort_scratch_ints(P, E));
+    const size_t small = sizeof(int) * (33 * (size_t)(E + 1) + 1);
+    if (P <= nq::kSortSmallPicks && small <= nq::kSortSmallShared)
+    {
+        nq::sort_small_kernel<<<1, 1024, small, st>>>(sel, (const __half*)rw, table, P, E, topk, start, hits, pe, pt, pos);
+        return nq::check_launch("nq_pf_sort");
+    }
     const int slices = (P + nq::kSortSlice - 1) / nq::kSortSlice, ctas = (slices + nq::kSortWarps - 1) / nq::kSortWarps;
     const size_t smem = sizeof(int) * nq::kSortWarps * (E + 1);
     nq::sort_count_kernel<<<ctas, 32 * nq::kSortWarps, smem, st>>>(sel, (const __half*)rw, table, P, E, scratch, hits);
     if (int e = nq::check_launch("nq_pf_sort(count)")) return e;
-    nq::sort_scan_kernel<<<1, 1024, 0, st>>>(scratch, slices, E, start);
-    if (int e = nq::check_launch("nq_pf_sort(scan)")) return e;
+    nq::sort_offset_kernel<<<(E + 1 + 31) / 32, 1024, 0, st>>>(scratch, slices, E);
+    if (int e = nq::check_launch("nq_pf_sort(offset)")) return e;
     nq::sort_place_kernel<<<ctas, 32 * nq::kSortWarps, smem, st>>>(sel, (const __half*)rw, table, P, E, topk, scratch, start, pe, pt, pos);
     return nq::check_launch("nq_pf_sort(place)");
 }

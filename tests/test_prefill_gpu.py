@@ -211,3 +211,56 @@ def test_pair_sort_is_a_stable_counting_sort():
     want_start[1:] = torch.cumsum(torch.bincount(key, minlength=NE + 1), 0)
     assert torch.equal(start.cpu().long(), want_start)
     assert torch.equal(hits.cpu().long(), torch.bincount(flat[valid], minlength=NE))
+
+
+@pytest.mark.parametrize("NE,topk,T", [(1, 1, 1), (5, 3, 11), (37, 1, 1024), (256, 8, 1023), (256, 8, 1024), (256, 8, 1025), (370, 7, 1170),
+                                       (371, 7, 1170), (1024, 4, 333), (1024, 8, 4500)])
+def test_pair_sort_and_plan_over_their_range(NE, topk, T):
+    """one-kernel sort (up to 8,192 picks and 371 bins) and three-kernel sort, and the pass lists from either form of the counts:
+    sizes around the lines between them, one slice and many, one expert and as many as a CTA has threads"""
+    from nestquant_b200 import ext
+    g = torch.Generator().manual_seed(NE + T)
+    table = torch.zeros(NE, 20, dtype=torch.int64)
+    table[:, 0] = torch.tensor([0, 2, 4, 4])[torch.randint(0, 4, (NE,), generator=g)]
+    table[0, 0] = 2
+    sel = (torch.rand(T, topk, generator=g) ** 3 * (NE + 1)).long() - (torch.rand(T, topk, generator=g) < 0.05).long()
+    rw = torch.rand(T, topk, generator=g).half()
+    rw[torch.rand(T, topk, generator=g) < 0.05] = 0
+    P = T * topk
+    mk = lambda n: torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    pe, pt, pos, start, dt = mk(P), mk(P), mk(P), mk(NE + 2), table.cuda()
+    hits = torch.zeros(NE, dtype=torch.int32, device="cuda")
+    ext.pf_sort(sel.cuda(), rw.cuda(), dt, pe, pt, pos, start, hits, mk(max(1, ext.pf_sort_scratch_ints(P, NE))))
+    flat, rwf = sel.reshape(-1), rw.reshape(-1)
+    valid = (flat >= 0) & (flat < NE) & (rwf != 0)
+    key = torch.where(valid & (table[flat.clamp(0, NE - 1), 0] > 0), flat, NE)
+    order = torch.argsort(key, stable=True)
+    assert torch.equal(pe.cpu().long(), key[order]) and torch.equal(pt.cpu().long(), order // topk)
+    inv = torch.empty(P, dtype=torch.long)
+    inv[order] = torch.arange(P)
+    assert torch.equal(pos.cpu().long(), inv)
+    want = torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum(torch.bincount(key, minlength=NE + 1), 0)])
+    assert torch.equal(start.cpu().long(), want)
+    assert torch.equal(hits.cpu().long(), torch.bincount(flat[valid], minlength=NE))
+
+    def passes(first, last, row0):      # pairs [first[e], last[e]) of expert e, rows counted from row0
+        return [(e, a - row0 + i, min(384, b - a - i)) for e, (a, b) in enumerate(zip(first, last)) if b > a and table[e, 0] > 0
+                for i in range(0, b - a, 384)]
+
+    def check(plan, expect):
+        p = plan.cpu().numpy()
+        assert list(p[:4]) == [len(expect), sum(n for _, _, n in expect), 0, 0]
+        rec = p[4:4 + 4 * len(expect)].reshape(-1, 4)
+        assert np.array_equal(rec, np.array([(e, r, n, 0) for e, r, n in expect], dtype=np.int32).reshape(-1, 4))
+
+    for pair0, n in ((0, P), (P // 3, max(1, P // 2))):
+        n = min(n, P - pair0)
+        plan = mk(ext.pf_plan_ints(NE, n))
+        ext.pf_plan_window(start, dt, plan, pair0, n)
+        lo, hi = [[min(max(int(v), pair0), pair0 + n) for v in w] for w in (want[:NE], want[1:NE + 1])]
+        check(plan, passes(lo, hi, pair0))
+    cnt = torch.bincount(flat[valid], minlength=NE)                   # experts that are not resident have pairs here
+    edge = [0] + torch.cumsum(cnt, 0).tolist()
+    plan = mk(ext.pf_plan_ints(NE, edge[-1]))
+    ext.pf_plan(cnt.int().cuda(), dt, plan, edge[-1])
+    check(plan, passes(edge[:-1], edge[1:], 0))
