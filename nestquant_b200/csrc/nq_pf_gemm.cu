@@ -9,7 +9,7 @@
 //   warps 2..17   decode: a warp streams every other chunk of one strip with cp.async, decodes each unit in registers
 //                 (bit-exact fp16) and stores it with tcgen05.st as two weight tiles [128 x 64] in TENSOR MEMORY
 //                 (k-blocks 2 c and 2 c + 1): the m16n8k16-style fragment a lane holds is exactly what the 16x256b
-//                 store shape takes, so a tile costs 4 stores per warp and no shared memory at all
+//                 store shape takes, so a tile costs one store per warp and no shared memory at all
 //   warp 1        one elected lane issues tcgen05.mma with the A operand in tensor memory (M 128 = weight rows, N =
 //                 tokens, K 16) into a [128 x 384] fp32 accumulator, also in tensor memory; tcgen05.commit frees the
 //                 stages.  Token tiles run 3..8 k-blocks ahead (160 KB), weight tiles 4 stages (32 columns each)

@@ -1,12 +1,12 @@
-// Asynchronous stream of packed planes into shared memory, shared by the decode-path GEMV, the prefill GEMM and the dense
-// decode kernel.
+// Streams of packed planes: into shared memory (RecordCursor: prefill GEMM, dense decode kernel) and straight into registers
+// (RecordReader: decode-path GEMV).
 //
 // Plane layout (sm120/moe.py:36-49): a record of BITS bits is cut into pieces - BITS / 128 pieces of 128 bits, then a
 // 64-, a 32- and a 16-bit piece as the binary digits of BITS % 128 say, then a tail of BITS % 16 bits - and every piece
 // kind is stored as its own array over all records of the plane (the tail bit-packed, followed by a 4-byte pad).  The
 // base plane of window code 0 is the special case of one 128-bit piece.
 //
-// Each lane copies the pieces of its own record with cp.async (global -> shared, no registers) a few units ahead and
+// RecordCursor: each lane copies the pieces of its own record with cp.async (global -> shared, no registers) a few units ahead and
 // later reads back only what it copied itself, so the ring needs no barrier at all.  Per warp and stage: 512 B for the
 // base records of a unit followed by 768 B for its residual records, one lane-indexed array per piece kind.
 // 32 records make a unit, so every piece array advances by a fixed number of bytes per unit and a lane's position
