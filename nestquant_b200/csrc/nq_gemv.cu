@@ -1282,6 +1282,9 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
             {
                 if (rest) cut_job(a, sh, R, L, job, l, job.stop, 0, lane);
                 else cut_share(a, sh, R, L, job, l, k, lane);
+                // a further share of list 0 may take all the room: the rows of list 1 that stood behind those of the first share are
+                // gone, list 1 prepares its own when it gets there
+                if (l == 0 && lane == 0) { R.job[1].staged = 0; R.job[1].rows_at = 0; }
             }
             __syncthreads();
         }
