@@ -6,9 +6,10 @@
 //
 //   route      every CTA groups the picks into runs (one expert + the tokens that picked it, level 4 first) in its own
 //              shared memory: no CTA waits for another one's routing.
-//   lists      the 16 x 128 units of the runs, in storage order, form up to four lists that every CTA goes through in order:
-//              gate|up of the first half of the runs, gate|up of the rest, down of the first half, down of the rest.  When a CTA
-//              gets to a down list the h it needs was finished while it worked on the list in between.
+//   lists      the 16 x 128 units of the runs, in storage order, form two lists, gate|up and down, that every CTA goes through in
+//              this order.  (Two lists per phase, each of half of the runs, would hide the hand-over of h, but their rows,
+//              barriers and cuts cost more than that: 1 token of the full layer 132 us against 117, 4 tokens 379 against 369,
+//              7 tokens over 90 experts at H = 2048, I = 640 101 against 75.)
 //   shares     a list is cut by cost into one share per CTA, at piece boundaries (a piece = 16-row strip x k-slice), and a share
 //              into one range per warp, at unit boundaries.  The cut points follow from the run list, so a CTA computes its
 //              own: no queue, and a warp walks a contiguous range of each plane.  (A share whose token rows do not fit into
@@ -76,7 +77,7 @@ struct MoeArgs
     float* part_d;     // [ks_dn][S][H]
     int* cnt_gu;       // [S * I/128] (run, group) arrivals, [S * I/128] (run, 512-block) arrivals, [S] finished groups per run
     int* cnt_d;        // [B][H/128] (token, group) arrivals
-    int* wq;           // [0], [2] shares drawn so far of lists 0 | 1 << 16 and 2 | 3 << 16, [1] CTAs that left ([3] unused)
+    int* wq;           // [0], [2] shares drawn so far of gate|up and down, [1] CTAs that left ([3] unused)
     float* zd;         // [S][I/128][4] down low-rank partials
     float* out;        // [B][H]
     int* hits;         // optional [E] pick counters (may be host-mapped)
@@ -153,21 +154,20 @@ __device__ __forceinline__ bool wait_counter(const int* p, int target, int* stat
 // Relative cost of a unit, by which the lists are cut: measured clocks of the unit loop, 410 at level 2 and 690 at level 4, and 64
 // (8 legacy MMAs) for a further column tile.
 constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f;
-constexpr int kUndecided = -1, kDeciding = -2, kLists = 4, kCachedRows = 2;
+constexpr int kUndecided = -1, kDeciding = -2, kLists = 2, kCachedRows = 2;
 // The units [at, stop) of list positions that this CTA is working on, and the token rows it needs for them.
 struct Job
 {
     int share, next;                 // share in work; the one to follow (kUndecided until the first warp is done)
     int at, stop, end;               // this job; the end of the share
-    int seq;                         // number of the job (of any list), never 0
-    int staged;                      // the rows are in place already
-    int run0, row0, nrows, rows_at;  // first run, its first row's number, rows, byte offset behind the slots
+    int seq;                         // number of the job (of either list), not 0 once it is cut
+    int run0, row0, nrows;           // first run, its first row's number, rows
     int bound[kWarps + 1];           // the warps' ranges
     int64_t row[kCachedRows][kTableWidth];   // table rows of run0 and the runs behind it
 };
 struct Shape
 {
-    int S, ng, ngH, KSg, KSd, nruns, split;      // split: runs of the first of the two lists of a phase
+    int S, ng, ngH, KSg, KSd, nruns;
     int nu_gu, nu_dn;                // units per run of the two projections (0: that half is not wanted)
 };
 // What a warp does with (part of) a piece: read by the decoder functions.
@@ -180,7 +180,7 @@ struct StripJob
     int c0, n;                       // first chunk, units
     uint32_t x;                      // shared-space address of the run's first token row
     int row_bytes, count;            // bytes from row to row, tokens of the run
-    // what becomes of the sums: list, run, strip, k-slice, units of the piece behind the warp's range, whether it begins in it
+    // what becomes of the sums: list (0 gate|up, 1 down), run, strip, k-slice, units of the piece behind the warp's range, whether it begins in it
     int l, r, strip, ks, left, starts;
 };
 // The state of a CTA, at the start of its shared memory.  (Reached through route(): the functions that are not inlined get
@@ -202,19 +202,19 @@ struct Route
     float cost[2][NQ_MAX_PICKS];          // cost of one unit of a run (gate|up, down)
     float base[2][NQ_MAX_PICKS + 1];      // cost of the units before a run
     int ks[2];                            // k-slices per strip in use
-    int draws[2];                         // this CTA's first shares of the lists, packed as in wq
+    int draws[kLists];                    // this CTA's first shares of the lists
     __align__(16) float zg[NQ_MAX_PICKS][4];   // low-rank inputs x V_gu^T of the picks of this CTA's gate|up shares
-    int slot_seq[2][kWarps];              // job whose share of a piece is in the warp's slot (lists 0, 2 and 1, 3)
+    int slot_seq[kWarps];                 // job whose share of a piece is in the warp's slot
     Job job[kLists];
 };
 constexpr int kRouteBytes = (sizeof(Route) + 127) / 128 * 128;
-extern __shared__ __align__(128) uint8_t nq_gemv_smem[];      // Route, [3][kWarps][slot_floats], token rows
+extern __shared__ __align__(128) uint8_t nq_gemv_smem[];      // Route, [2][kWarps][slot_floats], token rows
 __device__ __forceinline__ Route& route() { return *(Route*)nq_gemv_smem; }
-// slots of a warp: 0, 1 its share of a piece that an earlier warp adds up (lists 0, 2 and 1, 3), 2 the sums of its current
+// slots of a warp: 0 its share of a piece that an earlier warp adds up (read before the next job starts), 1 the sums of its current
 // piece; fragment order [tile][i][lane]
 __device__ __forceinline__ float* slot_of(const Route& R, int which, int warp) { return (float*)(nq_gemv_smem + kRouteBytes) + (which * kWarps + warp) * R.a.slot_floats; }
-__device__ __forceinline__ uint32_t rows_base(const Route& R) { return smem_addr(nq_gemv_smem) + kRouteBytes + 3 * kWarps * R.a.slot_floats * 4; }
-__host__ __device__ constexpr int rows_room(int slot_floats) { return kGemvSmem - kRouteBytes - 3 * kWarps * slot_floats * 4; }
+__device__ __forceinline__ uint32_t rows_base(const Route& R) { return smem_addr(nq_gemv_smem) + kRouteBytes + 2 * kWarps * R.a.slot_floats * 4; }
+__host__ __device__ constexpr int rows_room(int slot_floats) { return kGemvSmem - kRouteBytes - 2 * kWarps * slot_floats * 4; }
 
 // quotient of small non-negative integers (a < 2^20) without the ~130 clocks of an integer division
 __device__ __forceinline__ int quot(int a, int b) { return (int)__fdividef((float)a + 0.5f, (float)b); }
@@ -350,7 +350,7 @@ struct TokenSink
     }
 };
 
-// n units of one strip: stream, decode, multiply; the 16 x (8 NT) partial sums go to the warp's slot 2.  MODE 0: level 2, 1: level 4, 2: level 4 in
+// n units of one strip: stream, decode, multiply; the 16 x (8 NT) partial sums go to the warp's slot 1.  MODE 0: level 2, 1: level 4, 2: level 4 in
 // mask mode (chunks without a flag decode as level 2).  The records of the next unit are fetched into registers while the
 // current one is decoded.
 // Not inlined on purpose: each of the decoder variants gets a register allocation of its own, and the caller's state is
@@ -438,7 +438,7 @@ __device__ __noinline__ void strip_gemv()
             off += kRowStep;
         }
     }
-    float* out = slot_of(route(), 2, threadIdx.x >> 5) + lane;
+    float* out = slot_of(route(), 1, threadIdx.x >> 5) + lane;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -454,15 +454,14 @@ __device__ __forceinline__ void store4h_operand(__half* chunk, int lane, const f
     w[16] = *(const uint32_t*)&b;
 }
 
-// A list: units of the runs [run0, run1) of phase d; position p of the list is unit p mod NU of run run0 + p / NU.
-struct List { int d, run0, run1, C, NU, cps, NH; };        // chunks per strip, units per run, chunks per piece, units of a half (gate, up)
-__device__ __forceinline__ List list_of(const MoeArgs& a, const Shape& sh, int l)
+// A list (d = 0 gate|up, 1 down): position p is unit p mod NU of run p / NU.
+struct List { int d, C, NU, cps, NH; };        // chunks per strip, units per run, chunks per piece, units of a half (gate, up)
+__device__ __forceinline__ List list_of(const MoeArgs& a, const Shape& sh, int d)
 {
     List L;
-    L.d = l >> 1;
-    L.run0 = l & 1 ? sh.split : 0; L.run1 = l & 1 ? sh.nruns : sh.split;
-    L.C = (L.d ? a.I : a.H) >> 7; L.NU = L.d ? sh.nu_dn : sh.nu_gu; L.NH = L.d ? L.NU : L.NU >> 1;
-    const int KS = L.d ? sh.KSd : sh.KSg;
+    L.d = d;
+    L.C = (d ? a.I : a.H) >> 7; L.NU = d ? sh.nu_dn : sh.nu_gu; L.NH = d ? L.NU : L.NU >> 1;
+    const int KS = d ? sh.KSd : sh.KSg;
     L.cps = KS == 1 ? L.C : quot(L.C, KS);
     return L;
 }
@@ -477,12 +476,11 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // Rows are numbered run by run: gate|up has the gate rows of a run's picks, then their up rows, down one row per pick.
 __device__ __forceinline__ int row_id(const RunRec& run, int d, int up) { return d ? run.first : 2 * run.first + up * run.count; }
 // The rows of a gate|up job.  A warp task = eight blocks of 128 of one row: lanes 4 v .. 4 v + 3 hold block v (wht128_x8, map H).
-// Returns the number of warp tasks; w0: the warp that takes the first one.
-__device__ __forceinline__ int rotate_rows(const MoeArgs& a, const Shape& sh, const Route& R, const Job& job, uint32_t rows, int w0, int lane, int warp)
+__device__ __forceinline__ void rotate_rows(const MoeArgs& a, const Shape& sh, const Route& R, const Job& job, uint32_t rows, int lane, int warp)
 {
     const int oct = (sh.ngH + 7) >> 3, n = job.nrows * oct, q = lane & 3;
     int run = job.run0;
-    for (int t = warp >= w0 ? warp - w0 : warp + kWarps - w0; t < n; t += kWarps)
+    for (int t = warp; t < n; t += kWarps)
     {
         const int p = quot(t, oct), blk = (t - p * oct) * 8 + (lane >> 2);
         while (job.row0 + p >= 2 * (R.runs[run].first + R.runs[run].count)) ++run;
@@ -513,11 +511,11 @@ __device__ __forceinline__ int rotate_rows(const MoeArgs& a, const Shape& sh, co
                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + 64 * t4 + 16 * j), "r"(*(const uint32_t*)&h) : "memory");
             }
     }
-    return n;
 }
-// low-rank inputs x V_gu^T (unrotated input) of a gate|up job's picks, a warp per pick
-__device__ __forceinline__ void low_rank_inputs(const MoeArgs& a, Route& R, int p0, int p1, int lane, int warp)
+// low-rank inputs x V_gu^T (unrotated input) of the picks of a gate|up job that ends in run `last`, a warp per pick
+__device__ __forceinline__ void low_rank_inputs(const MoeArgs& a, Route& R, const Job& job, int last, int lane, int warp)
 {
+    const int p0 = R.runs[job.run0].first, p1 = R.runs[last].first + R.runs[last].count;
     for (int p = p0 + warp; p < p1; p += kWarps)
     {
         const int s = R.order[p];
@@ -849,16 +847,13 @@ __device__ __forceinline__ int choose_ksplit(int strips, int C, int ks, int ctas
     const unsigned good = __ballot_sync(0xffffffffu, load != 0x7fffffff && load * 32 <= best * 33);
     return good ? __ffs(good) : ks;
 }
-__device__ __forceinline__ Shape make_shape(const MoeArgs& a, int nruns, int ctas)
+__device__ __forceinline__ Shape make_shape(const MoeArgs& a, int nruns)
 {
     Shape sh;
     sh.S = a.B * a.topk; sh.ng = a.I >> 7; sh.ngH = a.H >> 7; sh.nruns = nruns;
     sh.nu_gu = (a.which & 1) ? (a.I >> 3) * sh.ngH : 0;
     sh.nu_dn = (a.which & 2) ? (a.H >> 4) * sh.ng : 0;
     sh.KSg = sh.KSd = 1;             // filled in once the lists are cut
-    // Two lists per phase hide the hand-over of h (the way from the last gate|up piece to the first down unit) but cost rows and
-    // barriers of their own: worth it from about a dozen units per warp on.
-    sh.split = a.which == 3 && nruns > 1 && nruns * (sh.nu_dn >> 2) >= ctas * kWarps ? (nruns + 1) >> 1 : nruns;
     return sh;
 }
 // costs of the units before each run of phase d, by one warp
@@ -878,36 +873,37 @@ __device__ __forceinline__ void prefix_costs(const Shape& sh, Route& R, int d, f
     if (lane == 0) R.base[d][sh.nruns] = run;
     __syncwarp();
 }
-// list position at which `cost` (counted from the phase's first run) has been passed, rounded to whole steps of `step` units.  The
+// list position at which `cost` has been passed, rounded to whole steps of `step` units.  The
 // arithmetic is approximate, but every CTA evaluates the same expression for the same cut.
 __device__ __forceinline__ int position_at(const Route& R, const List& L, float cost, int step)
 {
     const float* base = R.base[L.d];
-    int lo = L.run0, hi = L.run1;                // base[lo] <= cost < base[hi + 1]
+    const int nruns = R.nruns;
+    int lo = 0, hi = nruns;                      // base[lo] <= cost < base[hi + 1]
     while (lo < hi)
     {
         const int mid = (lo + hi + 1) >> 1;
         if (base[mid] <= cost) lo = mid; else hi = mid - 1;
     }
-    const int at = (lo - L.run0) * L.NU;
-    if (lo >= L.run1) return at;
+    const int at = lo * L.NU;
+    if (lo >= nruns) return at;
     const int n = __float2int_rn(__fdividef(cost - base[lo], R.cost[L.d][lo] * (float)step)) * step;
     return at + (n < 0 ? 0 : n < L.NU ? n : L.NU);
 }
 __device__ __forceinline__ float cost_at(const Route& R, const List& L, int p)
 {
     const int r = quot_any(p, L.NU);
-    return R.base[L.d][L.run0 + r] + (L.run0 + r < L.run1 ? (float)(p - r * L.NU) * R.cost[L.d][L.run0 + r] : 0.f);
+    return R.base[L.d][r] + (r < R.nruns ? (float)(p - r * L.NU) * R.cost[L.d][r] : 0.f);
 }
 // The job that starts at position `at` of the share in work, by one warp: how far its rows fit, the warps' ranges, the table rows
-// of its first runs.  rows_at: byte offset of its rows behind the slots.
-__device__ __forceinline__ void cut_job(const MoeArgs& a, const Shape& sh, Route& R, const List& L, Job& job, int l, int at, int rows_at, int lane)
+// of its first runs.
+__device__ __forceinline__ void cut_job(const MoeArgs& a, const Shape& sh, Route& R, const List& L, Job& job, int at, int lane)
 {
     int stop = job.end, run0 = 0, row0 = 0, nrows = 0;
     if (at < stop)
     {
-        const int row_bytes = (L.d ? sh.ng : sh.ngH) * kRowStep, room = quot(rows_room(a.slot_floats) - rows_at, row_bytes);
-        int h = quot_any(at, L.NH), up = L.d ? 0 : h & 1, run = L.run0 + (L.d ? h : h >> 1);
+        const int row_bytes = (L.d ? sh.ng : sh.ngH) * kRowStep, room = quot(rows_room(a.slot_floats), row_bytes);
+        int h = quot_any(at, L.NH), up = L.d ? 0 : h & 1, run = L.d ? h : h >> 1;
         run0 = run; row0 = row_id(R.runs[run], L.d, up);
         for (; h * L.NH < stop; ++h)           // (run) or (run, gate / up) by (run, gate / up)
         {
@@ -932,25 +928,25 @@ __device__ __forceinline__ void cut_job(const MoeArgs& a, const Shape& sh, Route
         for (int i = lane; i < kCachedRows * kTableWidth; i += 32)
         {
             const int k = i / kTableWidth, run = run0 + k;
-            if (run < L.run1) job.row[k][i - k * kTableWidth] = a.table[(int64_t)R.runs[run].expert * kTableWidth + i - k * kTableWidth];
+            if (run < R.nruns) job.row[k][i - k * kTableWidth] = a.table[(int64_t)R.runs[run].expert * kTableWidth + i - k * kTableWidth];
         }
     if (lane == 0)
     {
-        job.at = at; job.stop = stop; job.seq += kLists; job.staged = 0;
-        job.run0 = run0; job.row0 = row0; job.nrows = nrows; job.rows_at = rows_at;
+        job.at = at; job.stop = stop; job.seq += kLists;
+        job.run0 = run0; job.row0 = row0; job.nrows = nrows;
     }
     __syncwarp();
 }
 // share k of a list (an empty one if k >= the number of CTAs), by one warp
-__device__ __forceinline__ void cut_share(const MoeArgs& a, const Shape& sh, Route& R, const List& L, Job& job, int l, int k, int lane)
+__device__ __forceinline__ void cut_share(const MoeArgs& a, const Shape& sh, Route& R, const List& L, Job& job, int k, int lane)
 {
-    const float c0 = R.base[L.d][L.run0], each = __fdividef(R.base[L.d][L.run1] - c0, (float)gridDim.x);
-    const bool any = k < (int)gridDim.x && L.NU > 0 && L.run0 < L.run1;
-    const int A = any ? position_at(R, L, fmaf(each, (float)k, c0), L.cps) : 0;
-    const int B = !any ? 0 : k + 1 == (int)gridDim.x ? (L.run1 - L.run0) * L.NU : position_at(R, L, fmaf(each, (float)(k + 1), c0), L.cps);
+    const float each = __fdividef(R.base[L.d][R.nruns], (float)gridDim.x);
+    const bool any = k < (int)gridDim.x && L.NU > 0 && R.nruns > 0;
+    const int A = any ? position_at(R, L, __fmul_rn(each, (float)k), L.cps) : 0;
+    const int B = !any ? 0 : k + 1 == (int)gridDim.x ? R.nruns * L.NU : position_at(R, L, __fmul_rn(each, (float)(k + 1)), L.cps);
     if (lane == 0) { job.share = k; job.next = kUndecided; job.end = B; }
     __syncwarp();
-    cut_job(a, sh, R, L, job, l, A < B ? A : B, 0, lane);
+    cut_job(a, sh, R, L, job, A < B ? A : B, lane);
 }
 // this CTA's next share of a list (>= the number of CTAs: none left), decided once per share by the first warp that gets here
 __device__ __forceinline__ int next_share(const MoeArgs& a, Job& job, int l, int lane)
@@ -958,13 +954,13 @@ __device__ __forceinline__ int next_share(const MoeArgs& a, Job& job, int l, int
     int v = 0;
     if (lane == 0)
     {
-        const int ctas = (int)gridDim.x, shift = 16 * (l & 1);
+        const int ctas = (int)gridDim.x;
         v = atomicCAS(&job.next, kUndecided, kDeciding);
         if (v == kUndecided)
         {
             // with every CTA resident all shares are drawn by now: a plain read tells
-            int* q = a.wq + (l & 2);
-            v = (ld_relaxed(q) >> shift & 0xFFFF) < ctas ? atomicAdd(q, 1 << shift) >> shift & 0xFFFF : ctas;
+            int* q = a.wq + 2 * l;
+            v = ld_relaxed(q) < ctas ? atomicAdd(q, 1) : ctas;
             *(volatile int*)&job.next = v;
         }
         while (v == kDeciding) v = *(volatile int*)&job.next;
@@ -991,11 +987,11 @@ __device__ __noinline__ bool piece_done()
     const MoeArgs& a = R.a;
     const Shape& sh = R.sh;
     const Job& job = R.job[pc.l];
-    const int g = lane >> 2, t4 = lane & 3, d = pc.l >> 1, N = d ? a.H : 2 * a.I, buf = pc.l & 1;
+    const int g = lane >> 2, t4 = lane & 3, d = pc.l, N = d ? a.H : 2 * a.I;
     const RunRec run = R.runs[pc.r];
     float acc[NT][4];
     {
-        const float* from = slot_of(R, 2, warp) + lane;
+        const float* from = slot_of(R, 1, warp) + lane;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -1003,13 +999,13 @@ __device__ __noinline__ bool piece_done()
     }
     if (!pc.starts)
     {
-        float* to = slot_of(R, buf, warp) + lane;
+        float* to = slot_of(R, 0, warp) + lane;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int i = 0; i < 4; ++i) to[(nt * 4 + i) * 32] = acc[nt][i];
         __syncwarp();
-        if (lane == 0) asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(&R.slot_seq[buf][warp])), "r"(job.seq) : "memory");
+        if (lane == 0) asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(&R.slot_seq[warp])), "r"(job.seq) : "memory");
         return true;
     }
     int left = pc.left;
@@ -1018,7 +1014,7 @@ __device__ __noinline__ bool piece_done()
         const int n = job.bound[v + 1] - job.bound[v];
         if (n <= 0) continue;
         unsigned long long t0 = 0;
-        for (uint32_t i = 0; ld_slot_seq(&R.slot_seq[buf][v]) != job.seq; ++i)
+        for (uint32_t i = 0; ld_slot_seq(&R.slot_seq[v]) != job.seq; ++i)
             if ((i & 63u) == 63u)
             {
                 if (ld_relaxed(a.status) != 0) return false;
@@ -1028,7 +1024,7 @@ __device__ __noinline__ bool piece_done()
                 else if (t - t0 > kWaitNs) { atomicExch(a.status, 1); return false; }
             }
         __syncwarp();
-        const float* from = slot_of(R, buf, v) + lane;
+        const float* from = slot_of(R, 0, v) + lane;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -1105,11 +1101,11 @@ __device__ __noinline__ bool run_job(int l)
     const Job& job = R.job[l];
     StripJob& J = R.strip[warp];
     const int d = L.d, row_bytes = ((d ? a.I : a.H) >> 7) * kRowStep, NS = (d ? a.H : 2 * a.I) >> 4;
-    const uint32_t rows = rows_base(R) + job.rows_at;
+    const uint32_t rows = rows_base(R);
     const int end = job.bound[warp + 1];
     for (int at = job.bound[warp]; at < end;)
     {
-        const int k = quot_any(at, L.NU), r = L.run0 + k, u = at - k * L.NU, s = quot(u, L.C), ch = u - s * L.C, up = u >= L.NH;
+        const int r = quot_any(at, L.NU), u = at - r * L.NU, s = quot(u, L.C), ch = u - s * L.C, up = u >= L.NH;
         const int ks = L.cps == L.C ? 0 : quot(ch, L.cps), stop = (ks + 1) * L.cps, n = stop - ch < end - at ? stop - ch : end - at;
         at += n;
         const RunRec run = R.runs[r];
@@ -1144,7 +1140,7 @@ __device__ __forceinline__ void prefetch_job(const MoeArgs& a, const Route& R, c
 {
     const int at = job.bound[warp];
     if (at >= job.bound[warp + 1]) return;
-    const int k = quot_any(at, L.NU), u = at - k * L.NU, r = L.run0 + k;
+    const int r = quot_any(at, L.NU), u = at - r * L.NU;
     const RunRec run = R.runs[r];
     const int64_t* row = r - job.run0 < kCachedRows ? job.row[r - job.run0] : a.table + (int64_t)run.expert * kTableWidth;
     const ProjPlanes P = planes_from_row(row, L.d);
@@ -1168,9 +1164,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
     if (warp == kWarps - 1)
     {
         // this CTA's shares: one of each list that there is
-        if (lane < 2) R.draws[lane] = (a.which >> lane & 1) ? atomicAdd(a.wq + 2 * lane, 0x10001) : ctas | ctas << 16;
-        for (int i = lane; i < 2 * kWarps; i += 32) (&R.slot_seq[0][0])[i] = 0;
-        if (lane < kLists) R.job[lane].seq = lane;
+        if (lane < kLists) { R.draws[lane] = (a.which >> lane & 1) ? atomicAdd(a.wq + 2 * lane, 1) : ctas; R.job[lane].seq = lane; }
+        if (lane < kWarps) R.slot_seq[lane] = 0;
         for (int i = lane; i < (int)sizeof(MoeArgs) / 4; i += 32) ((int*)&R.a)[i] = ((const int*)&a)[i];
     }
     if (a.B * a.topk <= 32)
@@ -1184,40 +1179,30 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
     }
     else if (threadIdx.x == 0) s_small = 0;
     if (a.B * a.topk > 32 || !s_small) build_route_cta(a, R);
-    Shape sh = make_shape(a, R.nruns, ctas);
+    Shape sh = make_shape(a, R.nruns);
     if (warp < kLists)
     {
         // a warp per list
-        const int l = warp, d = l >> 1, ks = d ? a.ks_dn : a.ks_gu;
+        const int d = warp, ks = d ? a.ks_dn : a.ks_gu;
         const int use = a.which == 3 ? choose_ksplit(sh.nruns * (d ? a.H >> 4 : a.I >> 3), d ? sh.ng : sh.ngH, ks, ctas, lane) : ks;
-        if (lane == 0) R.ks[d] = use;                 // (the two warps of a phase store the same)
+        if (lane == 0) R.ks[d] = use;
         sh.KSg = sh.KSd = use;
         prefix_costs(sh, R, d, (float)(d ? sh.nu_dn : sh.nu_gu), lane);
-        cut_share(a, sh, R, list_of(a, sh, l), R.job[l], l, R.draws[d] >> (16 * (l & 1)) & 0xFFFF, lane);
+        cut_share(a, sh, R, list_of(a, sh, d), R.job[d], R.draws[d], lane);
     }
     __syncthreads();
     sh.KSg = R.ks[0]; sh.KSd = R.ks[1];
     const uint32_t rows = rows_base(R);
-    // the rows of both gate|up lists are prepared together when they fit
-    const bool both = R.job[0].stop == R.job[0].end && (R.job[0].nrows + R.job[1].nrows) * (sh.ngH * kRowStep) <= rows_room(a.slot_floats);
-    const int rows1 = both ? R.job[0].nrows * (sh.ngH * kRowStep) : 0;
-    if (threadIdx.x == 0)
-    {
-        R.sh = sh;
-        R.job[0].staged = 1; R.job[1].staged = both; R.job[1].rows_at = rows1;
-    }
+    if (threadIdx.x == 0) R.sh = sh;
     if (a.which & 1)
     {
-        int w0 = 0;
-        for (int l = 0; l < 1 + both; ++l)
+        const Job& job = R.job[0];
+        if (job.at < job.stop)
         {
-            const Job& job = R.job[l];
-            if (job.at >= job.stop) continue;
-            w0 += rotate_rows(a, sh, R, job, rows + (l ? rows1 : 0), w0 % kWarps, lane, warp);
-            const RunRec hi = R.runs[list_of(a, sh, l).run0 + quot_any(job.stop - 1, sh.nu_gu)];
-            low_rank_inputs(a, R, R.runs[job.run0].first, hi.first + hi.count, lane, warp);
+            rotate_rows(a, sh, R, job, rows, lane, warp);
+            low_rank_inputs(a, R, job, quot_any(job.stop - 1, sh.nu_gu), lane, warp);
         }
-        prefetch_job(a, R, list_of(a, sh, 0), R.job[0], lane, warp);
+        prefetch_job(a, R, list_of(a, sh, 0), job, lane, warp);
     }
     if (blockIdx.x == 0 && a.hits && (int)threadIdx.x < sh.S)
     {
@@ -1246,33 +1231,32 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
         }
     }
     __syncthreads();
-    bool ok = true;
+    bool ok = true, ready = a.which & 1;      // the rows of the first gate|up job are
 #pragma unroll 1
     for (int l = 0; l < kLists; ++l)
     {
-        if (!(a.which >> (l >> 1) & 1)) continue;
+        if (!(a.which >> l & 1) || sh.nruns == 0) continue;
         const List L = list_of(a, sh, l);
-        if (L.run0 >= L.run1) continue;
         Job& job = R.job[l];
         for (;;)
         {
             if (job.at < job.stop)
             {
-                if (!job.staged)
+                if (!ready)
                 {
-                    if (l >= 2) prefetch_job(a, R, L, job, lane, warp);
+                    if (l) prefetch_job(a, R, L, job, lane, warp);
                     __syncthreads();            // the rows of the job before are no longer needed
-                    if (l < 2)
+                    if (!l)
                     {
-                        rotate_rows(a, sh, R, job, rows + job.rows_at, 0, lane, warp);
-                        const RunRec hi = R.runs[L.run0 + quot_any(job.stop - 1, L.NU)];
-                        low_rank_inputs(a, R, R.runs[job.run0].first, hi.first + hi.count, lane, warp);
+                        rotate_rows(a, sh, R, job, rows, lane, warp);
+                        low_rank_inputs(a, R, job, quot_any(job.stop - 1, L.NU), lane, warp);
                     }
-                    else ok = copy_rows(a, sh, R, job, rows + job.rows_at, lane, warp) && ok;
+                    else ok = copy_rows(a, sh, R, job, rows, lane, warp) && ok;
                     __syncthreads();
                 }
                 if (ok) ok = run_job(l);
             }
+            ready = false;
             // the rest of the share, or (only if some CTA is not resident) a share that nobody has drawn
             const bool rest = job.stop < job.end;
             int k = 0;
@@ -1280,11 +1264,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
             __syncthreads();
             if (warp == 0)
             {
-                if (rest) cut_job(a, sh, R, L, job, l, job.stop, 0, lane);
-                else cut_share(a, sh, R, L, job, l, k, lane);
-                // a further share of list 0 may take all the room: the rows of list 1 that stood behind those of the first share are
-                // gone, list 1 prepares its own when it gets there
-                if (l == 0 && lane == 0) { R.job[1].staged = 0; R.job[1].rows_at = 0; }
+                if (rest) cut_job(a, sh, R, L, job, job.stop, lane);
+                else cut_share(a, sh, R, L, job, k, lane);
             }
             __syncthreads();
         }
