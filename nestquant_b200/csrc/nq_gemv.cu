@@ -155,6 +155,7 @@ __device__ __forceinline__ bool wait_counter(const int* p, int target, int* stat
 // (8 legacy MMAs) for a further column tile.
 constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f;
 constexpr int kUndecided = -1, kDeciding = -2, kLists = 2, kCachedRows = 2;
+constexpr int kQueue = 64;       // finishers waiting in a CTA
 // The units [at, stop) of list positions that this CTA is working on, and the token rows it needs for them.
 struct Job
 {
@@ -205,6 +206,9 @@ struct Route
     int draws[kLists];                    // this CTA's first shares of the lists
     __align__(16) float zg[NQ_MAX_PICKS][4];   // low-rank inputs x V_gu^T of the picks of this CTA's gate|up shares
     int slot_seq[kWarps];                 // job whose share of a piece is in the warp's slot
+    int queue[kQueue], q_head, q_tail;    // finishers to be done, [q_head, q_tail) of them not taken yet (0: entry not written yet)
+    int ended[kLists];                    // warps that are through with their ranges of the jobs of a list
+    int share_tasks;                      // some run has more than one token: finishers go through the queue
     Job job[kLists];
 };
 constexpr int kRouteBytes = (sizeof(Route) + 127) / 128 * 128;
@@ -555,7 +559,7 @@ __device__ __forceinline__ bool copy_rows(const MoeArgs& a, const Shape& sh, con
         while (job.row0 + p >= R.runs[run].first + R.runs[run].count) ++run;
         if ((a.which & 1) && run != seen)
         {
-            if (!wait_counter(a.cnt_gu + 2 * sh.S * sh.ng + run, sh.ng, a.status)) return false;
+            if (!wait_counter(a.cnt_gu + 2 * sh.S * sh.ng + run, sh.ng * R.runs[run].count, a.status)) return false;
             seen = run;
         }
         if (blk < sh.ng)
@@ -568,8 +572,7 @@ __device__ __forceinline__ bool copy_rows(const MoeArgs& a, const Shape& sh, con
 }
 
 // ---------------------------------------------------------------- finishers
-// (run, group) complete: WHT128, sv, (+ low rank), SwiGLU, su_d, WHT128 -> h, one token after the other; the sums of the
-// next token are fetched while the current one is transformed.
+// (run, group) complete, token j of the run: WHT128, sv, (+ low rank), SwiGLU, su_d, WHT128 -> h.
 __device__ __forceinline__ float4 sum_slices(const float* p, size_t stride, int KS)
 {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -580,84 +583,74 @@ __device__ __forceinline__ float4 sum_slices(const float* p, size_t stride, int 
     }
     return v;
 }
-__device__ __noinline__ void finish_gate_up(int r, int grp)
+__device__ __noinline__ void finish_gate_up(int r, int grp, int j)
 {
     const Route& R = route();
     const MoeArgs& a = R.a;
     const Shape& sh = R.sh;
     const int lane = threadIdx.x & 31;
-    __syncwarp();        // lane 0's acquiring arrival is ordered before every lane's loads below
+    __syncwarp();        // the acquiring look at the queue or at the counter is ordered before every lane's loads below
     const RunRec run = R.runs[r];
     const int64_t* row = a.table + (int64_t)run.expert * kTableWidth;
     const int S = sh.S, N = 2 * a.I, KS = sh.KSg, ng = sh.ng;
     const size_t slice = (size_t)S * N;
     const int col = grp * 128 + lane * 4;
     const float* part = a.part_gu + col;
-    int slot = R.order[run.first];
-    float4 fg = sum_slices(part + (size_t)slot * N, slice, KS), fu = sum_slices(part + (size_t)slot * N + a.I, slice, KS);
+    const int slot = R.order[run.first + j];
+    const float4 fg = sum_slices(part + (size_t)slot * N, slice, KS), fu = sum_slices(part + (size_t)slot * N + a.I, slice, KS);
     const __half* scales = R.scales[slot];
     const uint2 sv_g = *(const uint2*)(scales + a.H + col), sv_u = *(const uint2*)(scales + a.H + a.I + col),
                 su_d = *(const uint2*)(scales + a.H + 2 * a.I + col);
     const __half* lr = R.lr[slot];
     const int rg = lr ? (int)row[16] : 0, rd = lr ? (int)row[17] : 0, hw = (int)row[18];
     const __half* lr4 = lr && run.level == 4 ? (const __half*)row[15] : nullptr;
-#pragma unroll 1
-    for (int j = 0; j < run.count; ++j)
+    const float4 cur[2] = {fg, fu};
+    float z[4] = {0.f, 0.f, 0.f, 0.f};
+    if (rg)
     {
-        const float4 cur[2] = {fg, fu};
-        const int now = slot;
-        if (j + 1 < run.count)
-        {
-            slot = R.order[run.first + j + 1];
-            fg = sum_slices(part + (size_t)slot * N, slice, KS); fu = sum_slices(part + (size_t)slot * N + a.I, slice, KS);
-        }
-        float z[4] = {0.f, 0.f, 0.f, 0.f};
-        if (rg)
-        {
-            const float4 f = *(const float4*)R.zg[now];
-            z[0] = f.x; z[1] = f.y; z[2] = f.z; z[3] = f.w;
-        }
-        float gu[2][4];
+        const float4 f = *(const float4*)R.zg[slot];
+        z[0] = f.x; z[1] = f.y; z[2] = f.z; z[3] = f.w;
+    }
+    float gu[2][4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
-        {
-            float v[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w}, sc[4];
-            wht128(v, lane);
-            unpack4h(u ? sv_u : sv_g, sc);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] *= sc[i];
-            for (int q = 0; q < rg; ++q)
-            {
-                float u2[4], u4[4] = {0.f, 0.f, 0.f, 0.f};
-                const size_t o = (size_t)(u * rg + q) * a.I + col;
-                load4h(lr + (size_t)rg * a.H + o, u2);
-                if (lr4) load4h(lr4 + o, u4);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] += z[q] * u2[i] + z[q] * u4[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) gu[u][i] = v[i];
-        }
-        float v[4], sc[4];
-        unpack4h(su_d, sc);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = silu(gu[0][i]) * gu[1][i];
-        for (int q = 0; q < rd; ++q)          // this group's share of z_dn = sw V_dn^T
-        {
-            float w[4];
-            load4h(lr + (size_t)rg * a.H + 2 * (size_t)rg * a.I + (size_t)q * a.I + col, w);
-            float d = v[0] * w[0] + v[1] * w[1] + v[2] * w[2] + v[3] * w[3];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (lane == 0) a.zd[((size_t)now * ng + grp) * 4 + q] = d;
-        }
+    for (int u = 0; u < 2; ++u)
+    {
+        float v[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w}, sc[4];
+        wht128(v, lane);
+        unpack4h(u ? sv_u : sv_g, sc);
 #pragma unroll
         for (int i = 0; i < 4; ++i) v[i] *= sc[i];
-        wht128(v, lane);
-        if (hw <= 128) store4h_operand(a.h + (size_t)now * a.I + grp * 128, lane, v);
-        else __stcg((float4*)(a.part_gu + (size_t)now * N + col), make_float4(v[0], v[1], v[2], v[3]));   // fp32 stage: gate columns, k-slice 0
+        for (int q = 0; q < rg; ++q)
+        {
+            float u2[4], u4[4] = {0.f, 0.f, 0.f, 0.f};
+            const size_t o = (size_t)(u * rg + q) * a.I + col;
+            load4h(lr + (size_t)rg * a.H + o, u2);
+            if (lr4) load4h(lr4 + o, u4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] += z[q] * u2[i] + z[q] * u4[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) gu[u][i] = v[i];
     }
-    int done = 1;       // groups of this run whose h is now complete
+    float v[4], sc[4];
+    unpack4h(su_d, sc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = silu(gu[0][i]) * gu[1][i];
+    for (int q = 0; q < rd; ++q)          // this group's share of z_dn = sw V_dn^T
+    {
+        float w[4];
+        load4h(lr + (size_t)rg * a.H + 2 * (size_t)rg * a.I + (size_t)q * a.I + col, w);
+        float d = v[0] * w[0] + v[1] * w[1] + v[2] * w[2] + v[3] * w[3];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (lane == 0) a.zd[((size_t)slot * ng + grp) * 4 + q] = d;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] *= sc[i];
+    wht128(v, lane);
+    if (hw <= 128) store4h_operand(a.h + (size_t)slot * a.I + grp * 128, lane, v);
+    else __stcg((float4*)(a.part_gu + (size_t)slot * N + col), make_float4(v[0], v[1], v[2], v[3]));   // fp32 stage: gate columns, k-slice 0
+    int done = 1;       // groups of this token whose h is now complete
     if (hw > 128)
     {
         // 512-wide rotation = H_4 (x) WHT128 / 2: the last of the hw/128 groups of a block combines their fp32 results
@@ -666,7 +659,7 @@ __device__ __noinline__ void finish_gate_up(int r, int grp)
         int last = 0;
         if (lane == 0)
         {
-            int* ch = a.cnt_gu + S * ng + r * ng + b0;
+            int* ch = a.cnt_gu + (S + slot) * ng + b0;
             last = add_release(ch, 1) == nb - 1;
             if (last) { ld_acquire(ch); *ch = 0; }
         }
@@ -676,10 +669,9 @@ __device__ __noinline__ void finish_gate_up(int r, int grp)
         {
             __syncwarp();
             const float rs = rsqrtf((float)nb);
-            for (int task = 0; task < run.count * nb; ++task)
+            const float* p = a.part_gu + (size_t)slot * N + b0 * 128 + lane * 4;
+            for (int ob = 0; ob < nb; ++ob)
             {
-                const int j = task / nb, ob = task - j * nb, slot = R.order[run.first + j];
-                const float* p = a.part_gu + (size_t)slot * N + b0 * 128 + lane * 4;
                 float o[4] = {0.f, 0.f, 0.f, 0.f};
                 for (int b = 0; b < nb; ++b)
                 {
@@ -758,7 +750,7 @@ __device__ __noinline__ void finish_down(int b, int grp)
     const MoeArgs& a = R.a;
     const Shape& sh = R.sh;
     const int lane = threadIdx.x & 31;
-    __syncwarp();        // the acquiring arrival (some lane's) is ordered before every lane's loads below
+    __syncwarp();        // the acquiring look at the queue or at the counter is ordered before every lane's loads below
     const int N = a.H, KS = sh.KSd, col = grp * 128 + lane * 4, s0 = b * a.topk;
     const size_t slice = (size_t)sh.S * N;
     float o[4] = {0.f, 0.f, 0.f, 0.f};
@@ -827,6 +819,99 @@ __device__ __noinline__ void finish_down(int b, int grp)
     }
     if (a.world > 1) ep_send(a, sh, R.par, b, grp, lane, o);
     else *(float4*)(a.out + (size_t)b * a.H + col) = make_float4(o[0], o[1], o[2], o[3]);
+}
+
+// The finishers of a CTA's pieces: one entry per token of a gate|up (run, group) or per down (token, group).  The warp whose piece
+// arrives last puts them in, the warps that are through with their ranges take them out.  A finisher takes 3 to 11 us (chains of
+// loads and shuffles beside 19 busy warps); done by that one warp for all tokens of the run, they held up its range, its CTA and
+// whoever waits for the h: 24 tokens over 16 experts, H = 1024, I = 1280, low rank: 573 us per call against 148; 32 tokens
+// over 16 experts, H = 4096: 325 against 310; 15 tokens over 54 experts, H = 896: 52 against 43.
+// Calls in which no expert has two tokens gain nothing and do them in place; for one token (SHARE = false) the queue is not even
+// compiled in, as its code alone costs 1 to 1.5 us.
+constexpr int kTask = 1 << 30, kDownTask = 1 << 29;
+__device__ __forceinline__ void finish_task(int t)
+{
+    if (t & kDownTask) finish_down(t >> 16 & 0xFF, t >> 8 & 0xFF);
+    else finish_gate_up(t >> 16 & 0xFF, t >> 8 & 0xFF, t & 0xFF);
+}
+// every lane with `has` puts in its task; what does not fit is done here, and so is everything if the call does not share
+template <bool SHARE>
+__device__ __forceinline__ void put_tasks(Route& R, bool has, int task, int lane)
+{
+    const unsigned all = __ballot_sync(0xffffffffu, has);
+    if (!all) return;
+    __syncwarp();        // some lane's acquiring arrival is ordered before the releasing stores below
+    int at = kQueue;
+    if (SHARE && R.share_tasks)
+    {
+        if (lane == 0) at = atomicAdd(&R.q_tail, __popc(all));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(all & ((1u << lane) - 1u));
+    }
+    if (has && at < kQueue) asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(smem_addr(&R.queue[at])), "r"(task) : "memory");
+    unsigned left = __ballot_sync(0xffffffffu, has && at >= kQueue);
+    while (left)
+    {
+        const int src = __ffs(left) - 1;
+        left &= left - 1;
+        finish_task(__shfl_sync(0xffffffffu, task, src));
+    }
+}
+// lane 0: a task, 0 if there is none (or the next one is being written: its writer looks again when its range is through)
+__device__ __forceinline__ int take_task(Route& R)
+{
+    int h = *(volatile int*)&R.q_head;
+    for (;;)
+    {
+        const int tail = *(volatile int*)&R.q_tail;
+        if (h >= (tail < kQueue ? tail : kQueue)) return 0;
+        int t;
+        asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(t) : "r"(smem_addr(&R.queue[h])) : "memory");
+        if (!t) return 0;
+        const int seen = atomicCAS(&R.q_head, h, h + 1);
+        if (seen == h) return t;
+        h = seen;
+    }
+}
+// This warp is through with its range of list l's job: it takes finishers until no warp of the CTA can put in more (a barrier
+// follows).
+__device__ __noinline__ void do_tasks(int l)
+{
+    Route& R = route();
+    const int lane = threadIdx.x & 31;
+    int through = 0;
+    unsigned long long t0 = 0;
+    __syncwarp();
+    if (lane == 0) through = (atomicAdd(&R.ended[l], 1) / kWarps + 1) * kWarps;
+    for (uint32_t i = 0;; ++i)
+    {
+        int t = 0, more = 0;
+        if (lane == 0)
+        {
+            more = *(volatile int*)&R.ended[l] < through;
+            t = take_task(R);
+        }
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t) { finish_task(t); continue; }
+        if (!__shfl_sync(0xffffffffu, more, 0)) break;
+        if ((i & 63u) == 63u)
+        {
+            // (leaving early is harmless: whoever puts in a task takes it out again if nobody else does.  A warp that gave up a
+            // wait does not get here)
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            now = __shfl_sync(0xffffffffu, now, 0);
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > kWaitNs) break;
+            if (ld_relaxed(R.a.status) != 0) break;
+        }
+        __nanosleep(64);
+    }
+}
+// empties the queue; one warp, between two barriers of the CTA with no finisher left
+__device__ __forceinline__ void reset_queue(Route& R, int lane)
+{
+    for (int i = lane; i < kQueue; i += 32) R.queue[i] = 0;
+    if (lane == 0) { R.q_head = 0; R.q_tail = 0; }
 }
 
 // ---------------------------------------------------------------- shares and jobs
@@ -978,7 +1063,7 @@ __device__ __forceinline__ int ld_slot_seq(const int* p)
 // Part of a piece is through.  The warp in whose range the piece starts owns it: it adds the following warps' shares (if the
 // piece goes on behind its range), stores the sums to part[ks][slot][row] and counts the piece; the others leave theirs in
 // their slot (fragment order [tile][i][lane]).  false = a wait ran out.
-template <int NT>
+template <int NT, bool SHARE>
 __device__ __noinline__ bool piece_done()
 {
     Route& R = route();
@@ -1058,7 +1143,8 @@ __device__ __noinline__ bool piece_done()
             last = add_release(cnt, 1) == 2 * sh.KSg * 8 - 1;
             if (last) { ld_acquire(cnt); *cnt = 0; }
         }
-        if (__shfl_sync(0xffffffffu, last, 0)) finish_gate_up(pc.r, grp);
+        last = __shfl_sync(0xffffffffu, last, 0);
+        put_tasks<SHARE>(R, last && lane < run.count, kTask | pc.r << 16 | grp << 8 | lane, lane);
     }
     else
     {
@@ -1072,26 +1158,21 @@ __device__ __noinline__ bool piece_done()
             last = add_release(cnt, 1) == (int)R.nvalid[b] * sh.KSd * 8 - 1;
             if (last) { ld_acquire(cnt); *cnt = 0; }
         }
-        unsigned todo = __ballot_sync(0xffffffffu, last);
-        while (todo)
-        {
-            const int src = __ffs(todo) - 1;
-            todo &= todo - 1;
-            finish_down(__shfl_sync(0xffffffffu, b, src), grp);
-        }
+        put_tasks<SHARE>(R, last, kTask | kDownTask | b << 16 | grp << 8, lane);
     }
     return true;
 }
 
 // this warp's range of a job, piece by piece; false = a wait ran out
-template <int NT>
+template <int NT, bool SHARE>
 __device__ __forceinline__ bool run_piece(int mode, int rc, int bk)
 {
 #define NQ_RUN(RES, RCV, BKV) do { if (RES && mode == 2) strip_gemv<RES ? 2 : 0, RCV, BKV, NT>(); else strip_gemv<RES ? 1 : 0, RCV, BKV, NT>(); } while (0)
     NQ_WITH_CODES(mode > 0, rc, bk, NQ_GEMV_CODES, NQ_RUN);
 #undef NQ_RUN
-    return piece_done<NT>();
+    return piece_done<NT, SHARE>();
 }
+template <bool SHARE>
 __device__ __noinline__ bool run_job(int l)
 {
     Route& R = route();
@@ -1103,6 +1184,7 @@ __device__ __noinline__ bool run_job(int l)
     const int d = L.d, row_bytes = ((d ? a.I : a.H) >> 7) * kRowStep, NS = (d ? a.H : 2 * a.I) >> 4;
     const uint32_t rows = rows_base(R);
     const int end = job.bound[warp + 1];
+    bool ok = true;
     for (int at = job.bound[warp]; at < end;)
     {
         const int r = quot_any(at, L.NU), u = at - r * L.NU, s = quot(u, L.C), ch = u - s * L.C, up = u >= L.NH;
@@ -1126,14 +1208,14 @@ __device__ __noinline__ bool run_job(int l)
             J.l = l; J.r = r; J.strip = s; J.ks = ks; J.left = stop - ch - n; J.starts = ch == ks * L.cps;
         }
         __syncwarp();
-        bool ok;
-        if (run.count <= 8) ok = run_piece<1>(mode, rc, bk);
-        else if (run.count <= 16) ok = run_piece<2>(mode, rc, bk);
-        else ok = run_piece<kRunTiles>(mode, rc, bk);
-        if (!ok) return false;
+        if (run.count <= 8) ok = run_piece<1, SHARE>(mode, rc, bk);
+        else if (run.count <= 16) ok = run_piece<2, SHARE>(mode, rc, bk);
+        else ok = run_piece<kRunTiles, SHARE>(mode, rc, bk);
+        if (!ok) break;
         __syncwarp();
     }
-    return true;
+    if (SHARE && R.share_tasks) do_tasks(l);
+    return ok;
 }
 // the first unit of this warp's range on its way to L2, and the output scales of the strips of the job
 __device__ __forceinline__ void prefetch_job(const MoeArgs& a, const Route& R, const List& L, const Job& job, int lane, int warp)
@@ -1153,7 +1235,8 @@ __device__ __forceinline__ void prefetch_job(const MoeArgs& a, const Route& R, c
     if (lane == 1 && !L.d) prefetch_l2(sc + a.H + 2 * a.I + (col >= a.I ? col - a.I : col));
 }
 
-// one CTA per SM, warps independent of one another inside a job
+// one CTA per SM, warps independent of one another inside a job; SHARE: finishers may be shared (calls of two tokens or more)
+template <bool SHARE>
 __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_constant__ MoeArgs a)
 {
     Route& R = route();
@@ -1164,7 +1247,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
     if (warp == kWarps - 1)
     {
         // this CTA's shares: one of each list that there is
-        if (lane < kLists) { R.draws[lane] = (a.which >> lane & 1) ? atomicAdd(a.wq + 2 * lane, 1) : ctas; R.job[lane].seq = lane; }
+        if (SHARE) reset_queue(R, lane);
+        if (lane < kLists) { R.draws[lane] = (a.which >> lane & 1) ? atomicAdd(a.wq + 2 * lane, 1) : ctas; R.job[lane].seq = lane; R.ended[lane] = 0; }
         if (lane < kWarps) R.slot_seq[lane] = 0;
         for (int i = lane; i < (int)sizeof(MoeArgs) / 4; i += 32) ((int*)&R.a)[i] = ((const int*)&a)[i];
     }
@@ -1189,6 +1273,13 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
         sh.KSg = sh.KSd = use;
         prefix_costs(sh, R, d, (float)(d ? sh.nu_dn : sh.nu_gu), lane);
         cut_share(a, sh, R, list_of(a, sh, d), R.job[d], R.draws[d], lane);
+    }
+    else if (SHARE && warp == kLists)
+    {
+        bool any = false;
+        for (int r = lane; r < sh.nruns; r += 32) any = any || R.runs[r].count > 1;
+        any = __any_sync(0xffffffffu, any);
+        if (lane == 0) R.share_tasks = any;
     }
     __syncthreads();
     sh.KSg = R.ks[0]; sh.KSd = R.ks[1];
@@ -1246,6 +1337,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
                 {
                     if (l) prefetch_job(a, R, L, job, lane, warp);
                     __syncthreads();            // the rows of the job before are no longer needed
+                    if (SHARE && warp == kWarps - 1) reset_queue(R, lane);
                     if (!l)
                     {
                         rotate_rows(a, sh, R, job, rows, lane, warp);
@@ -1254,7 +1346,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
                     else ok = copy_rows(a, sh, R, job, rows, lane, warp) && ok;
                     __syncthreads();
                 }
-                if (ok) ok = run_job(l);
+                if (ok) ok = run_job<SHARE>(l);
             }
             ready = false;
             // the rest of the share, or (only if some CTA is not resident) a share that nobody has drawn
@@ -1306,9 +1398,14 @@ static int resident_ctas()
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
     if (cached[dev]) return cached[dev];
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaFuncSetAttribute((const void*)moe_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmem) != cudaSuccess) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)moe_decode_kernel, kThreads, kGemvSmem);
-    cached[dev] = per > 0 ? sms : 0;
+    int fits = 1;
+    for (const void* k : {(const void*)moe_decode_kernel<false>, (const void*)moe_decode_kernel<true>})
+    {
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemvSmem) != cudaSuccess) return 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kThreads, kGemvSmem);
+        fits = fits && per > 0;
+    }
+    cached[dev] = fits ? sms : 0;
     return cached[dev];
 }
 
@@ -1395,7 +1492,7 @@ static int moe_forward(const NqMoeForward* p, const NqMoeEp* ep, void* stream)
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, nq::moe_decode_kernel, a);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, p->B > 1 ? nq::moe_decode_kernel<true> : nq::moe_decode_kernel<false>, a);
     if (e != cudaSuccess) return nq::fail(NQ_ERR_CUDA, "nq_moe_forward: %s", cudaGetErrorString(e));
     return nq::check_launch("nq_moe_forward");
 }

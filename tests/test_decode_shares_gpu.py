@@ -5,14 +5,20 @@ import random
 import pytest
 import torch
 
-from tests.test_moe_layer_gpu import _routing
+from tests.test_moe_layer_gpu import _check, _routing
+from tests.util import expert_to_oracle
 
 pytestmark = pytest.mark.gpu
 
 
-def _layer(H, I, NE, levels, Bmax, topk, rk_gu=0, rk_dn=7):
+def _layer(H, I, NE, levels, Bmax, topk, rank=0, had=128):
     from nestquant_b200 import moe
-    exs = [moe.Expert(H, I, seed=900 + i, rk_gu=rk_gu, rk_dn=rk_dn, var=True, sv=0.02, gen_device="cuda") for i in range(NE)]
+    gen = torch.Generator().manual_seed(NE)
+    exs = [moe.Expert(H, I, seed=900 + i, rk_gu=0, rk_dn=7, var=True, sv=0.02, gen_device="cuda") for i in range(NE)]
+    for ex in exs:
+        ex.had_dn = had
+        if rank:
+            ex.set_lr(*[torch.randn(rank, n, generator=gen) * 0.02 for n in (H, I, I, I, I, I, H, H)])
     L = moe.MoELayer(NE, H, I, Bmax=Bmax, topk=topk)
     for e in range(NE):
         L.set(e, exs[e], levels[e])
@@ -47,3 +53,24 @@ def test_same_bits_when_other_work_holds_sms(H, I, NE, topk, B, level):
         assert torch.equal(alone, y), (held, int((alone != y).sum()), float((alone - y).abs().max()))
         for t in (L.cnt_gu, L.cnt_d, L.wq):
             assert int(t.abs().sum()) == 0
+
+
+# A CTA has room for 9 token rows at H = 6144, 13 at 4096, 6 at 8192 (of 136 bytes per 64 elements, beside 25 KB of routing and
+# 20 KB of partial sums), and one expert's tokens make a run of up to 8, 16 or 32 of them, as many as fit.
+@pytest.mark.parametrize("H,I,NE,topk,B,mode,rank,had", [
+    (6144, 128, 40, 8, 32, "rand", 0, 128),     # 207 units per CTA, 6 tokens per expert: a share over two runs' halves takes two jobs
+    (6144, 256, 4, 2, 32, "same", 0, 128),      # 32 tokens of one expert: runs of 8
+    (8192, 128, 8, 8, 8, "same", 0, 128),       # 8 tokens of one expert, rows for 6
+    (4096, 512, 6, 3, 17, "rand", 2, 512),      # runs of two column tiles, low rank, 512-wide rotation: finishers in two steps
+    (768, 512, 16, 8, 32, "rand", 1, 128),      # runs of up to 32 tokens, four column tiles
+    (128, 8192, 8, 8, 32, "same", 0, 128),      # 110 finishers per CTA and list: more than the queue holds
+    (1024, 1024, 3, 2, 2, "same", 3, 512),      # the smallest call that shares its finishers
+])
+def test_cuts_against_the_oracle(H, I, NE, topk, B, mode, rank, had):
+    levels = [(4, 2, 4, 4)[e % 4] for e in range(NE)]
+    L, exs = _layer(H, I, NE, levels, B, topk, rank, had)
+    rng = random.Random(NE + B)
+    sel, rw = _routing(B, NE, topk, rng, mode)
+    x = torch.randn(B, H, generator=torch.Generator().manual_seed(B)).bfloat16().half()
+    _check(L, [expert_to_oracle(e) for e in exs], levels, x, sel, rw, (H, I, B, mode))
+    assert L.status() == 0
