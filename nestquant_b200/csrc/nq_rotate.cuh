@@ -231,6 +231,16 @@ __device__ __forceinline__ void load16w_mapH(const __half* p, int q, uint32_t (&
         w[4 * j] = u.x; w[4 * j + 1] = u.y; w[4 * j + 2] = u.z; w[4 * j + 3] = u.w;
     }
 }
+// the same words from a vector that is aligned to 8 bytes only
+__device__ __forceinline__ void load16w_mapH_align8(const __half* p, int q, uint32_t (&w)[16])
+{
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+    {
+        const uint2 u = *(const uint2*)(p + 32 * (j >> 1) + 8 * q + 4 * (j & 1));
+        w[2 * j] = u.x; w[2 * j + 1] = u.y;
+    }
+}
 // v = x * s for the lane's 32 elements, both given as the packed fp16 words of map H (fp32 products)
 __device__ __forceinline__ void mul32w_mapH(const uint32_t (&xw)[16], const uint32_t (&sw)[16], float (&v)[32])
 {

@@ -74,3 +74,19 @@ def test_cuts_against_the_oracle(H, I, NE, topk, B, mode, rank, had):
     x = torch.randn(B, H, generator=torch.Generator().manual_seed(B)).bfloat16().half()
     _check(L, [expert_to_oracle(e) for e in exs], levels, x, sel, rw, (H, I, B, mode))
     assert L.status() == 0
+
+
+@pytest.mark.parametrize("B", [1, 4])
+def test_scale_vectors_aligned_to_8_bytes(B):
+    """a decode call asks 8 bytes of the scale vectors, which may be views into a larger array: same bits as from aligned ones"""
+    H, I, NE, topk = 1024, 512, 6, 3
+    L, exs = _layer(H, I, NE, [4, 2] * 3, B, topk)
+    sel, rw = (t.cuda() for t in _routing(B, NE, topk, random.Random(B)))
+    x = torch.randn(B, H, device="cuda").bfloat16().half()
+    want = L(x, sel, rw).clone()
+    for e, ex in enumerate(exs):
+        room = torch.zeros(ex.signs.numel() + 8, dtype=torch.float16, device="cuda")
+        ex.signs = room[4:4 + ex.signs.numel()].copy_(ex.signs)
+        assert ex.signs.data_ptr() % 16 == 8
+        L.set(e, ex, (4, 2)[e % 2])
+    assert torch.equal(L(x, sel, rw), want)
