@@ -154,12 +154,11 @@ __device__ __forceinline__ bool wait_counter(const int* p, int target, int* stat
 // Relative cost of a unit, by which the lists are cut: measured clocks of the unit loop, 410 at level 2 and 690 at level 4, and 64
 // (8 legacy MMAs) for a further column tile.
 constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f;
-constexpr int kUndecided = -1, kDeciding = -2, kLists = 2, kCachedRows = 2;
+constexpr int kLists = 2, kCachedRows = 2;
 constexpr int kQueue = 64;       // finishers waiting in a CTA
 // The units [at, stop) of list positions that this CTA is working on, and the token rows it needs for them.
 struct Job
 {
-    int share, next;                 // share in work; the one to follow (kUndecided until the first warp is done)
     int at, stop, end;               // this job; the end of the share
     int seq;                         // number of the job (of either list), not 0 once it is cut
     int run0, row0, nrows;           // first run, its first row's number, rows
@@ -203,7 +202,7 @@ struct Route
     float cost[2][NQ_MAX_PICKS];          // cost of one unit of a run (gate|up, down)
     float base[2][NQ_MAX_PICKS + 1];      // cost of the units before a run
     int ks[2];                            // k-slices per strip in use
-    int draws[kLists];                    // this CTA's first shares of the lists
+    int draws[kLists], drawn[kLists];     // this CTA's first shares of the lists, and how many shares were drawn when it last looked
     __align__(16) float zg[NQ_MAX_PICKS][4];   // low-rank inputs x V_gu^T of the picks of this CTA's gate|up shares
     int slot_seq[kWarps];                 // job whose share of a piece is in the warp's slot
     int queue[kQueue], q_head, q_tail;    // finishers to be done, [q_head, q_tail) of them not taken yet (0: entry not written yet)
@@ -1029,30 +1028,10 @@ __device__ __forceinline__ void cut_share(const MoeArgs& a, const Shape& sh, Rou
     const bool any = k < (int)gridDim.x && L.NU > 0 && R.nruns > 0;
     const int A = any ? position_at(R, L, __fmul_rn(each, (float)k), L.cps) : 0;
     const int B = !any ? 0 : k + 1 == (int)gridDim.x ? R.nruns * L.NU : position_at(R, L, __fmul_rn(each, (float)(k + 1)), L.cps);
-    if (lane == 0) { job.share = k; job.next = kUndecided; job.end = B; }
+    if (lane == 0) job.end = B;
     __syncwarp();
     cut_job(a, sh, R, L, job, A < B ? A : B, lane);
 }
-// this CTA's next share of a list (>= the number of CTAs: none left), decided once per share by the first warp that gets here
-__device__ __forceinline__ int next_share(const MoeArgs& a, Job& job, int l, int lane)
-{
-    int v = 0;
-    if (lane == 0)
-    {
-        const int ctas = (int)gridDim.x;
-        v = atomicCAS(&job.next, kUndecided, kDeciding);
-        if (v == kUndecided)
-        {
-            // with every CTA resident all shares are drawn by now: a plain read tells
-            int* q = a.wq + 2 * l;
-            v = ld_relaxed(q) < ctas ? atomicAdd(q, 1) : ctas;
-            *(volatile int*)&job.next = v;
-        }
-        while (v == kDeciding) v = *(volatile int*)&job.next;
-    }
-    return __shfl_sync(0xffffffffu, v, 0);
-}
-
 // ---------------------------------------------------------------- a warp's share of a job
 __device__ __forceinline__ int ld_slot_seq(const int* p)
 {
@@ -1285,6 +1264,8 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
     sh.KSg = R.ks[0]; sh.KSd = R.ks[1];
     const uint32_t rows = rows_base(R);
     if (threadIdx.x == 0) R.sh = sh;
+    int drawn = 0;
+    if (warp == kWarps - 1 && lane < kLists) drawn = ld_relaxed(a.wq + 2 * lane);      // (on its way while the rows are rotated)
     if (a.which & 1)
     {
         const Job& job = R.job[0];
@@ -1321,6 +1302,7 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
                 if (R.nvalid[task / sh.ngH] == 0) ep_send(a, sh, par, task / sh.ngH, task % sh.ngH, lane, zero);
         }
     }
+    if (warp == kWarps - 1 && lane < kLists) R.drawn[lane] = drawn;
     __syncthreads();
     bool ok = true, ready = a.which & 1;      // the rows of the first gate|up job are
 #pragma unroll 1
@@ -1349,15 +1331,21 @@ __global__ void __launch_bounds__(kThreads, 1) moe_decode_kernel(const __grid_co
                 if (ok) ok = run_job<SHARE>(l);
             }
             ready = false;
-            // the rest of the share, or (only if some CTA is not resident) a share that nobody has drawn
+            // the rest of the share, or a share that nobody has drawn (all of them were by the time the rows were rotated if every
+            // CTA was resident then; an empty share ends the list)
             const bool rest = job.stop < job.end;
-            int k = 0;
-            if (!rest && (k = next_share(a, job, l, lane)) >= ctas) break;
+            if (!rest && R.drawn[l] >= ctas) break;
             __syncthreads();
             if (warp == 0)
             {
                 if (rest) cut_job(a, sh, R, L, job, job.stop, lane);
-                else cut_share(a, sh, R, L, job, k, lane);
+                else
+                {
+                    int k = lane == 0 ? atomicAdd(a.wq + 2 * l, 1) : 0;
+                    k = __shfl_sync(0xffffffffu, k, 0);
+                    cut_share(a, sh, R, L, job, k, lane);
+                    if (lane == 0) R.drawn[l] = k + 1;
+                }
             }
             __syncthreads();
         }
