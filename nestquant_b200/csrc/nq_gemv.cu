@@ -29,7 +29,9 @@
 //   operand order   inside a 128-wide chunk the fp16 element k = 16 T + 2 t4 + 8 hi + e sits at position 32 t4 + 4 T + 2 hi + e,
 //              so lane (g, t4) finds the B fragments of all 8 k-steps of a unit in 64 contiguous bytes.
 // Split-k partial sums go to separate buffers and are added in a fixed order, so results are bitwise repeatable
-// (the reference accumulates with fp32 atomics and is not, sm120/check.py:21).
+// (the reference accumulates with fp32 atomics and is not, sm120/check.py:21).  The cut points follow from all picks of a call, so the
+// order in which a token's fp32 sums are added, and with it its last bits, depend on what the other tokens of the call picked; they do not
+// depend on timing nor on how many CTAs are resident.
 //
 // Bound: the integer decode.  A loop that does nothing but decode and multiply units from registers runs at 382 clocks per
 // unit and SM sub-partition at level 2 and 645 at level 4 (the multiplies and byte sums on the FMA-heavy pipe, half rate,
@@ -53,8 +55,8 @@ namespace nq {
 constexpr int kWarps = 20, kThreads = 32 * kWarps;
 static_assert(kThreads >= NQ_MAX_PICKS, "the run list is built by one thread per pick");
 // Shared memory of the CTA: route, slots, token rows.  It stays below 164 KB, which leaves 64 KB of L1: registers that the
-// decoder functions save live in local memory, and with all 227 KB taken every access to it went to L2 (a 1-token call
-// spent ~45 us outside the unit loop instead of ~20).
+// decoder functions save live in local memory.  With 224 KB calls take 2 to 4 us more (1 token of the full layer 117.7 -> 119.5,
+// 4 tokens 368.6 -> 375.2, 16 tokens of a small layer 65.1 -> 68.3).
 constexpr int kGemvSmem = 160 * 1024;
 constexpr int kRunTiles = 4;     // most column tiles (8 tokens each) of mma.m16n8k16 per run
 constexpr int kTileFloats = 4 * 32;      // accumulators of a column tile
@@ -151,8 +153,8 @@ __device__ __forceinline__ bool wait_counter(const int* p, int target, int* stat
 }
 
 // ---------------------------------------------------------------- shared state of a CTA
-// Relative cost of a unit, by which the lists are cut: measured clocks of the unit loop, 410 at level 2 and 690 at level 4, and 64
-// (8 legacy MMAs) for a further column tile.
+// Relative cost of a unit, by which the lists are cut: measured clocks of the unit loop, 410 at level 2 and 690 at level 4, and 80
+// for a further column tile (its 8 legacy MMAs are 64 of them, the reads of its fragments the rest).
 constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f;
 constexpr int kLists = 2, kCachedRows = 2;
 constexpr int kQueue = 64;       // finishers waiting in a CTA
@@ -223,8 +225,8 @@ __host__ __device__ constexpr int rows_room(int slot_floats) { return kGemvSmem 
 __device__ __forceinline__ int quot(int a, int b) { return (int)__fdividef((float)a + 0.5f, (float)b); }
 __device__ __forceinline__ int quot_any(int a, int b) { return a < (1 << 20) ? quot(a, b) : a / b; }
 
-// Group the picks into runs: a run = one expert and up to 32 of its picks in pick order; runs are numbered by first
-// pick, then ordered level 4 before level 2.  A run has at most run_cap picks.
+// Group the picks into runs: a run = one expert and up to run_cap of its picks in pick order; runs are numbered by first
+// pick, then ordered level 4 before level 2.
 __device__ __forceinline__ void set_costs(const MoeArgs& a, Route& R, int rank, const Pick& p, int count)
 {
     const int C[2] = {a.H / 128, a.I / 128}, nm[2] = {a.nm_gu, a.nm_dn};
@@ -1205,9 +1207,8 @@ __device__ __forceinline__ void prefetch_job(const MoeArgs& a, const Route& R, c
     const RunRec run = R.runs[r];
     const int64_t* row = r - job.run0 < kCachedRows ? job.row[r - job.run0] : a.table + (int64_t)run.expert * kTableWidth;
     const ProjPlanes P = planes_from_row(row, L.d);
-    // (the first sub-array of a plane holds 16 bytes per record, 8 for the codes below 128 bits)
-    prefetch_l2((const uint8_t*)P.base + ((size_t)u * 32 + lane) * ((row[19] >> (8 * L.d) & 0xFF) ? 8 : 16));
-    if (run.level >= 4 && !P.flags) prefetch_l2(P.p4 + ((size_t)u * 32 + lane) * (0x29D >> (int)row[10 + L.d] & 1 ? 16 : 8));
+    prefetch_l2((const uint8_t*)P.base + ((size_t)u * 32 + lane) * (kWideCodes >> (int)(row[19] >> (8 * L.d) & 0xFF) & 1 ? 16 : 8));
+    if (run.level >= 4 && !P.flags) prefetch_l2(P.p4 + ((size_t)u * 32 + lane) * (kWideCodes >> (int)row[10 + L.d] & 1 ? 16 : 8));
     const __half* sc = (const __half*)row[9];
     const int col = quot(u, L.C) * 16;
     if (lane == 0) prefetch_l2(L.d ? sc + a.H + 3 * a.I + col : sc + a.H + col);
@@ -1398,7 +1399,10 @@ static int resident_ctas()
 }
 
 // Most tokens of a run: their rows (of H or I halves) have to fit into shared memory behind the slots, whose size goes with the
-// number of column tiles.  Calls of up to 8 tokens have one tile.
+// number of column tiles.  Calls of up to 8 tokens have one tile.  An expert with more tokens than that (8 at 6,144 columns, 6 at 8,192,
+// 11 at 4,096, 32 up to about 900) is decoded once per run.  That costs less than it seems: a second decode of a unit keeps
+// every warp busy, while fragments of 32 tokens from L2 stalled the loop (an earlier version of this kernel): 32 tokens, top-8
+// of 16 experts, H = 6,144: 520 us against 1,070; all 32 tokens on one expert: 112 against 793.
 static void run_limits(int B, int H, int I, int* run_cap, int* slot_floats)
 {
     const int row = (H > I ? H : I) / 128 * kRowStep;

@@ -1,5 +1,5 @@
 // Prefill path, the permutation: the (token, pick) pairs of a window sorted by expert, as a stable counting sort in one kernel
-// (up to 8,192 picks) or three, and without a host sync.
+// (up to 8,192 picks and 369 experts, whose counts fit into 48 KB of shared memory) or three, and without a host sync.
 //
 // Replaces the host side of the reference's prefill (sm120/moe.py:293-298: torch.argsort of the flattened expert ids,
 // scatter_add for the counts, a .cpu() of the counts) and this library's earlier use of the same torch operators.

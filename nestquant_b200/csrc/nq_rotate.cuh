@@ -66,8 +66,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 // and register bits are index bits of the vector, see the maps below).  Five of the seven butterfly stages stay inside a
 // lane; two cross lanes (8 shuffles per vector instead of 20).  The passes that use it are bound by issue slots, so all but
 // the first stage work on pairs of registers: 208 instead of 320 instructions, the same sums in the same order
-// (b * -1 + a is a - b, rounded once).  Whole prefill calls on one GPU: 8,192 tokens
-// 8,786 -> 8,726 us, 3,001 tokens on one of four ranks 1,666 -> 1,656.
+// (b * -1 + a is a - b, rounded once).  Whole prefill calls are faster by less than their times spread (0.6 %).
 __device__ __forceinline__ void wht128_x8(float (&v)[32], int lane)
 {
     uint64_t w[16];

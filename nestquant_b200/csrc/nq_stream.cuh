@@ -25,12 +25,6 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
-// the same with compile-time byte offsets on both addresses
-template <int DOFF, int SOFF>
-__device__ __forceinline__ void cp_async16_at(uint32_t dst, const void* src)
-{
-    asm volatile("cp.async.cg.shared.global [%0 + %2], [%1 + %3], 16;" ::"r"(dst), "l"(src), "n"(DOFF), "n"(SOFF));
-}
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src));
@@ -75,6 +69,12 @@ struct RecordLayout
     // the tail lands in the upper half of the 16-bit piece's word when the pieces before it end on a half word
     static constexpr bool tail_joins = T != 0 && ((kBits - T) & 31) == 16;
 };
+
+// Window codes (bit c = code c) whose records have a 128-bit piece: the first sub-array of their planes has 16 bytes per record, that of the
+// others 8.
+template <int... C>
+constexpr uint32_t codes_with_128(std::integer_sequence<int, C...>) { return (0u | ... | ((uint32_t)(RecordLayout<C>::n128 != 0) << C)); }
+constexpr uint32_t kWideCodes = codes_with_128(std::make_integer_sequence<int, 10>{});
 
 // One lane's read position in a plane of `nrec` records, at unit `unit0`; copy(stage, u) fetches unit unit0 + u.
 template <int CODE>

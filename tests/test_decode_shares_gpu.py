@@ -55,7 +55,7 @@ def test_same_bits_when_other_work_holds_sms(H, I, NE, topk, B, level):
             assert int(t.abs().sum()) == 0
 
 
-# A CTA has room for 9 token rows at H = 6144, 13 at 4096, 6 at 8192 (of 136 bytes per 64 elements, beside 25 KB of routing and
+# A CTA has room for 9 token rows at H = 6144, 13 at 4096, 6 at 8192 (of 272 bytes per 128 elements, beside 23 KB of routing and
 # 20 KB of partial sums), and one expert's tokens make a run of up to 8, 16 or 32 of them, as many as fit.
 @pytest.mark.parametrize("H,I,NE,topk,B,mode,rank,had", [
     (6144, 128, 40, 8, 32, "rand", 0, 128),     # 207 units per CTA, 6 tokens per expert: a share over two runs' halves takes two jobs

@@ -213,10 +213,10 @@ def test_pair_sort_is_a_stable_counting_sort():
     assert torch.equal(hits.cpu().long(), torch.bincount(flat[valid], minlength=NE))
 
 
-@pytest.mark.parametrize("NE,topk,T", [(1, 1, 1), (5, 3, 11), (37, 1, 1024), (256, 8, 1023), (256, 8, 1024), (256, 8, 1025), (370, 7, 1170),
-                                       (371, 7, 1170), (1024, 4, 333), (1024, 8, 4500)])
+@pytest.mark.parametrize("NE,topk,T", [(1, 1, 1), (5, 3, 11), (37, 1, 1024), (256, 8, 1023), (256, 8, 1024), (256, 8, 1025), (369, 7, 1170),
+                                       (370, 7, 1170), (1024, 4, 333), (1024, 8, 4500)])
 def test_pair_sort_and_plan_over_their_range(NE, topk, T):
-    """one-kernel sort (up to 8,192 picks and 371 bins) and three-kernel sort, and the pass lists from either form of the counts:
+    """one-kernel sort (up to 8,192 picks and 370 bins) and three-kernel sort, and the pass lists from either form of the counts:
     sizes around the lines between them, one slice and many, one expert and as many as a CTA has threads"""
     from nestquant_b200 import ext
     g = torch.Generator().manual_seed(NE + T)
