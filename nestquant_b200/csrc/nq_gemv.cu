@@ -154,8 +154,10 @@ __device__ __forceinline__ bool wait_counter(const int* p, int target, int* stat
 
 // ---------------------------------------------------------------- shared state of a CTA
 // Relative cost of a unit, by which the lists are cut: measured clocks of the unit loop, 410 at level 2 and 690 at level 4, and 80
-// for a further column tile (its 8 legacy MMAs are 64 of them, the reads of its fragments the rest).
-constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f;
+// for a further column tile (its 8 legacy MMAs are 64 of them, the reads of its fragments the rest).  A unit of a strip in mask mode costs 75
+// more than its mix of refined and unrefined units (the loop decides unit by unit): without them, CTAs with masked experts took 455 us for a
+// gate|up share that took the others 400 (8 tokens of the full layer, a third of the level-4 experts masked).
+constexpr float kCostUnit = 410.f, kCostRefined = 280.f, kCostTile = 80.f, kCostMasked = 75.f;
 constexpr int kLists = 2, kCachedRows = 2;
 constexpr int kQueue = 64;       // finishers waiting in a CTA
 // The units [at, stop) of list positions that this CTA is working on, and the token rows it needs for them.
@@ -235,7 +237,7 @@ __device__ __forceinline__ void set_costs(const MoeArgs& a, Route& R, int rank, 
     {
         const bool masked = d ? p.masked_dn : p.masked_gu;
         const float refined = p.level < 4 ? 0.f : masked ? fminf(__fdividef((float)nm[d], (float)C[d]), 1.f) : 1.f;
-        R.cost[d][rank] = kCostUnit + kCostRefined * refined + kCostTile * (float)((count - 1) >> 3);
+        R.cost[d][rank] = kCostUnit + kCostRefined * refined + (p.level >= 4 && masked ? kCostMasked : 0.f) + kCostTile * (float)((count - 1) >> 3);
     }
 }
 // up to 32 picks, none of them more than run_cap times the same expert (false otherwise): one warp, a lane per pick
@@ -1426,7 +1428,7 @@ int nq_moe_workspace(int B, int topk, int H, int I, int ks_gu, int ks_dn, NqMoeW
     NQ_REQUIRE(ks_gu >= 1 && (H / 128) % ks_gu == 0 && ks_dn >= 1 && (I / 128) % ks_dn == 0, "nq_moe_workspace: k-splits %d / %d must divide %d / %d chunks", ks_gu, ks_dn, H / 128, I / 128);
     const size_t S = (size_t)B * topk;
     w->acc_gu_floats = (size_t)ks_gu * S * 2 * I;
-    w->h_halves = S * I + S * 2 * H;                    // h [S][I], the rest is spare
+    w->h_halves = S * I + S * 2 * H;                    // h [S][I]; the rest is not used (what the allocation-free entry refuses hangs on it)
     w->acc_d_floats = (size_t)ks_dn * S * H;
     w->cnt_gu_ints = 2 * S * (I / 128) + S;
     w->cnt_d_ints = (size_t)B * (H / 128);
@@ -1454,7 +1456,6 @@ static int moe_forward(const NqMoeForward* p, const NqMoeEp* ep, void* stream)
     NQ_REQUIRE(nq::aligned16(p->x) && nq::aligned16(p->out) && nq::aligned16(p->acc_gu) && nq::aligned16(p->acc_d) && nq::aligned16(p->h),
                "nq_moe_forward: x, out and workspaces must be 16-byte aligned");
     NQ_REQUIRE(p->force_level == 0 || p->force_level == 2 || p->force_level == 4, "nq_moe_forward: force_level = %d", p->force_level);
-    NQ_REQUIRE(((size_t)p->B * p->topk * p->I) % 8 == 0, "nq_moe_forward: h and the rotated inputs must both be 16-byte aligned");
     nq::MoeArgs a{};
     a.x = (const __half*)p->x; a.sel = p->sel; a.rw = (const __half*)p->rw;
     a.B = p->B; a.topk = p->topk; a.E = p->E; a.H = p->H; a.I = p->I; a.nm_gu = p->nm_gu; a.nm_dn = p->nm_dn;
