@@ -41,8 +41,8 @@ UNIT = "GB/s"
 N_LEVEL4 = 77
 SEED = 20240
 # DRAM bytes / algorithmic bytes of the decode kernel from the ncu capture summarised in
-# profiles/moe_decode_glm_1tok.md (127.24 MB read + 5.04 MB written for 126.05 MB of planes and scales)
-NCU_TRAFFIC_RATIO = 1.049
+# profiles/moe_decode_glm_1tok.md (116.64 MB read + 7.67 MB written for 126.05 MB of planes and scales)
+NCU_TRAFFIC_RATIO = 0.986
 
 
 # The timed CPU arm is this repository's C/OpenMP port of the reference's algorithm, not the reference's own torch code (which
@@ -820,7 +820,7 @@ def main():
                              "gate_up_alone": {"us": r1["gu_us"], "gbs": r1["gu_bytes"] / r1["gu_us"] / 1e3, "frac": r1["gu_bytes"] / r1["gu_us"] / 1e3 / peak},
                              "down_alone": {"us": r1["dn_us"], "gbs": (by_total / args.steps - r1["gu_bytes"]) / r1["dn_us"] / 1e3,
                                             "frac": (by_total / args.steps - r1["gu_bytes"]) / r1["dn_us"] / 1e3 / peak},
-                             "note": "gate_up_alone / down_alone launch the same kernel with one half of its pieces (which = 1 / 2); each includes the fixed cost of a launch, so their times add up to more than the full call's"},
+                             "note": "gate_up_alone / down_alone launch the same kernel with one of its two lists (which = 1 / 2); each includes the fixed cost of a launch, so their times add up to more than the full call's"},
                 "parity": parity,
                 "decode_4tok": None if r4 is None else {"layer_us": r4["us_total"] / s4, "value": r4["bytes_total"] / r4["us_total"] / 1e3, "unit": UNIT,
                                                         "bytes_per_step": r4["bytes_total"] / s4, "steps": s4},

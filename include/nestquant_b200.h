@@ -12,7 +12,8 @@
  *
  * Device table: int64 [E][20] per layer, one row per expert (sm120/nqmoe.cu:26-45, sm120/moe.py:216-229):
  *   [0] level (0 = not resident here, 2, 4)   [1..4] gate|up: base, p4, d4, flags (0 = dense)   [5..8] down: same
- *   [9] fp16 scales [H su_g | I sv_g | I sv_u | I su_d | H sv_o | H su_u]   [10],[11] residual window codes
+ *   [9] fp16 scales [H su_g | I sv_g | I sv_u | I su_d | H sv_o | H su_u] (aligned to 16 bytes; decode calls alone: to 8)
+ *   [10],[11] residual window codes
  *   [12],[13] ring-sign planes (0 = none)   [14] low-rank plane, [15] its level-4 part, [16] r_gu, [17] r_dn
  *   [18] width of the down-input rotation (0 or 128, or 512)   [19] base window codes bk_gu | bk_dn << 8 (0, or 1: see nq_bk_codes)
  */
@@ -155,9 +156,10 @@ int nq_pf_hits(const int32_t* counts, int32_t* hits, int E, void* stream);
  * tensor for its size.  Differences a caller can see:
  *   - up to 32 tokens per call (the reference: 8), B * topk <= 256;
  *   - split-k partial sums are written to acc_gu / acc_d and summed in a fixed order: results are bitwise repeatable,
- *     and those two buffers need no zeroing.  cnt_gu, cnt_d and wq must be zero on entry and are zero again on exit;
+ *     and those two buffers need no zeroing (the last bits of a token's sums depend on the picks of the whole call, not on
+ *     timing).  cnt_gu, cnt_d and wq must be zero on entry and are zero again on exit;
  *   - workspace sizes depend on the k-splits: ask nq_moe_workspace() (the reference sized them from B * topk alone);
- *     h also holds the rotated inputs;
+ *     h has room for [S][2][H] halves behind [S][I] that the call does not use;
  *   - cnt_h[0] is a status word: the call leaves it alone unless a device-side wait ran out (2 s), then it is 1 and the
  *     outputs are invalid.  Clear it before the first call and read it after synchronising if you want to know;
  *   - if no resident expert with a non-zero weight is picked at all, out is written with zeros
@@ -166,8 +168,8 @@ int nq_pf_hits(const int32_t* counts, int32_t* hits, int E, void* stream);
  * One persistent launch on `stream` does the routing, the input rotations, both GEMVs and the combine (the reference: two
  * launches); every routing, level and pointer decision is read on the device, so the call can be captured in a CUDA graph
  * and replayed while a mailbox flips table rows.
- * which = 1 stops after h (gate|up, SwiGLU); which = 2 starts from the h that is in the workspace.  Both h [S][I] and the
- * rotated inputs [S][2][H] behind it are fp16 in "operand order": inside every 128 consecutive k, element
+ * which = 1 stops after h (gate|up, SwiGLU); which = 2 starts from the h that is in the workspace.  h [S][I] is fp16 in
+ * "operand order": inside every 128 consecutive k, element
  * k = 16 T + 2 t4 + 8 hi + e (T < 8, t4 < 4, hi, e < 2) sits at position 32 t4 + 4 T + 2 hi + e.  With which = 1 the
  * split-k partial sums of the gate|up projection stay readable in acc_gu [ks_gu][S][2I], with which = 2 those of the down
  * projection in acc_d [ks_dn][S][H] (S = B * topk pick slots): fed one-hot inputs they hold columns of the decoded weight
@@ -234,7 +236,7 @@ int nq_moe_forward_ep(const NqMoeForward* args, const NqMoeEp* ep, void* stream)
  * (2, 1); 4 tokens at (4, 2) need 4.6 MB and are refused.  The call issues no cudaMalloc / cudaFree and no allocating library
  * routine.  The first call on a device looks up the array's device address (cudaGetSymbolAddress): make that call at
  * start-up, before any stream capture on the device.  All calls share the array, which keeps the previous call's
- * contents; the counters are cleared at the start of each call, and calls that overlap on the GPU race - keep them in
+ * contents; the counters and the status word are cleared at the start of each call, and calls that overlap on the GPU race - keep them in
  * one stream order.  x fp16 [B][H], sel int64 [B][topk], rw fp16 [B][topk], table int64 [E][20], out fp32 [B][H];
  * hits may be NULL. */
 size_t nq_moe_static_scratch_bytes(void);

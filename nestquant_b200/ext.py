@@ -168,8 +168,8 @@ def pf_hits(counts, hits_ptr):
 
 
 def operand_order(K):
-    """int64 [K]: position of element k of a row in the "operand order" of the decode path's internal fp16 rows (h and the
-    rotated inputs): inside every 128 consecutive k, k = 16 T + 2 t4 + 8 hi + e sits at 32 t4 + 4 T + 2 hi + e"""
+    """int64 [K]: position of element k of a row in the "operand order" of the decode path's internal fp16 rows (h, and the
+    rotated inputs in shared memory): inside every 128 consecutive k, k = 16 T + 2 t4 + 8 hi + e sits at 32 t4 + 4 T + 2 hi + e"""
     k = torch.arange(K)
     kk = k % 128
     T, q = kk >> 4, kk & 15
@@ -185,10 +185,11 @@ def kperm_order(K):
 
 
 def default_ksplit(B, H, I, share=1.0, topk=8):
-    """k-slices per strip (gate|up, down) for a B-token call.  The persistent kernel hands out pieces (a 16-row strip over
-    1 / k-slices of its chunks) to ~3,000 warps: the split aims at ~8 units (16 x 128 weights) per piece, between 3,000
-    and 8,192 gate|up pieces and between 1,536 and 6,144 down pieces - what sweeps of the GLM shape and of its
-    tensor-parallel shards (I / 2, I / 4, I / 8) at 1, 2 and 4 tokens settled on.
+    """k-slices per strip (gate|up, down) for a B-token call: the most the call may use (the workspaces are sized for them).  The
+    kernel itself uses a divisor of them, the fewest slices that still cut the runs of the call evenly over its CTAs; it only takes the
+    numbers as they are when one half of the layer is called alone.  The split aims at ~8 units (16 x 128 weights) per piece
+    (a 16-row strip over 1 / k-slices of its chunks), between 3,000 and 8,192 gate|up pieces and between 1,536 and 6,144 down
+    pieces.
     share: fraction of the layer's experts resident on this GPU (expert parallelism: 1 / ranks; 1 for one GPU and for
     tensor-parallel shards, whose I is the shard's)."""
     import math
