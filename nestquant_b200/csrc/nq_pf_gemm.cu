@@ -102,19 +102,33 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 // The producer and MMA warps run their loops with all 32 lanes converged (so that addresses, descriptors and
-// coordinates are warp-uniform values) and one elected lane issues the asynchronous instruction.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
+// coordinates are warp-uniform values) and one elected lane issues the asynchronous instruction.  Their waits leave the poll
+// together, on a vote; `bar` is a shared-space address.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+    unsigned long long t0 = 0;
+    for (uint32_t i = 0;; ++i)
+    {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (__all_sync(0xffffffffu, ok)) return true;
+        if (__any_sync(0xffffffffu, *abort_flag)) return false;
+        if ((i & 255u) == 255u)
+        {
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (t0 == 0) t0 = t;
+            else if (__any_sync(0xffffffffu, t - t0 > kPfWaitNs)) break;
+        }
+    }
+    *abort_flag = 1;
+    return false;
 }
 __device__ __forceinline__ void mbar_expect_tx_elect(uint64_t* bar, uint32_t bytes)
 {
     asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
                  "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(saddr(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_elect(uint64_t* bar)
-{
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(saddr(bar)) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d_elect(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
 {
@@ -122,12 +136,6 @@ __device__ __forceinline__ void tma_load_2d_elect(void* dst, const CUtensorMap* 
                  "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
                  ::"r"(saddr(dst)), "l"(map), "r"(saddr(bar)), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
-{
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(saddr(dst)), "l"(map), "r"(saddr(bar)), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit_elect(uint64_t* bar)
@@ -135,21 +143,13 @@ __device__ __forceinline__ void tc_commit_elect(uint64_t* bar)
     asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
                  "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(saddr(bar)) : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar)) : "memory");
-}
-// D[tmem] (+)= A[smem] * B[smem]; fp16 operands, fp32 accumulate
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// The four K = 16 steps of one 64-wide k-block, issued by one elected lane of a converged warp.  The weight operand is
-// in tensor memory (8 columns per step), the token operand in shared memory (descriptor advances by 32 B, in 16-byte
-// units on the low word: shared-memory addresses fit its 14-bit field).  first == 0: the first MMA overwrites the
-// accumulator.
-__device__ __forceinline__ void tc_mma_kblock(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t first)
+// The four K = 16 steps of one 64-wide k-block and the commits that release its two stages, issued by one elected lane of a
+// converged warp (one election for all six: the warp that issues shares its scheduler with four decode warps, and what it
+// spends per k-block is what paces the kernel when passes are narrow).  The weight operand is in tensor memory (8 columns per
+// step), the token operand in shared memory (descriptor advances by 32 B, in 16-byte units on the low word: shared-memory
+// addresses fit its 14-bit field).  first == 0: the first MMA overwrites the accumulator.
+__device__ __forceinline__ void tc_mma_kblock(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t first,
+                                              uint32_t free_a, uint32_t free_b)
 {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t.reg .b32 ta, tb;\n\t"
@@ -164,12 +164,14 @@ __device__ __forceinline__ void tc_mma_kblock(uint32_t tmem_d, uint32_t tmem_a, 
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %4, p;\n\t"
         "add.u32 ta, %1, 24;\n\tadd.u32 tb, %2, 6;\n\tmov.b64 db, {tb, %3};\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %4, p;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
         "}"
-        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first) : "memory");
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(free_a), "r"(free_b) : "memory");
 }
 // The same for a token tile cut into two column halves with their own accumulator columns (alternating chains).
 __device__ __forceinline__ void tc_mma_kblock2(uint32_t tmem_d0, uint32_t tmem_d1, uint32_t tmem_a, uint32_t b_lo0, uint32_t b_lo1,
-                                               uint32_t b_hi, uint32_t idesc0, uint32_t idesc1, uint32_t first)
+                                               uint32_t b_hi, uint32_t idesc0, uint32_t idesc1, uint32_t first, uint32_t free_a, uint32_t free_b)
 {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t.reg .b32 ta, tb;\n\t"
@@ -192,8 +194,11 @@ __device__ __forceinline__ void tc_mma_kblock2(uint32_t tmem_d0, uint32_t tmem_d
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %6, p;\n\t"
         "add.u32 tb, %4, 6;\n\tmov.b64 db, {tb, %5};\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [ta], db, %7, p;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%9];\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%10];\n\t"
         "}"
-        ::"r"(tmem_d0), "r"(tmem_d1), "r"(tmem_a), "r"(b_lo0), "r"(b_lo1), "r"(b_hi), "r"(idesc0), "r"(idesc1), "r"(first) : "memory");
+        ::"r"(tmem_d0), "r"(tmem_d1), "r"(tmem_a), "r"(b_lo0), "r"(b_lo1), "r"(b_hi), "r"(idesc0), "r"(idesc1), "r"(first), "r"(free_a), "r"(free_b)
+        : "memory");
 }
 // 16 lanes x 4 x 256 bits of tensor memory from a warp, for columns 8 i .. 8 i + 7: lane (g, t4) supplies lane g columns
 // 2 t4, 2 t4 + 1 (r[4 i], r[4 i + 1]) and lane g + 8, same columns (r[4 i + 2], r[4 i + 3]) - the layout of m16n8 fragments
@@ -231,7 +236,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
 // ---------------------------------------------------------------- decode warps
 struct PfShared
 {
-    uint64_t full_b[kPfBStages], empty_b[kPfBStages], full_a[kPfAStages], empty_a[kPfAStages], acc_full, acc_empty;
+    uint64_t full_b[kPfBStages], empty_b[kPfBStages], full_a[kPfGroups], empty_a[kPfAStages], acc_full, acc_empty;
     uint32_t tmem_base;
     volatile int abort_flag;
 };
@@ -260,23 +265,26 @@ struct UnitSink
         if constexpr ((T & 3) == 3)
         {
             const uint32_t it = it0 + (T >> 2), sa = it % kPfAStages;
-            if (*ok) *ok = mbar_wait_warp(&sh->empty_a[sa], ((it / kPfAStages) & 1u) ^ 1u, &sh->abort_flag);
+            if (*ok) *ok = mbar_wait_warp(saddr(&sh->empty_a[sa]), ((it / kPfAStages) & 1u) ^ 1u, &sh->abort_flag);
             tc_fence_after();
             // an aborted launch stores too (the columns are this CTA's until the end, the results are discarded) but signals nothing
             tmem_st_16x256b_x4(tmem_a + sa * kPfACols, frag);
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (*ok && lane == 0) mbar_arrive(&sh->full_a[sa]);
+            if constexpr (T == 7)
+            {
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (*ok && lane == 0) mbar_arrive(&sh->full_a[sa >> 1]);
+            }
         }
     }
 };
 
 // One decode warp, one item: its strip over the chunks c = GROUP, GROUP + 2, ... (the other group of 8 warps takes the
-// other parity), i.e. k-blocks 4 i + 2 GROUP and + 1.  it_base = k-blocks of earlier items.  false = aborted.
+// other parity), i.e. k-blocks 4 i + 2 GROUP and + 1.  unit0 = chunks of earlier items.  false = aborted.
 template <bool REFINED, int RC, int BK, class Mid>
 __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef& sr, int C, int NS, int lane, int group,
-                                             uint32_t tmem_a, uint32_t ring, PfShared* sh, uint32_t it_base, Mid& mid)
+                                             uint32_t tmem_a, uint32_t ring, PfShared* sh, uint32_t unit0, Mid& mid)
 {
     // per-unit scalars of this warp's chunks, one chunk (group + kPfGroups * lane) per lane: ring signs and, for refined units,
     // the block word with its fp16 multiplier / addend (computed once here instead of by every lane of every unit)
@@ -323,7 +331,7 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
         RecordCursor<BK>::read(wb, st, lane);
         uint32_t frag[16];
-        const UnitSink sink{tmem_a, sh, it_base + 2 * (uint32_t)ch, lane, &ok, frag};
+        const UnitSink sink{tmem_a, sh, 2 * (unit0 + (uint32_t)ch), lane, &ok, frag};
         bool refined = false;
         if constexpr (REFINED) refined = chunk_refined(sr, ch);
         if (refined)
@@ -342,11 +350,11 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
 
 template <class Mid>
 __device__ __forceinline__ bool decode_item(const ProjPlanes& P, int level, int rc, int bk, int strip, int C, int NS, int nm, int lane, int group,
-                                            uint32_t tmem_a, uint8_t* ring, PfShared* sh, uint32_t it_base, Mid& mid)
+                                            uint32_t tmem_a, uint8_t* ring, PfShared* sh, uint32_t unit0, Mid& mid)
 {
     const StripRef sr = locate_strip(P, strip, C, NS, nm, level >= 4);
     bool ok = true;
-#define NQ_RUN(REF, RCV, BKV) ok = decode_strip<REF, RCV, BKV>(P, sr, C, NS, lane, group, tmem_a, smem_addr(ring), sh, it_base, mid)
+#define NQ_RUN(REF, RCV, BKV) ok = decode_strip<REF, RCV, BKV>(P, sr, C, NS, lane, group, tmem_a, smem_addr(ring), sh, unit0, mid)
     NQ_WITH_CODES(level >= 4, rc, bk, 0x3FF, NQ_RUN);
 #undef NQ_RUN
     return ok;
@@ -366,7 +374,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < kPfBStages; ++s) { mbar_init(&sh->full_b[s], 1); mbar_init(&sh->empty_b[s], 1); }
-        for (int s = 0; s < kPfAStages; ++s) { mbar_init(&sh->full_a[s], 8); mbar_init(&sh->empty_a[s], 1); }
+        for (int s = 0; s < kPfGroups; ++s) mbar_init(&sh->full_a[s], 8);
+        for (int s = 0; s < kPfAStages; ++s) mbar_init(&sh->empty_a[s], 1);
         mbar_init(&sh->acc_full, 1); mbar_init(&sh->acc_empty, kPfDecodeWarps);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -384,7 +393,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     const int N = a.down ? a.H : 2 * a.I, K = a.down ? a.I : a.H, C = K / 128, NS = N / 16, groups = N / 128, nkb = K / 64;
     const int npass = a.plan[0], nitems = npass * groups;
     const PfPass* passes = (const PfPass*)(a.plan + 4);
-    uint32_t it = 0, nitem = 0;     // k-blocks / items handled so far by this role (phases of the A-stage and accumulator barriers)
+    uint32_t unit = 0, nitem = 0;        // chunks / items handled so far by this role (phases of the weight-tile and accumulator barriers)
+    const uint32_t full_a0 = saddr(sh->full_a), empty_a0 = saddr(sh->empty_a), full_b0 = saddr(sh->full_b), empty_b0 = saddr(sh->empty_b);
     uint32_t par_b = 0;                  // bit s: parity of the times token-tile stage s was used (its stage count changes from pass to pass)
     int last_sbox = 0;                   // producer: stage size of the previous item
 
@@ -429,11 +439,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const CUtensorMap* map = up ? &tmap1 : &tmap0;
             bool ok = true;
             if (sbox != last_sbox)
-                for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(&sh->empty_b[s], ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
+                for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
             last_sbox = sbox;
             for (int kb = 0, s = 0; ok && kb < nkb; ++kb, s = s + 1 == nb ? 0 : s + 1)
             {
-                if (!mbar_wait_warp(&sh->empty_b[s], ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag)) break;
+                if (!mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag)) break;
                 par_b ^= 1u << s;
                 mbar_expect_tx_elect(&sh->full_b[s], (uint32_t)nbox * kPfBoxBytes);
                 for (int j = 0; j < nbox; ++j)
@@ -443,7 +453,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         else if (warp == 1)
         {
             // ---- MMA issue
-            bool ok = mbar_wait_warp(&sh->acc_empty, (nitem & 1u) ^ 1u, &sh->abort_flag);   // epilogue of the previous item has drained TMEM
+            bool ok = mbar_wait_warp(saddr(&sh->acc_empty), (nitem & 1u) ^ 1u, &sh->abort_flag);   // epilogue of the previous item has drained TMEM
             tc_fence_after();
             // N <= 256 per instruction: one MMA per k-step, or two of (nearly) equal width
             const int n0 = ntok16 <= NQ_PF_SPLIT ? ntok16 : ((ntok16 / 2 + 15) & ~15), n1 = ntok16 - n0;
@@ -452,19 +462,24 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const uint32_t b_lo0 = (uint32_t)bdesc0, b_hi = (uint32_t)(bdesc0 >> 32);
             const uint32_t b_step = (uint32_t)(sbox * (kPfBoxBytes >> 4));
             uint32_t s = 0, b_lo = b_lo0;                 // token-tile stage of this k-block and its descriptor
-            for (int kb = 0; ok && kb < nkb; ++kb, ++it)
+            for (int c = 0; ok && c < C; ++c, ++unit)
             {
-                const uint32_t sa = it % kPfAStages;
-                if (!mbar_wait_warp(&sh->full_b[s], (par_b >> s) & 1u, &sh->abort_flag) ||
-                    !mbar_wait_warp(&sh->full_a[sa], (it / kPfAStages) & 1u, &sh->abort_flag)) { ok = false; break; }
-                par_b ^= 1u << s;
-                tc_fence_after();
-                const uint32_t ta = tmem + kPfAccCols + sa * kPfACols;
-                if (n1 > 0) tc_mma_kblock2(tmem, tmem + n0, ta, b_lo, b_lo + (uint32_t)(n0 * 8), b_hi, idesc0, idesc1, (uint32_t)kb);
-                else tc_mma_kblock(tmem, ta, b_lo, b_hi, idesc0, (uint32_t)kb);
-                tc_commit_elect(&sh->empty_a[sa]);       // both arrive when the MMAs above have read their operands
-                tc_commit_elect(&sh->empty_b[s]);
-                if (++s == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else b_lo += b_step;
+                const uint32_t ua = unit % kPfGroups;
+                ok = mbar_wait_warp(full_a0 + 8 * ua, (unit / kPfGroups) & 1u, &sh->abort_flag);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                {
+                    if (!ok) break;
+                    ok = mbar_wait_warp(full_b0 + 8 * s, (par_b >> s) & 1u, &sh->abort_flag);
+                    if (!ok) break;
+                    par_b ^= 1u << s;
+                    tc_fence_after();
+                    const uint32_t sa = 2 * ua + h, ta = tmem + kPfAccCols + sa * kPfACols, first = (uint32_t)c | h;
+                    if (n1 > 0)
+                        tc_mma_kblock2(tmem, tmem + n0, ta, b_lo, b_lo + (uint32_t)(n0 * 8), b_hi, idesc0, idesc1, first, empty_a0 + 8 * sa, empty_b0 + 8 * s);
+                    else tc_mma_kblock(tmem, ta, b_lo, b_hi, idesc0, first, empty_a0 + 8 * sa, empty_b0 + 8 * s);
+                    if (++s == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else b_lo += b_step;
+                }
             }
             if (ok) tc_commit_elect(&sh->acc_full);
         }
@@ -484,8 +499,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             // of the previous item runs after this item's first unit is decoded: the MMAs of the previous item's last
             // k-blocks finish meanwhile, and the tensor pipe finds tiles waiting when the accumulator is free again.
             auto mid = [&]() { if (have_prev) { epilogue(prev, prev_wg, prev_up, nitem - 1); have_prev = false; } };
-            const bool ok = decode_item(P, level, rc, bk, wg * 8 + sidx, C, NS, nm, lane, half, tmem_a, ring, sh, it, mid);
-            it += nkb;
+            const bool ok = decode_item(P, level, rc, bk, wg * 8 + sidx, C, NS, nm, lane, half, tmem_a, ring, sh, unit, mid);
+            unit += C;
             mid();                                   // (an item of fewer than two chunks: its second warp group decodes nothing)
             if (ok) { prev = ps; prev_wg = wg; prev_up = up; have_prev = true; }
         }
