@@ -32,25 +32,19 @@ namespace nq {
 #ifndef NQ_PF_SPLIT
 #define NQ_PF_SPLIT 256      // token tiles wider than this are multiplied as two column halves
 #endif
-#ifndef NQ_PF_GROUPS
-#define NQ_PF_GROUPS 2      // groups of 8 decode warps; group g takes the chunks c = g (mod groups) of its strips.  3 groups
-                            // (24 decode warps at 72 registers) measured the same time as 2: the kernel runs at the power cap
-#endif
-constexpr int kPfGroups = NQ_PF_GROUPS;
+constexpr int kPfGroups = 2;                         // groups of 8 decode warps; group g takes the chunks c = g (mod 2) of its strips.  (3 groups,
+                                                     // 24 decode warps at 72 registers, were slower on narrow passes and no faster on wide ones.)
 constexpr int kPfDecodeWarps = 8 * kPfGroups;
-constexpr int kPfAStages = 2 * kPfGroups;            // weight tiles in tensor memory: each unit fills two consecutive stages
-constexpr int kPfACols = 32;                         // [128 lanes x 64 k] fp16 = 32 columns
-constexpr int kPfTmemCols = 512;                     // [0, kPfAccCols) accumulator, the rest weight tiles
-constexpr int kPfAccCols = kPfTmemCols - kPfAStages * kPfACols;
-constexpr int kPfTokens = kPfAccCols;                // tokens per pass = accumulator columns (384 with 2 groups, 320 with 3)
+constexpr int kPfACols = 32;                         // weight tile [128 lanes x 64 k] fp16 = 32 columns; a unit stage is two of them
+constexpr int kPfTmemCols = 512;                     // the accumulator from column 0 on, unit stages from the top down
+constexpr int kPfTokens = 384;                       // most tokens per pass (accumulator columns)
+constexpr int kPfUnitStages = 6;                     // most unit stages
 constexpr int kPfBoxRows = 64;                       // token rows per TMA box
 constexpr int kPfBoxBytes = kPfBoxRows * 128;        // [64 rows][64 k] fp16
 constexpr int kPfBBoxes = 20;                        // token-tile region: 8 x 2, 5 x 4, 4 x 5 or 3 x 6 boxes per stage
 constexpr int kPfBStages = 8;                        // most token-tile stages
 constexpr int kPfRingDepth = 2;
 constexpr int kPfThreads = 32 * (2 + kPfDecodeWarps);
-constexpr int kPfSmem = kPfBBoxes * kPfBoxBytes + kPfDecodeWarps * kPfRingDepth * kStageBytes + 1024 + 256;
-static_assert(kPfSmem <= 232448, "shared memory of the prefill GEMM");
 constexpr unsigned long long kPfWaitNs = 2000000000ull;   // a wait that lasts 2 s is treated as a hang
 
 struct PfPass { int expert, row0, ntok, pad; };
@@ -102,17 +96,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 // The producer and MMA warps run their loops with all 32 lanes converged (so that addresses, descriptors and
-// coordinates are warp-uniform values) and one elected lane issues the asynchronous instruction.  Their waits leave the poll
-// together, on a vote; `bar` is a shared-space address.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
+// coordinates are warp-uniform values) and one elected lane issues the asynchronous instruction.
+// Waits of a whole warp, `bar` a shared-space address.  What a wait costs that finds its phase complete is the branches around the
+// poll, not the poll: 200 to 240 clocks as a loop (beside 16 busy warps), 95 as a poll, a vote and a branch that falls through, 15
+// the poll alone.  So the poll that nearly always succeeds stands in line and the bounded loop behind a call.
+__device__ __forceinline__ uint32_t mbar_poll(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok;
+}
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
     unsigned long long t0 = 0;
     for (uint32_t i = 0;; ++i)
     {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (__all_sync(0xffffffffu, ok)) return true;
+        if (__all_sync(0xffffffffu, mbar_poll(bar, parity))) return true;
         if (__any_sync(0xffffffffu, *abort_flag)) return false;
         if ((i & 255u) == 255u)
         {
@@ -125,16 +125,28 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
     *abort_flag = 1;
     return false;
 }
-__device__ __forceinline__ void mbar_expect_tx_elect(uint64_t* bar, uint32_t bytes)
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
 {
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(saddr(bar)), "r"(bytes) : "memory");
+    if (__builtin_expect(__all_sync(0xffffffffu, mbar_poll(bar, parity)), 1)) return true;
+    return mbar_wait_slow(bar, parity, abort_flag);
 }
-__device__ __forceinline__ void tma_load_2d_elect(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
+// Token boxes of the two k-blocks of a chunk, 64 columns apart, on one election.  first: with what the two barriers have to expect.
+__device__ __forceinline__ void tma_load_chunk_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar0, uint32_t bar1,
+                                                     uint32_t bytes)
 {
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
-                 ::"r"(saddr(dst)), "l"(map), "r"(saddr(bar)), "r"(x), "r"(y) : "memory");
+    asm volatile("{\n\t.reg .pred e;\n\t.reg .b32 x1;\n\telect.sync _|e, 0xffffffff;\n\tadd.s32 x1, %3, 64;\n\t"
+                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%5], %7;\n\t"
+                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%3, %4}], [%5];\n\t"
+                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%6], %7;\n\t"
+                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%6];\n\t}"
+                 ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar0), "r"(bar1), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load_more_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar0, uint32_t bar1)
+{
+    asm volatile("{\n\t.reg .pred e;\n\t.reg .b32 x1;\n\telect.sync _|e, 0xffffffff;\n\tadd.s32 x1, %3, 64;\n\t"
+                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%3, %4}], [%5];\n\t"
+                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%6];\n\t}"
+                 ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar0), "r"(bar1) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -236,10 +248,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
 // ---------------------------------------------------------------- decode warps
 struct PfShared
 {
-    uint64_t full_b[kPfBStages], empty_b[kPfBStages], full_a[kPfGroups], empty_a[kPfAStages], acc_full, acc_empty;
+    uint64_t full_b[kPfBStages], empty_b[kPfBStages], full_a[kPfUnitStages], empty_a[2 * kPfUnitStages], acc_full, acc_empty;
+    uint64_t head_full[2], head_empty[2];
+    // What the warps need to know of an item, put here by the producer warp one item ahead: read by every warp for itself, pass
+    // record and table row are two dependent loads from L2 (~0.7 us) at the start of an item of 10 to 30 us.
+    int64_t row[2][kTableWidth];
+    PfPass pass[2];
     uint32_t tmem_base;
     volatile int abort_flag;
 };
+constexpr int kPfSmem = kPfBBoxes * kPfBoxBytes + kPfDecodeWarps * kPfRingDepth * kStageBytes + 1024 + (int)sizeof(PfShared);
+static_assert(kPfSmem <= 232448, "shared memory of the prefill GEMM");
+// Unit stages beside the accumulator of a pass.  Group g uses the stages of its parity, so it is 1, 2 or 3 units ahead of the MMAs.
+// The stages of a narrow pass reach into columns that the accumulator of a wide one before it used (see decode_strip).
+__device__ __forceinline__ int unit_stages(int ntok) { return ntok <= 128 ? 6 : ntok <= 256 ? 4 : 2; }
 // The token-tile region (20 boxes) is cut into stages of 2, 4, 5 or 6 boxes (8, 5, 4 or 3 stages) for a pass of nbox
 // boxes per k-block.  Passes with the same stage size share the stage barriers freely; when the stage size changes
 // between two items of a CTA the new stages overlap old ones at other indices, so the producer first waits until every
@@ -254,37 +276,62 @@ __device__ __forceinline__ int b_stages(int nbox) { return nbox <= 2 ? 8 : nbox 
 // ten pieces that were scheduled one by one).
 struct UnitSink
 {
-    uint32_t tmem_a;      // tensor-memory address of the warp's 16 lanes in weight-tile stage 0
-    PfShared* sh; uint32_t it0; int lane; bool* ok; uint32_t* frag;      // frag: 16 registers
+    uint32_t tmem_a;      // tensor-memory address of the unit stage, at the warp's 16 lanes
+    PfShared* sh; uint32_t stage, parity; int lane; bool* ok; uint32_t* frag;      // frag: 16 registers
     template <int T>
     __device__ __forceinline__ void operator()(std::integral_constant<int, T>, const uint32_t (&a)[4]) const
     {
         // a[0], a[2]: row g, k = 2 t4 + {0,1} and 8 + 2 t4 + {0,1}; a[1], a[3]: row g + 8
-        constexpr int o = 4 * (T & 3);
+        constexpr int o = 4 * (T & 3), h = T >> 2;
         frag[o] = a[0]; frag[o + 1] = a[2]; frag[o + 2] = a[1]; frag[o + 3] = a[3];
         if constexpr ((T & 3) == 3)
         {
-            const uint32_t it = it0 + (T >> 2), sa = it % kPfAStages;
-            if (*ok) *ok = mbar_wait_warp(saddr(&sh->empty_a[sa]), ((it / kPfAStages) & 1u) ^ 1u, &sh->abort_flag);
+            if (*ok) *ok = mbar_wait_warp(saddr(&sh->empty_a[2 * stage + h]), parity ^ 1u, &sh->abort_flag);
             tc_fence_after();
             // an aborted launch stores too (the columns are this CTA's until the end, the results are discarded) but signals nothing
-            tmem_st_16x256b_x4(tmem_a + sa * kPfACols, frag);
+            tmem_st_16x256b_x4(tmem_a + h * kPfACols, frag);
             if constexpr (T == 7)
             {
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (*ok && lane == 0) mbar_arrive(&sh->full_a[sa >> 1]);
+                if (*ok && lane == 0) mbar_arrive(&sh->full_a[stage]);
             }
         }
     }
 };
 
+// Decode warps: accumulator [128 weight rows x ntok] of an item -> out (row of the item's first token, column of the weight group's
+// first row).  TMEM lanes 32 q .. 32 q + 31 (the quarter this warp may read) are weight rows; the four warps of a quarter take
+// 32-column chunks in turn.  Not inlined: it runs in the middle of a decode loop whose registers are all taken.
+__device__ __noinline__ void pf_epilogue(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (!mbar_wait_warp(saddr(&sh->acc_full), parity, &sh->abort_flag)) return;
+    tc_fence_after();
+    const int q = warp & 3, cpart = (warp - 2) >> 2;
+    for (int c0 = cpart * 32; c0 < ntok; c0 += 32 * (kPfDecodeWarps / 4))
+    {
+        uint32_t v[32];
+        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c0, v);
+        float* o = out + (size_t)c0 * ld + q * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < 32; ++j, o += ld)
+            if (c0 + j < ntok) *o = __uint_as_float(v[j]);
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->acc_empty);
+}
+
 // One decode warp, one item: its strip over the chunks c = GROUP, GROUP + 2, ... (the other group of 8 warps takes the
-// other parity), i.e. k-blocks 4 i + 2 GROUP and + 1.  unit0 = chunks of earlier items.  false = aborted.
+// other parity), i.e. k-blocks 4 i + 2 GROUP and + 1.  nstages = unit stages of this item, par_a =
+// parity of the times every stage was used; drain: the stages from 2 on lie where the accumulator of the previous item was, so their
+// first use waits until all warps have read it (acc_empty, phase `drain_parity`).  false = aborted.
 template <bool REFINED, int RC, int BK, class Mid>
 __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef& sr, int C, int NS, int lane, int group,
-                                             uint32_t tmem_a, uint32_t ring, PfShared* sh, uint32_t unit0, Mid& mid)
+                                             uint32_t tmem_a, uint32_t ring, PfShared* sh, int nstages, uint32_t& par_a, bool drain,
+                                             uint32_t drain_parity, Mid& mid)
 {
     // per-unit scalars of this warp's chunks, one chunk (group + kPfGroups * lane) per lane: ring signs and, for refined units,
     // the block word with its fp16 multiplier / addend (computed once here instead of by every lane of every unit)
@@ -317,7 +364,7 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         if (group + kPfGroups * d < C) issue(group + kPfGroups * d, ring + d * kStageBytes);
         cp_async_commit();
     }
-    int slot = 0, slot_in = kPfRingDepth - 1, i = 0;
+    int slot = 0, slot_in = kPfRingDepth - 1, i = 0, stage = group;
     bool ok = true;
     for (int ch = group; ch < C; ch += kPfGroups, ++i)
     {
@@ -331,7 +378,10 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
         RecordCursor<BK>::read(wb, st, lane);
         uint32_t frag[16];
-        const UnitSink sink{tmem_a, sh, 2 * (unit0 + (uint32_t)ch), lane, &ok, frag};
+        if (drain && i > 0 && ch < nstages && ok) ok = mbar_wait_warp(saddr(&sh->acc_empty), drain_parity, &sh->abort_flag);
+        const UnitSink sink{tmem_a - (uint32_t)stage * (2 * kPfACols), sh, (uint32_t)stage, (par_a >> stage) & 1u, lane, &ok, frag};
+        par_a ^= 1u << stage;
+        stage = stage + kPfGroups >= nstages ? group : stage + kPfGroups;
         bool refined = false;
         if constexpr (REFINED) refined = chunk_refined(sr, ch);
         if (refined)
@@ -350,15 +400,21 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
 
 template <class Mid>
 __device__ __forceinline__ bool decode_item(const ProjPlanes& P, int level, int rc, int bk, int strip, int C, int NS, int nm, int lane, int group,
-                                            uint32_t tmem_a, uint8_t* ring, PfShared* sh, uint32_t unit0, Mid& mid)
+                                            uint32_t tmem_a, uint8_t* ring, PfShared* sh, int nstages, uint32_t& par_a, bool drain,
+                                            uint32_t drain_parity, Mid& mid)
 {
     const StripRef sr = locate_strip(P, strip, C, NS, nm, level >= 4);
     bool ok = true;
-#define NQ_RUN(REF, RCV, BKV) ok = decode_strip<REF, RCV, BKV>(P, sr, C, NS, lane, group, tmem_a, smem_addr(ring), sh, unit0, mid)
+#define NQ_RUN(REF, RCV, BKV) ok = decode_strip<REF, RCV, BKV>(P, sr, C, NS, lane, group, tmem_a, smem_addr(ring), sh, nstages, par_a, drain, drain_parity, mid)
     NQ_WITH_CODES(level >= 4, rc, bk, 0x3FF, NQ_RUN);
 #undef NQ_RUN
     return ok;
 }
+
+// A value that is the same in all lanes, as one that the compiler knows to be: what it cannot tell from a lane's own value (anything
+// loaded, anything that depends on the thread index) reaches the uniform registers of an MMA or TMA instruction by a move of its own
+// in front of every one.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __reduce_or_sync(0xffffffffu, x); }
 
 // grid = resident CTAs (one per SM), 576 threads
 __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_constant__ CUtensorMap tmap0,
@@ -369,13 +425,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     uint8_t* b_tiles = smem;                                  // token tiles [rows][64 k] fp16, 128-byte swizzle (TMA boxes)
     uint8_t* rings = smem + kPfBBoxes * kPfBoxBytes;          // per decode warp: kPfRingDepth plane stages
     PfShared* sh = (PfShared*)(rings + kPfDecodeWarps * kPfRingDepth * kStageBytes);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < kPfBStages; ++s) { mbar_init(&sh->full_b[s], 1); mbar_init(&sh->empty_b[s], 1); }
-        for (int s = 0; s < kPfGroups; ++s) mbar_init(&sh->full_a[s], 8);
-        for (int s = 0; s < kPfAStages; ++s) mbar_init(&sh->empty_a[s], 1);
+        for (int s = 0; s < kPfUnitStages; ++s) mbar_init(&sh->full_a[s], 8);
+        for (int s = 0; s < 2 * kPfUnitStages; ++s) mbar_init(&sh->empty_a[s], 1);
+        for (int s = 0; s < 2; ++s) { mbar_init(&sh->head_full[s], 1); mbar_init(&sh->head_empty[s], 1 + kPfDecodeWarps); }
         mbar_init(&sh->acc_full, 1); mbar_init(&sh->acc_empty, kPfDecodeWarps);
         sh->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -388,71 +445,77 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = sh->tmem_base;
+    const uint32_t tmem = uniform(sh->tmem_base);
 
-    const int N = a.down ? a.H : 2 * a.I, K = a.down ? a.I : a.H, C = K / 128, NS = N / 16, groups = N / 128, nkb = K / 64;
-    const int npass = a.plan[0], nitems = npass * groups;
+    const int N = a.down ? a.H : 2 * a.I, K = a.down ? a.I : a.H, C = K / 128, NS = N / 16, groups = N / 128;
+    const int nitems = (int)uniform(a.plan[0]) * groups;
     const PfPass* passes = (const PfPass*)(a.plan + 4);
-    uint32_t unit = 0, nitem = 0;        // chunks / items handled so far by this role (phases of the weight-tile and accumulator barriers)
     const uint32_t full_a0 = saddr(sh->full_a), empty_a0 = saddr(sh->empty_a), full_b0 = saddr(sh->full_b), empty_b0 = saddr(sh->empty_b);
-    uint32_t par_b = 0;                  // bit s: parity of the times token-tile stage s was used (its stage count changes from pass to pass)
-    int last_sbox = 0;                   // producer: stage size of the previous item
-
-    // decode warps: accumulator [128 weight rows x ntok] of item number n of this CTA -> out.  TMEM lanes 32 q .. 32 q + 31
-    // (the quarter this warp may read) are weight rows; the four warps of a quarter take 32-column chunks in turn.
-    PfPass prev{};
-    int prev_wg = 0, prev_up = 0;
-    bool have_prev = false;
-    auto epilogue = [&](const PfPass& ps, int wg, int up, uint32_t n) {
-        bool ok = true;
-        if (lane == 0 && !mbar_wait(&sh->acc_full, n & 1u, &sh->abort_flag)) ok = false;
-        ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-        if (!ok) return;
-        tc_fence_after();
-        const int q = warp & 3, cpart = (warp - 2) >> 2;
-        const int ncol = (up ? wg - a.I / 128 : wg) * 128 + q * 32 + lane;
-        float* out = up ? a.out1 : a.out0;
-        const int ld = a.down ? a.H : a.I;
-        for (int c0 = cpart * 32; c0 < ps.ntok; c0 += 32 * (kPfDecodeWarps / 4))
-        {
-            uint32_t v[32];
-            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c0, v);
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (c0 + j < ps.ntok) out[(size_t)(ps.row0 + c0 + j) * ld + ncol] = __uint_as_float(v[j]);
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->acc_empty);
-    };
-
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
+    // item number n of this CTA: its header slot and the phase of its barriers
+    auto wait_head = [&](uint32_t n) { return mbar_wait_warp(saddr(&sh->head_full[n & 1u]), (n >> 1) & 1u, &sh->abort_flag); };
+    auto leave_head = [&](uint32_t n) { __syncwarp(); if (lane == 0) mbar_arrive(&sh->head_empty[n & 1u]); };
+    // Every role has its own loop over the items; nitem = items handled so far, par_a / par_b bit s = parity of the times unit stage /
+    // token-tile stage s was used (how many stages there are changes from pass to pass).
+    if (warp == 0)
     {
-        const int pi = item / groups, wg = item - pi * groups;
-        const PfPass ps = passes[pi];
-        const int ntok16 = (ps.ntok + 15) & ~15, nbox = (ps.ntok + kPfBoxRows - 1) / kPfBoxRows, nb = b_stages(nbox);
-        const int sbox = b_stage_boxes(nbox);
-        const int up = !a.down && wg >= a.I / 128;
-        if (warp == 0)
+        // ---- token tiles by TMA, up to nb k-blocks ahead of the MMAs; pass record and table row of the items, one item ahead
+        auto publish = [&](int item, uint32_t n) {
+            if (item >= nitems) return true;
+            const PfPass* pass = passes + item / groups;
+            const int64_t w = lane < kTableWidth ? a.table[(int64_t)pass->expert * kTableWidth + lane] : 0;
+            const uint32_t s = n & 1u;
+            if (!mbar_wait_warp(saddr(&sh->head_empty[s]), ((n >> 1) & 1u) ^ 1u, &sh->abort_flag)) return false;
+            if (lane < kTableWidth) sh->row[s][lane] = w;
+            if (lane == 0) sh->pass[s] = *pass;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->head_full[s]);
+            return true;
+        };
+        publish(blockIdx.x, 0);
+        uint32_t par_b = 0, nitem = 0;
+        int last_sbox = 0;                   // stage size of the previous item
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
         {
-            // ---- token tiles by TMA, up to nb k-blocks ahead of the MMAs
-            const CUtensorMap* map = up ? &tmap1 : &tmap0;
+            if (!publish(item + gridDim.x, nitem + 1) || !wait_head(nitem)) break;
+            const int wg = item % groups;
+            const int nbox = (int)uniform((sh->pass[nitem & 1u].ntok + kPfBoxRows - 1) / kPfBoxRows), row0 = (int)uniform(sh->pass[nitem & 1u].row0);
+            const int nb = b_stages(nbox), sbox = b_stage_boxes(nbox);
+            const CUtensorMap* map = uniform(!a.down && wg >= a.I / 128) ? &tmap1 : &tmap0;
             bool ok = true;
             if (sbox != last_sbox)
                 for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
             last_sbox = sbox;
-            for (int kb = 0, s = 0; ok && kb < nkb; ++kb, s = s + 1 == nb ? 0 : s + 1)
+            const uint32_t tiles0 = saddr(b_tiles), bytes = (uint32_t)nbox * kPfBoxBytes, step = (uint32_t)sbox * kPfBoxBytes;
+            for (int c = 0, s = 0; ok && c < C; ++c)
             {
-                if (!mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag)) break;
-                par_b ^= 1u << s;
-                mbar_expect_tx_elect(&sh->full_b[s], (uint32_t)nbox * kPfBoxBytes);
-                for (int j = 0; j < nbox; ++j)
-                    tma_load_2d_elect(b_tiles + (s * sbox + j) * kPfBoxBytes, map, kb * 64, ps.row0 + j * kPfBoxRows, &sh->full_b[s]);
+                const int s1 = s + 1 == nb ? 0 : s + 1;
+                const uint32_t p0 = ((par_b >> s) & 1u) ^ 1u, p1 = ((par_b >> s1) & 1u) ^ 1u;
+                const uint32_t free = mbar_poll(empty_b0 + 8 * s, p0) & mbar_poll(empty_b0 + 8 * s1, p1);
+                if (__builtin_expect(!__all_sync(0xffffffffu, free), 0))
+                {
+                    ok = mbar_wait_slow(empty_b0 + 8 * s, p0, &sh->abort_flag) && mbar_wait_slow(empty_b0 + 8 * s1, p1, &sh->abort_flag);
+                    if (!ok) break;
+                }
+                par_b ^= (1u << s) | (1u << s1);
+                const uint32_t d0 = tiles0 + s * step, d1 = tiles0 + s1 * step, f0 = full_b0 + 8 * s, f1 = full_b0 + 8 * s1;
+                tma_load_chunk_elect(d0, d1, map, c * 128, row0, f0, f1, bytes);
+                for (int j = 1; j < nbox; ++j)
+                    tma_load_more_elect(d0 + j * kPfBoxBytes, d1 + j * kPfBoxBytes, map, c * 128, row0 + j * kPfBoxRows, f0, f1);
+                s = s1 + 1 == nb ? 0 : s1 + 1;
             }
+            if (sh->abort_flag) break;
         }
-        else if (warp == 1)
+    }
+    else if (warp == 1)
+    {
+        // ---- MMA issue
+        uint32_t par_a = 0, par_b = 0, nitem = 0;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
         {
-            // ---- MMA issue
+            if (!wait_head(nitem)) break;
+            const int ntok = (int)uniform(sh->pass[nitem & 1u].ntok), ntok16 = (ntok + 15) & ~15, nbox = (ntok + kPfBoxRows - 1) / kPfBoxRows;
+            const int nb = b_stages(nbox), sbox = b_stage_boxes(nbox), nstages = unit_stages(ntok);
+            leave_head(nitem);
             bool ok = mbar_wait_warp(saddr(&sh->acc_empty), (nitem & 1u) ^ 1u, &sh->abort_flag);   // epilogue of the previous item has drained TMEM
             tc_fence_after();
             // N <= 256 per instruction: one MMA per k-step, or two of (nearly) equal width
@@ -462,51 +525,81 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const uint32_t b_lo0 = (uint32_t)bdesc0, b_hi = (uint32_t)(bdesc0 >> 32);
             const uint32_t b_step = (uint32_t)(sbox * (kPfBoxBytes >> 4));
             uint32_t s = 0, b_lo = b_lo0;                 // token-tile stage of this k-block and its descriptor
-            for (int c = 0; ok && c < C; ++c, ++unit)
+            for (int c = 0, ua = 0; ok && c < C; ++c, ua = ua + 1 == nstages ? 0 : ua + 1)
             {
-                const uint32_t ua = unit % kPfGroups;
-                ok = mbar_wait_warp(full_a0 + 8 * ua, (unit / kPfGroups) & 1u, &sh->abort_flag);
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
+                // the unit and its two token tiles: three polls, one vote, one branch
+                const uint32_t s1 = s + 1 == (uint32_t)nb ? 0 : s + 1, b_lo1 = s1 == 0 ? b_lo0 : b_lo + b_step;
+                const uint32_t pa = (par_a >> ua) & 1u, p0 = (par_b >> s) & 1u, p1 = (par_b >> s1) & 1u;
+                uint32_t ready = mbar_poll(full_a0 + 8 * ua, pa);
+                ready &= mbar_poll(full_b0 + 8 * s, p0);
+                ready &= mbar_poll(full_b0 + 8 * s1, p1);
+                if (__builtin_expect(!__all_sync(0xffffffffu, ready), 0))
                 {
+                    ok = mbar_wait_slow(full_a0 + 8 * ua, pa, &sh->abort_flag) && mbar_wait_slow(full_b0 + 8 * s, p0, &sh->abort_flag) &&
+                         mbar_wait_slow(full_b0 + 8 * s1, p1, &sh->abort_flag);
                     if (!ok) break;
-                    ok = mbar_wait_warp(full_b0 + 8 * s, (par_b >> s) & 1u, &sh->abort_flag);
-                    if (!ok) break;
-                    par_b ^= 1u << s;
-                    tc_fence_after();
-                    const uint32_t sa = 2 * ua + h, ta = tmem + kPfAccCols + sa * kPfACols, first = (uint32_t)c | h;
-                    if (n1 > 0)
-                        tc_mma_kblock2(tmem, tmem + n0, ta, b_lo, b_lo + (uint32_t)(n0 * 8), b_hi, idesc0, idesc1, first, empty_a0 + 8 * sa, empty_b0 + 8 * s);
-                    else tc_mma_kblock(tmem, ta, b_lo, b_hi, idesc0, first, empty_a0 + 8 * sa, empty_b0 + 8 * s);
-                    if (++s == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else b_lo += b_step;
                 }
+                par_a ^= 1u << ua;
+                par_b ^= (1u << s) | (1u << s1);
+                tc_fence_after();
+                const uint32_t ta = tmem + kPfTmemCols - 2 * kPfACols - ua * (2 * kPfACols), free_a = empty_a0 + 16 * ua;
+                if (n1 > 0)
+                {
+                    const uint32_t half = (uint32_t)(n0 * 8);
+                    tc_mma_kblock2(tmem, tmem + n0, ta, b_lo, b_lo + half, b_hi, idesc0, idesc1, (uint32_t)c, free_a, empty_b0 + 8 * s);
+                    tc_mma_kblock2(tmem, tmem + n0, ta + kPfACols, b_lo1, b_lo1 + half, b_hi, idesc0, idesc1, 1u, free_a + 8, empty_b0 + 8 * s1);
+                }
+                else
+                {
+                    tc_mma_kblock(tmem, ta, b_lo, b_hi, idesc0, (uint32_t)c, free_a, empty_b0 + 8 * s);
+                    tc_mma_kblock(tmem, ta + kPfACols, b_lo1, b_hi, idesc0, 1u, free_a + 8, empty_b0 + 8 * s1);
+                }
+                if (s1 + 1 == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else { s = s1 + 1; b_lo = b_lo1 + b_step; }
             }
             if (ok) tc_commit_elect(&sh->acc_full);
+            if (sh->abort_flag) break;
         }
-        else
+    }
+    else
+    {
+        // ---- decode, then epilogue
+        // A warp may touch only the 32 tensor-memory lanes of its quarter (warp % 4): the four decode warps of a
+        // quarter take its two strips x the chunk groups.
+        const int dw = warp - 2, qd = warp & 3, sub = (dw >> 2) & 1, half = dw >> 3, sidx = 2 * qd + sub;      // half = chunk group
+        const uint32_t tmem_a = tmem + ((uint32_t)(32 * qd + 16 * sub) << 16) + kPfTmemCols - 2 * kPfACols;
+        uint8_t* ring = rings + dw * kPfRingDepth * kStageBytes;
+        const int ld = a.down ? a.H : a.I;
+        uint32_t par_a = 0, nitem = 0;
+        float* prev_out = nullptr;           // the item whose accumulator this warp has still to write (prev_ntok 0: none)
+        int prev_ntok = 0, prev_stages = kPfUnitStages;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
         {
-            // ---- decode, then epilogue
-            // A warp may touch only the 32 tensor-memory lanes of its quarter (warp % 4): the four decode warps of a
-            // quarter take its two strips x the chunk groups.
-            const int dw = warp - 2, qd = warp & 3, sub = (dw >> 2) & 1, half = dw >> 3, sidx = 2 * qd + sub;      // half = chunk group
-            const uint32_t tmem_a = tmem + ((uint32_t)(32 * qd + 16 * sub) << 16) + kPfAccCols;
-            const int64_t* row = a.table + (int64_t)ps.expert * kTableWidth;
-            const int level = (int)row[0];
+            if (!wait_head(nitem)) break;
+            const int64_t* row = sh->row[nitem & 1u];
+            const PfPass ps = sh->pass[nitem & 1u];
+            const int level = (int)row[0], wg = item % groups, nstages = unit_stages(ps.ntok);
             const ProjPlanes P = planes_from_row(row, a.down);
             const int rc = (int)row[10 + a.down], nm = a.down ? a.nm_dn : a.nm_gu, bk = (int)(row[19] >> (8 * a.down)) & 0xFF;
-            uint8_t* ring = rings + dw * kPfRingDepth * kStageBytes;
+            leave_head(nitem);
             // group `half` of 8 warps decodes the chunks c = half (mod kPfGroups): k-blocks 2 c and 2 c + 1.  The epilogue
             // of the previous item runs after this item's first unit is decoded: the MMAs of the previous item's last
             // k-blocks finish meanwhile, and the tensor pipe finds tiles waiting when the accumulator is free again.
-            auto mid = [&]() { if (have_prev) { epilogue(prev, prev_wg, prev_up, nitem - 1); have_prev = false; } };
-            const bool ok = decode_item(P, level, rc, bk, wg * 8 + sidx, C, NS, nm, lane, half, tmem_a, ring, sh, unit, mid);
-            unit += C;
+            auto mid = [&]() { if (prev_ntok) { pf_epilogue(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u); prev_ntok = 0; } };
+            const bool ok = decode_item(P, level, rc, bk, wg * 8 + sidx, C, NS, nm, lane, half, tmem_a, ring, sh, nstages, par_a,
+                                        nstages > prev_stages, (nitem - 1) & 1u, mid);
             mid();                                   // (an item of fewer than two chunks: its second warp group decodes nothing)
-            if (ok) { prev = ps; prev_wg = wg; prev_up = up; have_prev = true; }
+            prev_stages = nstages;
+            if (ok)
+            {
+                const bool up = !a.down && wg >= a.I / 128;
+                prev_out = (up ? a.out1 : a.out0) + (size_t)ps.row0 * ld + (up ? wg - a.I / 128 : wg) * 128;
+                prev_ntok = ps.ntok;
+            }
+            if (sh->abort_flag) break;
         }
-        if (sh->abort_flag) break;
+        if (prev_ntok && !sh->abort_flag) pf_epilogue(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
     }
-    if (warp >= 2 && have_prev && !sh->abort_flag) epilogue(prev, prev_wg, prev_up, nitem - 1);
+    __syncwarp();
     if (sh->abort_flag && threadIdx.x == 0) atomicExch(a.status, 1);
     tc_fence_before();
     __syncthreads();
