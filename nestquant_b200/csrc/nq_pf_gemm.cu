@@ -277,7 +277,7 @@ __device__ __forceinline__ int b_stages(int nbox) { return nbox <= 2 ? 8 : nbox 
 struct UnitSink
 {
     uint32_t tmem_a;      // tensor-memory address of the unit stage, at the warp's 16 lanes
-    PfShared* sh; uint32_t stage, parity; int lane; bool* ok; uint32_t* frag;      // frag: 16 registers
+    PfShared* sh; uint32_t stage, parity; bool deep; int lane; bool* ok; uint32_t* frag;      // frag: 16 registers
     template <int T>
     __device__ __forceinline__ void operator()(std::integral_constant<int, T>, const uint32_t (&a)[4]) const
     {
@@ -286,7 +286,19 @@ struct UnitSink
         frag[o] = a[0]; frag[o + 1] = a[2]; frag[o + 2] = a[1]; frag[o + 3] = a[3];
         if constexpr ((T & 3) == 3)
         {
-            if (*ok) *ok = mbar_wait_warp(saddr(&sh->empty_a[2 * stage + h]), parity ^ 1u, &sh->abort_flag);
+            // two units or more ahead of the MMAs (deep), both halves are nearly always free when the first is written: one vote and
+            // branch for the two; one unit ahead, the second half comes back while the first is decoded
+            if (h == 0 ? *ok : *ok && !deep)
+            {
+                const uint32_t bar = saddr(&sh->empty_a[2 * stage + h]);
+                uint32_t free = mbar_poll(bar, parity ^ 1u);
+                if (h == 0) free &= mbar_poll(deep ? bar + 8 : bar, parity ^ 1u);
+                if (__builtin_expect(!__all_sync(0xffffffffu, free), 0))
+                {
+                    *ok = mbar_wait_slow(bar, parity ^ 1u, &sh->abort_flag);
+                    if (h == 0 && *ok && deep) *ok = mbar_wait_slow(bar + 8, parity ^ 1u, &sh->abort_flag);
+                }
+            }
             tc_fence_after();
             // an aborted launch stores too (the columns are this CTA's until the end, the results are discarded) but signals nothing
             tmem_st_16x256b_x4(tmem_a + h * kPfACols, frag);
@@ -379,7 +391,7 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         RecordCursor<BK>::read(wb, st, lane);
         uint32_t frag[16];
         if (drain && i > 0 && ch < nstages && ok) ok = mbar_wait_warp(saddr(&sh->acc_empty), drain_parity, &sh->abort_flag);
-        const UnitSink sink{tmem_a - (uint32_t)stage * (2 * kPfACols), sh, (uint32_t)stage, (par_a >> stage) & 1u, lane, &ok, frag};
+        const UnitSink sink{tmem_a - (uint32_t)stage * (2 * kPfACols), sh, (uint32_t)stage, (par_a >> stage) & 1u, nstages > kPfGroups, lane, &ok, frag};
         par_a ^= 1u << stage;
         stage = stage + kPfGroups >= nstages ? group : stage + kPfGroups;
         bool refined = false;
@@ -409,6 +421,38 @@ __device__ __forceinline__ bool decode_item(const ProjPlanes& P, int level, int 
     NQ_WITH_CODES(level >= 4, rc, bk, 0x3FF, NQ_RUN);
 #undef NQ_RUN
     return ok;
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// The planes' first lines of an item to L2, an item ahead (by one warp, lane i holding word i of the expert's table row): what a decode
+// warp reads before its first unit (flags, signs, block words, two units' records of the widest sub-arrays) is a chain of dependent
+// loads that an item of few chunks cannot hide.  Every address lies inside the plane it belongs to.  1 % of a 1,000-token call.
+__device__ __forceinline__ void prefetch_item(bool level4, int64_t row_word, int down, int wg, int C, int nm, int lane)
+{
+    const int o = down ? 5 : 1;
+    const char* base = (const char*)__shfl_sync(0xffffffffu, row_word, o);
+    const char* p4 = (const char*)__shfl_sync(0xffffffffu, row_word, o + 1);
+    const char* d4 = (const char*)__shfl_sync(0xffffffffu, row_word, o + 2);
+    const char* flags = (const char*)__shfl_sync(0xffffffffu, row_word, o + 3);
+    const char* var = (const char*)__shfl_sync(0xffffffffu, row_word, down ? 13 : 12);
+    const int rc = (int)__shfl_sync(0xffffffffu, row_word, 10 + down), bk = (int)(__shfl_sync(0xffffffffu, row_word, 19) >> (8 * down)) & 0xFF;
+    // eight strips, four lanes each: 256 bytes of the strip's first 1,024 per lane
+    const int strip = wg * 8 + (lane >> 2), part = (lane & 3) * 256;
+    const size_t unit0 = (size_t)strip * C;
+    if (bk == 0 && C > 1) { prefetch_l2(base + unit0 * 512 + part); prefetch_l2(base + unit0 * 512 + part + 128); }
+    if (part == 0 && var) prefetch_l2(var + unit0);
+    if (level4)
+    {
+        const bool compact = flags != nullptr;
+        const int refined = compact ? nm : C;
+        const size_t res0 = (size_t)strip * refined;
+        if (part == 0 && compact) prefetch_l2(flags + (size_t)strip * 8);
+        if (refined > 1)
+        {
+            if (part == 0) prefetch_l2(d4 + res0 * 4);
+            if ((kWideCodes >> rc) & 1u) { prefetch_l2(p4 + res0 * 512 + part); prefetch_l2(p4 + res0 * 512 + part + 128); }
+        }
+    }
 }
 
 // A value that is the same in all lanes, as one that the compiler knows to be: what it cannot tell from a lane's own value (anything
@@ -464,6 +508,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const PfPass* pass = passes + item / groups;
             const int64_t w = lane < kTableWidth ? a.table[(int64_t)pass->expert * kTableWidth + lane] : 0;
             const uint32_t s = n & 1u;
+            prefetch_item(__shfl_sync(0xffffffffu, w, 0) >= 4, w, a.down, item % groups, C, a.down ? a.nm_dn : a.nm_gu, lane);
             if (!mbar_wait_warp(saddr(&sh->head_empty[s]), ((n >> 1) & 1u) ^ 1u, &sh->abort_flag)) return false;
             if (lane < kTableWidth) sh->row[s][lane] = w;
             if (lane == 0) sh->pass[s] = *pass;
