@@ -5,21 +5,26 @@
 //
 // One work item = (pass, 128-row weight group): a pass is one expert and up to 384 of its tokens.  Per item a CTA
 // walks K in blocks of 64:
-//   warp 0        TMA: the tokens' activation tile [ntok x 64] fp16 (SWIZZLE_128B boxes of 64 rows) -> shared memory
+//   warp 0        TMA: the tokens' activation tiles [ntok x 64] fp16 (SWIZZLE_128B boxes of 64 rows) -> shared memory; the pass
+//                 record and table row of the next item -> shared memory, the first lines of its planes -> L2
 //   warps 2..17   decode: a warp streams every other chunk of one strip with cp.async, decodes each unit in registers
 //                 (bit-exact fp16) and stores it with tcgen05.st as two weight tiles [128 x 64] in TENSOR MEMORY
 //                 (k-blocks 2 c and 2 c + 1): the m16n8k16-style fragment a lane holds is exactly what the 16x256b
 //                 store shape takes, so a tile costs one store per warp and no shared memory at all
 //   warp 1        one elected lane issues tcgen05.mma with the A operand in tensor memory (M 128 = weight rows, N =
 //                 tokens, K 16) into a [128 x 384] fp32 accumulator, also in tensor memory; tcgen05.commit frees the
-//                 stages.  Token tiles run 3..8 k-blocks ahead (160 KB), weight tiles 4 stages (32 columns each)
+//                 stages.  Token tiles run 3..8 k-blocks ahead (160 KB), weight tiles 2, 4 or 6 units of two (64 columns each),
+//                 as many as the accumulator of the pass leaves room for
 //   warps 2..17   epilogue: tcgen05.ld the accumulator and store fp32 rows acc[pair][128 columns] (coalesced); it runs
 //                 after the first unit of the CTA's next item has been decoded
 // A lane's fragment registers of a k-step hold k = 2 t4 + {0, 1} and 8 + 2 t4 + {0, 1}; stored side by side they make
 // the tile's k order inside every 16: position 4 i + {0, 1} = k 2 i + {0, 1}, position 4 i + {2, 3} = k 8 + 2 i + {0, 1}.
 // The activation matrices must be in the same order (nq_pf_pre / nq_pf_mid with kperm = 1).
 // Each decoded weight is used for every token of the pass, so decode cost is paid once per expert (for up to 384
-// tokens).  Tensor-pipe bound by intent; the decode instruction rate is the practical limit.
+// tokens).  Tensor-pipe bound by intent; the decode instruction rate is the practical limit.  With 31 tokens per expert a unit takes a
+// scheduler ~1,000 clocks at level 4 and ~640 at level 2; the decode warps of this kernel alone, without MMAs, need ~810 and ~480, a bare
+// loop of decode and tensor-memory store 658 and 388.  Warps 0 and 1 share their schedulers with four decode warps each, so what
+// their loops cost is instructions, branches and operand moves, not memory or tensor time: see mbar_wait_warp and uniform.
 // Every mbarrier wait is bounded: on time-out the CTA raises status[0], drains and returns.
 #include <cuda.h>
 
@@ -271,7 +276,7 @@ __device__ __forceinline__ int b_stages(int nbox) { return nbox <= 2 ? 8 : nbox 
 
 // A unit is decoded whole (8 k-steps) by one warp: k-steps 0..3 fill the weight tile of k-block 2 c, k-steps 4..7 the
 // tile of k-block 2 c + 1.  The sink keeps the fragments of four k-steps in registers and hands them over as one: wait until
-// the MMAs that last read the stage are done, one 32-column store, wait for the store, signal "full".  The four k-steps are
+// the MMAs that last read the stage are done, one 32-column store, and after the second half wait for the stores and signal "full".  The four k-steps are
 // one straight run of arithmetic with nothing to wait for in it (a store and a branch after every k-step cut the unit into
 // ten pieces that were scheduled one by one).
 struct UnitSink
