@@ -500,7 +500,7 @@ __device__ __forceinline__ void rotate_rows(const MoeArgs& a, const Shape& sh, c
             uint32_t xw[16], sw[16];
             load16w_mapH(a.x + (size_t)quot(s, a.topk) * a.H + blk * 128, q, xw);
             load16w_mapH_align8(R.scales[s] + (u ? 2 * a.H + 3 * a.I : 0) + blk * 128, q, sw);
-            mul32w_mapH(xw, sw, v);
+            mul32w(xw, sw, v);
         }
         else
 #pragma unroll

@@ -78,6 +78,7 @@ __device__ __forceinline__ PairHead pair_head(const TokenRows& rows, const int* 
     h.xr = token_row(rows, pt[p], H);
     return h;
 }
+template <bool WIDE>
 __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows rows, const int* __restrict__ pt, const int* __restrict__ pe,
                                                      const int64_t* __restrict__ table, int E, __half* xg, __half* xu, float* zg, int H, int I,
                                                      int kperm, int R)
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows
         uint32_t sg[16], su[16], xw[16];
         int have = -1;                               // expert whose scales sg / su hold
         PairHead cur = pair_head(rows, pt, pe, table, E, H, p0, p1);
-        if (cur.live && in_row) load16w_mapH(cur.xr + k, q, xw);
+        if (cur.live && in_row) load16w_mapW<WIDE>(cur.xr + k, q, xw);
         for (int p = p0; p < p1; ++p)
         {
             const PairHead nxt = pair_head(rows, pt, pe, table, E, H, p + 1, p1);
@@ -101,25 +102,23 @@ __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows
                 if (cur.e != have)
                 {
                     const __half* scales = (const __half*)cur.row[9];
-                    if (in_row) { load16w_mapH(scales + k, q, sg); load16w_mapH(scales + 2 * H + 3 * I + k, q, su); }
+                    if (in_row) { load16w_mapW<false>(scales + k, q, sg); load16w_mapW<false>(scales + 2 * H + 3 * I + k, q, su); }
                     have = cur.e;
                 }
                 float v[32];
-                if (in_row) mul32w_mapH(xw, sg, v);
+                if (in_row) mul32w(xw, sg, v);
                 else
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = 0.f;
                 wht128_x8(v, lane);
-                if (kperm) store32h_mapH_kperm(xg + (size_t)p * H + k, q, v, in_row);
-                else if (in_row) store32h_mapH(xg + (size_t)p * H + k, q, v);
-                if (in_row) mul32w_mapH(xw, su, v);
+                if (in_row) store32h_mapW<WIDE>(xg + (size_t)p * H + k, q, v, kperm);
+                if (in_row) mul32w(xw, su, v);
                 // the row is consumed: fetch the next pair's while the second half of this one is transformed
-                if (nxt.live && in_row) load16w_mapH(nxt.xr + k, q, xw);
+                if (nxt.live && in_row) load16w_mapW<WIDE>(nxt.xr + k, q, xw);
                 wht128_x8(v, lane);
-                if (kperm) store32h_mapH_kperm(xu + (size_t)p * H + k, q, v, in_row);
-                else if (in_row) store32h_mapH(xu + (size_t)p * H + k, q, v);
+                if (in_row) store32h_mapW<WIDE>(xu + (size_t)p * H + k, q, v, kperm);
             }
-            else if (nxt.live && in_row) load16w_mapH(nxt.xr + k, q, xw);
+            else if (nxt.live && in_row) load16w_mapW<WIDE>(nxt.xr + k, q, xw);
             cur = nxt;
         }
     }
@@ -148,6 +147,7 @@ __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows
 }
 
 // one CTA per pair, one warp per 1024 columns; dynamic shared memory: I floats (staging for the 512-wide rotation)
+template <bool WIDE>
 __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, const float* __restrict__ zg,
                                                      const int* __restrict__ pe, const int64_t* __restrict__ table, int E, __half* h, float* zd, int H, int I, int kperm)
 {
@@ -173,19 +173,19 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const floa
 #pragma unroll
         for (int up = 0; up < 2; ++up)
         {
-            if (live) load32f_mapF((up ? acc_u : acc_g) + (size_t)p * I + col, q, v);
+            if (live) load32f_mapH<WIDE>((up ? acc_u : acc_g) + (size_t)p * I + col, q, v);
             else
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = 0.f;
             wht128_x8(v, lane);
             if (live)
             {
-                scale32h_mapF((up ? sv_u : sv_g) + col, q, v);
+                scale32h_mapH((up ? sv_u : sv_g) + col, q, v);
                 for (int r = 0; r < L.rg; ++r)
                 {
                     const size_t o = (size_t)(up * L.rg + r) * I + col;
-                    axpy32h_mapF(L.lr + (size_t)L.rg * H + o, q, z[r], v);
-                    if (L.lr4) axpy32h_mapF(L.lr4 + o, q, z[r], v);
+                    axpy32h_mapH(L.lr + (size_t)L.rg * H + o, q, z[r], v);
+                    if (L.lr4) axpy32h_mapH(L.lr4 + o, q, z[r], v);
                 }
             }
             if (up == 0)
@@ -197,17 +197,15 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const floa
         for (int r = 0; r < L.rd; ++r)
         {
             float d = 0.f;
-            if (live) d = dot32h_mapF(L.lr + (size_t)L.rg * H + 2 * (size_t)L.rg * I + (size_t)r * I + col, q, v);
+            if (live) d = dot32h_mapH(L.lr + (size_t)L.rg * H + 2 * (size_t)L.rg * I + (size_t)r * I + col, q, v);
             d = quad_sum(d);
             if (live && (lane & 3) == 0) zpart[grp][r] = d;
         }
-        if (live) scale32h_mapF(su_d + col, q, v);
+        if (live) scale32h_mapH(su_d + col, q, v);
         wht128_x8(v, lane);
-        if (live)
-        {
-            if (hw <= 128) { if (kperm) store32h_mapF_kperm(h + (size_t)p * I + col, q, v); else store32h_mapF(h + (size_t)p * I + col, q, v); }
-            else store32f_mapF(stage + col, q, v);
-        }
+        if (hw > 128) { if (live) store32f_mapH<false>(stage + col, q, v); }
+        else if (kperm) store32h_mapH_kperm(h + (size_t)p * I + col, q, v, live);
+        else if (live) store32h_mapH(h + (size_t)p * I + col, q, v);
     }
     __syncthreads();
     if (threadIdx.x < 4)      // column groups added in order: the same sum whatever the launch shape
@@ -241,9 +239,10 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const floa
 
 // v = rw * (WHT128(y) * sv_o + z_dn (U2_d [+ U4_d])) for the lane's 32 output columns of the group at col of pair p (live lanes
 // only load and scale; every lane takes part in the rotation); false if the pair adds nothing (warp-uniform)
+template <bool WIDE>
 __device__ __forceinline__ bool pair_output(const float* __restrict__ y, const float* __restrict__ zd, int p, int e, float w,
                                             const int64_t* __restrict__ table, int H, int I, int col, bool live, int lane, float (&v)[32])
-// (col = first column of the lane's group, columns by map F)
+// (col = first column of the lane's group, columns by map H)
 {
     const int64_t* row = table + (int64_t)e * kTableWidth;
     const int level = (int)row[0];
@@ -251,20 +250,20 @@ __device__ __forceinline__ bool pair_output(const float* __restrict__ y, const f
     const __half* sv_o = (const __half*)row[9] + H + 3 * I;
     const LowRank L = low_rank_of(row, level);
     const int q = lane & 3;
-    if (live) load32f_mapF(y + (size_t)p * H + col, q, v);
+    if (live) load32f_mapH<WIDE>(y + (size_t)p * H + col, q, v);
     else
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = 0.f;
     wht128_x8(v, lane);
     if (live)
     {
-        scale32h_mapF(sv_o + col, q, v);
+        scale32h_mapH(sv_o + col, q, v);
         const size_t ou = (size_t)L.rg * H + 2 * (size_t)L.rg * I + (size_t)L.rd * I;
         for (int r = 0; r < L.rd; ++r)
         {
             const float z = zd[(size_t)p * 4 + r];
-            axpy32h_mapF(L.lr + ou + (size_t)r * H + col, q, z, v);
-            if (L.lr4) axpy32h_mapF(L.lr4 + 2 * (size_t)L.rg * I + (size_t)r * H + col, q, z, v);
+            axpy32h_mapH(L.lr + ou + (size_t)r * H + col, q, z, v);
+            if (L.lr4) axpy32h_mapH(L.lr4 + 2 * (size_t)L.rg * I + (size_t)r * H + col, q, z, v);
         }
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] *= w;
@@ -286,10 +285,10 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const flo
         float v[32];
         const int grp = g0 + (lane >> 2), col = grp * 128;
         const bool live = grp < ng;
-        if (!pair_output(y, zd, p, pe[p], w, table, H, I, col, live, lane, v)) return;   // CTA-uniform
+        if (!pair_output<false>(y, zd, p, pe[p], w, table, H, I, col, live, lane, v)) return;   // CTA-uniform
         if (live)
 #pragma unroll
-            for (int i = 0; i < 32; ++i) atomicAdd(op + col + 16 * (i >> 2) + 4 * (lane & 3) + (i & 3), v[i]);
+            for (int i = 0; i < 32; ++i) atomicAdd(op + col + 32 * (i >> 3) + 8 * (lane & 3) + (i & 7), v[i]);
     }
 }
 
@@ -298,6 +297,7 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const flo
 // accumulate = 0: out[t] is overwritten (zeros if the token has no pick in the window); 1: the sum is added to out[t], and
 // tokens without a pick in the window are not touched.  Calling it window after window in a fixed order gives a bitwise
 // repeatable result without a pairs-sized buffer.
+template <bool WIDE>
 __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_combine_kernel(const float* __restrict__ y, const float* __restrict__ zd, const int* __restrict__ pos,
                                                          const int64_t* __restrict__ sel, const __half* __restrict__ rw,
                                                          const int64_t* __restrict__ table, float* out, int topk, int E, int H, int I,
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_combine_kernel(const 
         const int grp = g0 + (lane >> 2), col = grp * 128;
         const bool live = grp < ng;
         float o[32];
-        if (accumulate && live) load32f_mapF(out + (size_t)t * H + col, lane & 3, o);
+        if (accumulate && live) load32f_mapH<WIDE>(out + (size_t)t * H + col, lane & 3, o);
         else
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[i] = 0.f;
@@ -326,13 +326,13 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_combine_kernel(const 
             const int p = pos[(size_t)t * topk + k] - pair0;
             if (e < 0 || e >= E || p < 0 || p >= npairs) continue;
             float v[32];
-            if (!pair_output(y, zd, p, (int)e, __half2float(rw[(size_t)t * topk + k]), table, H, I, col, live, lane, v))
+            if (!pair_output<WIDE>(y, zd, p, (int)e, __half2float(rw[(size_t)t * topk + k]), table, H, I, col, live, lane, v))
                 continue;
             if (live)
 #pragma unroll
                 for (int i = 0; i < 32; ++i) o[i] += v[i];
         }
-        if (live) store32f_mapF(out + (size_t)t * H + col, lane & 3, o);
+        if (live) store32f_mapH<WIDE>(out + (size_t)t * H + col, lane & 3, o);
     }
 }
 
@@ -342,7 +342,6 @@ __global__ void pf_hits_kernel(const int* __restrict__ counts, int* hits, int E)
     if (e < E && counts[e]) atomicAdd(hits + e, counts[e]);
 }
 
-// threads per CTA of the passes above: one warp per 1024 columns of the row, at most 8 warps
 // CTAs of pf_pre: enough to fill the device a few times over, each with a run of consecutive pairs
 static int pf_pre_grid(int R)
 {
@@ -352,6 +351,10 @@ static int pf_pre_grid(int R)
     const int want = (sms > 0 ? sms : 148) * NQ_PF_PRE_BLOCKS * 4;
     return R < want ? R : want;
 }
+// 32-byte accesses where the arrays allow them (every row is a multiple of 256 bytes: aligned if the first one is); an array that is
+// aligned to 16 only takes the same elements in two pieces, with the same results
+static bool aligned32(const void* p) { return ((uintptr_t)p & 31u) == 0; }
+// threads per CTA of the passes above: one warp per 1024 columns of the row, at most 8 warps
 static int pf_threads(int cols) { const int w = (cols + 1023) / 1024; return 32 * (w > 8 ? 8 : w); }
 
 }  // namespace nq
@@ -371,7 +374,9 @@ int nq_pf_pre(const void* x, const int32_t* pt, const int32_t* pe, int R, const 
     NQ_REQUIRE(nq::aligned16(x) && nq::aligned16(xg) && nq::aligned16(xu), "nq_pf_pre: x, xg, xu must be 16-byte aligned");
     nq::TokenRows rows{};
     rows.base[0] = (const __half*)x; rows.tokens_per_rank = 0x7fffffff;
-    nq::pf_pre_kernel<<<nq::pf_pre_grid(R), nq::pf_threads(H), 0, (cudaStream_t)stream>>>(rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
+    const bool wide = nq::aligned32(x) && nq::aligned32(xg) && nq::aligned32(xu);
+    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R), nq::pf_threads(H), 0, (cudaStream_t)stream>>>(
+        rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
     return nq::check_launch("nq_pf_pre");
 }
 
@@ -386,13 +391,16 @@ int nq_pf_pre_ep(const void* const* peer_x, int world, int tokens_per_rank, cons
     NQ_REQUIRE(E >= 1, "nq_pf_pre_ep: E = %d", E);
     NQ_REQUIRE(nq::aligned16(xg) && nq::aligned16(xu), "nq_pf_pre_ep: xg, xu must be 16-byte aligned");
     nq::TokenRows rows{};
+    bool wide = nq::aligned32(xg) && nq::aligned32(xu);
     for (int r = 0; r < world; ++r)
     {
         NQ_REQUIRE(peer_x[r] && nq::aligned16(peer_x[r]), "nq_pf_pre_ep: input buffer of rank %d is null or misaligned", r);
         rows.base[r] = (const __half*)peer_x[r];
+        wide = wide && nq::aligned32(peer_x[r]);
     }
     rows.tokens_per_rank = tokens_per_rank;
-    nq::pf_pre_kernel<<<nq::pf_pre_grid(R), nq::pf_threads(H), 0, (cudaStream_t)stream>>>(rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
+    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R), nq::pf_threads(H), 0, (cudaStream_t)stream>>>(
+        rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
     return nq::check_launch("nq_pf_pre_ep");
 }
 
@@ -405,7 +413,8 @@ int nq_pf_mid(const float* acc_g, const float* acc_u, const float* zg, const int
     NQ_SHAPE_OK("nq_pf_mid");
     NQ_REQUIRE(E >= 1, "nq_pf_mid: E = %d", E);
     NQ_REQUIRE(nq::aligned16(acc_g) && nq::aligned16(acc_u) && nq::aligned16(h), "nq_pf_mid: acc_g, acc_u, h must be 16-byte aligned");
-    nq::pf_mid_kernel<<<R, nq::pf_threads(I), (size_t)I * 4, (cudaStream_t)stream>>>(acc_g, acc_u, zg, pe, table, E, (__half*)h, zd, H, I, kperm);
+    (nq::aligned32(acc_g) && nq::aligned32(acc_u) ? nq::pf_mid_kernel<true> : nq::pf_mid_kernel<false>)<<<R, nq::pf_threads(I), (size_t)I * 4, (cudaStream_t)stream>>>(
+        acc_g, acc_u, zg, pe, table, E, (__half*)h, zd, H, I, kperm);
     return nq::check_launch("nq_pf_mid");
 }
 
@@ -431,7 +440,8 @@ int nq_pf_combine(const float* y, const float* zd, const int32_t* pos, const int
     NQ_REQUIRE(y && zd && pos && sel && rw && table && out, "nq_pf_combine: null pointer");
     NQ_SHAPE_OK("nq_pf_combine");
     NQ_REQUIRE(nq::aligned16(y) && nq::aligned16(out), "nq_pf_combine: y and out must be 16-byte aligned");
-    nq::pf_combine_kernel<<<T, nq::pf_threads(H), 0, (cudaStream_t)stream>>>(y, zd, pos, sel, (const __half*)rw, table, out, topk, E, H, I, pair0, npairs, accumulate);
+    (nq::aligned32(y) && nq::aligned32(out) ? nq::pf_combine_kernel<true> : nq::pf_combine_kernel<false>)<<<T, nq::pf_threads(H), 0, (cudaStream_t)stream>>>(
+        y, zd, pos, sel, (const __half*)rw, table, out, topk, E, H, I, pair0, npairs, accumulate);
     return nq::check_launch("nq_pf_combine");
 }
 

@@ -101,23 +101,85 @@ __device__ __forceinline__ void wht128_x8(float (&v)[32], int lane)
 }
 // Which 32 elements of its vector a lane holds is free (any assignment of the 7 index bits to 5 register bits and 2
 // lane bits gives the same transform), so it is chosen for coalescing: the 4 lanes of a vector access adjacent pieces.
-//   map H (fp16 arrays, 16-byte accesses): register 8 j + e of lane q = element 32 j + 8 q + e   (j < 4, e < 8)
-//   map F (fp32 arrays, 16-byte accesses; fp16 vectors alongside them by 8-byte accesses):
-//                                          register 4 j + e of lane q = element 16 j + 4 q + e   (j < 8, e < 4)
+//   map H (fp16 arrays, 16-byte accesses; fp32 arrays, 32-byte accesses):
+//                                          register 8 j + e of lane q = element 32 j + 8 q + e   (j < 4, e < 8)
+//   map W (fp16 arrays, 32-byte accesses): register 16 j + e of lane q = element 64 j + 16 q + e (j < 2, e < 16)
+// With 32 bytes per lane the four lanes of a vector cover one 128-byte line per access; with 16 (or 8) an access of the warp touches
+// eight lines and half (or a quarter) of each.  WIDE: the array is aligned to 32 bytes; else the same elements go as two 16-byte pieces.
+// 65,536 pairs of 6,144 (2,048) columns, us, 16 or 8 bytes per lane / 32: first pass 573 / 525 (it also writes the GEMM's k order without
+// an exchange between lanes), middle pass 455 / 412, last pass 435 / 421.
 // p points at the vector's first element, q = lane & 3.
-__device__ __forceinline__ void load32h_mapH(const __half* p, int q, float (&f)[32])
+template <bool WIDE>
+__device__ __forceinline__ void load32b(const void* p, uint32_t* w)
+{
+    if constexpr (WIDE)
+        asm("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"      // (its users read what an earlier launch has written)
+            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
+    else
+    {
+        const uint4 a = ((const uint4*)p)[0], b = ((const uint4*)p)[1];
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    }
+}
+template <bool WIDE>
+__device__ __forceinline__ void store32b(void* p, const uint32_t* w)
+{
+    if constexpr (WIDE)
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                     ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+    else
+    {
+        ((uint4*)p)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        ((uint4*)p)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+template <bool WIDE>
+__device__ __forceinline__ void load32f_mapH(const float* p, int q, float (&f)[32])
 {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
     {
-        const uint4 u = *(const uint4*)(p + 32 * j + 8 * q);
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        uint32_t w[8];
+        load32b<WIDE>(p + 32 * j + 8 * q, w);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int e = 0; e < 8; ++e) f[8 * j + e] = __uint_as_float(w[e]);
+    }
+}
+template <bool WIDE>
+__device__ __forceinline__ void store32f_mapH(float* p, int q, const float (&v)[32])
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+        uint32_t w[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(v[8 * j + e]);
+        store32b<WIDE>(p + 32 * j + 8 * q, w);
+    }
+}
+template <bool WIDE>
+__device__ __forceinline__ void load16w_mapW(const __half* p, int q, uint32_t (&w)[16])
+{
+#pragma unroll
+    for (int j = 0; j < 2; ++j) load32b<WIDE>(p + 64 * j + 16 * q, w + 8 * j);
+}
+// kperm: the k order of the fused prefill GEMM (below); a lane holds whole groups of 16, so it is a choice of words
+template <bool WIDE>
+__device__ __forceinline__ void store32h_mapW(__half* p, int q, const float (&v)[32], bool kperm)
+{
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+    {
+        uint32_t w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
         {
-            const __half2 h = *(const __half2*)&w[i];
-            f[8 * j + 2 * i] = __low2float(h); f[8 * j + 2 * i + 1] = __high2float(h);
+            const __half2 h = __floats2half2_rn(v[16 * j + 2 * i], v[16 * j + 2 * i + 1]);
+            w[i] = *(const uint32_t*)&h;
         }
+        const uint32_t o[8] = {w[0], kperm ? w[4] : w[1], kperm ? w[1] : w[2], kperm ? w[5] : w[3],
+                               kperm ? w[2] : w[4], kperm ? w[6] : w[5], kperm ? w[3] : w[6], w[7]};
+        store32b<WIDE>(p + 64 * j + 16 * q, o);
     }
 }
 __device__ __forceinline__ void store32h_mapH(__half* p, int q, const float (&v)[32])
@@ -135,41 +197,6 @@ __device__ __forceinline__ void store32h_mapH(__half* p, int q, const float (&v)
         *(uint4*)(p + 32 * j + 8 * q) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
-__device__ __forceinline__ void load32f_mapF(const float* p, int q, float (&f)[32])
-{
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-    {
-        const float4 u = *(const float4*)(p + 16 * j + 4 * q);
-        f[4 * j] = u.x; f[4 * j + 1] = u.y; f[4 * j + 2] = u.z; f[4 * j + 3] = u.w;
-    }
-}
-__device__ __forceinline__ void store32f_mapF(float* p, int q, const float (&v)[32])
-{
-#pragma unroll
-    for (int j = 0; j < 8; ++j) *(float4*)(p + 16 * j + 4 * q) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-}
-__device__ __forceinline__ void load32h_mapF(const __half* p, int q, float (&f)[32])
-{
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-    {
-        const uint2 u = *(const uint2*)(p + 16 * j + 4 * q);
-        const __half2 a = *(const __half2*)&u.x, b = *(const __half2*)&u.y;
-        f[4 * j] = __low2float(a); f[4 * j + 1] = __high2float(a); f[4 * j + 2] = __low2float(b); f[4 * j + 3] = __high2float(b);
-    }
-}
-__device__ __forceinline__ void store32h_mapF(__half* p, int q, const float (&v)[32])
-{
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-    {
-        const __half2 a = __floats2half2_rn(v[4 * j], v[4 * j + 1]), b = __floats2half2_rn(v[4 * j + 2], v[4 * j + 3]);
-        uint2 u; u.x = *(const uint32_t*)&a; u.y = *(const uint32_t*)&b;
-        *(uint2*)(p + 16 * j + 4 * q) = u;
-    }
-}
-
 // k-permuted fp16 stores for the fused prefill GEMM, whose decode warps write weight fragments to tensor memory in
 // their register order: inside every group of 16 consecutive k, position 4 i + {0, 1} holds k = 2 i + {0, 1} and
 // position 4 i + {2, 3} holds k = 8 + 2 i + {0, 1} (i = 0 .. 3).
@@ -196,20 +223,6 @@ __device__ __forceinline__ void store32h_mapH_kperm(__half* p, int q, const floa
         if (live) *(uint4*)(p + 32 * j + 16 * (q >> 1) + 8 * (q & 1)) = o;      // every lane takes part in the exchange above
     }
 }
-// map F: lane q holds k = 4 q .. 4 q + 3 of the 16-group j: two packed words that land at two places
-__device__ __forceinline__ void store32h_mapF_kperm(__half* p, int q, const float (&v)[32])
-{
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-    {
-        const __half2 a = __floats2half2_rn(v[4 * j], v[4 * j + 1]), b = __floats2half2_rn(v[4 * j + 2], v[4 * j + 3]);
-        // k = 4 q + {0,1} -> pair index i = 2 q (mod 4) in half (q >> 1); k = 4 q + {2,3} -> i = 2 q + 1
-        const int half = q >> 1, i0 = (2 * q) & 3;
-        uint32_t* g = (uint32_t*)(p + 16 * j);
-        g[2 * i0 + half] = *(const uint32_t*)&a;
-        g[2 * (i0 + 1) + half] = *(const uint32_t*)&b;
-    }
-}
 // the same permutation for a lane holding 4 consecutive k (element 4 * lane + i of a 128-vector)
 __device__ __forceinline__ void store4h_kperm(__half* vec, int lane, const float (&v)[4])
 {
@@ -220,7 +233,8 @@ __device__ __forceinline__ void store4h_kperm(__half* vec, int lane, const float
     g[2 * (i0 + 1) + half] = *(const uint32_t*)&b;
 }
 
-// fused forms (no staging array): v = x * s for packed fp16 x (map H); v *= s, v += z * s, sum v * s for an fp16 vector s (map F)
+// fused forms (no staging array): v = x * s for packed fp16 x (map H); v *= s, v += z * s, sum v * s for an fp16 vector s (map H,
+// aligned to 8 bytes)
 __device__ __forceinline__ void load16w_mapH(const __half* p, int q, uint32_t (&w)[16])
 {
 #pragma unroll
@@ -240,8 +254,8 @@ __device__ __forceinline__ void load16w_mapH_align8(const __half* p, int q, uint
         w[2 * j] = u.x; w[2 * j + 1] = u.y;
     }
 }
-// v = x * s for the lane's 32 elements, both given as the packed fp16 words of map H (fp32 products)
-__device__ __forceinline__ void mul32w_mapH(const uint32_t (&xw)[16], const uint32_t (&sw)[16], float (&v)[32])
+// v = x * s for the lane's 32 elements, both given as packed fp16 words of one map (fp32 products)
+__device__ __forceinline__ void mul32w(const uint32_t (&xw)[16], const uint32_t (&sw)[16], float (&v)[32])
 {
 #pragma unroll
     for (int i = 0; i < 16; ++i)
@@ -251,22 +265,22 @@ __device__ __forceinline__ void mul32w_mapH(const uint32_t (&xw)[16], const uint
     }
 }
 template <class F>
-__device__ __forceinline__ void each32h_mapF(const __half* p, int q, F&& f)
+__device__ __forceinline__ void each32h_mapH(const __half* p, int q, F&& f)
 {
 #pragma unroll
     for (int j = 0; j < 8; ++j)
     {
-        const uint2 u = *(const uint2*)(p + 16 * j + 4 * q);
+        const uint2 u = *(const uint2*)(p + 32 * (j >> 1) + 8 * q + 4 * (j & 1));
         const __half2 a = *(const __half2*)&u.x, b = *(const __half2*)&u.y;
         f(4 * j, __low2float(a)); f(4 * j + 1, __high2float(a)); f(4 * j + 2, __low2float(b)); f(4 * j + 3, __high2float(b));
     }
 }
-__device__ __forceinline__ void scale32h_mapF(const __half* p, int q, float (&v)[32]) { each32h_mapF(p, q, [&](int i, float s) { v[i] *= s; }); }
-__device__ __forceinline__ void axpy32h_mapF(const __half* p, int q, float z, float (&v)[32]) { each32h_mapF(p, q, [&](int i, float s) { v[i] += z * s; }); }
-__device__ __forceinline__ float dot32h_mapF(const __half* p, int q, const float (&v)[32])
+__device__ __forceinline__ void scale32h_mapH(const __half* p, int q, float (&v)[32]) { each32h_mapH(p, q, [&](int i, float s) { v[i] *= s; }); }
+__device__ __forceinline__ void axpy32h_mapH(const __half* p, int q, float z, float (&v)[32]) { each32h_mapH(p, q, [&](int i, float s) { v[i] += z * s; }); }
+__device__ __forceinline__ float dot32h_mapH(const __half* p, int q, const float (&v)[32])
 {
     float d = 0.f;
-    each32h_mapF(p, q, [&](int i, float s) { d += v[i] * s; });
+    each32h_mapH(p, q, [&](int i, float s) { d += v[i] * s; });
     return d;
 }
 
