@@ -342,13 +342,21 @@ __global__ void pf_hits_kernel(const int* __restrict__ counts, int* hits, int E)
     if (e < E && counts[e]) atomicAdd(hits + e, counts[e]);
 }
 
-// CTAs of pf_pre: enough to fill the device a few times over, each with a run of consecutive pairs
-static int pf_pre_grid(int R)
+// pf_pre: a warp per 1,024 columns up to three, two rounds of half as many beyond.  At 128 registers an SM holds 512 threads: two CTAs of
+// six warps (H = 6,144) leave a quarter of them out, five of three do not.  CTAs: enough to fill the device a few times over, each
+// with a run of consecutive pairs (the runs of pairs that belong to no resident expert end at once, so more CTAs also balance better).
+// us, one round / two: 8,000 pairs 78 / 70, 24,008 of which a quarter is live 185 / 87, 65,536 525 / 482.
+static int pf_pre_threads(int cols)
+{
+    const int w = (cols + 1023) / 1024;
+    return 32 * (w > 3 ? (w + 1) / 2 : w);
+}
+static int pf_pre_grid(int R, int H)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int want = (sms > 0 ? sms : 148) * NQ_PF_PRE_BLOCKS * 4;
+    const int want = (sms > 0 ? sms : 148) * (256 * NQ_PF_PRE_BLOCKS / pf_pre_threads(H)) * 4;
     return R < want ? R : want;
 }
 // 32-byte accesses where the arrays allow them (every row is a multiple of 256 bytes: aligned if the first one is); an array that is
@@ -375,7 +383,7 @@ int nq_pf_pre(const void* x, const int32_t* pt, const int32_t* pe, int R, const 
     nq::TokenRows rows{};
     rows.base[0] = (const __half*)x; rows.tokens_per_rank = 0x7fffffff;
     const bool wide = nq::aligned32(x) && nq::aligned32(xg) && nq::aligned32(xu);
-    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R), nq::pf_threads(H), 0, (cudaStream_t)stream>>>(
+    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R, H), nq::pf_pre_threads(H), 0, (cudaStream_t)stream>>>(
         rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
     return nq::check_launch("nq_pf_pre");
 }
@@ -399,7 +407,7 @@ int nq_pf_pre_ep(const void* const* peer_x, int world, int tokens_per_rank, cons
         wide = wide && nq::aligned32(peer_x[r]);
     }
     rows.tokens_per_rank = tokens_per_rank;
-    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R), nq::pf_threads(H), 0, (cudaStream_t)stream>>>(
+    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R, H), nq::pf_pre_threads(H), 0, (cudaStream_t)stream>>>(
         rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
     return nq::check_launch("nq_pf_pre_ep");
 }
