@@ -13,8 +13,9 @@
 //                 store shape takes, so a tile costs one store per warp and no shared memory at all
 //   warp 1        one elected lane issues tcgen05.mma with the A operand in tensor memory (M 128 = weight rows, N =
 //                 tokens, K 16) into a [128 x 384] fp32 accumulator, also in tensor memory; tcgen05.commit frees the
-//                 stages.  Token tiles run 3..8 k-blocks ahead (160 KB), weight tiles 2, 4 or 6 units of two (64 columns each),
-//                 as many as the accumulator of the pass leaves room for
+//                 stages.  Token tiles run 2 or 4 chunks of two k-blocks ahead, 3 k-blocks in passes of more than 320 tokens
+//                 (160 KB), weight tiles 2, 4 or 6 units of two (64 columns each), as many as the accumulator of the pass leaves
+//                 room for
 //   warps 2..17   epilogue: tcgen05.ld the accumulator and store fp32 rows acc[pair][128 columns] (coalesced); it runs
 //                 after the first unit of the CTA's next item has been decoded
 // A lane's fragment registers of a k-step hold k = 2 t4 + {0, 1} and 8 + 2 t4 + {0, 1}; stored side by side they make
@@ -153,6 +154,16 @@ __device__ __forceinline__ void tma_load_more_elect(uint32_t dst0, uint32_t dst1
                  "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%6];\n\t}"
                  ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar0), "r"(bar1) : "memory");
 }
+// The boxes of one k-block, one below the other.
+__device__ __forceinline__ void tma_load_kblock_elect(uint32_t dst, const CUtensorMap* map, int x, int y, int nbox, uint32_t bar)
+{
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
+                 ::"r"(bar), "r"((uint32_t)(nbox * kPfBoxBytes)) : "memory");
+    for (int j = 0; j < nbox; ++j)
+        asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                     "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
+                     ::"r"(dst + j * kPfBoxBytes), "l"(map), "r"(x), "r"(y + j * kPfBoxRows), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit_elect(uint64_t* bar)
@@ -273,6 +284,12 @@ __device__ __forceinline__ int unit_stages(int ntok) { return ntok <= 128 ? 6 : 
 // stage of the old layout has been released.
 __device__ __forceinline__ int b_stage_boxes(int nbox) { return nbox <= 2 ? 2 : nbox <= 4 ? 4 : nbox <= 5 ? 5 : 6; }
 __device__ __forceinline__ int b_stages(int nbox) { return nbox <= 2 ? 8 : nbox <= 4 ? 5 : nbox <= 5 ? 4 : 3; }
+// Producer and MMA warp take the stages two at a time, the two k-blocks of a chunk at one wait, except where there are only three (passes
+// of more than 320 tokens): there a pair would come free only with the last k-block but one multiplied, and its load would find nothing
+// to hide behind.  16 experts x 384 tokens, H 6,144, I 2,048, us, pairs / one by one: gate|up 378 / 250 at level 2, 387 / 277 at level 4,
+// down 193 / 146 and 205 / 173 (the kernel that took every pass one by one: 277, 301, 166, 187).  (A poll does not help: try_wait may wait itself, so the second one of a pair does.)  Four stages one by
+// one: gate|up of 320 tokens 237 / 211 at level 2, 257 / 262 at level 4; five: 160 tokens 167 / 172 and 224 / 224.
+__device__ __forceinline__ bool stages_one_by_one(int nbox) { return b_stages(nbox) == 3; }
 
 // A unit is decoded whole (8 k-steps) by one warp: k-steps 0..3 fill the weight tile of k-block 2 c, k-steps 4..7 the
 // tile of k-block 2 c + 1.  The sink keeps the fragments of four k-steps in registers and hands them over as one: wait until
@@ -507,7 +524,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     // token-tile stage s was used (how many stages there are changes from pass to pass).
     if (warp == 0)
     {
-        // ---- token tiles by TMA, up to nb k-blocks ahead of the MMAs; pass record and table row of the items, one item ahead
+        // ---- token tiles by TMA, ahead of the MMAs as far as there are stages; pass record and table row of the items, one item ahead
         auto publish = [&](int item, uint32_t n) {
             if (item >= nitems) return true;
             const PfPass* pass = passes + item / groups;
@@ -536,6 +553,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
             last_sbox = sbox;
             const uint32_t tiles0 = saddr(b_tiles), bytes = (uint32_t)nbox * kPfBoxBytes, step = (uint32_t)sbox * kPfBoxBytes;
+            if (stages_one_by_one(nbox))
+                for (int kb = 0, s = 0; ok && kb < 2 * C; ++kb, s = s + 1 == nb ? 0 : s + 1)
+                {
+                    ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
+                    if (!ok) break;
+                    par_b ^= 1u << s;
+                    tma_load_kblock_elect(tiles0 + s * step, map, kb * 64, row0, nbox, full_b0 + 8 * s);
+                }
+            else
             for (int c = 0, s = 0; ok && c < C; ++c)
             {
                 const int s1 = s + 1 == nb ? 0 : s + 1;
@@ -575,6 +601,21 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const uint32_t b_lo0 = (uint32_t)bdesc0, b_hi = (uint32_t)(bdesc0 >> 32);
             const uint32_t b_step = (uint32_t)(sbox * (kPfBoxBytes >> 4));
             uint32_t s = 0, b_lo = b_lo0;                 // token-tile stage of this k-block and its descriptor
+            if (stages_one_by_one(nbox))
+                for (uint32_t kb = 0; ok && kb < 2u * C; ++kb)
+                {
+                    const uint32_t ua = (kb >> 1) & 1u, h = kb & 1u;           // (two unit stages, two column halves)
+                    ok = (h || mbar_wait_warp(full_a0 + 8 * ua, (par_a >> ua) & 1u, &sh->abort_flag)) &&
+                         mbar_wait_warp(full_b0 + 8 * s, (par_b >> s) & 1u, &sh->abort_flag);
+                    if (!ok) break;
+                    par_a ^= h << ua;
+                    par_b ^= 1u << s;
+                    tc_fence_after();
+                    tc_mma_kblock2(tmem, tmem + n0, tmem + kPfTmemCols - 2 * kPfACols - ua * (2 * kPfACols) + h * kPfACols, b_lo, b_lo + (uint32_t)(n0 * 8),
+                                   b_hi, idesc0, idesc1, kb, empty_a0 + 16 * ua + 8 * h, empty_b0 + 8 * s);
+                    if (++s == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else b_lo += b_step;
+                }
+            else
             for (int c = 0, ua = 0; ok && c < C; ++c, ua = ua + 1 == nstages ? 0 : ua + 1)
             {
                 // the unit and its two token tiles: three polls, one vote, one branch
