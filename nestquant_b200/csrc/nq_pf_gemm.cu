@@ -337,8 +337,8 @@ struct UnitSink
 
 // Decode warps: accumulator [128 weight rows x ntok] of an item -> out (row of the item's first token, column of the weight group's
 // first row).  TMEM lanes 32 q .. 32 q + 31 (the quarter this warp may read) are weight rows; the four warps of a quarter take
-// 32-column chunks in turn.  Not inlined: it runs in the middle of a decode loop whose registers are all taken.
-__device__ __noinline__ void pf_epilogue(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
+// 32-column chunks in turn.
+__device__ __forceinline__ void write_accumulator(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (!mbar_wait_warp(saddr(&sh->acc_full), parity, &sh->abort_flag)) return;
@@ -356,6 +356,14 @@ __device__ __noinline__ void pf_epilogue(PfShared* sh, uint32_t tmem, float* out
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh->acc_empty);
+}
+// Between two units it is a call, because the registers of the decode loop are all taken there; after the last unit it is in line.  A warp
+// with one unit per item has no other place for it than after that unit, and every item pays what the call costs: 128 experts x 31
+// tokens, H 6,144, down projection of 256 columns, us, call / in line: 153 / 122 at level 2, 225 / 187 at level 4.  In line between units
+// too, down projection of 2,048 columns, 64 experts: 255 / 246 and 404 / 415.
+__device__ __noinline__ void write_accumulator_between(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
+{
+    write_accumulator(sh, tmem, out, ld, ntok, parity);
 }
 
 // One decode warp, one item: its strip over the chunks c = GROUP, GROUP + 2, ... (the other group of 8 warps takes the
@@ -426,7 +434,7 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         }
         else
             decode_unit<false, 0, BK>(wb, wr, consts_level2(sign2), lane, sink);
-        if (i == 0) mid();      // the previous item's epilogue, once this item's first tiles are on their way
+        if (i == 0 && ch + kPfGroups < C) mid();      // the previous item's epilogue, once this item's first tiles are on their way
     }
     cp_async_wait<0>();
     return ok;
@@ -675,10 +683,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             // group `half` of 8 warps decodes the chunks c = half (mod kPfGroups): k-blocks 2 c and 2 c + 1.  The epilogue
             // of the previous item runs after this item's first unit is decoded: the MMAs of the previous item's last
             // k-blocks finish meanwhile, and the tensor pipe finds tiles waiting when the accumulator is free again.
-            auto mid = [&]() { if (prev_ntok) { pf_epilogue(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u); prev_ntok = 0; } };
+            auto mid = [&]() { if (prev_ntok) { write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u); prev_ntok = 0; } };
             const bool ok = decode_item(P, level, rc, bk, wg * 8 + sidx, C, NS, nm, lane, half, tmem_a, ring, sh, nstages, par_a,
                                         nstages > prev_stages, (nitem - 1) & 1u, mid);
-            mid();                                   // (an item of fewer than two chunks: its second warp group decodes nothing)
+            if (prev_ntok) { write_accumulator(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u); prev_ntok = 0; }     // (one unit or none)
             prev_stages = nstages;
             if (ok)
             {
@@ -688,7 +696,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             }
             if (sh->abort_flag) break;
         }
-        if (prev_ntok && !sh->abort_flag) pf_epilogue(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
+        if (prev_ntok && !sh->abort_flag) write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
     }
     __syncwarp();
     if (sh->abort_flag && threadIdx.x == 0) atomicExch(a.status, 1);

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 COUNTS = [384, 1, 128, 300, 129, 64, 256, 65, 385, 20, 257, 0, 127, 383, 16]
 
 
-@pytest.mark.parametrize("H,I", [(128, 2048), (384, 2048), (2048, 128), (2048, 1664)])
+@pytest.mark.parametrize("H,I", [(128, 2048), (256, 2048), (384, 2048), (2048, 128), (2048, 256), (2048, 1664)])
 def test_passes_of_every_width_in_turn(H, I):
     E, T = len(COUNTS), sum(COUNTS)
     # 16 passes x 32 (or 16) weight groups of a projection: every CTA takes several items, of passes that lie apart in the list
