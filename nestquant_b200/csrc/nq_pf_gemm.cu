@@ -74,38 +74,12 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(bar)), "r"(bytes) : "memory");
-}
-// bounded wait for the phase with the given parity; false = aborted (by this or another thread of the CTA)
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag)
-{
-    const uint32_t a = saddr(bar);
-    unsigned long long t0 = 0;
-    for (uint32_t i = 0;; ++i)
-    {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-        if (ok) return true;
-        if (*abort_flag) return false;
-        if ((i & 255u) == 255u)
-        {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > kPfWaitNs) break;
-        }
-    }
-    *abort_flag = 1;
-    return false;
-}
 // The producer and MMA warps run their loops with all 32 lanes converged (so that addresses, descriptors and
 // coordinates are warp-uniform values) and one elected lane issues the asynchronous instruction.
 // Waits of a whole warp, `bar` a shared-space address.  What a wait costs that finds its phase complete is the branches around the
 // poll, not the poll: 200 to 240 clocks as a loop (beside 16 busy warps), 95 as a poll, a vote and a branch that falls through, 15
 // the poll alone.  So the poll that nearly always succeeds stands in line and the bounded loop behind a call.
+// A wait returns false if it has run out, here or in another warp of the CTA.
 __device__ __forceinline__ uint32_t mbar_poll(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
