@@ -138,6 +138,8 @@ int nq_pf_combine(const float* y, const float* zd, const int32_t* pos, const int
  *                nq_pf_pre / nq_pf_mid write with kperm = 1.  Rows of pairs whose expert is not resident are not
  *                written.  status: int32 [1] on the device, set to 1 if a device-side wait timed out (bounded waits;
  *                the outputs are then invalid) - read it after synchronising.
+ *   nq_pf_gemm_within   the same with a limit of its own for every wait (ns; nq_pf_gemm: 2 s).  A launch whose wait runs out ends all
+ *                the same: it waits for its own loads and MMAs in flight and gives its tensor memory back.
  *   nq_pf_plan_window   the same from nq_pf_sort's start array for the pairs [pair0, pair0 + npairs) of the sorted list
  *                (rows counted from pair0): the pass list of one scratch chunk. */
 int nq_pf_plan_ints(int E, int pairs);
@@ -146,6 +148,8 @@ int nq_pf_plan_window(const int32_t* start, const int64_t* table, int E, int pai
 int nq_pf_plan(const int32_t* counts, const int64_t* table, int E, int pairs, int32_t* plan, int plan_ints, void* stream);
 int nq_pf_gemm(const int64_t* table, const int32_t* plan, const void* act0, const void* act1, int pairs, float* out0, float* out1,
                int H, int I, int nm_gu, int nm_dn, int down, int32_t* status, void* stream);
+int nq_pf_gemm_within(const int64_t* table, const int32_t* plan, const void* act0, const void* act1, int pairs, float* out0, float* out1,
+                      int H, int I, int nm_gu, int nm_dn, int down, int32_t* status, long long wait_ns, void* stream);
 
 /* hits[e] += counts[e] (hits may be host-mapped; NULL = no-op).  Replaces pf_hits() (sm120/nqmoe.cu:1241-1245,1288-1293). */
 int nq_pf_hits(const int32_t* counts, int32_t* hits, int E, void* stream);

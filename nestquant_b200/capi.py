@@ -71,6 +71,7 @@ SIGNATURES = {
     "nq_pf_plan_ints": (_i, [_i, _i]),
     "nq_pf_plan": (_i, [_p, _p, _i, _i, _p, _i, _p]),
     "nq_pf_gemm": (_i, [_p, _p, _p, _p, _i, _p, _p, _i, _i, _i, _i, _i, _p, _p]),
+    "nq_pf_gemm_within": (_i, [_p, _p, _p, _p, _i, _p, _p, _i, _i, _i, _i, _i, _p, C.c_longlong, _p]),
     "nq_moe_workspace": (_i, [_i, _i, _i, _i, _i, _i, C.POINTER(NqMoeWorkspace)]),
     "nq_moe_forward": (_i, [C.POINTER(NqMoeForward), _p]),
     "nq_moe_forward_ep": (_i, [C.POINTER(NqMoeForward), C.POINTER(NqMoeEp), _p]),

@@ -26,7 +26,8 @@
 // scheduler ~1,000 clocks at level 4 and ~640 at level 2; the decode warps of this kernel alone, without MMAs, need ~810 and ~480, a bare
 // loop of decode and tensor-memory store 658 and 388.  Warps 0 and 1 share their schedulers with four decode warps each, so what
 // their loops cost is instructions, branches and operand moves, not memory or tensor time: see mbar_wait_warp and uniform.
-// Every mbarrier wait is bounded: on time-out the CTA raises status[0], drains and returns.
+// Every mbarrier wait is bounded: on time-out the CTA raises status[0], waits for its TMA loads and MMAs in flight, frees its tensor
+// memory and returns.
 #include <cuda.h>
 
 #include "nq_common.cuh"
@@ -51,7 +52,7 @@ constexpr int kPfBBoxes = 20;                        // token-tile region: 8 x 2
 constexpr int kPfBStages = 8;                        // most token-tile stages
 constexpr int kPfRingDepth = 2;
 constexpr int kPfThreads = 32 * (2 + kPfDecodeWarps);
-constexpr unsigned long long kPfWaitNs = 2000000000ull;   // a wait that lasts 2 s is treated as a hang
+constexpr long long kPfWaitNs = 2000000000ll;             // a wait that lasts 2 s is treated as a hang, unless the caller has another limit
 
 struct PfPass { int expert, row0, ntok, pad; };
 
@@ -62,6 +63,13 @@ struct PfGemmArgs
     float* out0; float* out1; // gate|up: acc_g, acc_u [pairs][I]; down: y [pairs][H]
     int* status;              // [0] != 0: a wait timed out (device side), the results are invalid
     int H, I, nm_gu, nm_dn, down;
+    long long wait_ns;        // limit of a wait
+};
+// What the bounded waits of a CTA look at (shared memory).
+struct PfWaits
+{
+    volatile int aborted;                // a wait has run out
+    unsigned long long limit_ns;
 };
 
 // ---------------------------------------------------------------- mbarrier / tcgen05 / TMA primitives
@@ -87,28 +95,37 @@ __device__ __forceinline__ uint32_t mbar_poll(uint32_t bar, uint32_t parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag)
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, PfWaits* waits)
 {
     unsigned long long t0 = 0;
-    for (uint32_t i = 0;; ++i)
+    for (;;)
     {
         if (__all_sync(0xffffffffu, mbar_poll(bar, parity))) return true;
-        if (__any_sync(0xffffffffu, *abort_flag)) return false;
-        if ((i & 255u) == 255u)
-        {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            else if (__any_sync(0xffffffffu, t - t0 > kPfWaitNs)) break;
-        }
+        if (__any_sync(0xffffffffu, waits->aborted)) return false;
+        unsigned long long t;            // (a poll that fails has waited for some time itself)
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t0 == 0) t0 = t;
+        else if (__any_sync(0xffffffffu, t - t0 > waits->limit_ns)) break;
     }
-    *abort_flag = 1;
+    waits->aborted = 1;
     return false;
 }
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag)
+// Wait of a warp for what it has issued itself, whether or not the CTA has given up: no shared memory or tensor memory may be given back
+// that a load or an MMA still touches.
+__device__ __noinline__ void mbar_wait_own(uint32_t bar, uint32_t parity)
+{
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    do
+    {
+        if (__all_sync(0xffffffffu, mbar_poll(bar, parity))) return;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    } while (__all_sync(0xffffffffu, t - t0 < (unsigned long long)kPfWaitNs));
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, PfWaits* waits)
 {
     if (__builtin_expect(__all_sync(0xffffffffu, mbar_poll(bar, parity)), 1)) return true;
-    return mbar_wait_slow(bar, parity, abort_flag);
+    return mbar_wait_slow(bar, parity, waits);
 }
 // Token boxes of the two k-blocks of a chunk, 64 columns apart, on one election.  first: with what the two barriers have to expect.
 __device__ __forceinline__ void tma_load_chunk_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar0, uint32_t bar1,
@@ -239,13 +256,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
 struct PfShared
 {
     uint64_t full_b[kPfBStages], empty_b[kPfBStages], full_a[kPfUnitStages], empty_a[2 * kPfUnitStages], acc_full, acc_empty;
-    uint64_t head_full[2], head_empty[2];
+    uint64_t head_full[2], head_empty[2], mma_done;
     // What the warps need to know of an item, put here by the producer warp one item ahead: read by every warp for itself, pass
     // record and table row are two dependent loads from L2 (~0.7 us) at the start of an item of 10 to 30 us.
     int64_t row[2][kTableWidth];
     PfPass pass[2];
     uint32_t tmem_base;
-    volatile int abort_flag;
+    PfWaits waits;
 };
 constexpr int kPfSmem = kPfBBoxes * kPfBoxBytes + kPfDecodeWarps * kPfRingDepth * kStageBytes + 1024 + (int)sizeof(PfShared);
 static_assert(kPfSmem <= 232448, "shared memory of the prefill GEMM");
@@ -291,8 +308,8 @@ struct UnitSink
                 if (h == 0) free &= mbar_poll(deep ? bar + 8 : bar, parity ^ 1u);
                 if (__builtin_expect(!__all_sync(0xffffffffu, free), 0))
                 {
-                    *ok = mbar_wait_slow(bar, parity ^ 1u, &sh->abort_flag);
-                    if (h == 0 && *ok && deep) *ok = mbar_wait_slow(bar + 8, parity ^ 1u, &sh->abort_flag);
+                    *ok = mbar_wait_slow(bar, parity ^ 1u, &sh->waits);
+                    if (h == 0 && *ok && deep) *ok = mbar_wait_slow(bar + 8, parity ^ 1u, &sh->waits);
                 }
             }
             tc_fence_after();
@@ -315,7 +332,7 @@ struct UnitSink
 __device__ __forceinline__ void write_accumulator(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (!mbar_wait_warp(saddr(&sh->acc_full), parity, &sh->abort_flag)) return;
+    if (!mbar_wait_warp(saddr(&sh->acc_full), parity, &sh->waits)) return;
     tc_fence_after();
     const int q = warp & 3, cpart = (warp - 2) >> 2;
     for (int c0 = cpart * 32; c0 < ntok; c0 += 32 * (kPfDecodeWarps / 4))
@@ -394,7 +411,7 @@ __device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef
         uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
         RecordCursor<BK>::read(wb, st, lane);
         uint32_t frag[16];
-        if (drain && i > 0 && ch < nstages && ok) ok = mbar_wait_warp(saddr(&sh->acc_empty), drain_parity, &sh->abort_flag);
+        if (drain && i > 0 && ch < nstages && ok) ok = mbar_wait_warp(saddr(&sh->acc_empty), drain_parity, &sh->waits);
         const UnitSink sink{tmem_a - (uint32_t)stage * (2 * kPfACols), sh, (uint32_t)stage, (par_a >> stage) & 1u, nstages > kPfGroups, lane, &ok, frag};
         par_a ^= 1u << stage;
         stage = stage + kPfGroups >= nstages ? group : stage + kPfGroups;
@@ -482,7 +499,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         for (int s = 0; s < 2 * kPfUnitStages; ++s) mbar_init(&sh->empty_a[s], 1);
         for (int s = 0; s < 2; ++s) { mbar_init(&sh->head_full[s], 1); mbar_init(&sh->head_empty[s], 1 + kPfDecodeWarps); }
         mbar_init(&sh->acc_full, 1); mbar_init(&sh->acc_empty, kPfDecodeWarps);
-        sh->abort_flag = 0;
+        mbar_init(&sh->mma_done, 1);
+        sh->waits.aborted = 0; sh->waits.limit_ns = (unsigned long long)a.wait_ns;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1)
@@ -500,7 +518,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     const PfPass* passes = (const PfPass*)(a.plan + 4);
     const uint32_t full_a0 = saddr(sh->full_a), empty_a0 = saddr(sh->empty_a), full_b0 = saddr(sh->full_b), empty_b0 = saddr(sh->empty_b);
     // item number n of this CTA: its header slot and the phase of its barriers
-    auto wait_head = [&](uint32_t n) { return mbar_wait_warp(saddr(&sh->head_full[n & 1u]), (n >> 1) & 1u, &sh->abort_flag); };
+    auto wait_head = [&](uint32_t n) { return mbar_wait_warp(saddr(&sh->head_full[n & 1u]), (n >> 1) & 1u, &sh->waits); };
     auto leave_head = [&](uint32_t n) { __syncwarp(); if (lane == 0) mbar_arrive(&sh->head_empty[n & 1u]); };
     // Every role has its own loop over the items; nitem = items handled so far, par_a / par_b bit s = parity of the times unit stage /
     // token-tile stage s was used (how many stages there are changes from pass to pass).
@@ -513,7 +531,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const int64_t w = lane < kTableWidth ? a.table[(int64_t)pass->expert * kTableWidth + lane] : 0;
             const uint32_t s = n & 1u;
             prefetch_item(__shfl_sync(0xffffffffu, w, 0) >= 4, w, a.down, item % groups, C, a.down ? a.nm_dn : a.nm_gu, lane);
-            if (!mbar_wait_warp(saddr(&sh->head_empty[s]), ((n >> 1) & 1u) ^ 1u, &sh->abort_flag)) return false;
+            if (!mbar_wait_warp(saddr(&sh->head_empty[s]), ((n >> 1) & 1u) ^ 1u, &sh->waits)) return false;
             if (lane < kTableWidth) sh->row[s][lane] = w;
             if (lane == 0) sh->pass[s] = *pass;
             __syncwarp();
@@ -532,13 +550,13 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const CUtensorMap* map = uniform(!a.down && wg >= a.I / 128) ? &tmap1 : &tmap0;
             bool ok = true;
             if (sbox != last_sbox)
-                for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
+                for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->waits);
             last_sbox = sbox;
             const uint32_t tiles0 = saddr(b_tiles), bytes = (uint32_t)nbox * kPfBoxBytes, step = (uint32_t)sbox * kPfBoxBytes;
             if (stages_one_by_one(nbox))
                 for (int kb = 0, s = 0; ok && kb < 2 * C; ++kb, s = s + 1 == nb ? 0 : s + 1)
                 {
-                    ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->abort_flag);
+                    ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->waits);
                     if (!ok) break;
                     par_b ^= 1u << s;
                     tma_load_kblock_elect(tiles0 + s * step, map, kb * 64, row0, nbox, full_b0 + 8 * s);
@@ -551,7 +569,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 const uint32_t free = mbar_poll(empty_b0 + 8 * s, p0) & mbar_poll(empty_b0 + 8 * s1, p1);
                 if (__builtin_expect(!__all_sync(0xffffffffu, free), 0))
                 {
-                    ok = mbar_wait_slow(empty_b0 + 8 * s, p0, &sh->abort_flag) && mbar_wait_slow(empty_b0 + 8 * s1, p1, &sh->abort_flag);
+                    ok = mbar_wait_slow(empty_b0 + 8 * s, p0, &sh->waits) && mbar_wait_slow(empty_b0 + 8 * s1, p1, &sh->waits);
                     if (!ok) break;
                 }
                 par_b ^= (1u << s) | (1u << s1);
@@ -561,8 +579,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                     tma_load_more_elect(d0 + j * kPfBoxBytes, d1 + j * kPfBoxBytes, map, c * 128, row0 + j * kPfBoxRows, f0, f1);
                 s = s1 + 1 == nb ? 0 : s1 + 1;
             }
-            if (sh->abort_flag) break;
+            if (sh->waits.aborted) break;
         }
+        __syncwarp();
+        for (int s = 0; s < kPfBStages; ++s) mbar_wait_own(full_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u);      // loads on their way
     }
     else if (warp == 1)
     {
@@ -574,7 +594,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             const int ntok = (int)uniform(sh->pass[nitem & 1u].ntok), ntok16 = (ntok + 15) & ~15, nbox = (ntok + kPfBoxRows - 1) / kPfBoxRows;
             const int nb = b_stages(nbox), sbox = b_stage_boxes(nbox), nstages = unit_stages(ntok);
             leave_head(nitem);
-            bool ok = mbar_wait_warp(saddr(&sh->acc_empty), (nitem & 1u) ^ 1u, &sh->abort_flag);   // epilogue of the previous item has drained TMEM
+            bool ok = mbar_wait_warp(saddr(&sh->acc_empty), (nitem & 1u) ^ 1u, &sh->waits);   // epilogue of the previous item has drained TMEM
             tc_fence_after();
             // N <= 256 per instruction: one MMA per k-step, or two of (nearly) equal width
             const int n0 = ntok16 <= NQ_PF_SPLIT ? ntok16 : ((ntok16 / 2 + 15) & ~15), n1 = ntok16 - n0;
@@ -587,8 +607,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 for (uint32_t kb = 0; ok && kb < 2u * C; ++kb)
                 {
                     const uint32_t ua = (kb >> 1) & 1u, h = kb & 1u;           // (two unit stages, two column halves)
-                    ok = (h || mbar_wait_warp(full_a0 + 8 * ua, (par_a >> ua) & 1u, &sh->abort_flag)) &&
-                         mbar_wait_warp(full_b0 + 8 * s, (par_b >> s) & 1u, &sh->abort_flag);
+                    ok = (h || mbar_wait_warp(full_a0 + 8 * ua, (par_a >> ua) & 1u, &sh->waits)) &&
+                         mbar_wait_warp(full_b0 + 8 * s, (par_b >> s) & 1u, &sh->waits);
                     if (!ok) break;
                     par_a ^= h << ua;
                     par_b ^= 1u << s;
@@ -608,8 +628,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 ready &= mbar_poll(full_b0 + 8 * s1, p1);
                 if (__builtin_expect(!__all_sync(0xffffffffu, ready), 0))
                 {
-                    ok = mbar_wait_slow(full_a0 + 8 * ua, pa, &sh->abort_flag) && mbar_wait_slow(full_b0 + 8 * s, p0, &sh->abort_flag) &&
-                         mbar_wait_slow(full_b0 + 8 * s1, p1, &sh->abort_flag);
+                    ok = mbar_wait_slow(full_a0 + 8 * ua, pa, &sh->waits) && mbar_wait_slow(full_b0 + 8 * s, p0, &sh->waits) &&
+                         mbar_wait_slow(full_b0 + 8 * s1, p1, &sh->waits);
                     if (!ok) break;
                 }
                 par_a ^= 1u << ua;
@@ -630,8 +650,11 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 if (s1 + 1 == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else { s = s1 + 1; b_lo = b_lo1 + b_step; }
             }
             if (ok) tc_commit_elect(&sh->acc_full);
-            if (sh->abort_flag) break;
+            if (sh->waits.aborted) break;
         }
+        __syncwarp();
+        tc_commit_elect(&sh->mma_done);
+        mbar_wait_own(saddr(&sh->mma_done), 0);
     }
     else
     {
@@ -668,12 +691,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
                 prev_out = (up ? a.out1 : a.out0) + (size_t)ps.row0 * ld + (up ? wg - a.I / 128 : wg) * 128;
                 prev_ntok = ps.ntok;
             }
-            if (sh->abort_flag) break;
+            if (sh->waits.aborted) break;
         }
-        if (prev_ntok && !sh->abort_flag) write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
+        if (prev_ntok && !sh->waits.aborted) write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
     }
     __syncwarp();
-    if (sh->abort_flag && threadIdx.x == 0) atomicExch(a.status, 1);
+    if (sh->waits.aborted && threadIdx.x == 0) atomicExch(a.status, 1);
     tc_fence_before();
     __syncthreads();
     if (warp == 1)
@@ -780,9 +803,10 @@ int nq_pf_plan_window(const int32_t* start, const int64_t* table, int E, int pai
     return nq::check_launch("nq_pf_plan_window");
 }
 
-int nq_pf_gemm(const int64_t* table, const int32_t* plan, const void* act0, const void* act1, int pairs, float* out0, float* out1,
-               int H, int I, int nm_gu, int nm_dn, int down, int32_t* status, void* stream)
+int nq_pf_gemm_within(const int64_t* table, const int32_t* plan, const void* act0, const void* act1, int pairs, float* out0, float* out1,
+                      int H, int I, int nm_gu, int nm_dn, int down, int32_t* status, long long wait_ns, void* stream)
 {
+    NQ_REQUIRE(wait_ns >= 0, "nq_pf_gemm: wait_ns = %lld", wait_ns);
     NQ_REQUIRE(table && plan && act0 && out0 && status, "nq_pf_gemm: null pointer");
     NQ_REQUIRE(down || (act1 && out1), "nq_pf_gemm: the gate|up projection needs both activation matrices and both outputs");
     NQ_REQUIRE(H > 0 && I > 0 && H % 128 == 0 && I % 128 == 0 && H / 128 <= 64 && I / 128 <= 64, "nq_pf_gemm: H = %d, I = %d", H, I);
@@ -808,9 +832,15 @@ int nq_pf_gemm(const int64_t* table, const int32_t* plan, const void* act0, cons
     if (int e = nq::make_tile_map(&m1, down ? act0 : act1, (size_t)pairs, K)) return e;
     nq::PfGemmArgs a{};
     a.table = table; a.plan = plan; a.out0 = out0; a.out1 = out1; a.status = status;
-    a.H = H; a.I = I; a.nm_gu = nm_gu; a.nm_dn = nm_dn; a.down = down ? 1 : 0;
+    a.H = H; a.I = I; a.nm_gu = nm_gu; a.nm_dn = nm_dn; a.down = down ? 1 : 0; a.wait_ns = wait_ns;
     nq::pf_gemm_kernel<<<ctas, nq::kPfThreads, nq::kPfSmem, (cudaStream_t)stream>>>(m0, m1, a);
     return nq::check_launch("nq_pf_gemm");
+}
+
+int nq_pf_gemm(const int64_t* table, const int32_t* plan, const void* act0, const void* act1, int pairs, float* out0, float* out1,
+               int H, int I, int nm_gu, int nm_dn, int down, int32_t* status, void* stream)
+{
+    return nq_pf_gemm_within(table, plan, act0, act1, pairs, out0, out1, H, I, nm_gu, nm_dn, down, status, nq::kPfWaitNs, stream);
 }
 
 }  // extern "C"
