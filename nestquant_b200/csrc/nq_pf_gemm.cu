@@ -696,9 +696,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         if (prev_ntok && !sh->waits.aborted) write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
     }
     __syncwarp();
-    if (sh->waits.aborted && threadIdx.x == 0) atomicExch(a.status, 1);
     tc_fence_before();
     __syncthreads();
+    if (sh->waits.aborted && threadIdx.x == 0) atomicExch(a.status, 1);      // every warp is through: none can give up after this look
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kPfTmemCols) : "memory");
 }

@@ -1,5 +1,5 @@
-"""Launches of the fused prefill GEMM whose waits run out: they end by themselves, with nothing of theirs left in flight, and the next
-launch finds tensor memory and buffers as it should."""
+"""Launches of the fused prefill GEMM whose waits run out: they end by themselves, say so in the status word, leave nothing of theirs in
+flight, and the next launch finds tensor memory and buffers as it should."""
 import pytest
 import torch
 
@@ -61,3 +61,17 @@ def test_launch_that_gives_up_leaves_nothing_behind(down, E, H, I, tokens):
         assert run(None) == 0
         assert all(torch.equal(o, r) for o, r in zip(out, ref)), f"after a launch with a limit of {limit} ns"
     assert gave_up > 0
+
+
+@pytest.mark.parametrize("down,E,H,I,tokens", CASES)
+def test_launch_that_gives_up_says_so(down, E, H, I, tokens):
+    """whichever warp gives up, and whenever: with one item per CTA the warp that loads the tokens is long through by then"""
+    run, out = _launch(down, E, H, I, tokens)
+    assert run(None) == 0
+    ref = [o.clone() for o in out]
+    raised = 0
+    for limit in (0, 5000, 10000, 20000, 40000, 80000) * 3:
+        status = run(limit)
+        raised += status
+        assert status == 1 or all(torch.equal(o, r) for o, r in zip(out, ref)), f"limit {limit} ns: outputs missing, status 0"
+    assert raised > 0
