@@ -113,8 +113,8 @@ template <bool WIDE>
 __device__ __forceinline__ void load32b(const void* p, uint32_t* w)
 {
     if constexpr (WIDE)
-        asm("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"      // (its users read what an earlier launch has written)
-            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
+        asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"      // volatile, memory: stays behind a barrier or a wait in front of it
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p) : "memory");
     else
     {
         const uint4 a = ((const uint4*)p)[0], b = ((const uint4*)p)[1];
