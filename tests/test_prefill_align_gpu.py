@@ -59,3 +59,41 @@ def test_passes_do_not_depend_on_the_alignment(H, I, had, rank, kperm):
     assert float(a[0].abs().max()) > 0 and float(a[2].abs().max()) > 0 and float(a[4].abs().max()) > 0
     for s, t in zip(a, b):
         assert torch.equal(s, t)
+
+
+def test_rows_of_other_ranks_and_windows_of_pairs():
+    """the first pass with one buffer per rank (one that is aligned to 16 only is enough to leave the wide accesses), the last pass window by
+    window, adding to what is there"""
+    E, H, I, Tl, W, topk = 4, 1152, 512, 7, 3, 2
+    T, R = W * Tl, W * Tl * topk
+    L = moe.MoELayer(E, H, I, topk=topk)
+    exs = [moe.Expert(H, I, seed=9 + e, rk_gu=0, rk_dn=7, var=True, sv=0.02) for e in range(E)]
+    for e, lv in enumerate((2, 4, 0, 4)):
+        L.set(e, exs[e], lv)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    x0 = torch.randn(T, H, generator=gen, device="cuda").half()
+    sel = torch.randint(0, E, (T, topk), generator=gen, device="cuda")
+    rw = torch.rand(T, topk, generator=gen, device="cuda").half()
+    order = sel.flatten().argsort(stable=True)
+    pos = torch.empty_like(order).scatter_(0, order, torch.arange(R, device="cuda")).int()
+    pe, pt = sel.flatten()[order].int(), (order // topk).int()
+    y0 = torch.randn(R, H, generator=gen, device="cuda")
+    cut = R // 3
+
+    def passes(x_at, row_at, y_at, out_at):
+        xs = [_at((Tl, H), torch.float16, o) for o in x_at]
+        for r in range(W):
+            xs[r].copy_(x0[r * Tl:(r + 1) * Tl])
+        xg, xu, out = _at((R, H), torch.float16, row_at), _at((R, H), torch.float16, row_at), _at((T, H), torch.float32, out_at)
+        ext.pf_pre_ep([x.data_ptr() for x in xs], Tl, H, pt, pe, L.table, xg, xu, torch.zeros(R, 4, device="cuda"), I, kperm=True)
+        for a, b in ((0, cut), (cut, R)):
+            y = _at((b - a, H), torch.float32, y_at)
+            y.copy_(y0[a:b])
+            ext.pf_combine(y, torch.zeros(b - a, 4, device="cuda"), pos, sel, rw, L.table, out, I, pair0=a, npairs=b - a, accumulate=a > 0)
+        return xg.clone(), xu.clone(), out.clone()
+
+    ref = passes((0, 0, 0), 0, 0, 0)
+    assert all(float(t.abs().max()) > 0 for t in ref)
+    for at in (((16, 16, 16), 16, 16, 16), ((0, 0, 16), 0, 0, 16), ((0, 0, 0), 16, 16, 0), ((32, 32, 32), 32, 32, 32)):
+        for s, t in zip(ref, passes(*at)):
+            assert torch.equal(s, t), at

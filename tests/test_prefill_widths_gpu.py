@@ -13,10 +13,17 @@ pytestmark = pytest.mark.gpu
 COUNTS = [384, 1, 128, 300, 129, 64, 256, 65, 385, 20, 257, 0, 127, 383, 16]
 
 
-@pytest.mark.parametrize("H,I", [(128, 2048), (256, 2048), (384, 2048), (2048, 128), (2048, 256), (2048, 1664)])
-def test_passes_of_every_width_in_turn(H, I):
+# gate|up has 15 passes x I / 64 items of H / 128 chunks, down 15 x H / 128 items of I / 128.  `turns`: the projection whose CTAs take three
+# items or more, so that a layout follows another one twice; with three chunks or more it then also uses the unit stages that lie where
+# the accumulator before it was, which one and two chunks leave out.
+@pytest.mark.parametrize("H,I,turns", [(128, 2048, "gate|up"), (256, 2048, "gate|up"), (384, 2048, "gate|up"), (640, 2048, "gate|up"),
+                                       (1152, 1664, "gate|up"), (2048, 1664, "gate|up"), (2048, 128, None), (2048, 256, None),
+                                       (2560, 384, "down"), (2560, 640, "down")])
+def test_passes_of_every_width_in_turn(H, I, turns):
     E, T = len(COUNTS), sum(COUNTS)
-    # 16 passes x 32 (or 16) weight groups of a projection: every CTA takes several items, of passes that lie apart in the list
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    passes = sum((c + 383) // 384 for c in COUNTS)
+    assert passes == 15 and (turns is None or passes * (I // 64 if turns == "gate|up" else H // 128) > 2 * sms)
     exs = [moe.Expert(H, I, seed=60 + e, rk_gu=(0, 6)[e % 2], rk_dn=7, var=True, sv=0.02) for e in range(E)]
     L = moe.MoELayer(E, H, I, Bmax=1, topk=1)
     for e in range(E):
