@@ -24,7 +24,7 @@
 // Each decoded weight is used for every token of the pass, so decode cost is paid once per expert (for up to 384
 // tokens).  Tensor-pipe bound by intent; the decode instruction rate is the practical limit.  With 31 tokens per expert a unit takes a
 // scheduler ~1,000 clocks at level 4 and ~640 at level 2; the decode warps of this kernel alone, without MMAs, need ~810 and ~480, a bare
-// loop of decode and tensor-memory store 658 and 388.  Warps 0 and 1 share their schedulers with four decode warps each, so what
+// loop of records through the ring, decode and tensor-memory store 658 and 388 (without the ring 598 and 355).  Warps 0 and 1 share their schedulers with four decode warps each, so what
 // their loops cost is instructions, branches and operand moves, not memory or tensor time: see mbar_wait_warp and uniform.
 // Every mbarrier wait is bounded: on time-out the CTA raises status[0], waits for its TMA loads and MMAs in flight, frees its tensor
 // memory and returns.

@@ -345,7 +345,10 @@ __global__ void pf_hits_kernel(const int* __restrict__ counts, int* hits, int E)
 // pf_pre: a warp per 1,024 columns up to three, two rounds of half as many beyond.  At 128 registers an SM holds 512 threads: two CTAs of
 // six warps (H = 6,144) leave a quarter of them out, five of three do not.  CTAs: enough to fill the device a few times over, each
 // with a run of consecutive pairs (the runs of pairs that belong to no resident expert end at once, so more CTAs also balance better).
-// us, one round / two: 8,000 pairs 78 / 70, 24,008 of which a quarter is live 185 / 87, 65,536 525 / 482.
+// That also holds where one round fills the SM (four and eight warps); a low-rank plane, whose components the warps of a CTA take in
+// turn, gains most.  us, one round / two, 65,536 pairs: H 4,096 338 / 325, 5,120 428 / 444, 6,144 544 / 500, 7,168 606 / 566, 8,192
+// 640 / 616; with rank 2 643 / 505, 892 / 761, 1,372 / 872, 1,560 / 1,084, 1,755 / 1,205.  1,984 pairs: 31.2 / 30.4, 34.0 / 34.1, 39.5 / 36.5,
+// 43.0 / 42.8, 45.0 / 45.3.  6,144 columns, 24,008 pairs of which a quarter is live: 185 / 87.
 static int pf_pre_threads(int cols)
 {
     const int w = (cols + 1023) / 1024;
