@@ -5,27 +5,31 @@
 //
 // One work item = (pass, 128-row weight group): a pass is one expert and up to 384 of its tokens.  Per item a CTA
 // walks K in blocks of 64:
-//   warp 0        TMA: the tokens' activation tiles [ntok x 64] fp16 (SWIZZLE_128B boxes of 64 rows) -> shared memory; the pass
-//                 record and table row of the next item -> shared memory, the first lines of its planes -> L2
-//   warps 2..17   decode: a warp streams every other chunk of one strip with cp.async, decodes each unit in registers
-//                 (bit-exact fp16) and stores it with tcgen05.st as two weight tiles [128 x 64] in TENSOR MEMORY
+//   warp 0        TMA: the tokens' activation tiles [ntok x 64] fp16 (SWIZZLE_128B boxes of 64 rows) -> shared memory; the header
+//                 of the next item (everything the other warps need to know of it) -> shared memory, the first lines of its planes -> L2
+//   warps 2..17   decode: a warp streams every other chunk of one strip, the records of the next unit into registers while it
+//                 decodes this one (bit-exact fp16) and stores it with tcgen05.st as two weight tiles [128 x 64] in TENSOR MEMORY
 //                 (k-blocks 2 c and 2 c + 1): the m16n8k16-style fragment a lane holds is exactly what the 16x256b
 //                 store shape takes, so a tile costs one store per warp and no shared memory at all
-//   warp 1        one elected lane issues tcgen05.mma with the A operand in tensor memory (M 128 = weight rows, N =
-//                 tokens, K 16) into a [128 x 384] fp32 accumulator, also in tensor memory; tcgen05.commit frees the
-//                 stages.  Token tiles run 2 or 4 chunks of two k-blocks ahead, 3 k-blocks in passes of more than 320 tokens
-//                 (160 KB), weight tiles 2, 4 or 6 units of two (64 columns each), as many as the accumulator of the pass leaves
-//                 room for
+//   warps 1, 18   one elected lane issues tcgen05.mma with the A operand in tensor memory (M 128 = weight rows, N =
+//                 tokens, K 16) into a [128 x 384] fp32 accumulator, also in tensor memory; one tcgen05.commit per chunk of two
+//                 k-blocks frees its weight and token tiles.  Both run 6, 3 or 2 chunks ahead, as many as the accumulator of the pass
+//                 and 192 KB of shared memory leave room for.  Passes of up to 64 tokens are multiplied by both warps, wider ones by warp 1
 //   warps 2..17   epilogue: tcgen05.ld the accumulator and store fp32 rows acc[pair][128 columns] (coalesced); it runs
-//                 after the first unit of the CTA's next item has been decoded
+//                 after the first units of the CTA's next item have been decoded
 // A lane's fragment registers of a k-step hold k = 2 t4 + {0, 1} and 8 + 2 t4 + {0, 1}; stored side by side they make
 // the tile's k order inside every 16: position 4 i + {0, 1} = k 2 i + {0, 1}, position 4 i + {2, 3} = k 8 + 2 i + {0, 1}.
 // The activation matrices must be in the same order (nq_pf_pre / nq_pf_mid with kperm = 1).
 // Each decoded weight is used for every token of the pass, so decode cost is paid once per expert (for up to 384
-// tokens).  Tensor-pipe bound by intent; the decode instruction rate is the practical limit.  With 31 tokens per expert a unit takes a
-// scheduler ~1,000 clocks at level 4 and ~640 at level 2; the decode warps of this kernel alone, without MMAs, need ~810 and ~480, a bare
-// loop of records through the ring, decode and tensor-memory store 658 and 388 (without the ring 598 and 355).  Warps 0 and 1 share their schedulers with four decode warps each, so what
-// their loops cost is instructions, branches and operand moves, not memory or tensor time: see mbar_wait_warp and uniform.
+// tokens).  Tensor-pipe bound by intent; the decode instruction rate is the practical limit: with 31 tokens per expert a unit takes a
+// scheduler 790 clocks at level 4 and 490 at level 2 between two borders of items, of which the same loop without MMAs and item borders takes 662 and 393 (560
+// and 329 instructions, at most 0.84 per clock: the half-rate multiply and byte-sum pipe is busy for nine tenths of that).  What the two issuing warps
+// spend comes on top of the decode warps of their schedulers, and the slowest scheduler paces the others: with one issuing warp that scheduler ran
+// 671 instructions a unit at level 4, the average 626; see mbar_wait_warp, uniform and split_chunks.  An item costs a decode warp ~530 more instructions
+// and ~2,500 clocks without work.  128 experts x 31 tokens, H 6,144, I 2,048, us, gate|up / down, the kernel that kept records in a
+// shared-memory ring and all decoders in one function / this one: level 2 852 / 487 -> 757 / 437, level 4 1,344 / 789 -> 1,185 / 692, mask mode
+// 1,169 / 719 -> 1,093 / 711; 32 x 100 level 4 360 / 234 -> 330 / 213; 16 x 256 level 2 190 / 110 -> 175 / 116, level 4 231 / 149 -> 219 / 143;
+// 16 x 384 level 2 248 / 146 -> 262 / 156 (bound by the token tiles that come from L2), level 4 282 / 175 -> 275 / 175.
 // Every mbarrier wait is bounded: on time-out the CTA raises status[0], waits for its TMA loads and MMAs in flight, frees its tensor
 // memory and returns.
 #include <cuda.h>
@@ -36,22 +40,18 @@
 
 namespace nq {
 
-#ifndef NQ_PF_SPLIT
-#define NQ_PF_SPLIT 256      // token tiles wider than this are multiplied as two column halves
-#endif
 constexpr int kPfGroups = 2;                         // groups of 8 decode warps; group g takes the chunks c = g (mod 2) of its strips.  (3 groups,
                                                      // 24 decode warps at 72 registers, were slower on narrow passes and no faster on wide ones.)
 constexpr int kPfDecodeWarps = 8 * kPfGroups;
 constexpr int kPfACols = 32;                         // weight tile [128 lanes x 64 k] fp16 = 32 columns; a unit stage is two of them
 constexpr int kPfTmemCols = 512;                     // the accumulator from column 0 on, unit stages from the top down
 constexpr int kPfTokens = 384;                       // most tokens per pass (accumulator columns)
-constexpr int kPfUnitStages = 6;                     // most unit stages
+constexpr int kPfStages = 6;                         // most stages of a pass (chunk_stages)
 constexpr int kPfBoxRows = 64;                       // token rows per TMA box
 constexpr int kPfBoxBytes = kPfBoxRows * 128;        // [64 rows][64 k] fp16
-constexpr int kPfBBoxes = 20;                        // token-tile region: 8 x 2, 5 x 4, 4 x 5 or 3 x 6 boxes per stage
-constexpr int kPfBStages = 8;                        // most token-tile stages
-constexpr int kPfRingDepth = 2;
-constexpr int kPfThreads = 32 * (2 + kPfDecodeWarps);
+constexpr int kPfBBoxes = 24;                        // token-tile region: 6, 3 or 2 chunk stages of 2 x 2, 2 x 4 or 2 x 6 boxes
+constexpr int kPfSecondIssuer = 2 + kPfDecodeWarps;      // warp 1 and this one issue MMAs
+constexpr int kPfThreads = 32 * (kPfSecondIssuer + 1);
 constexpr long long kPfWaitNs = 2000000000ll;             // a wait that lasts 2 s is treated as a hang, unless the caller has another limit
 
 struct PfPass { int expert, row0, ntok, pad; };
@@ -78,10 +78,8 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, int count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(bar)), "r"(count));
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(bar)) : "memory");
-}
+__device__ __forceinline__ void mbar_arrive32(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { mbar_arrive32(saddr(bar)); }
 // The producer and MMA warps run their loops with all 32 lanes converged (so that addresses, descriptors and
 // coordinates are warp-uniform values) and one elected lane issues the asynchronous instruction.
 // Waits of a whole warp, `bar` a shared-space address.  What a wait costs that finds its phase complete is the branches around the
@@ -127,33 +125,21 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, Pf
     if (__builtin_expect(__all_sync(0xffffffffu, mbar_poll(bar, parity)), 1)) return true;
     return mbar_wait_slow(bar, parity, waits);
 }
-// Token boxes of the two k-blocks of a chunk, 64 columns apart, on one election.  first: with what the two barriers have to expect.
-__device__ __forceinline__ void tma_load_chunk_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar0, uint32_t bar1,
-                                                     uint32_t bytes)
+// Token boxes of the two k-blocks of a chunk, 64 columns apart, on one election.  first: with what the barrier has to expect.
+__device__ __forceinline__ void tma_load_chunk_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar, uint32_t bytes)
 {
     asm volatile("{\n\t.reg .pred e;\n\t.reg .b32 x1;\n\telect.sync _|e, 0xffffffff;\n\tadd.s32 x1, %3, 64;\n\t"
-                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%5], %7;\n\t"
+                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%5], %6;\n\t"
                  "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%3, %4}], [%5];\n\t"
-                 "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%6], %7;\n\t"
-                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%6];\n\t}"
-                 ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar0), "r"(bar1), "r"(bytes) : "memory");
+                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%5];\n\t}"
+                 ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void tma_load_more_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar0, uint32_t bar1)
+__device__ __forceinline__ void tma_load_more_elect(uint32_t dst0, uint32_t dst1, const CUtensorMap* map, int x, int y, uint32_t bar)
 {
     asm volatile("{\n\t.reg .pred e;\n\t.reg .b32 x1;\n\telect.sync _|e, 0xffffffff;\n\tadd.s32 x1, %3, 64;\n\t"
                  "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%2, {%3, %4}], [%5];\n\t"
-                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%6];\n\t}"
-                 ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar0), "r"(bar1) : "memory");
-}
-// The boxes of one k-block, one below the other.
-__device__ __forceinline__ void tma_load_kblock_elect(uint32_t dst, const CUtensorMap* map, int x, int y, int nbox, uint32_t bar)
-{
-    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
-                 ::"r"(bar), "r"((uint32_t)(nbox * kPfBoxBytes)) : "memory");
-    for (int j = 0; j < nbox; ++j)
-        asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
-                     "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
-                     ::"r"(dst + j * kPfBoxBytes), "l"(map), "r"(x), "r"(y + j * kPfBoxRows), "r"(bar) : "memory");
+                 "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%1], [%2, {x1, %4}], [%5];\n\t}"
+                 ::"r"(dst0), "r"(dst1), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -162,61 +148,122 @@ __device__ __forceinline__ void tc_commit_elect(uint64_t* bar)
     asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
                  "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(saddr(bar)) : "memory");
 }
-// The four K = 16 steps of one 64-wide k-block and the commits that release its two stages, issued by one elected lane of a
-// converged warp (one election for all six: the warp that issues shares its scheduler with four decode warps, and what it
-// spends per k-block is what paces the kernel when passes are narrow).  The weight operand is in tensor memory (8 columns per
-// step), the token operand in shared memory (descriptor advances by 32 B, in 16-byte units on the low word: shared-memory
-// addresses fit its 14-bit field).  first == 0: the first MMA overwrites the accumulator.
-__device__ __forceinline__ void tc_mma_kblock(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t first,
-                                              uint32_t free_a, uint32_t free_b)
+// The eight K = 16 steps of a chunk and the commit that releases its stage, issued by one elected lane of a converged warp (one election
+// for all nine: the warp that issues shares its scheduler with four decode warps, and what it spends per chunk is what paces the
+// kernel when passes are narrow).  The weight operand is in tensor memory (8 columns per step), the token operand in shared memory
+// (descriptor advances by 32 B, in 16-byte units on the low word: shared-memory addresses fit its 14-bit field; b_kb: from the first
+// k-block's tile to the second's).  first == 0: the first MMA overwrites the accumulator.
+__device__ __forceinline__ void tc_mma_chunk(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_kb, uint32_t b_hi, uint32_t idesc, uint32_t first,
+                                             uint32_t empty)
 {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t.reg .b32 ta, tb;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
-        "setp.eq.b32 p, %4, %4;\n\t"
-        "add.u32 ta, %1, 8;\n\tadd.u32 tb, %2, 2;\n\tmov.b64 db, {tb, %3};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %4, p;\n\t"
-        "add.u32 ta, %1, 16;\n\tadd.u32 tb, %2, 4;\n\tmov.b64 db, {tb, %3};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %4, p;\n\t"
-        "add.u32 ta, %1, 24;\n\tadd.u32 tb, %2, 6;\n\tmov.b64 db, {tb, %3};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %4, p;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b32 tb, %2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %5, p;\n\t"
+        "setp.eq.b32 p, %5, %5;\n\t"
+        "add.u32 ta, %1, 8;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, %1, 16;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, %1, 24;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, %1, 32;\n\t"
+        "add.u32 tb, %2, %3;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, %1, 40;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, %1, 48;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, %1, 56;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
         "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
         "}"
-        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(first), "r"(free_a), "r"(free_b) : "memory");
+        ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_kb), "r"(b_hi), "r"(idesc), "r"(first), "r"(empty) : "memory");
 }
-// The same for a token tile cut into two column halves with their own accumulator columns (alternating chains).
-__device__ __forceinline__ void tc_mma_kblock2(uint32_t tmem_d0, uint32_t tmem_d1, uint32_t tmem_a, uint32_t b_lo0, uint32_t b_lo1,
-                                               uint32_t b_hi, uint32_t idesc0, uint32_t idesc1, uint32_t first, uint32_t free_a, uint32_t free_b)
+// The same for a token tile cut into two column halves with their own accumulator columns (alternating chains); half_a is told when the
+// first k-block's weight tile has been read.
+__device__ __forceinline__ void tc_mma_chunk2(uint32_t tmem_d0, uint32_t tmem_d1, uint32_t tmem_a, uint32_t b_lo, uint32_t b_half, uint32_t b_kb, uint32_t b_hi,
+                                              uint32_t idesc0, uint32_t idesc1, uint32_t first, uint32_t half_a, uint32_t empty)
 {
     asm volatile(
         "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t.reg .b32 ta, tb;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %8, 0;\n\t"
-        "mov.b64 db, {%3, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], db, %6, p;\n\t"
-        "mov.b64 db, {%4, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], db, %7, p;\n\t"
-        "setp.eq.b32 p, %6, %6;\n\t"
-        "add.u32 ta, %2, 8;\n\tadd.u32 tb, %3, 2;\n\tmov.b64 db, {tb, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %6, p;\n\t"
-        "add.u32 tb, %4, 2;\n\tmov.b64 db, {tb, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [ta], db, %7, p;\n\t"
-        "add.u32 ta, %2, 16;\n\tadd.u32 tb, %3, 4;\n\tmov.b64 db, {tb, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %6, p;\n\t"
-        "add.u32 tb, %4, 4;\n\tmov.b64 db, {tb, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [ta], db, %7, p;\n\t"
-        "add.u32 ta, %2, 24;\n\tadd.u32 tb, %3, 6;\n\tmov.b64 db, {tb, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %6, p;\n\t"
-        "add.u32 tb, %4, 6;\n\tmov.b64 db, {tb, %5};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [ta], db, %7, p;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%9];\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%10];\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "mov.b32 tb, %2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [%1], db, %10, p;\n\t"
+        "setp.eq.b32 p, %5, %5;\n\t"
+        "add.u32 ta, %1, 8;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 8;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "add.u32 ta, %1, 16;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 16;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "add.u32 ta, %1, 24;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 24;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t"
+        "add.u32 ta, %1, 32;\n\t"
+        "add.u32 tb, %2, %3;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 32;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "add.u32 ta, %1, 40;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 40;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "add.u32 ta, %1, 48;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 48;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "add.u32 ta, %1, 56;\n\t"
+        "add.u32 tb, tb, 2;\n\t"
+        "mov.b64 db, {tb, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %5, p;\n\t"
+        "add.u32 ta, tb, %9;\n\tmov.b64 db, {ta, %4};\n\t"
+        "add.u32 ta, %1, 56;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%8], [ta], db, %10, p;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
         "}"
-        ::"r"(tmem_d0), "r"(tmem_d1), "r"(tmem_a), "r"(b_lo0), "r"(b_lo1), "r"(b_hi), "r"(idesc0), "r"(idesc1), "r"(first), "r"(free_a), "r"(free_b)
+        ::"r"(tmem_d0), "r"(tmem_a), "r"(b_lo), "r"(b_kb), "r"(b_hi), "r"(idesc0), "r"(first), "r"(empty), "r"(tmem_d1), "r"(b_half), "r"(idesc1), "r"(half_a)
         : "memory");
 }
 // 16 lanes x 4 x 256 bits of tensor memory from a warp, for columns 8 i .. 8 i + 7: lane (g, t4) supplies lane g columns
@@ -239,58 +286,89 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 // kind::f16 instruction descriptor: D fp32, A/B fp16 K-major, M 128, N tokens
 __device__ __forceinline__ uint32_t instr_desc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
+// 16 accumulator columns, and the same of the second accumulator; the wait is part of it, so nothing reads the registers in front of it
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, "
-                 "%26, %27, %28, %29, %30, %31}, [%32];"
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                   "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                   "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                   "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                   "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16_two(uint32_t taddr, uint32_t second, uint32_t (&v)[16], uint32_t (&w)[16])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                   "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                   "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]), "=r"(w[9]),
+                   "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+                 : "r"(taddr), "r"(second) : "memory");
 }
 
 // ---------------------------------------------------------------- decode warps
+// What the warps need to know of an item, put into shared memory by the producer warp one item ahead: pass record and table row are two
+// dependent loads from L2 (~0.7 us), and worked out by every decode warp for itself the rest takes 1,800 clocks of an item of 25,000
+// to 80,000 (four warps of a scheduler do it at the same time).
+struct PfItem
+{
+    ProjPlanes P;
+    uint32_t nrec, res_nrec;         // records of the base and of the residual plane
+    uint32_t unit0, res0;            // first strip of the weight group: its first unit, its first refined unit in the residual plane
+    float* out;                      // row of the item's first token, column of the weight group's first row
+    int strip0, res_strip;           // number of the first strip; refined units per strip
+    int ntok, nst, row0, up, variant;
+};
+constexpr int kPfCodes = kNumCodes + 2;     // window codes of a decoder function: the residual codes beside base code 0, 3 and 9 beside base code 1
+constexpr int kPfHeads = 3;          // this item, the one before it (its epilogue runs in this one) and the next
 struct PfShared
 {
-    uint64_t full_b[kPfBStages], empty_b[kPfBStages], full_a[kPfUnitStages], empty_a[2 * kPfUnitStages], acc_full, acc_empty;
-    uint64_t head_full[2], head_empty[2], mma_done;
-    // What the warps need to know of an item, put here by the producer warp one item ahead: read by every warp for itself, pass
-    // record and table row are two dependent loads from L2 (~0.7 us) at the start of an item of 10 to 30 us.
-    int64_t row[2][kTableWidth];
-    PfPass pass[2];
+    // full_a / full_b: weight / token tiles of a chunk are there; empty: the MMAs that read them are through; half_a: those of the first
+    // k-block (passes of two stages, i.e. one per group)
+    uint64_t full_a[kPfStages], full_b[kPfStages], empty[kPfStages], half_a[kPfGroups], acc_full[2], acc_empty[2];
+    uint64_t head_full[kPfHeads], head_empty[kPfHeads], mma_done[2];
+    PfItem item[kPfHeads];
+    int C, ld;                       // chunks of an item, floats from output row to output row
     uint32_t tmem_base;
     PfWaits waits;
 };
-constexpr int kPfSmem = kPfBBoxes * kPfBoxBytes + kPfDecodeWarps * kPfRingDepth * kStageBytes + 1024 + (int)sizeof(PfShared);
+constexpr int kPfSmem = kPfBBoxes * kPfBoxBytes + (int)sizeof(PfShared);
 static_assert(kPfSmem <= 232448, "shared memory of the prefill GEMM");
-// Unit stages beside the accumulator of a pass.  Group g uses the stages of its parity, so it is 1, 2 or 3 units ahead of the MMAs.
-// The stages of a narrow pass reach into columns that the accumulator of a wide one before it used (see decode_strip).
-__device__ __forceinline__ int unit_stages(int ntok) { return ntok <= 128 ? 6 : ntok <= 256 ? 4 : 2; }
-// The token-tile region (20 boxes) is cut into stages of 2, 4, 5 or 6 boxes (8, 5, 4 or 3 stages) for a pass of nbox
-// boxes per k-block.  Passes with the same stage size share the stage barriers freely; when the stage size changes
-// between two items of a CTA the new stages overlap old ones at other indices, so the producer first waits until every
-// stage of the old layout has been released.
-__device__ __forceinline__ int b_stage_boxes(int nbox) { return nbox <= 2 ? 2 : nbox <= 4 ? 4 : nbox <= 5 ? 5 : 6; }
-__device__ __forceinline__ int b_stages(int nbox) { return nbox <= 2 ? 8 : nbox <= 4 ? 5 : nbox <= 5 ? 4 : 3; }
-// Producer and MMA warp take the stages two at a time, the two k-blocks of a chunk at one wait, except where there are only three (passes
-// of more than 320 tokens): there a pair would come free only with the last k-block but one multiplied, and its load would find nothing
-// to hide behind.  16 experts x 384 tokens, H 6,144, I 2,048, us, pairs / one by one: gate|up 378 / 250 at level 2, 387 / 277 at level 4,
-// down 193 / 146 and 205 / 173 (the kernel that took every pass one by one: 277, 301, 166, 187).  (A poll does not help: try_wait may wait itself, so the second one of a pair does.)  Four stages one by
-// one: gate|up of 320 tokens 237 / 211 at level 2, 257 / 262 at level 4; five: 160 tokens 167 / 172 and 224 / 224.
-__device__ __forceinline__ bool stages_one_by_one(int nbox) { return b_stages(nbox) == 3; }
+extern __shared__ __align__(1024) uint8_t nq_pf_smem[];      // (the token tiles' swizzle needs the alignment; addresses in it are constants of the code)
+__device__ __forceinline__ uint8_t* pf_tiles() { return nq_pf_smem; }
+__device__ __forceinline__ PfShared* pf_shared() { return (PfShared*)(pf_tiles() + kPfBBoxes * kPfBoxBytes); }
+// Chunk stages of a pass: chunk c of an item uses stage c mod chunk_stages, its weight tiles in tensor memory (64 columns a stage, from the
+// top down beside the accumulator) and its token tiles in shared memory (2 x 12 / stages boxes).  One set of barriers serves both.  The
+// stages of a narrow pass reach into columns that the accumulator of a wide one before it used (see decode_strip), and when the number of
+// stages changes between two items of a CTA the new token tiles overlap old ones at other indices, so the producer first waits
+// until every stage of the old layout has been released.
+__device__ __forceinline__ int chunk_stages(int ntok) { return ntok <= 128 ? 6 : ntok <= 256 ? 3 : 2; }
+// Passes of up to 64 tokens: even and odd chunks are multiplied by two warps, each into an accumulator of its own that the epilogue adds up.
+// What a chunk costs the warp that issues its MMAs comes on top of the decode warps of its scheduler, and the slowest scheduler paces the
+// others: gate|up of 128 experts x 31 tokens with one warp / two, us: 785 / 757 at level 2, 1,226 / 1,193 at level 4.  Beyond 64 tokens the second
+// accumulator would leave four stages instead of six: 32 x 100 tokens, down, 164 / 149 at level 2, 229 / 217 at level 4 (four / six).
+__device__ __forceinline__ bool split_chunks(int ntok) { return ntok <= 64; }
+// First column of an item's accumulator, and from there to the second one.  Up to 32 tokens the items take turns with two pairs, so the MMAs
+// of the next item need not wait for the epilogue.
+__device__ __forceinline__ uint32_t acc_column(int ntok, uint32_t acc) { return ntok <= 32 ? 64u * acc : 0u; }
+__device__ __forceinline__ uint32_t acc_second(int ntok) { return ntok <= 32 ? 32u : 64u; }
+// bit s = parity of the times stage s was used, after an item of C chunks in nst stages
+__device__ __forceinline__ uint32_t stage_parities(uint32_t par, int C, int nst)
+{
+    const int rounds = C / nst;
+    return par ^ (rounds & 1 ? (1u << nst) - 1u : 0u) ^ ((1u << (C - rounds * nst)) - 1u);
+}
 
 // A unit is decoded whole (8 k-steps) by one warp: k-steps 0..3 fill the weight tile of k-block 2 c, k-steps 4..7 the
-// tile of k-block 2 c + 1.  The sink keeps the fragments of four k-steps in registers and hands them over as one: wait until
-// the MMAs that last read the stage are done, one 32-column store, and after the second half wait for the stores and signal "full".  The four k-steps are
-// one straight run of arithmetic with nothing to wait for in it (a store and a branch after every k-step cut the unit into
-// ten pieces that were scheduled one by one).
+// tile of k-block 2 c + 1.  The sink keeps the fragments of four k-steps in registers and hands them over as one 32-column store.
+// DEEP (two or three unit stages per group): the stage is free before the unit is begun, and the 64 weights are one straight run of
+// arithmetic with nothing to wait for in it.  One unit stage per group: each half is waited for when it is to be written.
+template <bool DEEP>
 struct UnitSink
 {
-    uint32_t tmem_a;      // tensor-memory address of the unit stage, at the warp's 16 lanes
-    PfShared* sh; uint32_t stage, parity; bool deep; int lane; bool* ok; uint32_t* frag;      // frag: 16 registers
+    uint32_t tmem_a;      // tensor-memory address of the stage, at the warp's 16 lanes
+    PfShared* sh; uint32_t stage, parity, half_parity; bool first; bool* ok; uint32_t* frag;      // frag: 16 registers
     template <int T>
     __device__ __forceinline__ void operator()(std::integral_constant<int, T>, const uint32_t (&a)[4]) const
     {
@@ -299,149 +377,187 @@ struct UnitSink
         frag[o] = a[0]; frag[o + 1] = a[2]; frag[o + 2] = a[1]; frag[o + 3] = a[3];
         if constexpr ((T & 3) == 3)
         {
-            // two units or more ahead of the MMAs (deep), both halves are nearly always free when the first is written: one vote and
-            // branch for the two; one unit ahead, the second half comes back while the first is decoded
-            if (h == 0 ? *ok : *ok && !deep)
+            if constexpr (!DEEP)
             {
-                const uint32_t bar = saddr(&sh->empty_a[2 * stage + h]);
-                uint32_t free = mbar_poll(bar, parity ^ 1u);
-                if (h == 0) free &= mbar_poll(deep ? bar + 8 : bar, parity ^ 1u);
-                if (__builtin_expect(!__all_sync(0xffffffffu, free), 0))
-                {
-                    *ok = mbar_wait_slow(bar, parity ^ 1u, &sh->waits);
-                    if (h == 0 && *ok && deep) *ok = mbar_wait_slow(bar + 8, parity ^ 1u, &sh->waits);
-                }
+                if (h == 0) *ok = mbar_wait_warp(saddr(&sh->half_a[stage]), half_parity, &sh->waits);
+                // (first unit of an item: the stage may have been used last by a pass that does not report halves)
+                if ((h == 1 || first) && *ok) *ok = mbar_wait_warp(saddr(&sh->empty[stage]), parity, &sh->waits);
+                tc_fence_after();
             }
-            tc_fence_after();
-            // an aborted launch stores too (the columns are this CTA's until the end, the results are discarded) but signals nothing
+            // (an aborted launch stores too: the columns are this CTA's until the end, the results are discarded)
             tmem_st_16x256b_x4(tmem_a + h * kPfACols, frag);
-            if constexpr (T == 7)
-            {
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (*ok && lane == 0) mbar_arrive(&sh->full_a[stage]);
-            }
         }
     }
 };
 
-// Decode warps: accumulator [128 weight rows x ntok] of an item -> out (row of the item's first token, column of the weight group's
-// first row).  TMEM lanes 32 q .. 32 q + 31 (the quarter this warp may read) are weight rows; the four warps of a quarter take
-// 32-column chunks in turn.
-__device__ __forceinline__ void write_accumulator(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
+// What a decoder function needs to know beside the item: in one word.
+struct PfInfo
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (!mbar_wait_warp(saddr(&sh->acc_full), parity, &sh->waits)) return;
+    uint32_t w;      // bits 0, 1 header slot of the item, 2, 3 of the one before it, 4 whose accumulator is to be written, 5 drain, 6 accumulator
+                     // barriers of the one before it, 7 their phase
+    __device__ __forceinline__ uint32_t slot() const { return w & 3u; }
+    __device__ __forceinline__ uint32_t prev() const { return w >> 2 & 3u; }
+    __device__ __forceinline__ bool has_prev() const { return w >> 4 & 1u; }
+    __device__ __forceinline__ bool drain() const { return w >> 5 & 1u; }
+    __device__ __forceinline__ uint32_t acc() const { return w >> 6 & 1u; }
+    __device__ __forceinline__ uint32_t phase() const { return w >> 7 & 1u; }
+};
+// Units of an item that a warp decodes before it writes the accumulator of the previous item, whose last MMAs finish meanwhile.  (Down
+// projection of 128 experts x 31 tokens at level 4, 2,048 / 256 columns, us: after two units 692 / 184, after one 694 / 181, at once 705 / 199;
+// 16 x 256 tokens, three stages: after one 143, at once 144.)
+__device__ __forceinline__ int units_before_epilogue(int nst, bool drain) { return nst == kPfStages && !drain ? 2 : 1; }
+
+// Decode warps: accumulator [128 weight rows x ntok] of the item before this one -> out.  TMEM lanes 32 q .. 32 q + 31 (the quarter this warp
+// may read) are weight rows; the four warps of a quarter take 16-column pieces in turn.
+__device__ __forceinline__ void write_accumulator(PfInfo info)
+{
+    PfShared* sh = pf_shared();
+    const PfItem& I = sh->item[info.prev()];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ntok = I.ntok, ld = sh->ld;
+    const bool both = split_chunks(ntok) && sh->C > 1;
+    const uint32_t tmem = sh->tmem_base + acc_column(ntok, info.acc());
+    if (!mbar_wait_warp(saddr(&sh->acc_full[info.acc()]), info.phase(), &sh->waits)) return;
     tc_fence_after();
     const int q = warp & 3, cpart = (warp - 2) >> 2;
-    for (int c0 = cpart * 32; c0 < ntok; c0 += 32 * (kPfDecodeWarps / 4))
+    for (int c0 = cpart * 16; c0 < ntok; c0 += 16 * (kPfDecodeWarps / 4))
     {
-        uint32_t v[32];
-        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c0, v);
-        float* o = out + (size_t)c0 * ld + q * 32 + lane;
+        const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + c0;
+        uint32_t v[16];
+        if (both)
+        {
+            uint32_t w[16];
+            tmem_ld16_two(at, at + acc_second(ntok), v, w);
 #pragma unroll
-        for (int j = 0; j < 32; ++j, o += ld)
+            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+        }
+        else tmem_ld16(at, v);
+        float* o = I.out + (size_t)c0 * ld + q * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < 16; ++j, o += ld)
             if (c0 + j < ntok) *o = __uint_as_float(v[j]);
     }
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sh->acc_empty);
+    if (lane == 0) { mbar_arrive(&sh->acc_empty[info.acc()]); mbar_arrive(&sh->head_empty[info.prev()]); }
 }
 // Between two units it is a call, because the registers of the decode loop are all taken there; after the last unit it is in line.  A warp
 // with one unit per item has no other place for it than after that unit, and every item pays what the call costs: 128 experts x 31
-// tokens, H 6,144, down projection of 256 columns, us, call / in line: 153 / 122 at level 2, 225 / 187 at level 4.  In line between units
-// too, down projection of 2,048 columns, 64 experts: 255 / 246 and 404 / 415.
-__device__ __noinline__ void write_accumulator_between(PfShared* sh, uint32_t tmem, float* out, int ld, int ntok, uint32_t parity)
-{
-    write_accumulator(sh, tmem, out, ld, ntok, parity);
-}
+// tokens, H 6,144, down projection of 256 columns, us, call / in line: 153 / 122 at level 2, 225 / 187 at level 4.
+__device__ __noinline__ void write_accumulator_between(uint32_t info) { write_accumulator(PfInfo{info}); }
 
-// One decode warp, one item: its strip over the chunks c = GROUP, GROUP + 2, ... (the other group of 8 warps takes the
-// other parity), i.e. k-blocks 4 i + 2 GROUP and + 1.  nstages = unit stages of this item, par_a =
-// parity of the times every stage was used; drain: the stages from 2 on lie where the accumulator of the previous item was, so their
-// first use waits until all warps have read it (acc_empty, phase `drain_parity`).  false = aborted.
-template <bool REFINED, int RC, int BK, class Mid>
-__device__ __forceinline__ bool decode_strip(const ProjPlanes& P, const StripRef& sr, int C, int NS, int lane, int group,
-                                             uint32_t tmem_a, uint32_t ring, PfShared* sh, int nstages, uint32_t& par_a, bool drain,
-                                             uint32_t drain_parity, Mid& mid)
+// One decode warp, one item: its strip over the chunks c = group, group + 2, ... (the other group of 8 warps takes the other
+// parity), i.e. k-blocks 4 i + 2 group and + 1.  MODE 0: level 2, 1: level 4, 2: level 4 in mask mode (chunks without a flag decode as
+// level 2).  The records of the next unit are fetched into registers while the current one is decoded.
+// par: bit s = parity of the times stage s was used before this item, bit kPfStages the same for half_a of this warp's group.
+// false: a wait ran out.
+// The epilogue of the previous item runs after this item's first units are decoded: the MMAs of the previous item's last k-blocks finish
+// meanwhile, and the tensor pipe finds tiles waiting when the accumulator is free again.  It stands between two runs of the
+// unit loop, not in it.  drain: the stages from 2 on lie where the accumulator of the previous item was, so they wait until all warps have
+// read it.
+template <int MODE, int RC, int BK, bool DEEP>
+__device__ __noinline__ bool decode_strip(uint32_t par, uint32_t info_word)
 {
-    // per-unit scalars of this warp's chunks, one chunk (group + kPfGroups * lane) per lane: ring signs and, for refined units,
-    // the block word with its fp16 multiplier / addend (computed once here instead of by every lane of every unit)
-    uint32_t var_b = 0, ac = 0, mbn = 0;
+    PfShared* sh = pf_shared();
+    const PfInfo info{info_word};
+    const int warp = (int)(threadIdx.x >> 5), lane = threadIdx.x & 31, group = (warp - 2) >> 3, nxt = ring_successor(lane);
+    const int sidx = 2 * (warp & 3) + (((warp - 2) >> 2) & 1);        // strip of the weight group: two to every quarter of the lanes
+    const PfItem& I = sh->item[info.slot()];
+    const int C = sh->C, n = (C - group + kPfGroups - 1) / kPfGroups;         // units of this warp: at most 32
+    if (n <= 0) return true;
+    const uint32_t unit0 = I.unit0 + (uint32_t)(sidx * C), res0 = I.res0 + (uint32_t)(sidx * I.res_strip);
+    const uint8_t *base = (const uint8_t*)I.P.base, *p4 = I.P.p4;
+    const uint32_t nrec = I.nrec, res_nrec = MODE == 1 ? nrec : I.res_nrec;
+    uint32_t rec = (unit0 + group) * 32 + lane, res = (MODE == 1 ? unit0 + group : res0) * 32 + lane;       // this unit's records (level 4 without flags: of both planes)
+    RecordValues<BK> rb;
+    rb.load_at(base, nrec, rec);
+    RecordValues<RC> rr;
+    unsigned long long flags = 0;        // refined chunks of the strip
+    uint32_t own = 0, other = 0;         // of them this warp's units, and the chunks behind those, from this unit on
+    if constexpr (MODE == 1) rr.load_at(p4, nrec, rec);
+    if constexpr (MODE == 2)
+    {
+        flags = (unsigned long long)__ldg((const unsigned long long*)I.P.flags + I.strip0 + sidx);
+        if (group) res += (uint32_t)(flags & 1ull) * 32u;
+        own = __ballot_sync(0xffffffffu, flags >> group >> (kPfGroups * lane) & 1ull);
+        other = __ballot_sync(0xffffffffu, flags >> group >> (kPfGroups * lane) >> 1 & 1ull);
+        if (own & 1u) rr.load_at(p4, res_nrec, res);
+    }
+    // per-unit scalars, one unit per lane: ring signs and block word (meta = word | signs << 16) and the block word's multipliers
+    uint32_t meta = 0, ac = 0;
+    if (lane < n)
     {
         const int ch = group + kPfGroups * lane;
-        if (ch < C)
+        if (I.P.var) meta = (uint32_t)__ldg(I.P.var + unit0 + ch) << 16;
+        if (MODE == 1 || (MODE == 2 && (flags >> ch & 1ull)))
         {
-            if (P.var) var_b = __ldg(P.var + sr.unit0 + ch);
-            if constexpr (REFINED)
-                if (chunk_refined(sr, ch))
+            const size_t at = res0 + (MODE == 1 ? ch : __popcll(flags & ((1ull << ch) - 1ull)));
+            const uint32_t word = __ldg(I.P.d4 + at) & 0xFFFFu;
+            meta |= word;
+            ac = block_multipliers(word);
+        }
+    }
+    const uint32_t tmem_a = sh->tmem_base + ((uint32_t)(16 * sidx) << 16) + kPfTmemCols - 2 * kPfACols, full_a0 = saddr(sh->full_a), empty0 = saddr(sh->empty);
+    const uint32_t nst = DEEP ? (uint32_t)I.nst : 2u;
+    const uint32_t half_par = par >> kPfStages;
+    uint32_t stage = (uint32_t)group, free = ~par;       // bit s of free: phase of `empty` that frees stage s for this round
+    int i = 0, end = info.has_prev() ? min(n, units_before_epilogue((int)nst, info.drain())) : n;
+    bool ok = true;
+#pragma unroll 1
+    for (;;)
+    {
+#pragma unroll 1
+        for (; i < end; ++i)
+        {
+            uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
+            const bool refined = MODE == 1 || (MODE == 2 && (own & 1u));
+            rb.words(wb, lane);
+            if constexpr (MODE > 0)
+                if (refined) rr.words(wr, lane);
+            if (i + 1 < n)
+            {
+                rec += kPfGroups * 32;
+                rb.load_at(base, nrec, rec);
+                if constexpr (MODE == 1) rr.load_at(p4, nrec, rec);
+                if constexpr (MODE == 2)
                 {
-                    mbn = __ldg(P.d4 + sr.res0 + refined_before(sr, ch)) & 0xFFFFu;
-                    ac = block_multipliers(mbn);
+                    res += ((own & 1u) + (other & 1u)) * 32u;
+                    own >>= 1; other >>= 1;
+                    if (own & 1u) rr.load_at(p4, res_nrec, res);
                 }
+            }
+            if constexpr (DEEP)
+            {
+                if (!mbar_wait_warp(empty0 + 8 * stage, (free >> stage) & 1u, &sh->waits)) return false;
+                tc_fence_after();
+            }
+            continue_stream<Pattern<BK>::kBits>(wb, __shfl_sync(0xffffffffu, wb[0], nxt));
+            const uint32_t um = __shfl_sync(0xffffffffu, meta, i), sign2 = sign_mask(um >> 16, lane);
+            uint32_t frag[16];
+            const UnitSink<DEEP> sink{tmem_a - stage * (2 * kPfACols), sh, stage, (free >> stage) & 1u, (half_par ^ i ^ 1u) & 1u, i == 0, &ok, frag};
+            if (MODE > 0 && refined)
+            {
+                if constexpr (MODE > 0)
+                {
+                    continue_stream<Pattern<RC>::kBits>(wr, __shfl_sync(0xffffffffu, wr[0], nxt));
+                    decode_words<true, RC, BK>(wb, wr, consts_level4(__shfl_sync(0xffffffffu, ac, i), um, sign2), sink);
+                }
+            }
+            else if constexpr (MODE != 1) decode_words<false, 0, BK>(wb, wr, consts_level2(sign2), sink);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if constexpr (!DEEP)
+                if (!ok) return false;
+            if (lane == 0) mbar_arrive32(full_a0 + 8 * stage);
+            stage += kPfGroups;
+            if (stage >= nst) { stage -= nst; free = ~free; }
         }
+        if (end == n) break;
+        write_accumulator_between(info_word);
+        if (info.drain() && !mbar_wait_warp(saddr(&sh->acc_empty[info.acc()]), info.phase(), &sh->waits)) return false;
+        end = n;
     }
-    RecordCursor<BK> cb;
-    cb.init(P.base, (size_t)NS * C * 32, sr.unit0, lane);
-    RecordCursor<RC> cr;
-    if constexpr (REFINED) cr.init(P.p4, sr.res_nrec, sr.res0, lane);
-    auto issue = [&](int ch, uint32_t st) {
-        cb.copy(st, ch, lane);
-        if constexpr (REFINED)
-            if (chunk_refined(sr, ch)) cr.copy(st + kStageBase, refined_before(sr, ch), lane);
-    };
-#pragma unroll
-    for (int d = 0; d < kPfRingDepth - 1; ++d)
-    {
-        if (group + kPfGroups * d < C) issue(group + kPfGroups * d, ring + d * kStageBytes);
-        cp_async_commit();
-    }
-    int slot = 0, slot_in = kPfRingDepth - 1, i = 0, stage = group;
-    bool ok = true;
-    for (int ch = group; ch < C; ch += kPfGroups, ++i)
-    {
-        if (ch + kPfGroups * (kPfRingDepth - 1) < C) issue(ch + kPfGroups * (kPfRingDepth - 1), ring + slot_in * kStageBytes);
-        cp_async_commit();
-        cp_async_wait<kPfRingDepth - 1>();
-        const uint32_t st = ring + slot * kStageBytes;
-        slot = slot + 1 == kPfRingDepth ? 0 : slot + 1;
-        slot_in = slot_in + 1 == kPfRingDepth ? 0 : slot_in + 1;
-        const uint32_t sign2 = sign_mask(__shfl_sync(0xffffffffu, var_b, i), lane);
-        uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
-        RecordCursor<BK>::read(wb, st, lane);
-        uint32_t frag[16];
-        if (drain && i > 0 && ch < nstages && ok) ok = mbar_wait_warp(saddr(&sh->acc_empty), drain_parity, &sh->waits);
-        const UnitSink sink{tmem_a - (uint32_t)stage * (2 * kPfACols), sh, (uint32_t)stage, (par_a >> stage) & 1u, nstages > kPfGroups, lane, &ok, frag};
-        par_a ^= 1u << stage;
-        stage = stage + kPfGroups >= nstages ? group : stage + kPfGroups;
-        bool refined = false;
-        if constexpr (REFINED) refined = chunk_refined(sr, ch);
-        if (refined)
-        {
-            const uint32_t acw = __shfl_sync(0xffffffffu, ac, i), mb = __shfl_sync(0xffffffffu, mbn, i);
-            RecordCursor<RC>::read(wr, st + kStageBase, lane);
-            decode_unit<true, RC, BK>(wb, wr, consts_level4(acw, mb, sign2), lane, sink);
-        }
-        else
-            decode_unit<false, 0, BK>(wb, wr, consts_level2(sign2), lane, sink);
-        if (i == 0 && ch + kPfGroups < C) mid();      // the previous item's epilogue, once this item's first tiles are on their way
-    }
-    cp_async_wait<0>();
-    return ok;
-}
-
-template <class Mid>
-__device__ __forceinline__ bool decode_item(const ProjPlanes& P, int level, int rc, int bk, int strip, int C, int NS, int nm, int lane, int group,
-                                            uint32_t tmem_a, uint8_t* ring, PfShared* sh, int nstages, uint32_t& par_a, bool drain,
-                                            uint32_t drain_parity, Mid& mid)
-{
-    const StripRef sr = locate_strip(P, strip, C, NS, nm, level >= 4);
-    bool ok = true;
-#define NQ_RUN(REF, RCV, BKV) ok = decode_strip<REF, RCV, BKV>(P, sr, C, NS, lane, group, tmem_a, smem_addr(ring), sh, nstages, par_a, drain, drain_parity, mid)
-    NQ_WITH_CODES(level >= 4, rc, bk, 0x3FF, NQ_RUN);
-#undef NQ_RUN
-    return ok;
+    return true;
 }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -481,26 +597,27 @@ __device__ __forceinline__ void prefetch_item(bool level4, int64_t row_word, int
 // in front of every one.
 __device__ __forceinline__ uint32_t uniform(uint32_t x) { return __reduce_or_sync(0xffffffffu, x); }
 
-// grid = resident CTAs (one per SM), 576 threads
+// grid = resident CTAs (one per SM), 608 threads
 __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_constant__ CUtensorMap tmap0,
                                                                 const __grid_constant__ CUtensorMap tmap1, PfGemmArgs a)
 {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* b_tiles = smem;                                  // token tiles [rows][64 k] fp16, 128-byte swizzle (TMA boxes)
-    uint8_t* rings = smem + kPfBBoxes * kPfBoxBytes;          // per decode warp: kPfRingDepth plane stages
-    PfShared* sh = (PfShared*)(rings + kPfDecodeWarps * kPfRingDepth * kStageBytes);
+    uint8_t* b_tiles = pf_tiles();                            // token tiles [rows][64 k] fp16, 128-byte swizzle (TMA boxes)
+    PfShared* sh = pf_shared();
     const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (saddr(b_tiles) & 1023u)          // (never: the swizzled tiles would be read from the wrong places)
+    {
+        if (threadIdx.x == 0) atomicExch(a.status, 1);
+        return;
+    }
 
     if (threadIdx.x == 0)
     {
-        for (int s = 0; s < kPfBStages; ++s) { mbar_init(&sh->full_b[s], 1); mbar_init(&sh->empty_b[s], 1); }
-        for (int s = 0; s < kPfUnitStages; ++s) mbar_init(&sh->full_a[s], 8);
-        for (int s = 0; s < 2 * kPfUnitStages; ++s) mbar_init(&sh->empty_a[s], 1);
-        for (int s = 0; s < 2; ++s) { mbar_init(&sh->head_full[s], 1); mbar_init(&sh->head_empty[s], 1 + kPfDecodeWarps); }
-        mbar_init(&sh->acc_full, 1); mbar_init(&sh->acc_empty, kPfDecodeWarps);
-        mbar_init(&sh->mma_done, 1);
+        for (int s = 0; s < kPfStages; ++s) { mbar_init(&sh->full_a[s], 8); mbar_init(&sh->full_b[s], 1); mbar_init(&sh->empty[s], 1); }
+        for (int s = 0; s < kPfGroups; ++s) mbar_init(&sh->half_a[s], 1);
+        for (int s = 0; s < kPfHeads; ++s) { mbar_init(&sh->head_full[s], 1); mbar_init(&sh->head_empty[s], 2 + kPfDecodeWarps); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&sh->acc_full[s], 2); mbar_init(&sh->acc_empty[s], kPfDecodeWarps); mbar_init(&sh->mma_done[s], 1); }
         sh->waits.aborted = 0; sh->waits.limit_ns = (unsigned long long)a.wait_ns;
+        sh->C = (a.down ? a.I : a.H) / 128; sh->ld = a.down ? a.H : a.I;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1)
@@ -516,184 +633,195 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     const int N = a.down ? a.H : 2 * a.I, K = a.down ? a.I : a.H, C = K / 128, NS = N / 16, groups = N / 128;
     const int nitems = (int)uniform(a.plan[0]) * groups;
     const PfPass* passes = (const PfPass*)(a.plan + 4);
-    const uint32_t full_a0 = saddr(sh->full_a), empty_a0 = saddr(sh->empty_a), full_b0 = saddr(sh->full_b), empty_b0 = saddr(sh->empty_b);
-    // item number n of this CTA: its header slot and the phase of its barriers
-    auto wait_head = [&](uint32_t n) { return mbar_wait_warp(saddr(&sh->head_full[n & 1u]), (n >> 1) & 1u, &sh->waits); };
-    auto leave_head = [&](uint32_t n) { __syncwarp(); if (lane == 0) mbar_arrive(&sh->head_empty[n & 1u]); };
-    // Every role has its own loop over the items; nitem = items handled so far, par_a / par_b bit s = parity of the times unit stage /
-    // token-tile stage s was used (how many stages there are changes from pass to pass).
+    const uint32_t full_a0 = saddr(sh->full_a), full_b0 = saddr(sh->full_b), empty0 = saddr(sh->empty), half_a0 = saddr(sh->half_a);
+    // header slot of an item of this CTA and the phase of its barriers
+    struct Head
+    {
+        uint32_t slot = 0, phase = 0;
+        __device__ __forceinline__ void next() { if (++slot == kPfHeads) { slot = 0; phase ^= 1u; } }
+    };
+    auto wait_head = [&](const Head& h) { return mbar_wait_warp(saddr(&sh->head_full[h.slot]), h.phase, &sh->waits); };
+    // Every role has its own loop over the items; nitem = items handled so far, par bit s = parity of the times stage s was used (how many
+    // stages there are changes from pass to pass).
     if (warp == 0)
     {
-        // ---- token tiles by TMA, ahead of the MMAs as far as there are stages; pass record and table row of the items, one item ahead
-        auto publish = [&](int item, uint32_t n) {
-            if (item >= nitems) return true;
-            const PfPass* pass = passes + item / groups;
-            const int64_t w = lane < kTableWidth ? a.table[(int64_t)pass->expert * kTableWidth + lane] : 0;
-            const uint32_t s = n & 1u;
-            prefetch_item(__shfl_sync(0xffffffffu, w, 0) >= 4, w, a.down, item % groups, C, a.down ? a.nm_dn : a.nm_gu, lane);
-            if (!mbar_wait_warp(saddr(&sh->head_empty[s]), ((n >> 1) & 1u) ^ 1u, &sh->waits)) return false;
-            if (lane < kTableWidth) sh->row[s][lane] = w;
-            if (lane == 0) sh->pass[s] = *pass;
+        // ---- token tiles by TMA, ahead of the MMAs as far as there are stages; the headers of the items, one item ahead: the pass record
+        // is fetched two items ahead of that, the table row one
+        struct At { int pass, wg; } at0{(int)blockIdx.x / groups, (int)blockIdx.x % groups}, at1, at2;
+        const int step_pass = (int)gridDim.x / groups, step_wg = (int)gridDim.x % groups, npass = nitems / groups;
+        auto behind = [&](At t) {
+            t.pass += step_pass; t.wg += step_wg;
+            if (t.wg >= groups) { t.wg -= groups; ++t.pass; }
+            return t;
+        };
+        auto pass_of = [&](const At& t) { return t.pass < npass ? __ldg((const int4*)(passes + t.pass)) : make_int4(0, 0, 0, 0); };
+        auto row_of = [&](const At& t, const int4& p) { return t.pass < npass && lane < kTableWidth ? a.table[(int64_t)p.x * kTableWidth + lane] : 0; };
+        auto publish = [&](const At& t, const int4& p, int64_t w, const Head& h) {
+            if (t.pass >= npass) return true;
+            auto field = [&](int i) { return __shfl_sync(0xffffffffu, w, i); };
+            const int down = a.down, o = down ? 5 : 1, nm = down ? a.nm_dn : a.nm_gu;
+            const bool level4 = (int)field(0) >= 4;
+            prefetch_item(level4, w, down, t.wg, C, nm, lane);
+            const int64_t base = field(o), p4 = field(o + 1), d4 = field(o + 2), flags = field(o + 3), var = field(down ? 13 : 12);
+            const int rc = (int)field(10 + down), bk = (int)(field(19) >> (8 * down)) & 0xFF, mode = !level4 ? 0 : flags ? 2 : 1;
+            const int code = bk == 1 ? (mode && rc == 9 ? 11 : 10) : mode && rc >= 0 && rc < kNumCodes ? rc : 0;
+            const int refined = mode == 2 ? nm : C, nst = chunk_stages(p.z), up = !down && t.wg >= a.I / 128;
+            if (!mbar_wait_warp(saddr(&sh->head_empty[h.slot]), h.phase ^ 1u, &sh->waits)) return false;
+            if (lane == 0)
+            {
+                PfItem& I = sh->item[h.slot];
+                I.P.base = (const uint4*)base; I.P.p4 = (const uint8_t*)p4; I.P.d4 = (const uint32_t*)d4; I.P.flags = (const uint64_t*)flags;
+                I.P.var = (const uint8_t*)var;
+                I.nrec = (uint32_t)(NS * C * 32); I.res_nrec = (uint32_t)(NS * refined * 32);
+                I.strip0 = t.wg * 8; I.unit0 = (uint32_t)(t.wg * 8 * C); I.res0 = (uint32_t)(t.wg * 8 * refined); I.res_strip = refined;
+                I.out = (up ? a.out1 : a.out0) + (size_t)p.y * sh->ld + (up ? t.wg - a.I / 128 : t.wg) * 128;
+                I.ntok = p.z; I.nst = nst; I.row0 = p.y; I.up = up; I.variant = (mode * kPfCodes + code) * 2 + (nst > 2);
+            }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->head_full[s]);
+            if (lane == 0) mbar_arrive(&sh->head_full[h.slot]);
             return true;
         };
-        publish(blockIdx.x, 0);
-        uint32_t par_b = 0, nitem = 0;
-        int last_sbox = 0;                   // stage size of the previous item
-        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
+        int4 p0 = pass_of(at0), p1;
+        int64_t w1;
+        Head head, ahead;
+        publish(at0, p0, row_of(at0, p0), ahead);
+        at1 = behind(at0); p1 = pass_of(at1); w1 = row_of(at1, p1);
+        at2 = behind(at1);
+        int4 p2 = pass_of(at2);
+        uint32_t par = 0;
+        int last_nst = 0;                    // stages of the previous item
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, head.next())
         {
-            if (!publish(item + gridDim.x, nitem + 1) || !wait_head(nitem)) break;
-            const int wg = item % groups;
-            const int nbox = (int)uniform((sh->pass[nitem & 1u].ntok + kPfBoxRows - 1) / kPfBoxRows), row0 = (int)uniform(sh->pass[nitem & 1u].row0);
-            const int nb = b_stages(nbox), sbox = b_stage_boxes(nbox);
-            const CUtensorMap* map = uniform(!a.down && wg >= a.I / 128) ? &tmap1 : &tmap0;
+            if (!wait_head(head)) break;
+            const PfItem& I = sh->item[head.slot];
+            const int ntok = (int)uniform(I.ntok), nbox = (ntok + kPfBoxRows - 1) / kPfBoxRows, row0 = (int)uniform(I.row0);
+            const int nst = chunk_stages(ntok);
+            const CUtensorMap* map = uniform(I.up) ? &tmap1 : &tmap0;
             bool ok = true;
-            if (sbox != last_sbox)
-                for (int s = 0; ok && s < kPfBStages; ++s) ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->waits);
-            last_sbox = sbox;
-            const uint32_t tiles0 = saddr(b_tiles), bytes = (uint32_t)nbox * kPfBoxBytes, step = (uint32_t)sbox * kPfBoxBytes;
-            if (stages_one_by_one(nbox))
-                for (int kb = 0, s = 0; ok && kb < 2 * C; ++kb, s = s + 1 == nb ? 0 : s + 1)
-                {
-                    ok = mbar_wait_warp(empty_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u, &sh->waits);
-                    if (!ok) break;
-                    par_b ^= 1u << s;
-                    tma_load_kblock_elect(tiles0 + s * step, map, kb * 64, row0, nbox, full_b0 + 8 * s);
-                }
-            else
-            for (int c = 0, s = 0; ok && c < C; ++c)
+            if (nst != last_nst)
+                for (int s = 0; ok && s < kPfStages; ++s) ok = mbar_wait_warp(empty0 + 8 * s, ((par >> s) & 1u) ^ 1u, &sh->waits);
+            last_nst = nst;
+            const uint32_t tiles0 = saddr(b_tiles), bytes = 2u * (uint32_t)nbox * kPfBoxBytes, step = (uint32_t)(kPfBBoxes / nst) * kPfBoxBytes;
+            uint32_t free = ~par, loaded = par;
+            for (int c = 0, s = 0; c < C; ++c)
             {
-                const int s1 = s + 1 == nb ? 0 : s + 1;
-                const uint32_t p0 = ((par_b >> s) & 1u) ^ 1u, p1 = ((par_b >> s1) & 1u) ^ 1u;
-                const uint32_t free = mbar_poll(empty_b0 + 8 * s, p0) & mbar_poll(empty_b0 + 8 * s1, p1);
-                if (__builtin_expect(!__all_sync(0xffffffffu, free), 0))
-                {
-                    ok = mbar_wait_slow(empty_b0 + 8 * s, p0, &sh->waits) && mbar_wait_slow(empty_b0 + 8 * s1, p1, &sh->waits);
-                    if (!ok) break;
-                }
-                par_b ^= (1u << s) | (1u << s1);
-                const uint32_t d0 = tiles0 + s * step, d1 = tiles0 + s1 * step, f0 = full_b0 + 8 * s, f1 = full_b0 + 8 * s1;
-                tma_load_chunk_elect(d0, d1, map, c * 128, row0, f0, f1, bytes);
-                for (int j = 1; j < nbox; ++j)
-                    tma_load_more_elect(d0 + j * kPfBoxBytes, d1 + j * kPfBoxBytes, map, c * 128, row0 + j * kPfBoxRows, f0, f1);
-                s = s1 + 1 == nb ? 0 : s1 + 1;
+                ok = ok && mbar_wait_warp(empty0 + 8 * s, (free >> s) & 1u, &sh->waits);
+                if (!ok) break;
+                loaded ^= 1u << s;
+                const uint32_t d0 = tiles0 + s * step, d1 = d0 + step / 2, f = full_b0 + 8 * s;
+                tma_load_chunk_elect(d0, d1, map, c * 128, row0, f, bytes);
+                for (int j = 1; j < nbox; ++j) tma_load_more_elect(d0 + j * kPfBoxBytes, d1 + j * kPfBoxBytes, map, c * 128, row0 + j * kPfBoxRows, f);
+                if (++s == nst) { s = 0; free = ~free; }
             }
-            if (sh->waits.aborted) break;
+            par = loaded;
+            if (!ok || sh->waits.aborted) break;
+            ahead.next();
+            if (!publish(at1, p1, w1, ahead)) break;
+            w1 = row_of(at2, p2);
+            at1 = at2; p1 = p2;
+            at2 = behind(at2); p2 = pass_of(at2);
         }
         __syncwarp();
-        for (int s = 0; s < kPfBStages; ++s) mbar_wait_own(full_b0 + 8 * s, ((par_b >> s) & 1u) ^ 1u);      // loads on their way
+        for (int s = 0; s < kPfStages; ++s) mbar_wait_own(full_b0 + 8 * s, ((par >> s) & 1u) ^ 1u);      // loads on their way
     }
-    else if (warp == 1)
+    else if (warp == 1 || warp == kPfSecondIssuer)
     {
         // ---- MMA issue
-        uint32_t par_a = 0, par_b = 0, nitem = 0;
-        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
+        const int who = warp == 1 ? 0 : 1;
+        uint32_t par = 0, nitem = 0;
+        bool turns_before = true;            // the previous item's accumulators are one of the two pairs
+        Head head;
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem, head.next())
         {
-            if (!wait_head(nitem)) break;
-            const int ntok = (int)uniform(sh->pass[nitem & 1u].ntok), ntok16 = (ntok + 15) & ~15, nbox = (ntok + kPfBoxRows - 1) / kPfBoxRows;
-            const int nb = b_stages(nbox), sbox = b_stage_boxes(nbox), nstages = unit_stages(ntok);
-            leave_head(nitem);
-            bool ok = mbar_wait_warp(saddr(&sh->acc_empty), (nitem & 1u) ^ 1u, &sh->waits);   // epilogue of the previous item has drained TMEM
+            if (!wait_head(head)) break;
+            const int ntok = (int)uniform(sh->item[head.slot].ntok), ntok16 = (ntok + 15) & ~15, nst = chunk_stages(ntok);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh->head_empty[head.slot]);
+            // the epilogues that have to be through: that of the item before the previous one, and that of the previous one where the two
+            // share columns
+            const uint32_t acc = nitem & 1u, phase = (nitem >> 1) & 1u;
+            const bool turns = ntok <= 32;
+            bool ok = mbar_wait_warp(saddr(&sh->acc_empty[acc]), phase ^ 1u, &sh->waits);
+            if (ok && nitem > 0 && !(turns && turns_before)) ok = mbar_wait_warp(saddr(&sh->acc_empty[acc ^ 1u]), ((nitem - 1) >> 1) & 1u, &sh->waits);
+            turns_before = turns;
             tc_fence_after();
+            const bool split = split_chunks(ntok);
+            const int first = split ? who : who ? C : 0, step = split ? 2 : 1;
+            const uint32_t tmem_d = tmem + acc_column(ntok, acc) + (who ? acc_second(ntok) : 0u);
             // N <= 256 per instruction: one MMA per k-step, or two of (nearly) equal width
-            const int n0 = ntok16 <= NQ_PF_SPLIT ? ntok16 : ((ntok16 / 2 + 15) & ~15), n1 = ntok16 - n0;
+            const int n0 = nst > 2 ? ntok16 : ((ntok16 / 2 + 15) & ~15), n1 = ntok16 - n0;
             const uint32_t idesc0 = instr_desc(n0), idesc1 = instr_desc(n1 > 0 ? n1 : 16);
             const uint64_t bdesc0 = smem_desc(saddr(b_tiles), 16, 1024, 2);
             const uint32_t b_lo0 = (uint32_t)bdesc0, b_hi = (uint32_t)(bdesc0 >> 32);
-            const uint32_t b_step = (uint32_t)(sbox * (kPfBoxBytes >> 4));
-            uint32_t s = 0, b_lo = b_lo0;                 // token-tile stage of this k-block and its descriptor
-            if (stages_one_by_one(nbox))
-                for (uint32_t kb = 0; ok && kb < 2u * C; ++kb)
-                {
-                    const uint32_t ua = (kb >> 1) & 1u, h = kb & 1u;           // (two unit stages, two column halves)
-                    ok = (h || mbar_wait_warp(full_a0 + 8 * ua, (par_a >> ua) & 1u, &sh->waits)) &&
-                         mbar_wait_warp(full_b0 + 8 * s, (par_b >> s) & 1u, &sh->waits);
-                    if (!ok) break;
-                    par_a ^= h << ua;
-                    par_b ^= 1u << s;
-                    tc_fence_after();
-                    tc_mma_kblock2(tmem, tmem + n0, tmem + kPfTmemCols - 2 * kPfACols - ua * (2 * kPfACols) + h * kPfACols, b_lo, b_lo + (uint32_t)(n0 * 8),
-                                   b_hi, idesc0, idesc1, kb, empty_a0 + 16 * ua + 8 * h, empty_b0 + 8 * s);
-                    if (++s == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else b_lo += b_step;
-                }
-            else
-            for (int c = 0, ua = 0; ok && c < C; ++c, ua = ua + 1 == nstages ? 0 : ua + 1)
+            const uint32_t b_step = (uint32_t)(kPfBBoxes / nst) * (kPfBoxBytes >> 4), b_kb = b_step / 2;
+            uint32_t full = par, s = split ? (uint32_t)who : 0u;
+            for (int c = first; ok && c < C; c += step)
             {
-                // the unit and its two token tiles: three polls, one vote, one branch
-                const uint32_t s1 = s + 1 == (uint32_t)nb ? 0 : s + 1, b_lo1 = s1 == 0 ? b_lo0 : b_lo + b_step;
-                const uint32_t pa = (par_a >> ua) & 1u, p0 = (par_b >> s) & 1u, p1 = (par_b >> s1) & 1u;
-                uint32_t ready = mbar_poll(full_a0 + 8 * ua, pa);
-                ready &= mbar_poll(full_b0 + 8 * s, p0);
-                ready &= mbar_poll(full_b0 + 8 * s1, p1);
+                // weight and token tiles: two polls, one vote, one branch
+                const uint32_t p = (full >> s) & 1u;
+                uint32_t ready = mbar_poll(full_a0 + 8 * s, p);
+                ready &= mbar_poll(full_b0 + 8 * s, p);
                 if (__builtin_expect(!__all_sync(0xffffffffu, ready), 0))
                 {
-                    ok = mbar_wait_slow(full_a0 + 8 * ua, pa, &sh->waits) && mbar_wait_slow(full_b0 + 8 * s, p0, &sh->waits) &&
-                         mbar_wait_slow(full_b0 + 8 * s1, p1, &sh->waits);
+                    ok = mbar_wait_slow(full_a0 + 8 * s, p, &sh->waits) && mbar_wait_slow(full_b0 + 8 * s, p, &sh->waits);
                     if (!ok) break;
                 }
-                par_a ^= 1u << ua;
-                par_b ^= (1u << s) | (1u << s1);
                 tc_fence_after();
-                const uint32_t ta = tmem + kPfTmemCols - 2 * kPfACols - ua * (2 * kPfACols), free_a = empty_a0 + 16 * ua;
-                if (n1 > 0)
-                {
-                    const uint32_t half = (uint32_t)(n0 * 8);
-                    tc_mma_kblock2(tmem, tmem + n0, ta, b_lo, b_lo + half, b_hi, idesc0, idesc1, (uint32_t)c, free_a, empty_b0 + 8 * s);
-                    tc_mma_kblock2(tmem, tmem + n0, ta + kPfACols, b_lo1, b_lo1 + half, b_hi, idesc0, idesc1, 1u, free_a + 8, empty_b0 + 8 * s1);
-                }
-                else
-                {
-                    tc_mma_kblock(tmem, ta, b_lo, b_hi, idesc0, (uint32_t)c, free_a, empty_b0 + 8 * s);
-                    tc_mma_kblock(tmem, ta + kPfACols, b_lo1, b_hi, idesc0, 1u, free_a + 8, empty_b0 + 8 * s1);
-                }
-                if (s1 + 1 == (uint32_t)nb) { s = 0; b_lo = b_lo0; } else { s = s1 + 1; b_lo = b_lo1 + b_step; }
+                const uint32_t b_lo = b_lo0 + s * b_step, ta = tmem + kPfTmemCols - 2 * kPfACols - s * (2 * kPfACols);
+                if (nst == 2) tc_mma_chunk2(tmem_d, tmem_d + n0, ta, b_lo, (uint32_t)(n0 * 8), b_kb, b_hi, idesc0, idesc1, (uint32_t)c, half_a0 + 8 * s, empty0 + 8 * s);
+                else tc_mma_chunk(tmem_d, ta, b_lo, b_kb, b_hi, idesc0, (uint32_t)(c - first), empty0 + 8 * s);
+                s += (uint32_t)step;
+                if (s >= (uint32_t)nst) { s -= (uint32_t)nst; full = ~full; }
             }
-            if (ok) tc_commit_elect(&sh->acc_full);
+            if (ok) tc_commit_elect(&sh->acc_full[acc]);
+            par = stage_parities(par, C, nst);
             if (sh->waits.aborted) break;
         }
         __syncwarp();
-        tc_commit_elect(&sh->mma_done);
-        mbar_wait_own(saddr(&sh->mma_done), 0);
+        tc_commit_elect(&sh->mma_done[who]);
+        mbar_wait_own(saddr(&sh->mma_done[who]), 0);
     }
     else
     {
-        // ---- decode, then epilogue
-        // A warp may touch only the 32 tensor-memory lanes of its quarter (warp % 4): the four decode warps of a
-        // quarter take its two strips x the chunk groups.
-        const int dw = warp - 2, qd = warp & 3, sub = (dw >> 2) & 1, half = dw >> 3, sidx = 2 * qd + sub;      // half = chunk group
-        const uint32_t tmem_a = tmem + ((uint32_t)(32 * qd + 16 * sub) << 16) + kPfTmemCols - 2 * kPfACols;
-        uint8_t* ring = rings + dw * kPfRingDepth * kStageBytes;
-        const int ld = a.down ? a.H : a.I;
-        uint32_t par_a = 0, nitem = 0;
-        float* prev_out = nullptr;           // the item whose accumulator this warp has still to write (prev_ntok 0: none)
-        int prev_ntok = 0, prev_stages = kPfUnitStages;
-        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem)
+        // ---- decode, then epilogue.  A warp may touch only the 32 tensor-memory lanes of its quarter (warp % 4): the four decode warps of a
+        // quarter take its two strips x the chunk groups.  Group `half` of 8 warps decodes the chunks c = half (mod kPfGroups).
+        const int half = (warp - 2) >> 3, units = (C - half + kPfGroups - 1) / kPfGroups;
+        uint32_t par = 0, nitem = 0, info = 0;
+        int prev_nst = kPfStages;
+        Head head;
+        bool left = false;                   // the previous item's accumulator is still to be written
+        for (int item = blockIdx.x; item < nitems; item += gridDim.x, ++nitem, head.next())
         {
-            if (!wait_head(nitem)) break;
-            const int64_t* row = sh->row[nitem & 1u];
-            const PfPass ps = sh->pass[nitem & 1u];
-            const int level = (int)row[0], wg = item % groups, nstages = unit_stages(ps.ntok);
-            const ProjPlanes P = planes_from_row(row, a.down);
-            const int rc = (int)row[10 + a.down], nm = a.down ? a.nm_dn : a.nm_gu, bk = (int)(row[19] >> (8 * a.down)) & 0xFF;
-            leave_head(nitem);
-            // group `half` of 8 warps decodes the chunks c = half (mod kPfGroups): k-blocks 2 c and 2 c + 1.  The epilogue
-            // of the previous item runs after this item's first unit is decoded: the MMAs of the previous item's last
-            // k-blocks finish meanwhile, and the tensor pipe finds tiles waiting when the accumulator is free again.
-            auto mid = [&]() { if (prev_ntok) { write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u); prev_ntok = 0; } };
-            const bool ok = decode_item(P, level, rc, bk, wg * 8 + sidx, C, NS, nm, lane, half, tmem_a, ring, sh, nstages, par_a,
-                                        nstages > prev_stages, (nitem - 1) & 1u, mid);
-            if (prev_ntok) { write_accumulator(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u); prev_ntok = 0; }     // (one unit or none)
-            prev_stages = nstages;
-            if (ok)
+            if (!wait_head(head)) break;
+            const PfItem& I = sh->item[head.slot];
+            const int nst = I.nst;
+            const bool drain = nst > prev_nst;
+            const uint32_t before = nitem - 1;
+            info = head.slot | (head.slot ? head.slot - 1 : kPfHeads - 1) << 2 | (uint32_t)left << 4 | (uint32_t)drain << 5 | (before & 1u) << 6 | (before >> 1 & 1u) << 7;
+            bool ok = true;
+#define NQ_RUN(MODE, CODE, RC, BK) \
+    case ((MODE) * kPfCodes + (CODE)) * 2: ok = decode_strip<MODE, RC, BK, false>(par, info); break; \
+    case ((MODE) * kPfCodes + (CODE)) * 2 + 1: ok = decode_strip<MODE, RC, BK, true>(par, info); break;
+#define NQ_RUN4(MODE) \
+    NQ_RUN(MODE, 0, 0, 0) NQ_RUN(MODE, 1, 1, 0) NQ_RUN(MODE, 2, 2, 0) NQ_RUN(MODE, 3, 3, 0) NQ_RUN(MODE, 4, 4, 0) NQ_RUN(MODE, 5, 5, 0) \
+    NQ_RUN(MODE, 6, 6, 0) NQ_RUN(MODE, 7, 7, 0) NQ_RUN(MODE, 8, 8, 0) NQ_RUN(MODE, 9, 9, 0) NQ_RUN(MODE, 10, 3, 1) NQ_RUN(MODE, 11, 9, 1)
+            switch (I.variant)
             {
-                const bool up = !a.down && wg >= a.I / 128;
-                prev_out = (up ? a.out1 : a.out0) + (size_t)ps.row0 * ld + (up ? wg - a.I / 128 : wg) * 128;
-                prev_ntok = ps.ntok;
+                NQ_RUN(0, 0, 0, 0) NQ_RUN(0, 10, 0, 1) NQ_RUN4(1) NQ_RUN4(2)
             }
-            if (sh->waits.aborted) break;
+#undef NQ_RUN4
+#undef NQ_RUN
+            par = stage_parities(par, C, nst) ^ (nst == 2 ? (units & 1u) << kPfStages : 0u);
+            if (left && units <= units_before_epilogue(nst, drain)) write_accumulator(PfInfo{info});     // (the decoder function had no unit left behind it)
+            prev_nst = nst;
+            left = ok;
+            if (!ok || sh->waits.aborted) break;
         }
-        if (prev_ntok && !sh->waits.aborted) write_accumulator_between(sh, tmem, prev_out, ld, prev_ntok, (nitem - 1) & 1u);
+        if (left && !sh->waits.aborted)
+        {
+            const uint32_t before = nitem - 1;
+            write_accumulator_between((head.slot ? head.slot - 1 : kPfHeads - 1) << 2 | (before & 1u) << 6 | (before >> 1 & 1u) << 7);
+        }
     }
     __syncwarp();
     tc_fence_before();

@@ -1,5 +1,5 @@
-// Streams of packed planes: into shared memory (RecordCursor: prefill GEMM, dense decode kernel) and straight into registers
-// (RecordReader: decode-path GEMV).
+// Streams of packed planes: into shared memory (RecordCursor: dense decode kernel) and straight into registers (RecordReader: decode-path
+// GEMV, prefill GEMM).
 //
 // Plane layout (sm120/moe.py:36-49): a record of BITS bits is cut into pieces - BITS / 128 pieces of 128 bits, then a
 // 64-, a 32- and a 16-bit piece as the binary digits of BITS % 128 say, then a tail of BITS % 16 bits - and every piece
@@ -131,7 +131,7 @@ struct RecordCursor
     }
 };
 
-// The same records read straight into registers, one unit ahead of their use (the decode-path kernel): a warp that decodes
+// The same records read straight into registers, one unit ahead of their use (decode-path kernel and prefill GEMM): a warp that decodes
 // for ~1 us between two loads needs no deeper pipeline, and the copies into shared memory, their stage addresses and the
 // reads back are gone.  Plane bytes are used once: they bypass L1, which holds the token rows.
 __device__ __forceinline__ uint4 ldg_stream128(const void* p)
@@ -160,33 +160,25 @@ __device__ __forceinline__ uint32_t ldg_stream16(const void* p)
 }
 
 template <int CODE>
-struct RecordReader
+struct RecordValues
 {
     using L = RecordLayout<CODE>;
-    const uint8_t *p128, *p64, *p32, *p16, *ptail;
     uint4 v128; uint2 v64, vtail; uint32_t v32, v16;      // pieces in flight
 
-    __device__ __forceinline__ void init(const void* plane, size_t nrec, size_t unit0, int lane)
+    // fetch record r of a plane of nrec records.  One index and one address for all pieces (a plane is far below 4 GB: offsets are 32-bit), where
+    // the reader below keeps an address per piece: the prefill GEMM has no registers for up to six of them.
+    __device__ __forceinline__ void load_at(const uint8_t* plane, uint32_t nrec, uint32_t r)
     {
-        const uint8_t* p = (const uint8_t*)plane;
-        if constexpr (L::n128) { p128 = p + unit0 * 512 + lane * 16; p += nrec * 16; }
-        if constexpr (L::has64) { p64 = p + unit0 * 256 + lane * 8; p += nrec * 8; }
-        if constexpr (L::has32) { p32 = p + unit0 * 128 + lane * 4; p += nrec * 4; }
-        if constexpr (L::has16) { p16 = p + unit0 * 64 + lane * 2; p += nrec * 2; }
-        if constexpr (L::T != 0) ptail = p + unit0 * (4 * L::T) + ((lane * L::T) >> 5) * 4;
-    }
-    // fetch the unit at the read position and move on
-    __device__ __forceinline__ void fetch()
-    {
-        if constexpr (L::n128) { v128 = ldg_stream128(p128); p128 += 512; }
-        if constexpr (L::has64) { v64 = ldg_stream64(p64); p64 += 256; }
-        if constexpr (L::has32) { v32 = ldg_stream32(p32); p32 += 128; }
-        if constexpr (L::has16) { v16 = ldg_stream16(p16); p16 += 64; }
+        constexpr uint32_t b64 = 16 * L::n128, b32 = b64 + (L::has64 ? 8 : 0), b16 = b32 + (L::has32 ? 4 : 0), bt = b16 + (L::has16 ? 2 : 0);
+        if constexpr (L::n128) v128 = ldg_stream128(plane + (size_t)r * 16);
+        if constexpr (L::has64) v64 = ldg_stream64(plane + (nrec * b64 + r * 8u));
+        if constexpr (L::has32) v32 = ldg_stream32(plane + (nrec * b32 + r * 4u));
+        if constexpr (L::has16) v16 = ldg_stream16(plane + (nrec * b16 + r * 2u));
         if constexpr (L::T != 0)
         {
-            vtail.x = ldg_stream32(ptail);
-            if constexpr (L::tail2) vtail.y = ldg_stream32(ptail + 4);
-            ptail += 4 * L::T;
+            const uint8_t* p = plane + (nrec * bt + ((r * (uint32_t)L::T) >> 5) * 4u);
+            vtail.x = ldg_stream32(p);
+            if constexpr (L::tail2) vtail.y = ldg_stream32(p + 4);
         }
     }
     // the fetched record as stream words w[0 .. kWords), bits past the record zero
@@ -204,6 +196,37 @@ struct RecordReader
             v &= (1u << L::T) - 1u;
             if constexpr (L::tail_joins) w[k - 1] |= v << 16;
             else w[k++] = v;
+        }
+    }
+};
+template <int CODE>
+struct RecordReader : RecordValues<CODE>
+{
+    using L = RecordLayout<CODE>;
+    using V = RecordValues<CODE>;
+    const uint8_t *p128, *p64, *p32, *p16, *ptail;
+
+    __device__ __forceinline__ void init(const void* plane, size_t nrec, size_t unit0, int lane)
+    {
+        const uint8_t* p = (const uint8_t*)plane;
+        if constexpr (L::n128) { p128 = p + unit0 * 512 + lane * 16; p += nrec * 16; }
+        if constexpr (L::has64) { p64 = p + unit0 * 256 + lane * 8; p += nrec * 8; }
+        if constexpr (L::has32) { p32 = p + unit0 * 128 + lane * 4; p += nrec * 4; }
+        if constexpr (L::has16) { p16 = p + unit0 * 64 + lane * 2; p += nrec * 2; }
+        if constexpr (L::T != 0) ptail = p + unit0 * (4 * L::T) + ((lane * L::T) >> 5) * 4;
+    }
+    // fetch the unit at the read position and move on
+    __device__ __forceinline__ void fetch()
+    {
+        if constexpr (L::n128) { V::v128 = ldg_stream128(p128); p128 += 512; }
+        if constexpr (L::has64) { V::v64 = ldg_stream64(p64); p64 += 256; }
+        if constexpr (L::has32) { V::v32 = ldg_stream32(p32); p32 += 128; }
+        if constexpr (L::has16) { V::v16 = ldg_stream16(p16); p16 += 64; }
+        if constexpr (L::T != 0)
+        {
+            V::vtail.x = ldg_stream32(ptail);
+            if constexpr (L::tail2) V::vtail.y = ldg_stream32(ptail + 4);
+            ptail += 4 * L::T;
         }
     }
 };

@@ -1,5 +1,5 @@
-"""The fused prefill GEMM changes its tensor-memory layout with the width of a pass (2, 4 or 6 unit stages beside the accumulator): passes of
-every width one after the other on the same CTAs, for few and odd numbers of chunks."""
+"""The fused prefill GEMM changes its layout with the width of a pass (2, 3 or 6 stages beside the accumulator; up to 64 tokens two accumulators,
+up to 32 two pairs of them in turn): passes of every width one after the other on the same CTAs, for few and odd numbers of chunks."""
 import pytest
 import torch
 
@@ -20,16 +20,29 @@ COUNTS = [384, 1, 128, 300, 129, 64, 256, 65, 385, 20, 257, 0, 127, 383, 16]
                                        (1152, 1664, "gate|up"), (2048, 1664, "gate|up"), (2048, 128, None), (2048, 256, None),
                                        (2560, 384, "down"), (2560, 640, "down")])
 def test_passes_of_every_width_in_turn(H, I, turns):
-    E, T = len(COUNTS), sum(COUNTS)
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     passes = sum((c + 383) // 384 for c in COUNTS)
     assert passes == 15 and (turns is None or passes * (I // 64 if turns == "gate|up" else H // 128) > 2 * sms)
+    _check(COUNTS, H, I)
+
+
+# Narrow passes in a row, with a wide one between: accumulators in turn and not, one chunk (nothing for the second issuing warp) to seven.
+NARROW = [31, 1, 32, 16, 33, 5, 32, 64, 2, 30, 65, 8, 31, 384, 17, 32, 129, 24]
+
+
+@pytest.mark.parametrize("H,I", [(128, 2048), (256, 2048), (384, 2048), (896, 2048), (2048, 128), (2560, 256), (2560, 640)])
+def test_narrow_passes_in_a_row(H, I):
+    _check(NARROW, H, I)
+
+
+def _check(counts, H, I):
+    E, T = len(counts), sum(counts)
     exs = [moe.Expert(H, I, seed=60 + e, rk_gu=(0, 6)[e % 2], rk_dn=7, var=True, sv=0.02) for e in range(E)]
     L = moe.MoELayer(E, H, I, Bmax=1, topk=1)
     for e in range(E):
         L.set(e, exs[e], (4, 4, 2)[e % 3])
     gen = torch.Generator().manual_seed(7)
-    sel = torch.repeat_interleave(torch.arange(E), torch.tensor(COUNTS))[torch.randperm(T, generator=gen)].view(T, 1).cuda()
+    sel = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T, generator=gen)].view(T, 1).cuda()
     x = torch.randn(T, H, generator=gen).bfloat16().half().cuda()
     rw = torch.rand(T, 1, generator=gen).half().cuda()
     ref = prefill_library(L, x, sel, rw)
