@@ -154,6 +154,22 @@ int nq_pf_gemm_within(const int64_t* table, const int32_t* plan, const void* act
 /* hits[e] += counts[e] (hits may be host-mapped; NULL = no-op).  Replaces pf_hits() (sm120/nqmoe.cu:1241-1245,1288-1293). */
 int nq_pf_hits(const int32_t* counts, int32_t* hits, int E, void* stream);
 
+/* A whole prefill call (the host side of sm120/moe.py:282-327): the entries above in order - nq_pf_sort, then for every chunk of R pairs the
+ * pass list, nq_pf_pre (or nq_pf_pre_ep, if world > 0), nq_pf_gemm, nq_pf_mid, nq_pf_gemm, nq_pf_combine.  Everything is caller-owned:
+ *   x [T][H] fp16 (not read if world > 0), sel [T][topk], rw [T][topk] fp16, out [T][H] fp32;
+ *   pe, pt, pos [T * topk], start [E + 2], sort_scratch [nq_pf_sort_scratch_ints];  hits [E] (may be host-mapped) with hit_counts [E] of
+ *   scratch, or both NULL;
+ *   for chunks of R pairs: plan [plan_ints >= nq_pf_plan_ints(E, min(R, T * topk))], xg, xu [R][H] fp16, y [R][H] fp32 (may overlay xg | xu), acc_g,
+ *   acc_u [R][I] fp32, h [R][I] fp16, zg, zd [R][4] fp32;  status int32 [1], see nq_pf_gemm. */
+typedef struct {
+    const void* x; const int64_t* sel; const void* rw; const int64_t* table; float* out;
+    int32_t *pe, *pt, *pos, *start, *sort_scratch, *hit_counts, *hits, *plan;
+    void *xg, *xu; float *y, *acc_g, *acc_u; void* h; float *zg, *zd; int32_t* status;
+    const void* const* peer_x;
+    int T, topk, E, H, I, nm_gu, nm_dn, R, plan_ints, sort_scratch_ints, world, tokens_per_rank;
+} NqPrefill;
+int nq_prefill(const NqPrefill* p, void* stream);
+
 /* ---- decode path: one MoE layer call for 1..NQ_MAX_TOKENS tokens -------------------------------------------
  * Replaces moe_forward() (sm120/nqmoe.cu:858-907).  The argument block carries the same tensors, in the same roles,
  * as the reference's positional arguments; element counts travel with the pointers because nothing here can ask a

@@ -32,6 +32,13 @@ class NqMoeForward(C.Structure):
                                    "which")])
 
 
+class NqPrefill(C.Structure):
+    _fields_ = ([(n, _p) for n in ("x", "sel", "rw", "table", "out", "pe", "pt", "pos", "start", "sort_scratch", "hit_counts", "hits", "plan",
+                                   "xg", "xu", "y", "acc_g", "acc_u", "h", "zg", "zd", "status", "peer_x")] +
+                [(n, _i) for n in ("T", "topk", "E", "H", "I", "nm_gu", "nm_dn", "R", "plan_ints", "sort_scratch_ints", "world",
+                                   "tokens_per_rank")])
+
+
 class NqMoeEp(C.Structure):
     _fields_ = [("world", _i), ("rank", _i), ("peer_recv", C.POINTER(_p)), ("peer_counters", C.POINTER(_p)), ("epoch", _p)]
 
@@ -72,6 +79,7 @@ SIGNATURES = {
     "nq_pf_plan": (_i, [_p, _p, _i, _i, _p, _i, _p]),
     "nq_pf_gemm": (_i, [_p, _p, _p, _p, _i, _p, _p, _i, _i, _i, _i, _i, _p, _p]),
     "nq_pf_gemm_within": (_i, [_p, _p, _p, _p, _i, _p, _p, _i, _i, _i, _i, _i, _p, C.c_longlong, _p]),
+    "nq_prefill": (_i, [C.POINTER(NqPrefill), _p]),
     "nq_moe_workspace": (_i, [_i, _i, _i, _i, _i, _i, C.POINTER(NqMoeWorkspace)]),
     "nq_moe_forward": (_i, [C.POINTER(NqMoeForward), _p]),
     "nq_moe_forward_ep": (_i, [C.POINTER(NqMoeForward), C.POINTER(NqMoeEp), _p]),

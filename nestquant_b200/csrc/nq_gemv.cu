@@ -104,12 +104,6 @@ __device__ __forceinline__ bool read_pick(const MoeArgs& a, int s, Pick& p)
     return (int)lv > 0 && __half2float(w) != 0.f;
 }
 
-// Programmatic dependent launch: a kernel lets its successor in the stream start launching early (launch_dependents)
-// and the successor blocks (grid_dependency_wait) until the whole predecessor grid has completed and its writes are
-// visible, before it touches anything.
-__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ int ld_acquire(const int* p)
 {
     int v;

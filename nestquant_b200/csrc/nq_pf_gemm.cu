@@ -35,7 +35,7 @@
 #include <cuda.h>
 
 #include "nq_common.cuh"
-#include "nq_scan.cuh"
+#include "nq_plan.cuh"
 #include "nq_unit.cuh"
 
 namespace nq {
@@ -45,7 +45,6 @@ constexpr int kPfGroups = 2;                         // groups of 8 decode warps
 constexpr int kPfDecodeWarps = 8 * kPfGroups;
 constexpr int kPfACols = 32;                         // weight tile [128 lanes x 64 k] fp16 = 32 columns; a unit stage is two of them
 constexpr int kPfTmemCols = 512;                     // the accumulator from column 0 on, unit stages from the top down
-constexpr int kPfTokens = 384;                       // most tokens per pass (accumulator columns)
 constexpr int kPfStages = 6;                         // most stages of a pass (chunk_stages)
 constexpr int kPfBoxRows = 64;                       // token rows per TMA box
 constexpr int kPfBoxBytes = kPfBoxRows * 128;        // [64 rows][64 k] fp16
@@ -53,8 +52,6 @@ constexpr int kPfBBoxes = 24;                        // token-tile region: 6, 3 
 constexpr int kPfSecondIssuer = 2 + kPfDecodeWarps;      // warp 1 and this one issue MMAs
 constexpr int kPfThreads = 32 * (kPfSecondIssuer + 1);
 constexpr long long kPfWaitNs = 2000000000ll;             // a wait that lasts 2 s is treated as a hang, unless the caller has another limit
-
-struct PfPass { int expert, row0, ntok, pad; };
 
 struct PfGemmArgs
 {
@@ -606,6 +603,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     const int warp = (int)uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (saddr(b_tiles) & 1023u)          // (never: the swizzled tiles would be read from the wrong places)
     {
+        grid_dependency_wait();
         if (threadIdx.x == 0) atomicExch(a.status, 1);
         return;
     }
@@ -628,6 +626,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();
     const uint32_t tmem = uniform(sh->tmem_base);
 
     const int N = a.down ? a.H : 2 * a.I, K = a.down ? a.I : a.H, C = K / 128, NS = N / 16, groups = N / 128;
@@ -823,6 +822,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             write_accumulator_between((head.slot ? head.slot - 1 : kPfHeads - 1) << 2 | (before & 1u) << 6 | (before >> 1 & 1u) << 7);
         }
     }
+    // Not at the start: with CTAs of the next pass waiting beside this one's, whole prefill calls took 7 % longer (geometric mean over 54 of 50 to 1,200 us).
+    launch_dependents();
     __syncwarp();
     tc_fence_before();
     __syncthreads();
@@ -831,57 +832,15 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kPfTmemCols) : "memory");
 }
 
-// ---------------------------------------------------------------- pass plan (device side, no host sync)
-// A pass = one expert x up to 384 of its pairs (pairs are sorted by expert); experts at level 0 get none.  plan: [0] passes,
-// [1] pairs covered, then PfPass records from int 4 on, in expert order.
-//   WINDOW = false  from[e] = routed pairs of expert e, in the order of the pair list; the plan covers the whole list
-//   WINDOW = true   from[e] = first pair of expert e in the sorted list (from[E] = end of the last expert's pairs); the plan covers
-//                   the pairs [pair0, pair0 + npairs) with rows counted from pair0
-// One CTA, a thread per expert: sums over the CTA (passes before the expert, pairs before it) place every record.  One thread
-// that walks the experts alone pays two dependent loads for each of them.
-constexpr int kPlanThreads = 1024;
-
+// ---------------------------------------------------------------- pass plan (device side, no host sync), see nq_plan.cuh
 template <bool WINDOW>
 __global__ void __launch_bounds__(kPlanThreads) pf_plan_kernel(const int* __restrict__ from, const int64_t* __restrict__ table, int E,
                                                                int pair0, int npairs, int* plan, int max_passes)
 {
     __shared__ int s_warp[kPlanThreads / 32];
-    PfPass* out = (PfPass*)(plan + 4);
-    int n = 0, rows = 0, covered = 0;     // passes, pairs and covered pairs of the experts handled so far
-    for (int e0 = 0; e0 < E; e0 += kPlanThreads)
-    {
-        const int e = e0 + (int)threadIdx.x;
-        int first = 0, c = 0, total;
-        bool live = false;
-        if (e < E)
-        {
-            live = table[(int64_t)e * kTableWidth] > 0;
-            if constexpr (WINDOW)
-            {
-                const int a = max(from[e], pair0), b = min(from[e + 1], pair0 + npairs);
-                first = a - pair0; c = b - a;
-            }
-            else c = from[e];
-        }
-        if constexpr (!WINDOW)
-        {
-            first = rows + cta_exclusive_sum(c, s_warp, total);
-            rows += total;
-        }
-        const int np = live && c > 0 ? (c + kPfTokens - 1) / kPfTokens : 0;
-        const int at = n + cta_exclusive_sum(np, s_warp, total);
-        const int kept = max(min(np, max_passes - at), 0);
-        for (int i = 0; i < kept; ++i)
-        {
-            PfPass ps;
-            ps.expert = e; ps.row0 = first + i * kPfTokens; ps.ntok = min(c - i * kPfTokens, kPfTokens); ps.pad = 0;
-            out[at + i] = ps;
-        }
-        n = min(n + total, max_passes);
-        cta_exclusive_sum(kept > 0 ? min(c, kept * kPfTokens) : 0, s_warp, total);
-        covered += total;
-    }
-    if (threadIdx.x == 0) { plan[0] = n; plan[1] = covered; plan[2] = plan[3] = 0; }
+    launch_dependents();
+    grid_dependency_wait();
+    plan_passes<WINDOW>(from, table, E, pair0, npairs, plan, max_passes, s_warp);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -919,7 +878,7 @@ int nq_pf_plan(const int32_t* counts, const int64_t* table, int E, int pairs, in
 {
     NQ_REQUIRE(counts && table && plan && E > 0 && pairs >= 0, "nq_pf_plan: bad arguments");
     NQ_REQUIRE(plan_ints >= nq_pf_plan_ints(E, pairs), "nq_pf_plan: plan needs %d ints", nq_pf_plan_ints(E, pairs));
-    nq::pf_plan_kernel<false><<<1, nq::kPlanThreads, 0, (cudaStream_t)stream>>>(counts, table, E, 0, 0, plan, (plan_ints - 4) / 4);
+    nq::launch_dependent(nq::pf_plan_kernel<false>, dim3(1), dim3(nq::kPlanThreads), 0, (cudaStream_t)stream, counts, table, E, 0, 0, plan, (plan_ints - 4) / 4);
     return nq::check_launch("nq_pf_plan");
 }
 
@@ -927,7 +886,7 @@ int nq_pf_plan_window(const int32_t* start, const int64_t* table, int E, int pai
 {
     NQ_REQUIRE(start && table && plan && E > 0 && pair0 >= 0 && npairs >= 0, "nq_pf_plan_window: bad arguments");
     NQ_REQUIRE(plan_ints >= nq_pf_plan_ints(E, npairs), "nq_pf_plan_window: plan needs %d ints", nq_pf_plan_ints(E, npairs));
-    nq::pf_plan_kernel<true><<<1, nq::kPlanThreads, 0, (cudaStream_t)stream>>>(start, table, E, pair0, npairs, plan, (plan_ints - 4) / 4);
+    nq::launch_dependent(nq::pf_plan_kernel<true>, dim3(1), dim3(nq::kPlanThreads), 0, (cudaStream_t)stream, start, table, E, pair0, npairs, plan, (plan_ints - 4) / 4);
     return nq::check_launch("nq_pf_plan_window");
 }
 
@@ -957,11 +916,13 @@ int nq_pf_gemm_within(const int64_t* table, const int32_t* plan, const void* act
     CUtensorMap m0, m1;
     const size_t K = down ? I : H;
     if (int e = nq::make_tile_map(&m0, act0, (size_t)pairs, K)) return e;
-    if (int e = nq::make_tile_map(&m1, down ? act0 : act1, (size_t)pairs, K)) return e;
+    m1 = m0;
+    if (!down)
+        if (int e = nq::make_tile_map(&m1, act1, (size_t)pairs, K)) return e;
     nq::PfGemmArgs a{};
     a.table = table; a.plan = plan; a.out0 = out0; a.out1 = out1; a.status = status;
     a.H = H; a.I = I; a.nm_gu = nm_gu; a.nm_dn = nm_dn; a.down = down ? 1 : 0; a.wait_ns = wait_ns;
-    nq::pf_gemm_kernel<<<ctas, nq::kPfThreads, nq::kPfSmem, (cudaStream_t)stream>>>(m0, m1, a);
+    nq::launch_dependent(nq::pf_gemm_kernel, dim3(ctas), dim3(nq::kPfThreads), nq::kPfSmem, (cudaStream_t)stream, m0, m1, a);
     return nq::check_launch("nq_pf_gemm");
 }
 

@@ -21,7 +21,7 @@
 
 #include "nq_common.cuh"
 #include "nq_format.cuh"
-#include "nq_scan.cuh"
+#include "nq_plan.cuh"
 
 namespace nq {
 
@@ -43,6 +43,8 @@ __device__ __forceinline__ int pick_bin(const int64_t* __restrict__ sel, const _
 __global__ void __launch_bounds__(32 * kSortWarps) sort_count_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
                                                                     const int64_t* __restrict__ table, int P, int E, int* hist, int* hits)
 {
+    launch_dependents();
+    grid_dependency_wait();
     extern __shared__ int s_hist[];      // [kSortWarps][E + 1]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slice = blockIdx.x * kSortWarps + warp, nb = E + 1;
     int* h = s_hist + warp * nb;
@@ -65,6 +67,8 @@ __global__ void __launch_bounds__(32 * kSortWarps) sort_count_kernel(const int64
 // the bin instead.  A CTA takes 32 bins (a lane each), its 32 warps equal runs of slices: every load is independent.
 __global__ void __launch_bounds__(1024) sort_offset_kernel(int* hist, int nslices, int E)
 {
+    launch_dependents();
+    grid_dependency_wait();
     __shared__ int s_sum[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = E + 1, b = blockIdx.x * 32 + lane;
     const int per = (nslices + 31) / 32, s0 = warp * per, s1 = min(s0 + per, nslices);
@@ -85,20 +89,24 @@ __global__ void __launch_bounds__(1024) sort_offset_kernel(int* hist, int nslice
     if (b >= nb) return;
     for (int s = s0; s < s1; ++s)
     {
-        const int c = hist[(size_t)s * nb + b];
+        const int c = __ldcg(hist + (size_t)s * nb + b);
         hist[(size_t)s * nb + b] = s ? run : total;
         run += c;
     }
 }
 
 // size[b] -> s_start[b] = picks of earlier bins, s_start[nb] = all picks; whole CTA.  size and s_start may be the same array.
+// GLOBAL: size is an array that the kernel before this one both read and wrote (its CTAs share lines of it), so it comes from L2, not from what
+// that kernel left in this SM's L1.
+template <bool GLOBAL>
 __device__ __forceinline__ void scan_bins(const int* size, int nb, int* s_start, int* s_warp)
 {
+    auto at = [&](int b) { return GLOBAL ? __ldcg(size + b) : size[b]; };
     const int per = (nb + (int)blockDim.x - 1) / (int)blockDim.x, b0 = (int)threadIdx.x * per, b1 = min(b0 + per, nb);
     int sum = 0, total;
-    for (int b = b0; b < b1; ++b) sum += size[b];
+    for (int b = b0; b < b1; ++b) sum += at(b);
     int run = cta_exclusive_sum(sum, s_warp, total);
-    for (int b = b0; b < b1; ++b) { const int c = size[b]; s_start[b] = run; run += c; }
+    for (int b = b0; b < b1; ++b) { const int c = at(b); s_start[b] = run; run += c; }
     if (threadIdx.x == 0) s_start[nb] = total;
     __syncthreads();
 }
@@ -120,18 +128,20 @@ __device__ __forceinline__ void place_picks(int* nx, int b, int i, int topk, int
 // pass 3: place every pick.  Every CTA adds up the bin sizes itself (row 0 of hist); CTA 0 writes them out as start.
 __global__ void __launch_bounds__(32 * kSortWarps) sort_place_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
                                                                     const int64_t* __restrict__ table, int P, int E, int topk,
-                                                                    const int* __restrict__ hist, int* start, int* pe, int* pt, int* pos)
+                                                                    const int* hist, int* start, int* pe, int* pt, int* pos)
 {
+    launch_dependents();
+    grid_dependency_wait();
     extern __shared__ int s_next[];      // [kSortWarps][E + 1]: next free place of each bin for this slice
     __shared__ int s_start[kSortMaxBins + 1], s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slice = blockIdx.x * kSortWarps + warp, nb = E + 1;
-    scan_bins(hist, nb, s_start, s_warp);
+    scan_bins<true>(hist, nb, s_start, s_warp);
     if (blockIdx.x == 0)
         for (int b = threadIdx.x; b <= nb; b += blockDim.x) start[b] = s_start[b];
     int* nx = s_next + warp * nb;
     const int i0 = slice * kSortSlice;
     if (i0 >= P) return;                 // warp-uniform
-    for (int b = lane; b < nb; b += 32) nx[b] = s_start[b] + (slice ? hist[(size_t)slice * nb + b] : 0);
+    for (int b = lane; b < nb; b += 32) nx[b] = s_start[b] + (slice ? __ldcg(hist + (size_t)slice * nb + b) : 0);
     __syncwarp();
     for (int base = i0; base < i0 + kSortSlice && base < P; base += 32)
     {
@@ -142,12 +152,15 @@ __global__ void __launch_bounds__(32 * kSortWarps) sort_place_kernel(const int64
 }
 
 // The three passes in one CTA of 32 warps, the counts in shared memory: up to 32 slices (8,192 picks).  A slice is a multiple of
-// 32 picks, no longer than needed, and a lane keeps its picks' bins in registers between the passes.
+// 32 picks, no longer than needed, and a lane keeps its picks' bins in registers between the passes.  If the whole list is one chunk, its
+// pass list too.
 constexpr int kSortSmallPicks = 32 * kSortSlice;
 __global__ void __launch_bounds__(1024) sort_small_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
                                                           const int64_t* __restrict__ table, int P, int E, int topk, int* start, int* hits,
-                                                          int* pe, int* pt, int* pos)
+                                                          int* pe, int* pt, int* pos, int* plan, int max_passes)
 {
+    launch_dependents();
+    grid_dependency_wait();
     extern __shared__ int s_hist[];      // [32][E + 1] counts, then next free places; [E + 2] bin sizes, then starts
     __shared__ int s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = E + 1;
@@ -181,13 +194,43 @@ __global__ void __launch_bounds__(1024) sort_small_kernel(const int64_t* __restr
         s_start[b] = run;
     }
     __syncthreads();
-    scan_bins(s_start, nb, s_start, s_warp);
+    scan_bins<false>(s_start, nb, s_start, s_warp);
     for (int b = threadIdx.x; b <= nb; b += blockDim.x) start[b] = s_start[b];
     for (int b = lane; b < nb; b += 32) h[b] += s_start[b];
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < kSortSlice / 32; ++j)
         if (32 * j < slice) place_picks(h, bin[j], i0 + 32 * j + lane, topk, lane, pe, pt, pos);
+    if (plan) plan_passes<true>(s_start, table, E, 0, P, plan, max_passes, s_warp);
+}
+
+// the sort, and the pass list of the whole window if plan is given
+int sort_pairs(const int64_t* sel, const void* rw, const int64_t* table, int T, int topk, int E, int32_t* pe, int32_t* pt, int32_t* pos, int32_t* start,
+               int32_t* hits, int32_t* scratch, int scratch_ints, int32_t* plan, int plan_ints, void* stream)
+{
+    NQ_REQUIRE(T >= 0 && topk >= 1 && E >= 1 && E + 1 <= kSortMaxBins, "nq_pf_sort: T = %d, topk = %d, E = %d", T, topk, E);
+    NQ_REQUIRE((long long)T * topk <= 0x7fffffffLL, "nq_pf_sort: too many pairs");
+    const int P = T * topk;
+    NQ_REQUIRE(start, "nq_pf_sort: null start array");
+    cudaStream_t st = (cudaStream_t)stream;
+    if (P == 0) return cudaMemsetAsync(start, 0, sizeof(int32_t) * (E + 2), st) == cudaSuccess ? NQ_OK : fail(NQ_ERR_CUDA, "nq_pf_sort: memset failed");
+    NQ_REQUIRE(sel && rw && table && pe && pt && pos && scratch, "nq_pf_sort: null pointer");
+    NQ_REQUIRE(scratch_ints >= nq_pf_sort_scratch_ints(P, E), "nq_pf_sort: scratch needs %d ints", nq_pf_sort_scratch_ints(P, E));
+    const size_t small = sizeof(int) * (33 * (size_t)(E + 1) + 1);
+    if (P <= kSortSmallPicks && small <= kSortSmallShared)
+    {
+        launch_dependent(sort_small_kernel, dim3(1), dim3(1024), small, st, sel, (const __half*)rw, table, P, E, topk, start, hits, pe, pt, pos, plan, (plan_ints - 4) / 4);
+        return check_launch("nq_pf_sort");
+    }
+    const int slices = (P + kSortSlice - 1) / kSortSlice, ctas = (slices + kSortWarps - 1) / kSortWarps;
+    const size_t smem = sizeof(int) * kSortWarps * (E + 1);
+    launch_dependent(sort_count_kernel, dim3(ctas), dim3(32 * kSortWarps), smem, st, sel, (const __half*)rw, table, P, E, scratch, hits);
+    if (int e = check_launch("nq_pf_sort(count)")) return e;
+    launch_dependent(sort_offset_kernel, dim3((E + 1 + 31) / 32), dim3(1024), 0, st, scratch, slices, E);
+    if (int e = check_launch("nq_pf_sort(offset)")) return e;
+    launch_dependent(sort_place_kernel, dim3(ctas), dim3(32 * kSortWarps), smem, st, sel, (const __half*)rw, table, P, E, topk, scratch, start, pe, pt, pos);
+    if (int e = check_launch("nq_pf_sort(place)")) return e;
+    return plan ? nq_pf_plan_window(start, table, E, 0, P, plan, plan_ints, stream) : NQ_OK;
 }
 
 }  // namespace nq
@@ -205,28 +248,7 @@ int nq_pf_sort_scratch_ints(int pairs, int E)
 int nq_pf_sort(const int64_t* sel, const void* rw, const int64_t* table, int T, int topk, int E, int32_t* pe, int32_t* pt, int32_t* pos,
                int32_t* start, int32_t* hits, int32_t* scratch, int scratch_ints, void* stream)
 {
-    NQ_REQUIRE(T >= 0 && topk >= 1 && E >= 1 && E + 1 <= nq::kSortMaxBins, "nq_pf_sort: T = %d, topk = %d, E = %d", T, topk, E);
-    NQ_REQUIRE((long long)T * topk <= 0x7fffffffLL, "nq_pf_sort: too many pairs");
-    const int P = T * topk;
-    NQ_REQUIRE(start, "nq_pf_sort: null start array");
-    cudaStream_t st = (cudaStream_t)stream;
-    if (P == 0) return cudaMemsetAsync(start, 0, sizeof(int32_t) * (E + 2), st) == cudaSuccess ? NQ_OK : nq::fail(NQ_ERR_CUDA, "nq_pf_sort: memset failed");
-    NQ_REQUIRE(sel && rw && table && pe && pt && pos && scratch, "nq_pf_sort: null pointer");
-    NQ_REQUIRE(scratch_ints >= nq_pf_sort_scratch_ints(P, E), "nq_pf_sort: scratch needs %d ints", nq_pf_sort_scratch_ints(P, E));
-    const size_t small = sizeof(int) * (33 * (size_t)(E + 1) + 1);
-    if (P <= nq::kSortSmallPicks && small <= nq::kSortSmallShared)
-    {
-        nq::sort_small_kernel<<<1, 1024, small, st>>>(sel, (const __half*)rw, table, P, E, topk, start, hits, pe, pt, pos);
-        return nq::check_launch("nq_pf_sort");
-    }
-    const int slices = (P + nq::kSortSlice - 1) / nq::kSortSlice, ctas = (slices + nq::kSortWarps - 1) / nq::kSortWarps;
-    const size_t smem = sizeof(int) * nq::kSortWarps * (E + 1);
-    nq::sort_count_kernel<<<ctas, 32 * nq::kSortWarps, smem, st>>>(sel, (const __half*)rw, table, P, E, scratch, hits);
-    if (int e = nq::check_launch("nq_pf_sort(count)")) return e;
-    nq::sort_offset_kernel<<<(E + 1 + 31) / 32, 1024, 0, st>>>(scratch, slices, E);
-    if (int e = nq::check_launch("nq_pf_sort(offset)")) return e;
-    nq::sort_place_kernel<<<ctas, 32 * nq::kSortWarps, smem, st>>>(sel, (const __half*)rw, table, P, E, topk, scratch, start, pe, pt, pos);
-    return nq::check_launch("nq_pf_sort(place)");
+    return nq::sort_pairs(sel, rw, table, T, topk, E, pe, pt, pos, start, hits, scratch, scratch_ints, nullptr, 4, stream);
 }
 
 }  // extern "C"

@@ -83,6 +83,8 @@ __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows
                                                      const int64_t* __restrict__ table, int E, __half* xg, __half* xu, float* zg, int H, int I,
                                                      int kperm, int R)
 {
+    launch_dependents();
+    grid_dependency_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = H / 128;
     const int per = (R + (int)gridDim.x - 1) / (int)gridDim.x, p0 = (int)blockIdx.x * per, p1 = p0 + per < R ? p0 + per : R;
     const int q = lane & 3;
@@ -151,6 +153,8 @@ template <bool WIDE>
 __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, const float* __restrict__ zg,
                                                      const int* __restrict__ pe, const int64_t* __restrict__ table, int E, __half* h, float* zd, int H, int I, int kperm)
 {
+    launch_dependents();
+    grid_dependency_wait();
     extern __shared__ float stage[];
     __shared__ float zpart[64][4];
     const int p = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = I / 128;
@@ -276,6 +280,8 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const flo
                                                       const int* __restrict__ pe, const __half* __restrict__ prw,
                                                       const int64_t* __restrict__ table, int E, float* out, int H, int I)
 {
+    launch_dependents();
+    grid_dependency_wait();
     const int p = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = H / 128;
     if (pe[p] < 0 || pe[p] >= E) return;
     const float w = __half2float(prw[p]);
@@ -303,6 +309,8 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_combine_kernel(const 
                                                          const int64_t* __restrict__ table, float* out, int topk, int E, int H, int I,
                                                          int pair0, int npairs, int accumulate)
 {
+    launch_dependents();
+    grid_dependency_wait();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = H / 128;
     bool any = false;
     for (int k = 0; k < topk; ++k)
@@ -386,7 +394,7 @@ int nq_pf_pre(const void* x, const int32_t* pt, const int32_t* pe, int R, const 
     nq::TokenRows rows{};
     rows.base[0] = (const __half*)x; rows.tokens_per_rank = 0x7fffffff;
     const bool wide = nq::aligned32(x) && nq::aligned32(xg) && nq::aligned32(xu);
-    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R, H), nq::pf_pre_threads(H), 0, (cudaStream_t)stream>>>(
+    nq::launch_dependent(wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>, dim3(nq::pf_pre_grid(R, H)), dim3(nq::pf_pre_threads(H)), 0, (cudaStream_t)stream,
         rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
     return nq::check_launch("nq_pf_pre");
 }
@@ -410,7 +418,7 @@ int nq_pf_pre_ep(const void* const* peer_x, int world, int tokens_per_rank, cons
         wide = wide && nq::aligned32(peer_x[r]);
     }
     rows.tokens_per_rank = tokens_per_rank;
-    (wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>)<<<nq::pf_pre_grid(R, H), nq::pf_pre_threads(H), 0, (cudaStream_t)stream>>>(
+    nq::launch_dependent(wide ? nq::pf_pre_kernel<true> : nq::pf_pre_kernel<false>, dim3(nq::pf_pre_grid(R, H)), dim3(nq::pf_pre_threads(H)), 0, (cudaStream_t)stream,
         rows, pt, pe, table, E, (__half*)xg, (__half*)xu, zg, H, I, kperm, R);
     return nq::check_launch("nq_pf_pre_ep");
 }
@@ -424,7 +432,7 @@ int nq_pf_mid(const float* acc_g, const float* acc_u, const float* zg, const int
     NQ_SHAPE_OK("nq_pf_mid");
     NQ_REQUIRE(E >= 1, "nq_pf_mid: E = %d", E);
     NQ_REQUIRE(nq::aligned16(acc_g) && nq::aligned16(acc_u) && nq::aligned16(h), "nq_pf_mid: acc_g, acc_u, h must be 16-byte aligned");
-    (nq::aligned32(acc_g) && nq::aligned32(acc_u) ? nq::pf_mid_kernel<true> : nq::pf_mid_kernel<false>)<<<R, nq::pf_threads(I), (size_t)I * 4, (cudaStream_t)stream>>>(
+    nq::launch_dependent(nq::aligned32(acc_g) && nq::aligned32(acc_u) ? nq::pf_mid_kernel<true> : nq::pf_mid_kernel<false>, dim3(R), dim3(nq::pf_threads(I)), (size_t)I * 4, (cudaStream_t)stream,
         acc_g, acc_u, zg, pe, table, E, (__half*)h, zd, H, I, kperm);
     return nq::check_launch("nq_pf_mid");
 }
@@ -438,7 +446,7 @@ int nq_pf_post(const float* y, const float* zd, const int32_t* pt, const int32_t
     NQ_SHAPE_OK("nq_pf_post");
     NQ_REQUIRE(E >= 1, "nq_pf_post: E = %d", E);
     NQ_REQUIRE(nq::aligned16(y) && nq::aligned16(out), "nq_pf_post: y and out must be 16-byte aligned");
-    nq::pf_post_kernel<<<R, nq::pf_threads(H), 0, (cudaStream_t)stream>>>(y, zd, pt, pe, (const __half*)prw, table, E, out, H, I);
+    nq::launch_dependent(nq::pf_post_kernel, dim3(R), dim3(nq::pf_threads(H)), 0, (cudaStream_t)stream, y, zd, pt, pe, (const __half*)prw, table, E, out, H, I);
     return nq::check_launch("nq_pf_post");
 }
 
@@ -451,7 +459,7 @@ int nq_pf_combine(const float* y, const float* zd, const int32_t* pos, const int
     NQ_REQUIRE(y && zd && pos && sel && rw && table && out, "nq_pf_combine: null pointer");
     NQ_SHAPE_OK("nq_pf_combine");
     NQ_REQUIRE(nq::aligned16(y) && nq::aligned16(out), "nq_pf_combine: y and out must be 16-byte aligned");
-    (nq::aligned32(y) && nq::aligned32(out) ? nq::pf_combine_kernel<true> : nq::pf_combine_kernel<false>)<<<T, nq::pf_threads(H), 0, (cudaStream_t)stream>>>(
+    nq::launch_dependent(nq::aligned32(y) && nq::aligned32(out) ? nq::pf_combine_kernel<true> : nq::pf_combine_kernel<false>, dim3(T), dim3(nq::pf_threads(H)), 0, (cudaStream_t)stream,
         y, zd, pos, sel, (const __half*)rw, table, out, topk, E, H, I, pair0, npairs, accumulate);
     return nq::check_launch("nq_pf_combine");
 }

@@ -167,6 +167,38 @@ def pf_hits(counts, hits_ptr):
     check(lib().nq_pf_hits(ptr(counts), hits_ptr, counts.numel(), current_stream()), "pf_hits")
 
 
+def prefill(x, sel, rw, table, out, perm, scratch, R, I, nm_gu, nm_dn, hits_ptr=0, x_peers=None):
+    """One whole prefill call (nq_prefill): sel int64 / rw fp16 [T,topk], x fp16 [T,H] (ignored if x_peers = (device addresses of the ranks' input
+    buffers, tokens per rank) is given), out fp32 [T,H].  perm: pe, pt, pos, start, hit, scratch as for pf_sort; scratch: xg, xu, y, acc_g,
+    acc_u, h, zg, zd, plan, status with at least R rows each, for chunks of R pairs"""
+    _need(sel, torch.int64, "sel"); _need(rw, torch.float16, "rw"); _need(table, torch.int64, "table"); _need(out, torch.float32, "out")
+    T, topk = sel.shape
+    H, E, P = scratch["y"].shape[1], table.shape[0], T * topk
+    if rw.numel() < P or out.numel() < T * H or R > scratch["R"] or P > perm["P"]:
+        raise NestQuantError("prefill sizes: rw [T,topk], out [T,H], scratch for R pairs, index arrays for T * topk")
+    a, peers = capi.NqPrefill(), None
+    if x_peers is None:
+        _need(x, torch.float16, "x")
+        if x.dim() != 2 or x.shape[1] != H or x.shape[0] < T:
+            raise NestQuantError(f"prefill: x {tuple(x.shape)}, expected [{T}, {H}]")
+        a.x = x.data_ptr()
+    else:
+        peers = (C.c_void_p * len(x_peers[0]))(*x_peers[0])         # (lives until the call below)
+        a.peer_x = C.addressof(peers)
+        a.world, a.tokens_per_rank = len(x_peers[0]), x_peers[1]
+    a.sel, a.rw, a.table, a.out = sel.data_ptr(), rw.data_ptr(), table.data_ptr(), out.data_ptr()
+    for n in ("pe", "pt", "pos", "start"):
+        setattr(a, n, perm[n].data_ptr())
+    a.sort_scratch, a.sort_scratch_ints = perm["scratch"].data_ptr(), perm["scratch"].numel()
+    if hits_ptr:
+        a.hit_counts, a.hits = perm["hit"].data_ptr(), hits_ptr
+    for n in ("xg", "xu", "y", "acc_g", "acc_u", "h", "zg", "zd", "plan", "status"):
+        setattr(a, n, scratch[n].data_ptr())
+    a.plan_ints = scratch["plan"].numel()
+    a.T, a.topk, a.E, a.H, a.I, a.nm_gu, a.nm_dn, a.R = T, topk, E, H, I, nm_gu, nm_dn, R
+    check(lib().nq_prefill(C.byref(a), current_stream()), "prefill")
+
+
 def operand_order(K):
     """int64 [K]: position of element k of a row in the "operand order" of the decode path's internal fp16 rows (h, and the
     rotated inputs in shared memory): inside every 128 consecutive k, k = 16 T + 2 t4 + 8 hi + e sits at 32 t4 + 4 T + 2 hi + e"""

@@ -376,7 +376,7 @@ class MoELayer:
         TMEM; dense weights never touch HBM), same math as __call__.  x fp16 [T,H], sel int64 [T,topk], rw fp16 [T,topk] ->
         fp32 [T,H].  Same call shape as the reference's prefill (sm120/moe.py:282-327).
         R: pairs per scratch chunk (default 65536 = an 8192-token window of top-8 picks; the scratch, ~45 KB per pair at
-        the GLM shape, is allocated once per R and kept).  The expert-sorted pair list is processed chunk by chunk and each
+        the GLM shape, is kept between calls and grows with them).  The expert-sorted pair list is processed chunk by chunk and each
         token's picks are added chunk after chunk in pick order, so the result is bitwise repeatable for a given R.
         G (experts decoded per group in the reference) is accepted and ignored: nothing is decoded ahead of the GEMM.
         Picks whose expert id is outside [0, E) (e.g. -1 padding) are ignored, as on the decode path.
@@ -387,7 +387,7 @@ class MoELayer:
         prefill_status() reads."""
         assert x.dtype == torch.float16 and rw.dtype == torch.float16 and sel.dtype == torch.int64, (x.dtype, rw.dtype, sel.dtype)
         T, k = sel.shape
-        H, I, E, M, dev = s.H, s.I, s.E, s.M, sel.device
+        H, I, M, dev = s.H, s.I, s.M, sel.device
         tb = s.table if table is None else table
         P = T * k
         R = max(1, min(R or 65536, P))
@@ -395,40 +395,22 @@ class MoELayer:
         if P == 0:
             return out
         sc = s._prefill_scratch(R, dev)
-        # pairs sorted by expert on the device: pe / pt of each sorted pair, pos of each pick, first pair of each expert.  Picks
-        # that contribute nothing (no valid expert id, expert not resident here, zero weight) sort behind every real pair.
+        # one call for all of it: the pairs sorted by expert on the device (picks that contribute nothing - no valid expert id, expert not
+        # resident here, zero weight - sort behind every real pair), then chunk by chunk pass list, rotations, GEMMs and combine, where y
+        # overwrites xg | xu
         sel, rw = sel.contiguous(), rw.contiguous()
-        perm = s._prefill_perm(P, dev)
-        pe, pt, pos = perm["pe"][:P], perm["pt"][:P], perm["pos"][:P]
-        hit = None
-        if s.hits_ptr:
-            hit = perm["hit"].zero_()
-        M.pf_sort(sel, rw, tb, pe, pt, pos, perm["start"], hit, perm["scratch"])
-        if s.hits_ptr:
-            M.pf_hits(hit, s.hits_ptr)
-        for c0 in range(0, P, R):
-            n = min(R, P - c0)
-            M.pf_plan_window(perm["start"], tb, sc["plan"], c0, n)       # pass list of this chunk, built on the device
-            xg, xu, y = sc["xg"][:n], sc["xu"][:n], sc["y"][:n]
-            if x_peers is None:
-                M.pf_pre(x, pt[c0:c0 + n], pe[c0:c0 + n], tb, xg, xu, sc["zg"], I, kperm=True)
-            else:
-                M.pf_pre_ep(x_peers[0], x_peers[1], H, pt[c0:c0 + n], pe[c0:c0 + n], tb, xg, xu, sc["zg"], I, kperm=True)
-            M.pf_gemm(tb, sc["plan"], xg, xu, sc["acc_g"], sc["acc_u"], H, I, s.nm_gu, s.nm_dn, False, sc["status"])
-            M.pf_mid(sc["acc_g"], sc["acc_u"], sc["zg"], pe[c0:c0 + n], tb, sc["h"], sc["zd"], H, I, kperm=True)
-            M.pf_gemm(tb, sc["plan"], sc["h"][:n], None, y, None, H, I, s.nm_gu, s.nm_dn, True, sc["status"])     # y overwrites xg | xu
-            M.pf_combine(y, sc["zd"], pos, sel, rw, tb, out, I, pair0=c0, npairs=n, accumulate=c0 > 0)
+        M.prefill(x, sel, rw, tb, out, s._prefill_perm(P, dev), sc, R, I, s.nm_gu, s.nm_dn, s.hits_ptr, x_peers)
         return out
 
     def _prefill_scratch(s, R, dev):
-        """scratch of the prefill path for chunks of R pairs, kept between calls (the reference's pf_scratch,
+        """scratch of the prefill path for chunks of up to R pairs, kept between calls, the largest asked for so far (the reference's pf_scratch,
         sm120/moe.py:263-275, without its dense weight buffers): xg | xu fp16 [R,H] each, aliased by y fp32 [R,H];
         acc_g, acc_u fp32 [R,I]; h fp16 [R,I]; zg, zd fp32 [R,4]; the pass list; the status word"""
         owner = getattr(s, "_pf_owner", None)
         if owner is not None:
             return owner._prefill_scratch(R, dev)
         sc = getattr(s, "_pf_sc", None)
-        if sc is not None and sc["R"] == R and sc["y"].device == dev:
+        if sc is not None and sc["R"] >= R and sc["y"].device == dev:
             return sc
         H, I, E = s.H, s.I, s.E
         f16, f32, i32 = torch.float16, torch.float32, torch.int32
