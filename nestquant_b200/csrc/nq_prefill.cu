@@ -6,7 +6,7 @@
 //   pf_hits     routing-hit export
 // Replaces nq_pf_pre / nq_pf_mid / nq_pf_post / nq_pf_hits of the reference (sm120/nqmoe.cu:1081-1245,1258-1293).
 // All of them are elementwise passes over [pairs][H] or [pairs][I] arrays; a CTA owns a pair, a token or (pf_pre) a run of pairs, a
-// warp eight 128-wide groups (Hadamard blocks) at a time, 32 consecutive columns per lane.
+// warp eight 128-wide groups (Hadamard blocks) at a time - of one row, or of several short ones -, 32 consecutive columns per lane.
 #include "nq_common.cuh"
 #include "nq_format.cuh"
 #include "nq_rotate.cuh"
@@ -152,31 +152,42 @@ __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows
     }
 }
 
-// one CTA per pair, one warp per 1024 columns; dynamic shared memory: I floats (staging for the 512-wide rotation)
-template <bool WIDE>
-__global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, const float* __restrict__ zg,
-                                                     const int* __restrict__ pe, const int64_t* __restrict__ table, int E, __half* h, float* zd, int H, int I, int kperm)
+// One CTA per pair, one warp per 1024 columns; dynamic shared memory: I floats (staging for the 512-wide rotation).
+// SEVERAL (rows of at most 512 columns): a warp takes 8 / slots pairs, slots = 1, 2 or 4 groups of its eight each, and no other warp has
+// a part in them; the lanes of a pair follow its own expert.  Dynamic shared memory: 1,024 floats per warp.
+// us, a CTA per pair / this: 24,576 pairs x 256 columns 77.8 / 33.7, x 512 82.8 / 57.4, 6,144 x 384 32.8 / 28.6.  With all eight groups for one pair:
+// 16,384 x 640 61.4 / 67.6, x 768 63.5 / 69.6, x 1,024 in rotations of 512 79.9 / 92.2.  At 96 registers (20 warps on an SM) it spills: 37.8, 62.4, 30.8.
+constexpr int kMidWarps = 2;      // warps of a CTA that takes several pairs per warp
+template <bool WIDE, bool SEVERAL>
+__global__ void __launch_bounds__(SEVERAL ? 32 * kMidWarps : 256, SEVERAL ? 16 / kMidWarps : NQ_PF_EW_BLOCKS)
+pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, const float* __restrict__ zg, const int* __restrict__ pe,
+              const int64_t* __restrict__ table, int E, __half* h, float* zd, int R, int H, int I, int kperm, int slots)
 {
     launch_dependents();
     grid_dependency_wait();
     extern __shared__ float stage[];
     __shared__ float zpart[64][4];
-    const int p = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = I / 128;
-    if (pe[p] < 0 || pe[p] >= E) return;
-    const int64_t* row = table + (int64_t)pe[p] * kTableWidth;
-    const int level = (int)row[0];
-    if (level <= 0) return;
-    const __half* scales = (const __half*)row[9];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = I / 128;
+    const int vec = lane >> 2, q = lane & 3, pairs = SEVERAL ? 8 / slots : 1;
+    const int first = SEVERAL ? ((int)blockIdx.x * nwarp + warp) * pairs : (int)blockIdx.x, p = SEVERAL ? first + vec / slots : first;
+    const int e = p < R ? pe[p] : -1;
+    const int64_t* row = table + (int64_t)(e >= 0 && e < E ? e : 0) * kTableWidth;
+    const int level = e >= 0 && e < E ? (int)row[0] : 0;
+    const bool valid = level > 0;        // of the lane's pair
+    if (!SEVERAL && !valid) return;
+    if (SEVERAL && __ballot_sync(0xffffffffu, valid) == 0u) return;      // its warp's shared memory is its own: __syncwarp below
+    const __half* scales = valid ? (const __half*)row[9] : nullptr;
     const __half *sv_g = scales + H, *sv_u = sv_g + I, *su_d = sv_u + I;
-    const LowRank L = low_rank_of(row, level);
-    const int hw = (int)row[18];
+    LowRank L{nullptr, nullptr, 0, 0};
+    if (valid) L = low_rank_of(row, level);
+    const int hw = valid ? (int)row[18] : 128, rd = SEVERAL ? __reduce_max_sync(0xffffffffu, L.rd) : L.rd;
     float z[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) z[r] = zg[(size_t)p * 4 + r];
-    for (int g0 = warp * 8; g0 < ng; g0 += nwarp * 8)
+    for (int r = 0; r < 4; ++r) z[r] = valid ? zg[(size_t)p * 4 + r] : 0.f;
+    for (int g0 = SEVERAL ? 0 : warp * 8; g0 < (SEVERAL ? 1 : ng); g0 += nwarp * 8)
     {
-        const int grp = g0 + (lane >> 2), col = grp * 128, q = lane & 3;
-        const bool live = grp < ng;
+        const int grp = SEVERAL ? vec & (slots - 1) : g0 + vec, col = grp * 128, at = SEVERAL ? warp * 8 + vec : grp;
+        const bool live = valid && grp < ng;
         float g[32], v[32];
 #pragma unroll
         for (int up = 0; up < 2; ++up)
@@ -202,45 +213,58 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_mid_kernel(const floa
         }
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = live ? silu(g[i]) * v[i] : 0.f;
-        for (int r = 0; r < L.rd; ++r)
+        for (int r = 0; r < rd; ++r)
         {
+            const bool mine = live && (!SEVERAL || r < L.rd);
             float d = 0.f;
-            if (live) d = dot32h_mapH(L.lr + (size_t)L.rg * H + 2 * (size_t)L.rg * I + (size_t)r * I + col, q, v);
+            if (mine) d = dot32h_mapH(L.lr + (size_t)L.rg * H + 2 * (size_t)L.rg * I + (size_t)r * I + col, q, v);
             d = quad_sum(d);
-            if (live && (lane & 3) == 0) zpart[grp][r] = d;
+            if (mine && q == 0) zpart[at][r] = d;
         }
         if (live) scale32h_mapH(su_d + col, q, v);
         wht128_x8(v, lane);
-        if (hw > 128) { if (live) store32f_mapH<false>(stage + col, q, v); }
-        else if (kperm) store32h_mapH_kperm(h + (size_t)p * I + col, q, v, live);
-        else if (live) store32h_mapH(h + (size_t)p * I + col, q, v);
+        const bool plain = live && hw <= 128;
+        if (kperm && (SEVERAL || hw <= 128)) store32h_mapH_kperm(h + (size_t)p * I + col, q, v, plain);
+        else if (plain) store32h_mapH(h + (size_t)p * I + col, q, v);
+        if (live && hw > 128) store32f_mapH<false>(stage + at * 128, q, v);
     }
-    __syncthreads();
-    if (threadIdx.x < 4)      // column groups added in order: the same sum whatever the launch shape
-    {
-        float s = 0.f;
-        if ((int)threadIdx.x < L.rd)
-            for (int q = 0; q < ng; ++q) s += zpart[q][threadIdx.x];
-        zd[(size_t)p * 4 + threadIdx.x] = s;
-    }
-    if (hw > 128)             // WHT_hw = H_(hw/128) (x) WHT128: combine the hw/128 rotated blocks of each hw-wide group
-    {
-        const int nb = hw / 128;
-        const float rs = rsqrtf((float)nb);
-        for (int blk = warp; blk < ng; blk += nwarp)
+    if (SEVERAL) __syncwarp();
+    else __syncthreads();
+    {      // column groups added in order: the same sum whatever the launch shape
+        const int sub = SEVERAL ? lane >> 2 : 0, r = SEVERAL ? q : (int)threadIdx.x, src = sub * slots * 4 & 31;
+        const int n = SEVERAL ? __shfl_sync(0xffffffffu, L.rd, src) : L.rd;
+        const bool on = SEVERAL ? __shfl_sync(0xffffffffu, valid, src) && sub < pairs : r < 4;
+        if (on)
         {
-            const int b0 = blk / nb * nb, ob = blk - b0;
+            float s = 0.f;
+            if (r < n)
+                for (int g = 0; g < ng; ++g) s += zpart[SEVERAL ? warp * 8 + sub * slots + g : g][r];
+            zd[(size_t)(first + sub) * 4 + r] = s;
+        }
+    }
+    // WHT_hw = H_(hw/128) (x) WHT128: combine the hw/128 rotated blocks of each hw-wide group
+    if (SEVERAL ? __reduce_max_sync(0xffffffffu, hw) > 128 : hw > 128)
+    {
+        for (int i = SEVERAL ? 0 : warp; i < (SEVERAL ? 8 : ng); i += SEVERAL ? 1 : nwarp)
+        {
+            const int sub = SEVERAL ? i / slots : 0, blk = SEVERAL ? i & (slots - 1) : i;
+            const int w = SEVERAL ? __shfl_sync(0xffffffffu, hw, 4 * i) : hw;
+            if (SEVERAL && (w <= 128 || blk >= ng)) continue;      // warp-uniform; a pair without an expert has w = 128
+            const int nb = w / 128, b0 = blk / nb * nb, ob = blk - b0;
+            const float rs = rsqrtf((float)nb);
+            const float* from = stage + (SEVERAL ? warp * 8 + sub * slots : 0) * 128;
             float o[4] = {0.f, 0.f, 0.f, 0.f};
             for (int b = 0; b < nb; ++b)
             {
-                const float4 f = *(const float4*)(stage + (b0 + b) * 128 + lane * 4);
+                const float4 f = *(const float4*)(from + (b0 + b) * 128 + lane * 4);
                 const float sg = (__popc(ob & b) & 1) ? -1.f : 1.f;
                 o[0] += sg * f.x; o[1] += sg * f.y; o[2] += sg * f.z; o[3] += sg * f.w;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] *= rs;
-            if (kperm) store4h_kperm(h + (size_t)p * I + blk * 128, lane, o);
-            else store4h(h + (size_t)p * I + blk * 128 + lane * 4, o);
+            for (int k = 0; k < 4; ++k) o[k] *= rs;
+            __half* out = h + (size_t)(first + sub) * I + blk * 128;
+            if (kperm) store4h_kperm(out, lane, o);
+            else store4h(out + lane * 4, o);
         }
     }
 }
@@ -444,8 +468,14 @@ int nq_pf_mid(const float* acc_g, const float* acc_u, const float* zg, const int
     NQ_SHAPE_OK("nq_pf_mid");
     NQ_REQUIRE(E >= 1, "nq_pf_mid: E = %d", E);
     NQ_REQUIRE(nq::aligned16(acc_g) && nq::aligned16(acc_u) && nq::aligned16(h), "nq_pf_mid: acc_g, acc_u, h must be 16-byte aligned");
-    nq::launch_dependent(nq::aligned32(acc_g) && nq::aligned32(acc_u) ? nq::pf_mid_kernel<true> : nq::pf_mid_kernel<false>, dim3(R), dim3(nq::pf_threads(I)), (size_t)I * 4, (cudaStream_t)stream,
-        acc_g, acc_u, zg, pe, table, E, (__half*)h, zd, H, I, kperm);
+    const bool wide = nq::aligned32(acc_g) && nq::aligned32(acc_u);
+    const int ng = I / 128, slots = ng <= 2 ? ng : 4, per = nq::kMidWarps * 8 / slots;
+    if (ng <= 4)      // two pairs per warp or more: a CTA per pair would leave half of the lanes idle
+        nq::launch_dependent(wide ? nq::pf_mid_kernel<true, true> : nq::pf_mid_kernel<false, true>, dim3((R + per - 1) / per), dim3(32 * nq::kMidWarps),
+            (size_t)nq::kMidWarps * 4096, (cudaStream_t)stream, acc_g, acc_u, zg, pe, table, E, (__half*)h, zd, R, H, I, kperm, slots);
+    else
+        nq::launch_dependent(wide ? nq::pf_mid_kernel<true, false> : nq::pf_mid_kernel<false, false>, dim3(R), dim3(nq::pf_threads(I)), (size_t)I * 4, (cudaStream_t)stream,
+            acc_g, acc_u, zg, pe, table, E, (__half*)h, zd, R, H, I, kperm, 1);
     return nq::check_launch("nq_pf_mid");
 }
 
