@@ -37,6 +37,12 @@ __device__ __forceinline__ LowRank low_rank_of(const int64_t* row, int level)
     l.lr4 = level == 4 ? (const __half*)row[15] : nullptr;
     return l;
 }
+// Passes of one CTA per pair or token let the next kernel in early only where they are small: the signal costs a CTA more than its launch does, and
+// a rank's pairs are mostly without an expert (54,944 pairs of which a quarter is live, middle pass 111.2 us with it, 91.2 without).
+__device__ __forceinline__ void launch_dependents_of_few()
+{
+    if (gridDim.x <= 2048) launch_dependents();
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ float warp_sum(float d)
 {
@@ -163,7 +169,7 @@ __global__ void __launch_bounds__(SEVERAL ? 32 * kMidWarps : 256, SEVERAL ? 16 /
 pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, const float* __restrict__ zg, const int* __restrict__ pe,
               const int64_t* __restrict__ table, int E, __half* h, float* zd, int R, int H, int I, int kperm, int slots)
 {
-    launch_dependents();
+    launch_dependents_of_few();
     grid_dependency_wait();
     extern __shared__ float stage[];
     __shared__ float zpart[64][4];
@@ -171,6 +177,7 @@ pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, 
     const int vec = lane >> 2, q = lane & 3, pairs = SEVERAL ? 8 / slots : 1;
     const int first = SEVERAL ? ((int)blockIdx.x * nwarp + warp) * pairs : (int)blockIdx.x, p = SEVERAL ? first + vec / slots : first;
     const int e = p < R ? pe[p] : -1;
+    if (!SEVERAL && (e < 0 || e >= E)) return;      // before anything of the table is read: most pairs of a rank may be without an expert
     const int64_t* row = table + (int64_t)(e >= 0 && e < E ? e : 0) * kTableWidth;
     const int level = e >= 0 && e < E ? (int)row[0] : 0;
     const bool valid = level > 0;        // of the lane's pair
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const flo
                                                       const int* __restrict__ pe, const __half* __restrict__ prw,
                                                       const int64_t* __restrict__ table, int E, float* out, int H, int I)
 {
-    launch_dependents();
+    launch_dependents_of_few();
     grid_dependency_wait();
     const int p = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = H / 128;
     if (pe[p] < 0 || pe[p] >= E) return;
@@ -331,16 +338,18 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const flo
 // accumulate = 0: out[t] is overwritten (zeros if the token has no pick in the window); 1: the sum is added to out[t], and
 // tokens without a pick in the window are not touched.  Calling it window after window in a fixed order gives a bitwise
 // repeatable result without a pairs-sized buffer.
-// Bound by the latency of a pick's rows: the one two picks ahead is asked into L2 meanwhile, one 128-byte line per lane.  us, 80
+// Bound by the latency of a pick's rows: the one two picks ahead is asked into L2 meanwhile, one 128-byte line per lane.  A lane looks up one
+// pick; those that add nothing (experts not resident, zero weights) cost no more.  us, 80
 // registers with spills and no prefetch / this, picks x H: 16,384 x 6,144 120.9 / 116.7 (with rank 2 170.0 / 163.8), x 4,096 88.1 / 74.7,
-// x 2,048 56.3 / 45.1; 24,576 x 1,024 47.8 / 38.9; 65,536 x 6,144 416.6 / 414.8 (446.5 without the prefetch).
+// x 2,048 56.3 / 45.1; 24,576 x 1,024 47.8 / 38.9; 65,536 x 6,144 416.6 / 414.8 (446.5 without the prefetch); 54,944 x 1,792 of which a
+// quarter adds something 67.3 / 58.7.
 template <bool WIDE>
 __global__ void __launch_bounds__(256, NQ_PF_COMBINE_BLOCKS) pf_combine_kernel(const float* __restrict__ y, const float* __restrict__ zd, const int* __restrict__ pos,
                                                          const int64_t* __restrict__ sel, const __half* __restrict__ rw,
                                                          const int64_t* __restrict__ table, float* out, int topk, int E, int H, int I,
                                                          int pair0, int npairs, int accumulate)
 {
-    launch_dependents();
+    launch_dependents_of_few();
     grid_dependency_wait();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, ng = H / 128;
     bool any = false;
@@ -359,22 +368,31 @@ __global__ void __launch_bounds__(256, NQ_PF_COMBINE_BLOCKS) pf_combine_kernel(c
         else
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[i] = 0.f;
-        for (int k = 0; k < topk; ++k)
+        for (int k0 = 0; k0 < topk; k0 += 32)
         {
-            const int64_t e = sel[(size_t)t * topk + k];
-            const int p = pos[(size_t)t * topk + k] - pair0;
-            if (k + 2 < topk)
+            int e = -1, p = 0;
+            float w = 0.f;
+            if (k0 + lane < topk)
             {
-                const int ahead = pos[(size_t)t * topk + k + 2] - pair0, c = g0 * 128 + lane * 32;
-                if (ahead >= 0 && ahead < npairs && c < H) prefetch_l2(y + (size_t)ahead * H + c);
+                const size_t at = (size_t)t * topk + k0 + lane;
+                const int64_t id = sel[at];
+                p = pos[at] - pair0;
+                w = __half2float(rw[at]);
+                if (id >= 0 && id < E && p >= 0 && p < npairs && w != 0.f && table[id * kTableWidth] > 0) e = (int)id;
             }
-            if (e < 0 || e >= E || p < 0 || p >= npairs) continue;
-            float v[32];
-            if (!pair_output<WIDE>(y, zd, p, (int)e, __half2float(rw[(size_t)t * topk + k]), table, H, I, col, live, lane, v))
-                continue;
-            if (live)
+            for (uint32_t left = __ballot_sync(0xffffffffu, e >= 0), todo = left; todo; todo = left)
+            {
+                const int k = __ffs(todo) - 1;
+                left = todo & (todo - 1u);
+                const uint32_t after = left & (left - 1u);
+                const int ahead = __shfl_sync(0xffffffffu, p, after ? __ffs(after) - 1 : 0), c = g0 * 128 + lane * 32;
+                if (after && c < H) prefetch_l2(y + (size_t)ahead * H + c);
+                float v[32];
+                pair_output<WIDE>(y, zd, __shfl_sync(0xffffffffu, p, k), __shfl_sync(0xffffffffu, e, k), __shfl_sync(0xffffffffu, w, k), table, H, I, col, live, lane, v);
+                if (live)
 #pragma unroll
-                for (int i = 0; i < 32; ++i) o[i] += v[i];
+                    for (int i = 0; i < 32; ++i) o[i] += v[i];
+            }
         }
         if (live) store32f_mapH<WIDE>(out + (size_t)t * H + col, lane & 3, o);
     }
