@@ -13,7 +13,7 @@
 //                 store shape takes, so a tile costs one store per warp and no shared memory at all
 //   warps 1, 18   one elected lane issues tcgen05.mma with the A operand in tensor memory (M 128 = weight rows, N =
 //                 tokens, K 16) into a [128 x 384] fp32 accumulator, also in tensor memory; one tcgen05.commit per chunk of two
-//                 k-blocks frees its weight and token tiles.  Both run 6, 3 or 2 chunks ahead, as many as the accumulator of the pass
+//                 k-blocks frees its weight and token tiles.  Both run 6, 4, 3 or 2 chunks ahead, as many as the accumulator of the pass
 //                 and 192 KB of shared memory leave room for.  Passes of up to 64 tokens are multiplied by both warps, wider ones by warp 1
 //   warps 2..17   epilogue: tcgen05.ld the accumulator and store fp32 rows acc[pair][128 columns] (coalesced); it runs
 //                 after the first units of the CTA's next item have been decoded
@@ -48,7 +48,7 @@ constexpr int kPfTmemCols = 512;                     // the accumulator from col
 constexpr int kPfStages = 6;                         // most stages of a pass (chunk_stages)
 constexpr int kPfBoxRows = 64;                       // token rows per TMA box
 constexpr int kPfBoxBytes = kPfBoxRows * 128;        // [64 rows][64 k] fp16
-constexpr int kPfBBoxes = 24;                        // token-tile region: 6, 3 or 2 chunk stages of 2 x 2, 2 x 4 or 2 x 6 boxes
+constexpr int kPfBBoxes = 24;                        // token-tile region: 6, 4, 3 or 2 chunk stages of 2 x 2, 2 x 3, 2 x 4 or 2 x 6 boxes
 constexpr int kPfSecondIssuer = 2 + kPfDecodeWarps;      // warp 1 and this one issue MMAs
 constexpr int kPfThreads = 32 * (kPfSecondIssuer + 1);
 constexpr long long kPfWaitNs = 2000000000ll;             // a wait that lasts 2 s is treated as a hang, unless the caller has another limit
@@ -339,8 +339,10 @@ __device__ __forceinline__ PfShared* pf_shared() { return (PfShared*)(pf_tiles()
 // top down beside the accumulator) and its token tiles in shared memory (2 x 12 / stages boxes).  One set of barriers serves both.  The
 // stages of a narrow pass reach into columns that the accumulator of a wide one before it used (see decode_strip), and when the number of
 // stages changes between two items of a CTA the new token tiles overlap old ones at other indices, so the producer first waits
-// until every stage of the old layout has been released.
-__device__ __forceinline__ int chunk_stages(int ntok) { return ntok <= 128 ? 6 : ntok <= 256 ? 3 : 2; }
+// until every stage of the old layout has been released.  Where the chunks of a strip take different times (mask mode) the stages even them
+// out: 16 experts, H 6,144, I 2,048, gate|up / down, us, with three / four stages: 160 tokens 199 / 192 and 140 / 136, at level 4 202.3 / 200.6 and 129.1 /
+// 127.9; 192 tokens 202 / 196 and 145 / 139, at level 4 204.9 / 203.9 and 132.1 / 130.2.
+__device__ __forceinline__ int chunk_stages(int ntok) { return ntok <= 128 ? 6 : ntok <= 192 ? 4 : ntok <= 256 ? 3 : 2; }
 // Passes of up to 64 tokens: even and odd chunks are multiplied by two warps, each into an accumulator of its own that the epilogue adds up.
 // What a chunk costs the warp that issues its MMAs comes on top of the decode warps of its scheduler, and the slowest scheduler paces the
 // others: gate|up of 128 experts x 31 tokens with one warp / two, us: 785 / 757 at level 2, 1,226 / 1,193 at level 4.  Beyond 64 tokens the second

@@ -1,4 +1,4 @@
-"""The fused prefill GEMM changes its layout with the width of a pass (2, 3 or 6 stages beside the accumulator; up to 64 tokens two accumulators,
+"""The fused prefill GEMM changes its layout with the width of a pass (2, 3, 4 or 6 stages beside the accumulator; up to 64 tokens two accumulators,
 up to 32 two pairs of them in turn): passes of every width one after the other on the same CTAs, for few and odd numbers of chunks."""
 import pytest
 import torch
@@ -33,6 +33,15 @@ NARROW = [31, 1, 32, 16, 33, 5, 32, 64, 2, 30, 65, 8, 31, 384, 17, 32, 129, 24]
 @pytest.mark.parametrize("H,I", [(128, 2048), (256, 2048), (384, 2048), (896, 2048), (2048, 128), (2560, 256), (2560, 640)])
 def test_narrow_passes_in_a_row(H, I):
     _check(NARROW, H, I)
+
+
+# Every layout behind every other one, at both ends of the four-stage widths.
+MIDDLE = [192, 129, 193, 160, 384, 144, 16, 191, 128, 130, 257, 192, 256, 40, 384, 193, 65, 300, 8, 256, 176]
+
+
+@pytest.mark.parametrize("H,I", [(128, 2048), (384, 2048), (640, 2048), (1152, 1664), (2560, 640)])
+def test_four_stage_passes_in_turn(H, I):
+    _check(MIDDLE, H, I)
 
 
 def _check(counts, H, I):
