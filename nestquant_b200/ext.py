@@ -174,8 +174,13 @@ def prefill(x, sel, rw, table, out, perm, scratch, R, I, nm_gu, nm_dn, hits_ptr=
     _need(sel, torch.int64, "sel"); _need(rw, torch.float16, "rw"); _need(table, torch.int64, "table"); _need(out, torch.float32, "out")
     T, topk = sel.shape
     H, E, P = scratch["y"].shape[1], table.shape[0], T * topk
-    if rw.numel() < P or out.numel() < T * H or R > scratch["R"] or P > perm["P"]:
-        raise NestQuantError("prefill sizes: rw [T,topk], out [T,H], scratch for R pairs, index arrays for T * topk")
+    # the arrays are sized by the layer's own number of experts, the table may come from the caller
+    if perm["start"].numel() < E + 2 or (hits_ptr and perm["hit"].numel() < E):
+        raise NestQuantError(f"prefill sizes: a table of {E} experts, index arrays for fewer")
+    if rw.numel() < P or out.dim() < 2 or out.shape[1] != H or out.numel() < T * H or min(perm[n].numel() for n in ("pe", "pt", "pos")) < P:
+        raise NestQuantError("prefill sizes: rw [T,topk], out [T,H], index arrays for T * topk pairs")
+    if any(scratch[n].numel() < R * w for n, w in (("xg", H), ("xu", H), ("y", H), ("acc_g", I), ("acc_u", I), ("h", I), ("zg", 4), ("zd", 4))):
+        raise NestQuantError(f"prefill sizes: scratch for chunks of {R} pairs of {H} and {I} columns")
     a, peers = capi.NqPrefill(), None
     if x_peers is None:
         _need(x, torch.float16, "x")

@@ -69,3 +69,16 @@ def test_refused_inputs():
             L.prefill(bad, sel, rw)
     with pytest.raises(NestQuantError):
         L.prefill(x, sel, rw, out=torch.empty(39, 256, device="cuda"))
+
+
+def test_table_of_more_experts_than_the_layer_is_refused():
+    """also where an earlier, larger call has left scratch that would be large enough for it"""
+    L, exs = _layer(16, 4)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    L.prefill(*_inputs(16, 4, 8192, 256, gen))
+    x, sel, rw = _inputs(16, 4, 10, 256, gen)
+    with pytest.raises(NestQuantError):
+        L.prefill(x, sel, rw, table=L.table.repeat(19, 1)[:300].contiguous())
+    fewer = L.prefill(x, sel % 12, rw, table=L.table[:12].contiguous())
+    torch.cuda.synchronize()
+    assert torch.equal(fewer, L.prefill(x, sel % 12, rw))
