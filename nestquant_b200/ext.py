@@ -177,9 +177,9 @@ def prefill(x, sel, rw, table, out, perm, scratch, R, I, nm_gu, nm_dn, hits_ptr=
     # the arrays are sized by the layer's own number of experts, the table may come from the caller
     if perm["start"].numel() < E + 2 or (hits_ptr and perm["hit"].numel() < E):
         raise NestQuantError(f"prefill sizes: a table of {E} experts, index arrays for fewer")
-    if rw.numel() < P or out.dim() < 2 or out.shape[1] != H or out.numel() < T * H or min(perm[n].numel() for n in ("pe", "pt", "pos")) < P:
+    if rw.numel() < P or out.dim() < 2 or out.shape[1] != H or out.numel() < T * H or P > perm["P"]:
         raise NestQuantError("prefill sizes: rw [T,topk], out [T,H], index arrays for T * topk pairs")
-    if any(scratch[n].numel() < R * w for n, w in (("xg", H), ("xu", H), ("y", H), ("acc_g", I), ("acc_u", I), ("h", I), ("zg", 4), ("zd", 4))):
+    if R > scratch["R"] or scratch["acc_g"].numel() < R * I:
         raise NestQuantError(f"prefill sizes: scratch for chunks of {R} pairs of {H} and {I} columns")
     a, peers = capi.NqPrefill(), None
     if x_peers is None:

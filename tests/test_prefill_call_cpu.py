@@ -59,11 +59,9 @@ def test_fitting_sizes_reach_the_library(library):
     dict(out=torch.empty(2560)),
     dict(out=torch.empty(9, 256)),
     dict(rw=torch.empty(9, 4, dtype=torch.float16)),
-    dict(pos=torch.empty(39, dtype=torch.int32)),
+    dict(T=11),
     dict(chunk=41),
-    dict(h=torch.empty(39, 128, dtype=torch.float16)),
-    dict(acc_u=torch.empty(40, 64)),
-    dict(zd=torch.empty(39, 4)),
+    dict(acc_g=torch.empty(40, 64)),
 ], ids=lambda o: ",".join(o))
 def test_sizes_that_do_not_fit_are_refused(library, over):
     with pytest.raises(NestQuantError):
