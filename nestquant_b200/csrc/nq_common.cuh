@@ -27,7 +27,10 @@ inline int check_launch(const char* what)
 // Programmatic dependent launch: a kernel lets its successor in the stream start launching early (its CTAs take their places, set up their shared
 // memory and block), and itself waits until the whole predecessor grid has completed and its writes are visible, before it touches
 // anything.  Every thread of every CTA passes through it, also where there is nothing to do: a grid that ended before its predecessor would
-// release the one behind it too early.
+// release the one behind it too early.  What such a kernel reads may be written while it is already there, so its parameters are not
+// const __restrict__ and it reads them without __ldg: both tell the compiler that the memory does not change during the kernel, and loads of such
+// memory may be non-coherent and may move in front of the wait.  (What it finds through a table row, planes and scales, is read behind
+// the row and so behind the wait.)
 #ifdef __CUDACC__
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

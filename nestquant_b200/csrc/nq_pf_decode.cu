@@ -145,7 +145,7 @@ __device__ __noinline__ void dense_run()
 }
 
 // grid (ceil(units / (8 run)), n_experts, 2 = gate|up / down); run = units of a run
-__global__ void __launch_bounds__(32 * kDenseWarps, kDenseCtas) pf_decode_kernel(const int64_t* __restrict__ table, const int32_t* __restrict__ experts,
+__global__ void __launch_bounds__(32 * kDenseWarps, kDenseCtas) pf_decode_kernel(const int64_t* table, const int32_t* experts,
                                                                                 __half* Wgu, __half* Wdn, int H, int I, int nm_gu, int nm_dn,
                                                                                 int force_level, int run)
 {
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, kDenseCtas) pf_decode_kernel
     const int N = down ? H : 2 * I, K = down ? I : H, C = K / 128, NS = N / 16, units = NS * C, nm = down ? nm_dn : nm_gu;
     const int unit = ((int)blockIdx.x * kDenseWarps + warp) * run;
     if (!W || unit >= units) return;     // warp-uniform
-    const int64_t* row = table + (int64_t)__ldg(experts + blockIdx.y) * kTableWidth;
+    const int64_t* row = table + (int64_t)experts[blockIdx.y] * kTableWidth;
     int level = (int)row[0];
     if (force_level > 0 && level > 0) level = force_level;
     const ProjPlanes P = planes_from_row(row, down);

@@ -655,7 +655,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
             if (t.wg >= groups) { t.wg -= groups; ++t.pass; }
             return t;
         };
-        auto pass_of = [&](const At& t) { return t.pass < npass ? __ldg((const int4*)(passes + t.pass)) : make_int4(0, 0, 0, 0); };
+        auto pass_of = [&](const At& t) {
+            const PfPass ps = t.pass < npass ? passes[t.pass] : PfPass{0, 0, 0, 0};
+            return make_int4(ps.expert, ps.row0, ps.ntok, 0);
+        };
         auto row_of = [&](const At& t, const int4& p) { return t.pass < npass && lane < kTableWidth ? a.table[(int64_t)p.x * kTableWidth + lane] : 0; };
         auto publish = [&](const At& t, const int4& p, int64_t w, const Head& h) {
             if (t.pass >= npass) return true;
@@ -825,6 +828,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
         }
     }
     // Not at the start: with CTAs of the next pass waiting beside this one's, whole prefill calls took 7 % longer (geometric mean over 54 of 50 to 1,200 us).
+    // It also keeps the chain's scratch safe: no kernel comes up before a GEMM has ended that lies between two uses of an array (zg, zd, y, the
+    // pass list and the index arrays are written again call after call), so none can hold a line of its former contents in L1.
     launch_dependents();
     __syncwarp();
     tc_fence_before();
@@ -836,7 +841,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) pf_gemm_kernel(const __grid_con
 
 // ---------------------------------------------------------------- pass plan (device side, no host sync), see nq_plan.cuh
 template <bool WINDOW>
-__global__ void __launch_bounds__(kPlanThreads) pf_plan_kernel(const int* __restrict__ from, const int64_t* __restrict__ table, int E,
+__global__ void __launch_bounds__(kPlanThreads) pf_plan_kernel(const int* from, const int64_t* table, int E,
                                                                int pair0, int npairs, int* plan, int max_passes)
 {
     __shared__ int s_warp[kPlanThreads / 32];

@@ -30,7 +30,7 @@ constexpr int kSortWarps = 8;        // warps per CTA
 constexpr int kSortMaxBins = 1025;   // experts + 1
 constexpr size_t kSortSmallShared = 48 * 1024 - 256;      // the one-kernel form stays within the default shared memory of a CTA
 
-__device__ __forceinline__ int pick_bin(const int64_t* __restrict__ sel, const __half* __restrict__ rw, const int64_t* __restrict__ table,
+__device__ __forceinline__ int pick_bin(const int64_t* sel, const __half* rw, const int64_t* table,
                                         int E, int i, bool* hit)
 {
     const int64_t e = sel[i];
@@ -40,8 +40,8 @@ __device__ __forceinline__ int pick_bin(const int64_t* __restrict__ sel, const _
 }
 
 // pass 1: hist[slice][bin] (and hits[e] += picks with a weight)
-__global__ void __launch_bounds__(32 * kSortWarps) sort_count_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
-                                                                    const int64_t* __restrict__ table, int P, int E, int* hist, int* hits)
+__global__ void __launch_bounds__(32 * kSortWarps) sort_count_kernel(const int64_t* sel, const __half* rw,
+                                                                    const int64_t* table, int P, int E, int* hist, int* hits)
 {
     launch_dependents();
     grid_dependency_wait();
@@ -126,8 +126,8 @@ __device__ __forceinline__ void place_picks(int* nx, int b, int i, int topk, int
 }
 
 // pass 3: place every pick.  Every CTA adds up the bin sizes itself (row 0 of hist); CTA 0 writes them out as start.
-__global__ void __launch_bounds__(32 * kSortWarps) sort_place_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
-                                                                    const int64_t* __restrict__ table, int P, int E, int topk,
+__global__ void __launch_bounds__(32 * kSortWarps) sort_place_kernel(const int64_t* sel, const __half* rw,
+                                                                    const int64_t* table, int P, int E, int topk,
                                                                     const int* hist, int* start, int* pe, int* pt, int* pos)
 {
     launch_dependents();
@@ -155,8 +155,8 @@ __global__ void __launch_bounds__(32 * kSortWarps) sort_place_kernel(const int64
 // 32 picks, no longer than needed, and a lane keeps its picks' bins in registers between the passes.  If the whole list is one chunk, its
 // pass list too.
 constexpr int kSortSmallPicks = 32 * kSortSlice;
-__global__ void __launch_bounds__(1024) sort_small_kernel(const int64_t* __restrict__ sel, const __half* __restrict__ rw,
-                                                          const int64_t* __restrict__ table, int P, int E, int topk, int* start, int* hits,
+__global__ void __launch_bounds__(1024) sort_small_kernel(const int64_t* sel, const __half* rw,
+                                                          const int64_t* table, int P, int E, int topk, int* start, int* hits,
                                                           int* pe, int* pt, int* pos, int* plan, int max_passes)
 {
     launch_dependents();

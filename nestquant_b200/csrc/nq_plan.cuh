@@ -18,7 +18,7 @@ struct PfPass { int expert, row0, ntok, pad; };
 constexpr int kPlanThreads = 1024;
 
 template <bool WINDOW>
-__device__ __forceinline__ void plan_passes(const int* from, const int64_t* __restrict__ table, int E, int pair0, int npairs, int* plan, int max_passes,
+__device__ __forceinline__ void plan_passes(const int* from, const int64_t* table, int E, int pair0, int npairs, int* plan, int max_passes,
                                             int* s_warp)
 {
     PfPass* out = (PfPass*)(plan + 4);

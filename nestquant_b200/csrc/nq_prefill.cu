@@ -74,8 +74,8 @@ __device__ __forceinline__ const __half* token_row(const TokenRows& r, int t, in
 // vectors of those columns stay in registers while the expert stays the same (the pairs of an expert are consecutive),
 // and the input row of the next pair is fetched before the current one is transformed.
 struct PairHead { int e; bool live; const __half* xr; const int64_t* row; int level; };
-__device__ __forceinline__ PairHead pair_head(const TokenRows& rows, const int* __restrict__ pt, const int* __restrict__ pe,
-                                              const int64_t* __restrict__ table, int E, int H, int p, int p1)
+__device__ __forceinline__ PairHead pair_head(const TokenRows& rows, const int* pt, const int* pe,
+                                              const int64_t* table, int E, int H, int p, int p1)
 {
     PairHead h{-1, false, nullptr, nullptr, 0};
     if (p >= p1) return h;
@@ -89,8 +89,8 @@ __device__ __forceinline__ PairHead pair_head(const TokenRows& rows, const int* 
     return h;
 }
 template <bool WIDE>
-__global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows rows, const int* __restrict__ pt, const int* __restrict__ pe,
-                                                     const int64_t* __restrict__ table, int E, __half* xg, __half* xu, float* zg, int H, int I,
+__global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows rows, const int* pt, const int* pe,
+                                                     const int64_t* table, int E, __half* xg, __half* xu, float* zg, int H, int I,
                                                      int kperm, int R)
 {
     launch_dependents();
@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(256, NQ_PF_PRE_BLOCKS) pf_pre_kernel(TokenRows
 constexpr int kMidWarps = 2;      // warps of a CTA that takes several pairs per warp
 template <bool WIDE, bool SEVERAL>
 __global__ void __launch_bounds__(SEVERAL ? 32 * kMidWarps : 256, SEVERAL ? 16 / kMidWarps : NQ_PF_EW_BLOCKS)
-pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, const float* __restrict__ zg, const int* __restrict__ pe,
-              const int64_t* __restrict__ table, int E, __half* h, float* zd, int R, int H, int I, int kperm, int slots)
+pf_mid_kernel(const float* acc_g, const float* acc_u, const float* zg, const int* pe,
+              const int64_t* table, int E, __half* h, float* zd, int R, int H, int I, int kperm, int slots)
 {
     launch_dependents_of_few();
     grid_dependency_wait();
@@ -279,8 +279,8 @@ pf_mid_kernel(const float* __restrict__ acc_g, const float* __restrict__ acc_u, 
 // v = rw * (WHT128(y) * sv_o + z_dn (U2_d [+ U4_d])) for the lane's 32 output columns of the group at col of pair p (live lanes
 // only load and scale; every lane takes part in the rotation); false if the pair adds nothing (warp-uniform)
 template <bool WIDE>
-__device__ __forceinline__ bool pair_output(const float* __restrict__ y, const float* __restrict__ zd, int p, int e, float w,
-                                            const int64_t* __restrict__ table, int H, int I, int col, bool live, int lane, float (&v)[32])
+__device__ __forceinline__ bool pair_output(const float* y, const float* zd, int p, int e, float w,
+                                            const int64_t* table, int H, int I, int col, bool live, int lane, float (&v)[32])
 // (col = first column of the lane's group, columns by map H)
 {
     const int64_t* row = table + (int64_t)e * kTableWidth;
@@ -311,9 +311,9 @@ __device__ __forceinline__ bool pair_output(const float* __restrict__ y, const f
 }
 
 // one CTA per pair: atomic accumulation into out[token]
-__global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const float* __restrict__ y, const float* __restrict__ zd, const int* __restrict__ pt,
-                                                      const int* __restrict__ pe, const __half* __restrict__ prw,
-                                                      const int64_t* __restrict__ table, int E, float* out, int H, int I)
+__global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const float* y, const float* zd, const int* pt,
+                                                      const int* pe, const __half* prw,
+                                                      const int64_t* table, int E, float* out, int H, int I)
 {
     launch_dependents_of_few();
     grid_dependency_wait();
@@ -344,9 +344,9 @@ __global__ void __launch_bounds__(256, NQ_PF_EW_BLOCKS) pf_post_kernel(const flo
 // x 2,048 56.3 / 45.1; 24,576 x 1,024 47.8 / 38.9; 65,536 x 6,144 416.6 / 414.8 (446.5 without the prefetch); 54,944 x 1,792 of which a
 // quarter adds something 67.3 / 58.7.
 template <bool WIDE>
-__global__ void __launch_bounds__(256, NQ_PF_COMBINE_BLOCKS) pf_combine_kernel(const float* __restrict__ y, const float* __restrict__ zd, const int* __restrict__ pos,
-                                                         const int64_t* __restrict__ sel, const __half* __restrict__ rw,
-                                                         const int64_t* __restrict__ table, float* out, int topk, int E, int H, int I,
+__global__ void __launch_bounds__(256, NQ_PF_COMBINE_BLOCKS) pf_combine_kernel(const float* y, const float* zd, const int* pos,
+                                                         const int64_t* sel, const __half* rw,
+                                                         const int64_t* table, float* out, int topk, int E, int H, int I,
                                                          int pair0, int npairs, int accumulate)
 {
     launch_dependents_of_few();

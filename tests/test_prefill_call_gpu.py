@@ -82,3 +82,27 @@ def test_table_of_more_experts_than_the_layer_is_refused():
     fewer = L.prefill(x, sel % 12, rw, table=L.table[:12].contiguous())
     torch.cuda.synchronize()
     assert torch.equal(fewer, L.prefill(x, sel % 12, rw))
+
+
+def test_calls_in_a_row_over_arrays_aligned_to_16_bytes():
+    """the forms of the passes for arrays that are not aligned to 32 bytes, call after call in several chunks"""
+    L, exs = _layer(16, 4, H=512, I=256)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    ins = [_inputs(16, 4, T, 512, gen) for T in (300, 77, 513)]
+    want = [L.prefill(*a, R=200) for a in ins]
+    torch.cuda.synchronize()
+
+    def shifted(t):
+        n = 16 // t.element_size()
+        return torch.empty(t.numel() + n, dtype=t.dtype, device="cuda")[n:].view(t.shape)
+
+    sc = L._prefill_scratch(200, torch.device("cuda", torch.cuda.current_device()))
+    sc.update({n: shifted(sc[n]) for n in ("acc_g", "acc_u", "h", "xg", "xu", "y")})
+    ins = [(shifted(x).copy_(x), sel, rw) for x, sel, rw in ins]
+    outs = [shifted(w) for w in want]
+    for _ in range(10):
+        for a, o in zip(ins, outs):
+            L.prefill(*a, R=200, out=o.fill_(7.0))
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, w) for o, w in zip(outs, want))
+    assert L.prefill_status() == 0
