@@ -18,6 +18,8 @@ extern "C" int nq_prefill(const NqPrefill* p, void* stream)
     NQ_REQUIRE(p->R >= 1 && p->xg && p->xu && p->y && p->acc_g && p->acc_u && p->h && p->zg && p->zd && p->plan && p->status && p->start,
                "nq_prefill: null scratch or R = %d", p->R);
     NQ_REQUIRE(!p->hits || p->hit_counts, "nq_prefill: hits without hit_counts");
+    NQ_REQUIRE(p->world <= 0 || (p->peer_x && (long long)p->world * p->tokens_per_rank >= p->T), "nq_prefill: %d tokens on %d ranks of %d", p->T, p->world,
+               p->tokens_per_rank);      // (a token behind them would be looked for in a buffer that is not there)
     const int H = p->H, I = p->I, E = p->E, R = p->R < P ? p->R : P;
     NQ_REQUIRE(E >= 1 && p->plan_ints >= nq_pf_plan_ints(E, R), "nq_prefill: plan needs %d ints", nq_pf_plan_ints(E, R));
     if (p->hits && cudaMemsetAsync(p->hit_counts, 0, sizeof(int32_t) * E, (cudaStream_t)stream) != cudaSuccess)

@@ -1,9 +1,11 @@
 """What a prefill call refuses before anything is enqueued: sizes that do not fit one another.  The checks look at shapes only, so CPU
 tensors and a library that records what reaches it do."""
+import ctypes as C
+
 import pytest
 import torch
 
-from nestquant_b200 import ext
+from nestquant_b200 import capi, ext
 from nestquant_b200.capi import NestQuantError
 
 
@@ -67,3 +69,19 @@ def test_sizes_that_do_not_fit_are_refused(library, over):
     with pytest.raises(NestQuantError):
         _call(**over)
     assert library.calls == 0
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the arguments are not device addresses")
+@pytest.mark.parametrize("world,per,T", [(2, 20, 41), (8, 5, 100), (4, 0, 1), (4, -3, 12)])
+def test_tokens_that_no_rank_has_are_refused(world, per, T):
+    """before anything is enqueued: an argument error, where a call that reached the device would fail for want of one"""
+    a = capi.NqPrefill()
+    for n, t in capi.NqPrefill._fields_:
+        setattr(a, n, 4096 if t is C.c_void_p else 0)
+    a.hits = a.hit_counts = None
+    a.T, a.topk, a.E, a.H, a.I, a.nm_gu, a.nm_dn, a.R = T, 4, 16, 256, 128, 1, 1, 400
+    a.plan_ints = a.sort_scratch_ints = 1 << 20
+    peers = (C.c_void_p * 8)(*[4096] * 8)
+    a.peer_x, a.world, a.tokens_per_rank = C.addressof(peers), world, per
+    assert capi.lib().nq_prefill(C.byref(a), None) == -1          # NQ_ERR_ARG
+    assert b"ranks" in capi.lib().nq_last_error()

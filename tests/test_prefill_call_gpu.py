@@ -98,6 +98,7 @@ def test_calls_in_a_row_over_arrays_aligned_to_16_bytes():
 
     sc = L._prefill_scratch(200, torch.device("cuda", torch.cuda.current_device()))
     sc.update({n: shifted(sc[n]) for n in ("acc_g", "acc_u", "h", "xg", "xu", "y")})
+    sc["plan"] = torch.empty(sc["plan"].numel() + 1, dtype=torch.int32, device="cuda")[1:]      # (4 bytes: any int array will do)
     ins = [(shifted(x).copy_(x), sel, rw) for x, sel, rw in ins]
     outs = [shifted(w) for w in want]
     for _ in range(10):
