@@ -30,9 +30,9 @@ extern "C" int nq_prefill(const NqPrefill* p, void* stream)
         return e;
     if (p->hits)
         if (int e = nq_pf_hits(p->hit_counts, p->hits, E, stream)) return e;
-    for (int c0 = 0; c0 < P; c0 += R)
+    for (int c0 = 0, n; c0 < P; c0 += n)
     {
-        const int n = P - c0 < R ? P - c0 : R;
+        n = P - c0 < R ? P - c0 : R;
         if (R < P)
             if (int e = nq_pf_plan_window(p->start, p->table, E, c0, n, p->plan, p->plan_ints, stream)) return e;
         const int32_t *pt = p->pt + c0, *pe = p->pe + c0;
