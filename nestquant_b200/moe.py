@@ -286,6 +286,7 @@ class MoELayer:
         s.wq = torch.zeros(n["wq_ints"], dtype=i32, device=dev)
         s.zd = torch.zeros(n["zd_floats"], dtype=f32, device=dev)
         s.cnt_h = torch.zeros(n["cnt_h_ints"], dtype=i32, device=dev)
+        s._pf_status = torch.zeros(1, dtype=i32, device=dev)       # raised by the prefill GEMM; here, so that no captured call clears it
 
     def set(s, e, ex, level):
         w = had_dn(ex)
@@ -376,13 +377,16 @@ class MoELayer:
         TMEM; dense weights never touch HBM), same math as __call__.  x fp16 [T,H], sel int64 [T,topk], rw fp16 [T,topk] ->
         fp32 [T,H].  Same call shape as the reference's prefill (sm120/moe.py:282-327).
         R: pairs per scratch chunk (default 65536 = an 8192-token window of top-8 picks; the scratch, ~45 KB per pair at
-        the GLM shape, is kept between calls and grows with them).  The expert-sorted pair list is processed chunk by chunk and each
+        the GLM shape, is kept between calls and grows with them, up to the R that is asked for: a call that names a smaller one gives the
+        rest back).  The expert-sorted pair list is processed chunk by chunk and each
         token's picks are added chunk after chunk in pick order, so the result is bitwise repeatable for a given R.
         G (experts decoded per group in the reference) is accepted and ignored: nothing is decoded ahead of the GEMM.
         Picks whose expert id is outside [0, E) (e.g. -1 padding) are ignored, as on the decode path.
         x_peers = (device addresses of every rank's input buffer, tokens per rank): expert parallelism - x is ignored (pass
         any fp16 [*, H] tensor on the device), token t of sel / rw is read from buffer t // tokens_per_rank by the first pass
         itself (see nq_pf_pre_ep).
+        Under torch.cuda.graph a call's scratch comes from the graph's own pool and lives as long as the graph: replays and eager calls, whatever
+        their sizes, do not disturb one another.
         Nothing here synchronises with the host; a device-side time-out inside the GEMM raises a flag that
         prefill_status() reads."""
         assert x.dtype == torch.float16 and rw.dtype == torch.float16 and sel.dtype == torch.int64, (x.dtype, rw.dtype, sel.dtype)
@@ -390,11 +394,12 @@ class MoELayer:
         H, I, M, dev = s.H, s.I, s.M, sel.device
         tb = s.table if table is None else table
         P = T * k
+        most = R
         R = max(1, min(R or 65536, P))
         out = torch.empty(T, H, dtype=torch.float32, device=dev) if out is None else out
         if P == 0:
             return out
-        sc = s._prefill_scratch(R, dev)
+        sc = s._prefill_scratch(R, dev, most)
         # one call for all of it: the pairs sorted by expert on the device (picks that contribute nothing - no valid expert id, expert not
         # resident here, zero weight - sort behind every real pair), then chunk by chunk pass list, rotations, GEMMs and combine, where y
         # overwrites xg | xu
@@ -402,40 +407,46 @@ class MoELayer:
         M.prefill(x, sel, rw, tb, out, s._prefill_perm(P, dev), sc, R, I, s.nm_gu, s.nm_dn, s.hits_ptr, x_peers)
         return out
 
-    def _prefill_scratch(s, R, dev):
-        """scratch of the prefill path for chunks of up to R pairs, kept between calls, the largest asked for so far (the reference's pf_scratch,
-        sm120/moe.py:263-275, without its dense weight buffers): xg | xu fp16 [R,H] each, aliased by y fp32 [R,H];
-        acc_g, acc_u fp32 [R,I]; h fp16 [R,I]; zg, zd fp32 [R,4]; the pass list; the status word"""
+    def _prefill_scratch(s, R, dev, most=None):
+        """scratch of the prefill path for chunks of up to R pairs (the reference's pf_scratch, sm120/moe.py:263-275, without its dense weight
+        buffers): xg | xu fp16 [R,H] each, aliased by y fp32 [R,H]; acc_g, acc_u fp32 [R,I]; h fp16 [R,I]; zg, zd fp32 [R,4]; the pass
+        list; the status word.  Kept between calls, the largest asked for so far unless that is more than `most` rows (None: no limit).  Not
+        kept by a call under capture: its tensors are the graph's, as all that torch allocates during one, and they stay as they are for it."""
         owner = getattr(s, "_pf_owner", None)
         if owner is not None:
-            return owner._prefill_scratch(R, dev)
-        sc = getattr(s, "_pf_sc", None)
-        if sc is not None and sc["R"] >= R and sc["y"].device == dev:
+            return owner._prefill_scratch(R, dev, most)
+        captured, sc = torch.cuda.is_current_stream_capturing(), getattr(s, "_pf_sc", None)
+        if not captured and sc is not None and sc["R"] >= R and (not most or sc["R"] <= max(1, most)) and sc["y"].device == dev:
             return sc
         H, I, E = s.H, s.I, s.E
         f16, f32, i32 = torch.float16, torch.float32, torch.int32
+        if not captured:
+            s._pf_sc = sc = None      # (before the new one is there)
         y = torch.empty(R, H, dtype=f32, device=dev)
         halves = y.view(-1).view(f16)
-        status = sc["status"] if sc is not None and sc["status"].device == dev else torch.zeros(1, dtype=i32, device=dev)
-        s._pf_sc = dict(R=R, y=y, xg=halves[:R * H].view(R, H), xu=halves[R * H:].view(R, H),
-                        acc_g=torch.empty(R, I, dtype=f32, device=dev), acc_u=torch.empty(R, I, dtype=f32, device=dev),
-                        h=torch.empty(R, I, dtype=f16, device=dev), zg=torch.zeros(R, 4, dtype=f32, device=dev),
-                        zd=torch.zeros(R, 4, dtype=f32, device=dev),
-                        plan=torch.empty(s.M.pf_plan_ints(E, R), dtype=i32, device=dev), status=status)
-        return s._pf_sc
+        sc = dict(R=R, y=y, xg=halves[:R * H].view(R, H), xu=halves[R * H:].view(R, H),
+                  acc_g=torch.empty(R, I, dtype=f32, device=dev), acc_u=torch.empty(R, I, dtype=f32, device=dev),
+                  h=torch.empty(R, I, dtype=f16, device=dev), zg=torch.empty(R, 4, dtype=f32, device=dev),
+                  zd=torch.empty(R, 4, dtype=f32, device=dev),
+                  plan=torch.empty(s.M.pf_plan_ints(E, R), dtype=i32, device=dev), status=s._pf_status)
+        if not captured:
+            s._pf_sc = sc
+        return sc
 
     def _prefill_perm(s, P, dev):
-        """index arrays of the pair sort for windows of up to P pairs, kept between calls"""
+        """index arrays of the pair sort for windows of up to P pairs, kept between calls as the scratch is"""
         owner = getattr(s, "_pf_owner", None)
         if owner is not None:
             return owner._prefill_perm(P, dev)
-        pm = getattr(s, "_pf_perm", None)
-        if pm is not None and pm["P"] >= P and pm["pe"].device == dev:
+        captured, pm = torch.cuda.is_current_stream_capturing(), getattr(s, "_pf_perm", None)
+        if not captured and pm is not None and pm["P"] >= P and pm["pe"].device == dev:
             return pm
         i32 = torch.int32
         mk = lambda n: torch.empty(n, dtype=i32, device=dev)
-        s._pf_perm = dict(P=P, pe=mk(P), pt=mk(P), pos=mk(P), start=mk(s.E + 2), hit=mk(s.E), scratch=mk(max(1, s.M.pf_sort_scratch_ints(P, s.E))))
-        return s._pf_perm
+        pm = dict(P=P, pe=mk(P), pt=mk(P), pos=mk(P), start=mk(s.E + 2), hit=mk(s.E), scratch=mk(max(1, s.M.pf_sort_scratch_ints(P, s.E))))
+        if not captured:
+            s._pf_perm = pm
+        return pm
 
     def share_prefill_scratch(s, other):
         """use the prefill scratch (and status word) of another layer of the same shape: the layers of a stack run one after
@@ -449,8 +460,7 @@ class MoELayer:
         owner = getattr(s, "_pf_owner", None)
         if owner is not None:
             return owner.prefill_status()
-        sc = getattr(s, "_pf_sc", None)
-        return 0 if sc is None else int(sc["status"].item())
+        return int(s._pf_status.item())
 
 
 class _Captured:

@@ -107,3 +107,38 @@ def test_calls_in_a_row_over_arrays_aligned_to_16_bytes():
         torch.cuda.synchronize()
         assert all(torch.equal(o, w) for o, w in zip(outs, want))
     assert L.prefill_status() == 0
+
+
+@pytest.mark.parametrize("R", [None, 200])
+def test_captured_calls(R):
+    """replays over other inputs, beside larger and smaller eager calls that replace the layer's scratch, against eager calls; the first call of
+    a layer may be the captured one, and a raised status word outlives replays"""
+    L, exs = _layer(16, 4, H=512, I=256)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    ins = [_inputs(16, 4, 130, 512, gen) for _ in range(3)]
+    big = _inputs(16, 4, 900, 512, gen)
+    _layer(16, 4, H=512, I=256)[0].prefill(*ins[0])      # (the kernels are loaded)
+    x, sel, rw = (t.clone() for t in ins[0])
+    out = torch.empty(130, 512, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        L.prefill(x, sel, rw, out=out, R=R)
+    want = [L.prefill(*a, R=R) for a in ins]
+    large = L.prefill(*big)
+    spare = [torch.full((n,), 3.0, device="cuda") for n in (1 << 14, 1 << 17, 1 << 20) for _ in range(4)]      # where freed scratch would have been
+    for i in (1, 0, 2, 1):
+        for dst, src in zip((x, sel, rw), ins[i]):
+            dst.copy_(src)
+        out.fill_(7.0)
+        graph.replay()
+        assert torch.equal(L.prefill(*big), large)
+        assert torch.equal(L.prefill(*ins[i], R=R), want[i])
+        torch.cuda.synchronize()
+        assert torch.equal(out, want[i])
+    assert all((t == 3.0).all() for t in spare)
+    assert L.prefill_status() == 0
+    L._pf_status.fill_(1)
+    graph.replay()
+    assert L.prefill_status() == 1
+    del graph
