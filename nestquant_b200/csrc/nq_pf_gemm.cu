@@ -469,7 +469,11 @@ __device__ __noinline__ bool decode_strip(uint32_t par, uint32_t info_word)
     uint32_t rec = (unit0 + group) * 32 + lane, res = (MODE == 1 ? unit0 + group : res0) * 32 + lane;       // this unit's records (level 4 without flags: of both planes)
     RecordValues<BK> rb;
     rb.load_at(base, nrec, rec);
-    RecordValues<RC> rr;
+    // Zeroed, and taken apart for every unit: a record that holds nothing yet, or is taken apart on refined units only, costs the compiler
+    // registers beside the words made of it, 2,480 bytes of spill loads over all decoders without the one, 1,440 without the other, none with both.
+    // us, gate|up / down, without both / with: 128 experts x 31 tokens in mask mode 1,074 / 705 -> 984 / 583, level 2 759 / 435 -> 710 / 407,
+    // level 4 1,165 / 679 -> 1,146 / 641; 16 x 256 in mask mode 212 / 152 -> 192 / 127; 225 x 244, H 1,792, I 640, 307 / 250 -> 276 / 205.
+    RecordValues<RC> rr = {};
     unsigned long long flags = 0;        // refined chunks of the strip
     uint32_t own = 0, other = 0;         // of them this warp's units, and the chunks behind those, from this unit on
     if constexpr (MODE == 1) rr.load_at(p4, nrec, rec);
@@ -510,8 +514,7 @@ __device__ __noinline__ bool decode_strip(uint32_t par, uint32_t info_word)
             uint32_t wb[Pattern<BK>::kWords + 2], wr[Pattern<RC>::kWords + 2];
             const bool refined = MODE == 1 || (MODE == 2 && (own & 1u));
             rb.words(wb, lane);
-            if constexpr (MODE > 0)
-                if (refined) rr.words(wr, lane);
+            if constexpr (MODE > 0) rr.words(wr, lane);      // (mask mode: also of a unit that is not refined, where nothing uses them)
             if (i + 1 < n)
             {
                 rec += kPfGroups * 32;
