@@ -361,8 +361,9 @@ __device__ __forceinline__ uint32_t stage_parities(uint32_t par, int C, int nst)
 
 // A unit is decoded whole (8 k-steps) by one warp: k-steps 0..3 fill the weight tile of k-block 2 c, k-steps 4..7 the
 // tile of k-block 2 c + 1.  The sink keeps the fragments of four k-steps in registers and hands them over as one 32-column store.
-// DEEP (two or three unit stages per group): the stage is free before the unit is begun, and the 64 weights are one straight run of
-// arithmetic with nothing to wait for in it.  One unit stage per group: each half is waited for when it is to be written.
+// DEEP (more stages than groups: six or four, of which a group uses its own three or two, or three that both go round): the stage is free before
+// the unit is begun, and the 64 weights are one straight run of arithmetic with nothing to wait for in it.  Two stages, one per group: each half
+// is waited for when it is to be written.
 template <bool DEEP>
 struct UnitSink
 {

@@ -1,5 +1,5 @@
-"""The widest passes of the fused prefill GEMM (321 to 384 tokens) have three token-tile stages instead of four: what they take must follow
-their tokens, not the stages."""
+"""Passes on both sides of the prefill GEMM's borders between layouts: what they take must follow their tokens, not the number of stages
+(four up to 192 tokens, three up to 256, two beyond)."""
 import pytest
 import torch
 
@@ -8,7 +8,7 @@ from nestquant_b200 import ext, moe
 pytestmark = pytest.mark.gpu
 
 
-def test_widest_passes_cost_what_their_tokens_cost():
+def test_wide_passes_cost_what_their_tokens_cost():
     E, H, I = 4, 4096, 2048      # 4 passes x 32 weight groups: one item per CTA, 64 k-blocks each
     exs = [moe.Expert(H, I, seed=90 + e, rk_gu=0, rk_dn=7, var=True, sv=0.02) for e in range(E)]
     L = moe.MoELayer(E, H, I, Bmax=1, topk=1)
@@ -29,9 +29,10 @@ def test_widest_passes_cost_what_their_tokens_cost():
         torch.cuda.synchronize()
         return a.elapsed_time(b)
 
-    four, three = gemm(320), gemm(384)
-    times = [(once(four), once(three)) for _ in range(25)][5:]
-    t4, t3 = min(t for t, _ in times), min(t for _, t in times)
-    # 1.2 times the tokens; taken in pairs the three stages made it 1.5 times the time
-    assert t3 <= 1.3 * t4, (t3, t4)
+    widths = (192, 256, 272, 384)
+    fs = [gemm(n) for n in widths]
+    t = {n: min(ts) for n, ts in zip(widths, zip(*[[once(f) for f in fs] for _ in range(25)][5:]))}
+    # tokens 1.33, 1.06 and 1.41 times as many; a layout whose loads do not hide costs 1.4 times and more what its tokens do (378 instead of 250 us
+    # for 384, 16 experts of H 6,144)
+    assert t[256] <= 1.4 * t[192] and t[272] <= 1.4 * t[256] and t[384] <= 1.6 * t[272], t
     assert int(status) == 0

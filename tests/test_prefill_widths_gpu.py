@@ -1,5 +1,6 @@
 """The fused prefill GEMM changes its layout with the width of a pass (2, 3, 4 or 6 stages beside the accumulator; up to 64 tokens two accumulators,
-up to 32 two pairs of them in turn): passes of every width one after the other on the same CTAs, for few and odd numbers of chunks."""
+up to 32 two pairs of them in turn): passes of every width one after the other on the same CTAs, for few and odd numbers of chunks, experts of
+every mode (level 2, level 4, mask mode) and both base codes among them."""
 import pytest
 import torch
 
@@ -45,11 +46,30 @@ def test_four_stage_passes_in_turn(H, I):
 
 
 def _check(counts, H, I):
+    nm = [max(1, k // 256) for k in (H, I)]
+    exs, levels = [], []
+    for e in range(len(counts)):
+        masked, base = e % 5 in (1, 3), int(e % 5 == 4 or e % 10 == 3)
+        exs.append(moe.Expert(H, I, seed=60 + e, nm_gu=nm[0] if masked else None, nm_dn=nm[1] if masked else None, rk_gu=3 if base else (0, 6)[e % 2],
+                              rk_dn=9 if base else 7, var=True, sv=0.02, bk_gu=base, bk_dn=base))
+        levels.append(4 if masked else (4, 4, 2)[e % 3])
+    _compare(counts, H, I, exs, levels, nm)
+
+
+# Every residual code in mask mode and with either base code, in passes of two stages, of three and of six with an odd number of chunks.
+@pytest.mark.parametrize("rk,base", [(rk, 0) for rk in range(10)] + [(3, 1), (9, 1)])
+def test_every_code_in_wide_passes(rk, base):
+    H, I, nm = 640, 384, (2, 1)
+    exs = [moe.Expert(H, I, seed=300 + 10 * rk + e, nm_gu=nm[0] if e % 2 == 0 else None, nm_dn=nm[1] if e % 2 == 0 else None, rk_gu=rk, rk_dn=rk, var=e != 2,
+                      sv=0.02, bk_gu=base, bk_dn=base) for e in range(6)]
+    _compare([384, 300, 257, 200, 30, 250], H, I, exs, [4] * 6, nm)
+
+
+def _compare(counts, H, I, exs, levels, nm):
     E, T = len(counts), sum(counts)
-    exs = [moe.Expert(H, I, seed=60 + e, rk_gu=(0, 6)[e % 2], rk_dn=7, var=True, sv=0.02) for e in range(E)]
-    L = moe.MoELayer(E, H, I, Bmax=1, topk=1)
+    L = moe.MoELayer(E, H, I, *nm, Bmax=1, topk=1)
     for e in range(E):
-        L.set(e, exs[e], (4, 4, 2)[e % 3])
+        L.set(e, exs[e], levels[e])
     gen = torch.Generator().manual_seed(7)
     sel = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T, generator=gen)].view(T, 1).cuda()
     x = torch.randn(T, H, generator=gen).bfloat16().half().cuda()
