@@ -1,7 +1,7 @@
 // A whole prefill call: sort, pass list, and chunk by chunk the two GEMMs with the passes around them, enqueued by one call of the host.
-// The reference's host side (sm120/moe.py:282-327) and an earlier one of this library made one call per kernel; from Python those cost
-// 107 to 112 us, more than the GPU takes for a short prompt on a small layer: 75 tokens, 64 experts, H 1,024, I 512: 109 -> 91 us a call,
-// 110 tokens, 25 experts, H 768, I 640: 110 -> 54, of which the launches on the heels of one another (nq_common.cuh) 4 to 6.
+// The reference's host side (sm120/moe.py:282-327) makes one call per kernel; from Python those take 92 to 94 us, more than the GPU needs for a short
+// prompt on a small layer.  A call per kernel / this, the same kernels, us back to back: 75 tokens, 64 experts, H 1,024, I 512: 94.3 / 80.3;
+// 110 tokens, 25 experts, H 768, I 640: 92.4 / 51.8.
 #include "nq_common.cuh"
 
 namespace nq {

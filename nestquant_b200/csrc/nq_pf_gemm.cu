@@ -22,14 +22,14 @@
 // The activation matrices must be in the same order (nq_pf_pre / nq_pf_mid with kperm = 1).
 // Each decoded weight is used for every token of the pass, so decode cost is paid once per expert (for up to 384
 // tokens).  Tensor-pipe bound by intent; the decode instruction rate is the practical limit: with 31 tokens per expert a unit takes a
-// scheduler 790 clocks at level 4 and 490 at level 2 between two borders of items, of which the same loop without MMAs and item borders takes 662 and 393 (560
-// and 329 instructions, at most 0.84 per clock: the half-rate multiply and byte-sum pipe is busy for nine tenths of that).  What the two issuing warps
-// spend comes on top of the decode warps of their schedulers, and the slowest scheduler paces the others: with one issuing warp that scheduler ran
-// 671 instructions a unit at level 4, the average 626; see mbar_wait_warp, uniform and split_chunks.  An item costs a decode warp ~530 more instructions
-// and ~2,500 clocks without work.  128 experts x 31 tokens, H 6,144, I 2,048, us, gate|up / down, the kernel that kept records in a
-// shared-memory ring and all decoders in one function / this one: level 2 852 / 487 -> 757 / 437, level 4 1,344 / 789 -> 1,185 / 692, mask mode
-// 1,169 / 719 -> 1,093 / 711; 32 x 100 level 4 360 / 234 -> 330 / 213; 16 x 256 level 2 190 / 110 -> 175 / 116, level 4 231 / 149 -> 219 / 143;
-// 16 x 384 level 2 248 / 146 -> 262 / 156 (bound by the token tiles that come from L2), level 4 282 / 175 -> 275 / 175.
+// scheduler 777 clocks at level 4, 663 in mask mode and 475 at level 2, borders of items included (gate|up of H 6,144: 613, 523 and 376 instructions,
+// at most 0.84 per clock: the half-rate multiply and byte-sum pipe is busy for nine tenths of that); a loop that only decodes and stores takes 662 at
+// level 4 and 393 at level 2.  What the two issuing warps spend comes on top of the decode warps of their schedulers, and the slowest scheduler
+// paces the others; see mbar_wait_warp, uniform and split_chunks.  H 6,144, I 2,048, us, gate|up / down:
+//     experts x tokens    128 x 31       32 x 100     16 x 160     16 x 256     16 x 384
+//     level 2             712 / 409      229 / 143    148 / 93     175 / 109    255 / 147 (bound by the token tiles that come from L2)
+//     level 4             1,147 / 641    318 / 199    197 / 120    209 / 131    265 / 166
+//     mask mode           985 / 583      279 / 183    175 / 113    194 / 125    261 / 159
 // Every mbarrier wait is bounded: on time-out the CTA raises status[0], waits for its TMA loads and MMAs in flight, frees its tensor
 // memory and returns.
 #include <cuda.h>
@@ -340,13 +340,16 @@ __device__ __forceinline__ PfShared* pf_shared() { return (PfShared*)(pf_tiles()
 // stages of a narrow pass reach into columns that the accumulator of a wide one before it used (see decode_strip), and when the number of
 // stages changes between two items of a CTA the new token tiles overlap old ones at other indices, so the producer first waits
 // until every stage of the old layout has been released.  Where the chunks of a strip take different times (mask mode) the stages even them
-// out: 16 experts, H 6,144, I 2,048, gate|up / down, us, with three / four stages: 160 tokens 199 / 192 and 140 / 136, at level 4 202.3 / 200.6 and 129.1 /
-// 127.9; 192 tokens 202 / 196 and 145 / 139, at level 4 204.9 / 203.9 and 132.1 / 130.2.
+// out: 16 experts, H 6,144, I 2,048, gate|up / down, us, with three / four stages: 160 tokens 177 / 175 and 114 / 112, at level 2 153 / 148 and 94 / 93; 192 tokens
+// 181 / 180 and 118 / 115, at level 2 159 / 158 and 99.1 / 98.5; at level 4 the same.
 __device__ __forceinline__ int chunk_stages(int ntok) { return ntok <= 128 ? 6 : ntok <= 192 ? 4 : ntok <= 256 ? 3 : 2; }
 // Passes of up to 64 tokens: even and odd chunks are multiplied by two warps, each into an accumulator of its own that the epilogue adds up.
 // What a chunk costs the warp that issues its MMAs comes on top of the decode warps of its scheduler, and the slowest scheduler paces the
-// others: gate|up of 128 experts x 31 tokens with one warp / two, us: 785 / 757 at level 2, 1,226 / 1,193 at level 4.  Beyond 64 tokens the second
-// accumulator would leave four stages instead of six: 32 x 100 tokens, down, 164 / 149 at level 2, 229 / 217 at level 4 (four / six).
+// others: 128 experts x 31 tokens, H 6,144, I 2,048, gate|up / down, with one warp / two, us: level 2 766 / 712 and 426 / 409, level 4 1,183 / 1,147 and
+// 666 / 641, mask mode 1,009 / 985 and 601 / 583; strips of two chunks lose by it (I 256, down: 114 / 119, 154 / 156, 158 / 165).  Beyond 64 tokens the second
+// accumulator would leave four stages instead of six, which comes out even or a little better (32 x 100 tokens, six stages and one warp / four and
+// two: level 2 229 / 221 and 143 / 143, level 4 318 / 311 and 199 / 197, mask mode 279 / 275 and 183 / 183); before the decoders kept clear of
+// spills it was 7 to 10 % slower.
 __device__ __forceinline__ bool split_chunks(int ntok) { return ntok <= 64; }
 // First column of an item's accumulator, and from there to the second one.  Up to 32 tokens the items take turns with two pairs, so the MMAs
 // of the next item need not wait for the epilogue.
@@ -402,9 +405,9 @@ struct PfInfo
     __device__ __forceinline__ uint32_t acc() const { return w >> 6 & 1u; }
     __device__ __forceinline__ uint32_t phase() const { return w >> 7 & 1u; }
 };
-// Units of an item that a warp decodes before it writes the accumulator of the previous item, whose last MMAs finish meanwhile.  (Down
-// projection of 128 experts x 31 tokens at level 4, 2,048 / 256 columns, us: after two units 692 / 184, after one 694 / 181, at once 705 / 199;
-// 16 x 256 tokens, three stages: after one 143, at once 144.)
+// Units of an item that a warp decodes before it writes the accumulator of the previous item, whose last MMAs finish meanwhile.  128 experts x 31
+// tokens, H 6,144, I 2,048, gate|up / down, us, after two units, after one, at once: level 2 712 / 409, 721 / 411, 722 / 415; level 4 1,147 / 641, 1,162 /
+// 640, 1,155 / 668; with I 256, whose down strips have one unit per warp, down after it 119, 156 at level 4, at once 130, 180.
 __device__ __forceinline__ int units_before_epilogue(int nst, bool drain) { return nst == kPfStages && !drain ? 2 : 1; }
 
 // Decode warps: accumulator [128 weight rows x ntok] of the item before this one -> out.  TMEM lanes 32 q .. 32 q + 31 (the quarter this warp
@@ -442,7 +445,7 @@ __device__ __forceinline__ void write_accumulator(PfInfo info)
 }
 // Between two units it is a call, because the registers of the decode loop are all taken there; after the last unit it is in line.  A warp
 // with one unit per item has no other place for it than after that unit, and every item pays what the call costs: 128 experts x 31
-// tokens, H 6,144, down projection of 256 columns, us, call / in line: 153 / 122 at level 2, 225 / 187 at level 4.
+// tokens, H 6,144, down projection of 256 columns, us, call / in line: 126 / 120 at level 2, 170 / 156 at level 4; of 512 columns 164 / 158, 243 / 228.
 __device__ __noinline__ void write_accumulator_between(uint32_t info) { write_accumulator(PfInfo{info}); }
 
 // One decode warp, one item: its strip over the chunks c = group, group + 2, ... (the other group of 8 warps takes the other
