@@ -156,7 +156,7 @@ int nq_pf_hits(const int32_t* counts, int32_t* hits, int E, void* stream);
 
 /* A whole prefill call (the host side of sm120/moe.py:282-327): the entries above in order - nq_pf_sort, then for every chunk of R pairs the
  * pass list, nq_pf_pre (or nq_pf_pre_ep, if world > 0), nq_pf_gemm, nq_pf_mid, nq_pf_gemm, nq_pf_combine.  Everything is caller-owned:
- *   x [T][H] fp16 (not read if world > 0), sel [T][topk], rw [T][topk] fp16, out [T][H] fp32;
+ *   x [T][H] fp16 (not read if world > 0; then T <= world * tokens_per_rank), sel [T][topk], rw [T][topk] fp16, out [T][H] fp32;
  *   pe, pt, pos [T * topk], start [E + 2], sort_scratch [nq_pf_sort_scratch_ints];  hits [E] (may be host-mapped) with hit_counts [E] of
  *   scratch, or both NULL;
  *   for chunks of R pairs: plan [plan_ints >= nq_pf_plan_ints(E, min(R, T * topk))], xg, xu [R][H] fp16, y [R][H] fp32 (may overlay xg | xu), acc_g,
