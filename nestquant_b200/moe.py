@@ -386,7 +386,7 @@ class MoELayer:
         any fp16 [*, H] tensor on the device), token t of sel / rw is read from buffer t // tokens_per_rank by the first pass
         itself (see nq_pf_pre_ep).
         Under torch.cuda.graph a call's scratch comes from the graph's own pool and lives as long as the graph: replays and eager calls, whatever
-        their sizes, do not disturb one another.
+        their sizes, do not disturb one another.  (A capture that torch does not know of has no such pool: ext.prefill with scratch that the caller keeps.)
         Nothing here synchronises with the host; a device-side time-out inside the GEMM raises a flag that
         prefill_status() reads."""
         assert x.dtype == torch.float16 and rw.dtype == torch.float16 and sel.dtype == torch.int64, (x.dtype, rw.dtype, sel.dtype)
